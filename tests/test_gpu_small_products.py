@@ -1,0 +1,52 @@
+"""Products outside the prepared-weight tensor-core kernel: few rows, two activations, the LSTM recurrence."""
+from ctypes import byref
+
+import numpy as np
+import pytest
+
+from oracle import ref_runner
+
+from util import max_err_rel_linf, run_cuda, single_op_model
+
+pytestmark = pytest.mark.gpu
+
+
+def _gemm(ctx, a, b, c=None, alpha=1.0, beta=0.0, relu=0, trans_a=False, trans_b=False):
+    """wdc_gemm on [batch, m, k] x [batch, k, n]; trans_*: the operand is stored transposed."""
+    from webdnn_b200.backend import CPUTensor
+    from webdnn_b200.lib import GemmDesc
+    batch, m, k = a.shape
+    n = b.shape[2]
+    put = lambda x: ctx.move_tensor(CPUTensor.from_array(np.ascontiguousarray(x)))  # noqa: E731
+    da = put(a.transpose(0, 2, 1) if trans_a else a)
+    db = put(b.transpose(0, 2, 1) if trans_b else b)
+    dc = put(c) if c is not None else None
+    y = ctx.empty_tensor([batch, m, n])
+    d = GemmDesc(batch=batch, m=m, n=n, k=k, sab=m * k, sa0=1 if trans_a else k, sa1=m if trans_a else 1,
+                 sbb=k * n, sb0=1 if trans_b else n, sb1=k if trans_b else 1,
+                 sc0=n if c is not None and c.ndim == 2 else 0, sc1=1, alpha=alpha, beta=beta, relu=relu)
+    ctx.gemm(d, da, db, dc, y)
+    got = y.get_data().reshape(batch, m, n)
+    for t in (da, db, dc, y):
+        if t is not None:
+            t.dispose()
+    return got
+
+
+def _want(a, b, c=None, alpha=1.0, beta=0.0, relu=0):
+    y = alpha * np.matmul(a.astype(np.float64), b.astype(np.float64))
+    if c is not None:
+        y = y + beta * c
+    return np.maximum(y, 0) if relu else y
+
+
+# rows around the kernels' row counts (1, 2, 4, 8 and their multiples), K around one load per lane and warp
+@pytest.mark.parametrize("m", [1, 2, 3, 5, 8, 9, 31])
+@pytest.mark.parametrize("n,k,batch", [(1, 1, 1), (10, 512, 1), (33, 127, 3), (1000, 2048, 1), (130, 1028, 2), (7, 36, 1)])
+@pytest.mark.parametrize("trans_b", [False, True])
+def test_few_rows(cuda_context, m, n, k, batch, trans_b):
+    rng = np.random.default_rng(m * 1000 + n)
+    a, b = (rng.standard_normal(s).astype(np.float32) for s in ((batch, m, k), (batch, k, n)))
+    c = rng.standard_normal(n).astype(np.float32)
+    got = _gemm(cuda_context, a, b, c, 0.5, 2.0, 1, trans_b=trans_b)
+    assert max_err_rel_linf(got, _want(a, b, c, 0.5, 2.0, 1)) <= 2e-6

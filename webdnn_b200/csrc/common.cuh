@@ -139,6 +139,8 @@ int wdc_tc_conv2d(wdc_context* ctx, const wdc_conv_desc* d, const float* x, cons
                   const float* scale, const float* shift, const float* residual, float* y);
 int wdc_tc_gemm(wdc_context* ctx, const wdc_gemm_desc* d, const float* A, const float* B,
                 const float* C, float* Y);
+// Few-row Gemm on the CUDA cores (gemm_skinny.cu); WDC_ERR_UNSUPPORTED for strides of B it does not take.
+int wdc_skinny_gemm(wdc_context* ctx, const wdc_gemm_desc* d, const float* A, const float* B, const float* C, float* Y);
 void wdc_tc_destroy(wdc_context* ctx);
 // Looks up the device address of wdc_lstm_static's scratch array for ctx's (current) device (lstm.cu).
 int wdc_lstm_static_setup(wdc_context* ctx);

@@ -218,6 +218,12 @@ extern "C" int wdc_gemm(wdc_context* ctx, const wdc_gemm_desc* d, const float* A
   // Y = alpha*A*B + beta*Y (C aliasing the output) is served by the CUDA-core kernel's in-place mode only
   int s = (C != nullptr && C == Y) ? WDC_ERR_UNSUPPORTED : wdc_tc_gemm(ctx, d, A, B, C, Y);
   if (s != WDC_ERR_UNSUPPORTED) return s;
+  // Below 32 rows the tensor-core path declines (a 128-row tile would be three quarters empty and B would have to be
+  // split first): such a product is a few dot products per column, bound by reading B.
+  if (d->m < 32 && (C == nullptr || C != Y)) {
+    s = wdc_skinny_gemm(ctx, d, A, B, C, Y);
+    if (s != WDC_ERR_UNSUPPORTED) return s;
+  }
   return wdc_simt_gemm(ctx, d, A, B, C, Y);
 }
 
