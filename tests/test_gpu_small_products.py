@@ -50,3 +50,32 @@ def test_few_rows(cuda_context, m, n, k, batch, trans_b):
     c = rng.standard_normal(n).astype(np.float32)
     got = _gemm(cuda_context, a, b, c, 0.5, 2.0, 1, trans_b=trans_b)
     assert max_err_rel_linf(got, _want(a, b, c, 0.5, 2.0, 1)) <= 2e-6
+
+
+# edges of the 128-row tile, of the three tile widths, of a K block (32), a TMEM segment (128) and the two stages
+@pytest.mark.parametrize("batch,m,n,k", [(3, 32, 17, 1), (1, 129, 33, 31), (2, 128, 64, 32), (5, 127, 65, 33), (2, 40, 129, 128),
+                                         (2, 300, 260, 129), (1, 64, 50, 161), (2, 96, 128, 256), (1, 1, 1, 5), (64, 257, 130, 67),
+                                         (8, 850, 850, 32), (8, 850, 32, 850), (40, 130, 257, 1000)])
+@pytest.mark.parametrize("trans_a,trans_b", [(False, False), (True, True), (False, True)])
+def test_two_activations(cuda_context, batch, m, n, k, trans_a, trans_b):
+    rng = np.random.default_rng(m + n + k)
+    a, b = (rng.standard_normal(s).astype(np.float32) for s in ((batch, m, k), (batch, k, n)))
+    got = _gemm(cuda_context, a, b, trans_a=trans_a, trans_b=trans_b)
+    assert max_err_rel_linf(got, _want(a, b)) <= 2e-6
+
+
+def test_two_activations_addend_and_non_finite(cuda_context):
+    rng = np.random.default_rng(3)
+    a, b = (rng.standard_normal(s).astype(np.float32) for s in ((2, 200, 45), (2, 45, 150)))
+    c = rng.standard_normal((200, 150)).astype(np.float32)
+    got = _gemm(cuda_context, a, b, c, -1.5, 0.5, 1)
+    assert max_err_rel_linf(got, _want(a, b, c, -1.5, 0.5, 1)) <= 2e-6
+    a[0, 3, 7], a[1, 150, 2], b[1, 11, 140] = np.inf, np.nan, 3.4e38
+    a[1, :, 11] = 1e-3
+    got = _gemm(cuda_context, a, b)
+    with np.errstate(invalid="ignore"):
+        want = _want(a, b)
+    assert np.array_equal(np.isnan(got), np.isnan(want))
+    m = np.isfinite(want)
+    assert np.array_equal(got[~m & ~np.isnan(want)], want[~m & ~np.isnan(want)].astype(np.float32))
+    assert np.all(np.abs(got[m] - want[m]) <= 1e-5 * np.maximum(np.abs(want[m]), 1.0))

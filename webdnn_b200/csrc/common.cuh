@@ -141,6 +141,9 @@ int wdc_tc_gemm(wdc_context* ctx, const wdc_gemm_desc* d, const float* A, const 
                 const float* C, float* Y);
 // Few-row Gemm on the CUDA cores (gemm_skinny.cu); WDC_ERR_UNSUPPORTED for strides of B it does not take.
 int wdc_skinny_gemm(wdc_context* ctx, const wdc_gemm_desc* d, const float* A, const float* B, const float* C, float* Y);
+// Tensor-core Gemm that splits both operands as it loads them (gemm_tc_direct.cu): any strides, ragged K, batches.
+int wdc_tc_gemm_direct(wdc_context* ctx, const wdc_gemm_desc* d, const float* A, const float* B, const float* C,
+                       float* Y);
 void wdc_tc_destroy(wdc_context* ctx);
 // Looks up the device address of wdc_lstm_static's scratch array for ctx's (current) device (lstm.cu).
 int wdc_lstm_static_setup(wdc_context* ctx);

@@ -223,6 +223,9 @@ extern "C" int wdc_gemm(wdc_context* ctx, const wdc_gemm_desc* d, const float* A
   if (d->m < 32 && (C == nullptr || C != Y)) {
     s = wdc_skinny_gemm(ctx, d, A, B, C, Y);
     if (s != WDC_ERR_UNSUPPORTED) return s;
+  } else if (C != Y || C == nullptr) {
+    s = wdc_tc_gemm_direct(ctx, d, A, B, C, Y);
+    if (s != WDC_ERR_UNSUPPORTED) return s;
   }
   return wdc_simt_gemm(ctx, d, A, B, C, Y);
 }
