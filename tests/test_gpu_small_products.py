@@ -79,3 +79,35 @@ def test_two_activations_addend_and_non_finite(cuda_context):
     m = np.isfinite(want)
     assert np.array_equal(got[~m & ~np.isnan(want)], want[~m & ~np.isnan(want)].astype(np.float32))
     assert np.all(np.abs(got[m] - want[m]) <= 1e-5 * np.maximum(np.abs(want[m]), 1.0))
+
+
+# hidden sizes around the 32 units of a cluster and the K slices (8, 4 CTAs), batches around an MMA's 16 columns, the
+# spread over groups of clusters, and more rows than one launch takes; 800 and 36 x 100 leave the kernel's range
+@pytest.mark.parametrize("seq,batch,inp,hidden,state", [
+    (1, 1, 4, 4, False), (2, 3, 32, 36, True), (17, 16, 40, 64, False), (5, 17, 12, 100, True), (9, 96, 64, 216, True),
+    (23, 5, 100, 344, False), (12, 64, 256, 512, True), (6, 70, 32, 512, False), (5, 33, 36, 516, True), (7, 96, 48, 768, True),
+    (4, 130, 32, 764, False), (3, 9, 32, 800, True), (128, 1, 80, 256, False)])
+def test_lstm_recurrence(cuda_context, seq, batch, inp, hidden, state):
+    rng = np.random.default_rng(seq * batch)
+    lim = 1 / np.sqrt(hidden)
+    uni = lambda *s: rng.uniform(-lim, lim, s).astype(np.float32)  # noqa: E731
+    ins = [rng.standard_normal((seq, batch, inp)).astype(np.float32), uni(1, 4 * hidden, inp), uni(1, 4 * hidden, hidden),
+           uni(1, 8 * hidden)]
+    ctx = cuda_context
+    if not state:
+        model = single_op_model("LSTM", {"hidden_size": hidden}, ins, n_out=3, n_graph_inputs=1)
+        want = ref_runner.run_model(model, ins[:1])
+        got = run_cuda(model, ins[:1], ctx)
+    else:
+        from oracle import ops
+        from webdnn_b200.backend import CPUTensor
+        h0, c0 = (rng.uniform(-1, 1, (1, batch, hidden)).astype(np.float32) for _ in range(2))
+        want = ops.lstm(*ins, h0, c0)
+        dev = [ctx.move_tensor(CPUTensor.from_array(x)) for x in (*ins, h0, c0)]
+        outs = [ctx.empty_tensor(s) for s in ((seq, 1, batch, hidden), (1, batch, hidden), (1, batch, hidden))]
+        ctx._call("wdc_lstm", *(t.ptr for t in dev + outs), seq, batch, inp, hidden)
+        got = [o.get_data().reshape(o.dims) for o in outs]
+        for t in dev + outs:
+            t.dispose()
+    for g, w in zip(got, want):
+        assert max_err_rel_linf(g, np.asarray(w).reshape(g.shape)) <= 1e-5
