@@ -69,6 +69,27 @@ int wdc_capture_begin(wdc_context* ctx);
 int wdc_capture_end(wdc_context* ctx, wdc_graph** graph);
 int wdc_graph_launch(wdc_context* ctx, wdc_graph* graph);
 int wdc_graph_destroy(wdc_context* ctx, wdc_graph* graph);
+/* wdc_graph_launch between the transfers of a whole run, in one call: input i is copied from src[i] (host memory where
+ * in_on_host[i] != 0, else device memory) into the recorded input buffer dst[i] first; afterwards the n_out recorded
+ * outputs are copied to host[] and the call waits for them (n_out == 0: it only queues). */
+int wdc_graph_run(wdc_context* ctx, wdc_graph* graph, int n_in, void* const* dst, const void* const* src,
+                  const int64_t* in_bytes, const int32_t* in_on_host, int n_out, void* const* host,
+                  const void* const* out, const int64_t* out_bytes);
+/* A tape is the list of calls of one run, for a host whose own work per operator is longer than the device's (no
+ * counterpart in the reference either).  Unlike a graph it owns no device memory and takes new buffers every time.
+ * wdc_tape_begin names the run's device inputs; every following call of this thread on the context executes and is
+ * noted, allocations included, until wdc_tape_end names the run's results.  *tape is NULL when the run cannot be
+ * repeated: it moved host data, waited, freed a buffer that is not its own, kept one that is no result, or returns an
+ * input (n_out < 0: the recording is given up).  Device memory that is neither input nor allocated by the run (weights) is taken to stay where it is.
+ * wdc_tape_run repeats the calls on new inputs (host memory where in_on_host[i] != 0).  out_host == NULL: out[]
+ * receives the results' device buffers, which the caller frees; else the results are copied to out_host[], the call
+ * waits for them and frees everything. */
+typedef struct wdc_tape wdc_tape;
+int wdc_tape_begin(wdc_context* ctx, int n_in, void* const* in, const int64_t* bytes);
+int wdc_tape_end(wdc_context* ctx, int n_out, void* const* out, wdc_tape** tape);
+int wdc_tape_run(wdc_context* ctx, wdc_tape* tape, const void* const* in, const int32_t* in_on_host, void** out,
+                 void* const* out_host, const int64_t* out_bytes);
+int wdc_tape_destroy(wdc_context* ctx, wdc_tape* tape);
 int wdc_upload_async(wdc_context* ctx, void* dst, const void* host, int64_t bytes, int64_t* ticket);
 int wdc_wait_upload(wdc_context* ctx, int64_t ticket);
 /* wdc_upload_async for a destination that no queued work has touched since wdc_alloc returned it (a tensor created

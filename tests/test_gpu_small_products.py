@@ -82,9 +82,9 @@ def test_two_activations_addend_and_non_finite(cuda_context):
 
 
 # hidden sizes around the 32 units of a cluster and the K slices (8, 4 CTAs), batches around an MMA's 16 columns, the
-# spread over groups of clusters, and more rows than one launch takes; 800 and 36 x 100 leave the kernel's range
+# spread over groups of clusters, and more rows than one launch takes; 3 steps, 28 and 800 units leave the kernel's range
 @pytest.mark.parametrize("seq,batch,inp,hidden,state", [
-    (1, 1, 4, 4, False), (2, 3, 32, 36, True), (17, 16, 40, 64, False), (5, 17, 12, 100, True), (9, 96, 64, 216, True),
+    (3, 3, 8, 32, False), (4, 1, 4, 32, False), (5, 2, 12, 28, True), (6, 3, 32, 36, True), (17, 16, 40, 64, False), (5, 17, 12, 100, True), (9, 96, 64, 216, True),
     (23, 5, 100, 344, False), (12, 64, 256, 512, True), (6, 70, 32, 512, False), (5, 33, 36, 516, True), (7, 96, 48, 768, True),
     (4, 130, 32, 764, False), (3, 9, 32, 800, True), (128, 1, 80, 256, False)])
 def test_lstm_recurrence(cuda_context, seq, batch, inp, hidden, state):

@@ -120,6 +120,15 @@ class EightbitCPUTensor(CPUTensor):
         return self._decoded
 
 
+def like_cpu_tensor(template: TensorImpl, data: np.ndarray) -> CPUTensor:
+    """A CPUTensor of the template's dims and dtype over `data` (flat, of that length and dtype)."""
+    t = CPUTensor.__new__(CPUTensor)
+    t.dims, t.ndim, t.data_type, t.backend = list(template.dims), template.ndim, template.data_type, "cpu"
+    t.strides, t.length = list(template.strides), template.length
+    t.data, t.use_external_buffer = data, True
+    return t
+
+
 class CudaSharedBuffer:
     """Refcounted device allocation shared by aliases of one tensor."""
 
@@ -154,6 +163,18 @@ class CudaTensor(TensorImpl):
         self.aux: Dict[str, "CudaTensor"] = {}  # derived device data that lives and dies with this tensor
         self.upload_ticket: Optional[int] = None  # pending transfer on the copy stream (prefetch_tensor)
         self.disposed = False
+
+    @classmethod
+    def adopt(cls, template: "CudaTensor", ptr: int) -> "CudaTensor":
+        """A tensor of the template's dims, dtype and layout that owns the arena allocation at ``ptr``."""
+        buf = CudaSharedBuffer.__new__(CudaSharedBuffer)
+        buf.context, buf.byte_length, buf.ptr, buf.ref_count = template.context, template.byte_length, ptr, 1
+        t = cls.__new__(cls)
+        t.dims, t.ndim, t.data_type, t.backend = list(template.dims), template.ndim, template.data_type, "cuda"
+        t.strides, t.length = list(template.strides), template.length
+        t.context, t.byte_length, t.shared_buffer, t.layout = template.context, template.byte_length, buf, template.layout
+        t.aux, t.upload_ticket, t.disposed = {}, None, False
+        return t
 
     @property
     def ptr(self) -> int:
@@ -284,8 +305,8 @@ class WebDNNCudaContext:
             self._call("wdc_free", c_void_p(ptr))
 
     def _upload(self, ptr: int, arr: np.ndarray) -> None:
-        # cudaMemcpyAsync from pageable memory returns once the source has been staged, so the
-        # caller may release `arr` right away; pinned sources must outlive the copy
+        # a pageable source has been staged when the call returns, so the caller may release `arr` right away;
+        # pinned sources must outlive the copy
         self._call("wdc_upload", c_void_p(ptr), arr.ctypes.data_as(c_void_p), arr.nbytes)
 
     def _download(self, out: np.ndarray, ptr: int, nbytes: int) -> None:
@@ -405,6 +426,22 @@ class WebDNNCudaContext:
         dst.upload_ticket = ticket.value
         dst._prefetch_source = arr  # keeps the host memory alive until the tensor goes away
         return dst
+
+    # --- tape of a run's calls
+    def tape_begin(self, inputs: Sequence[CudaTensor]) -> None:
+        n = len(inputs)
+        self._call("wdc_tape_begin", n, (c_void_p * n)(*(t.ptr for t in inputs)), i64_array([t.length * 4 for t in inputs]))
+
+    def tape_end(self, outputs: Optional[Sequence[CudaTensor]]) -> Optional[int]:
+        """The tape, or None where the run cannot be repeated; ``outputs=None`` gives the recording up."""
+        tape = c_void_p()
+        n = -1 if outputs is None else len(outputs)
+        self._call("wdc_tape_end", n, (c_void_p * max(n, 1))(*(t.ptr for t in outputs or [])), byref(tape))
+        return tape.value
+
+    def tape_destroy(self, tape: int) -> None:
+        if self.handle is not None:
+            self._call("wdc_tape_destroy", c_void_p(tape))
 
     # --- capture of a run into a CUDA graph
     def capture_begin(self) -> None:

@@ -9,7 +9,7 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB_PATH = os.path.join(HERE, "libwebdnn_cuda.so")
-SOURCES = ["context.cu", "pointwise.cu", "rowops.cu", "pool.cu", "layout.cu", "gemm_simt.cu", "gemm_skinny.cu",
+SOURCES = ["context.cu", "transfer.cu", "tape.cu", "pointwise.cu", "rowops.cu", "pool.cu", "layout.cu", "gemm_simt.cu", "gemm_skinny.cu",
            "conv_tc.cu", "gemm_tc_direct.cu", "lstm.cu", "lstm_persistent.cu", "lstm_cluster.cu", "extra_ops.cu", "attention.cu", "attention_tc.cu"]
 # WDC_BUILD_DEVELOP=1 in the environment adds -DWDC_TC_DEVELOP: the contraction kernel then carries its development
 # knock-out switches (read from WDC_TC_DEBUG); the shipped build has none.

@@ -18,7 +18,7 @@
 // are not stored.
 #include <math.h>
 
-#include "common.cuh"
+#include "tape.cuh"
 
 namespace {
 
@@ -208,6 +208,7 @@ int wdc_attention_tc(wdc_context* ctx, const wdc_attention_desc* d, const float*
 extern "C" int wdc_attention(wdc_context* ctx, const wdc_attention_desc* d, const float* q, const float* k,
                              const float* v, float* y) {
   if (!ctx) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_attention: null context");
+  WDC_TAPE(ctx, wdc_attention, tape_desc(d), q, k, v, y);
   wdc_note_write(ctx, y);
   WDC_REQUIRE(ctx, d && q && k && v && y, "wdc_attention: null argument");
   WDC_REQUIRE(ctx, d->batch > 0 && d->heads > 0 && d->tq > 0 && d->tk > 0, "wdc_attention: bad shape");

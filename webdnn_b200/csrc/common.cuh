@@ -39,8 +39,9 @@ struct wdc_context {
   std::mutex mu;
   int64_t n_alloc = 0, n_free = 0, n_launch = 0, h2d_bytes = 0, d2h_bytes = 0, n_tc_launch = 0;
   int sm_count = 0;
-  int* status_word = nullptr;       // device word set by kernels whose bounded waits expire
-  int* status_word_host = nullptr;  // pinned mirror
+  int* status_word = nullptr;       // word set by kernels whose bounded waits expire: the mapping of ...
+  int* status_word_host = nullptr;  // ... page-locked host memory
+  struct wdc_stager* stager = nullptr;   // page-locked ring of the host transfers (transfer.cu), made at first use
   void* tc_state = nullptr;         // tensor-map cache of the tcgen05 path
   // While a run is being captured into a CUDA graph, allocations come from (and return to) a private
   // arena that the finished graph keeps: replays reuse exactly the addresses the capture saw.
@@ -145,6 +146,12 @@ int wdc_skinny_gemm(wdc_context* ctx, const wdc_gemm_desc* d, const float* A, co
 int wdc_tc_gemm_direct(wdc_context* ctx, const wdc_gemm_desc* d, const float* A, const float* B, const float* C,
                        float* Y);
 void wdc_tc_destroy(wdc_context* ctx);
+// Transfers on the compute stream through page-locked chunks (transfer.cu).
+int wdc_stage_in(wdc_context* ctx, void* dst, const void* host, int64_t bytes);
+int wdc_stage_out(wdc_context* ctx, int count, void* const* host, const void* const* src, const int64_t* bytes);
+void wdc_stager_destroy(wdc_context* ctx);
+void wdc_tape_note_alloc(struct wdc_tape* t, void* p, int64_t bytes);
+void wdc_tape_note_free(struct wdc_tape* t, void* p);
 // Looks up the device address of wdc_lstm_static's scratch array for ctx's (current) device (lstm.cu).
 int wdc_lstm_static_setup(wdc_context* ctx);
 // Drops every cached hi/lo split whose source (weight matrix or per-channel scale vector) overlaps the

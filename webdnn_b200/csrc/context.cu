@@ -5,7 +5,7 @@
 
 #include <nvtx3/nvToolsExt.h>   // header-only: ranges reach a profiler only when one has injected its library
 
-#include "common.cuh"
+#include "tape.cuh"
 
 static std::string g_last_error;  // for failures before a context exists
 static std::mutex g_mu;
@@ -75,9 +75,10 @@ extern "C" int wdc_create(int device, int64_t arena_limit_bytes, wdc_context** o
   ctx->sm_count = prop.multiProcessorCount;
   ctx->arena.limit = arena_limit_bytes;
   e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&ctx->status_word, 256);
-  if (e == cudaSuccess) e = cudaMemset(ctx->status_word, 0, 256);
-  if (e == cudaSuccess) e = cudaMallocHost((void**)&ctx->status_word_host, 256);
+  // the word kernels report an expired wait in: host memory they write through its mapping, so that a waiting call
+  // reads it without a transfer of its own
+  if (e == cudaSuccess) e = cudaHostAlloc((void**)&ctx->status_word_host, 256, cudaHostAllocMapped);
+  if (e == cudaSuccess) e = cudaHostGetDevicePointer((void**)&ctx->status_word, ctx->status_word_host, 0);
   if (e != cudaSuccess) {
     int s = wdc_check_cuda(nullptr, e, "wdc_create");
     delete ctx;
@@ -111,7 +112,7 @@ extern "C" int wdc_destroy(wdc_context* ctx) {
     for (auto& s : a->slabs) cudaFree(s.base);
     delete a;
   }
-  cudaFree(ctx->status_word);
+  wdc_stager_destroy(ctx);
   cudaFreeHost(ctx->status_word_host);
   if (ctx->d2h_stream) {
     cudaStreamSynchronize(ctx->d2h_stream);
@@ -150,6 +151,7 @@ extern "C" int wdc_alloc(wdc_context* ctx, int64_t bytes, void** dptr) {
   if (!ctx || !dptr) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_alloc: null argument");
   *dptr = nullptr;
   if (bytes < 0) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_alloc: negative size %lld", (long long)bytes);
+  TapeScope tape_scope(ctx);
   std::lock_guard<std::mutex> lk(ctx->mu);
   wdc_arena& a = ctx->capture_arena ? *ctx->capture_arena : ctx->arena;
   int64_t need = ((bytes > 0 ? bytes : 1) + kAlign - 1) / kAlign * kAlign;
@@ -198,6 +200,7 @@ extern "C" int wdc_alloc(wdc_context* ctx, int64_t bytes, void** dptr) {
   if (a.in_use > a.high_water) a.high_water = a.in_use;
   ctx->n_alloc++;
   *dptr = p;
+  if (tape_scope.tape) wdc_tape_note_alloc(tape_scope.tape, p, bytes);
   return WDC_OK;
 }
 
@@ -227,6 +230,8 @@ bool wdc_arena_extent(wdc_context* ctx, const void* p, const char** lo, const ch
 extern "C" int wdc_free(wdc_context* ctx, void* dptr) {
   if (!ctx) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_free: null context");
   if (!dptr) return WDC_OK;
+  TapeScope tape_scope(ctx);
+  if (tape_scope.tape) wdc_tape_note_free(tape_scope.tape, dptr);
   wdc_tc_evict(ctx, dptr, 0);   // widened to the block's extent
   std::lock_guard<std::mutex> lk(ctx->mu);
   wdc_arena* owner = &ctx->arena;
@@ -292,20 +297,10 @@ extern "C" int wdc_host_free(wdc_context* ctx, void* hptr) {
   return WDC_OK;
 }
 
-extern "C" int wdc_upload(wdc_context* ctx, void* dst, const void* host, int64_t bytes) {
-  if (!ctx || bytes < 0 || (bytes > 0 && (!dst || !host)))
-    return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_upload: bad argument");
-  if (bytes == 0) return WDC_OK;
-  DeviceGuard g(ctx->device);
-  wdc_tc_evict(ctx, dst, bytes);
-  WDC_CUDA(ctx, cudaMemcpyAsync(dst, host, (size_t)bytes, cudaMemcpyHostToDevice, ctx->stream));
-  ctx->h2d_bytes += bytes;
-  return WDC_OK;
-}
-
 static int upload_async(wdc_context* ctx, void* dst, const void* host, int64_t bytes, int64_t* ticket, bool fresh) {
   if (!ctx || !ticket || bytes < 0 || (bytes > 0 && (!dst || !host)))
     return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_upload_async: bad argument");
+  WDC_NO_TAPE(ctx);
   DeviceGuard g(ctx->device);
   if (!ctx->copy_stream) {
     WDC_CUDA(ctx, cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking));
@@ -375,6 +370,7 @@ void wdc_graphs_note_evicted(wdc_context* ctx, int64_t born) {
 
 extern "C" int wdc_capture_begin(wdc_context* ctx) {
   if (!ctx) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_capture_begin: null context");
+  WDC_NO_TAPE(ctx);
   if (ctx->capture_arena) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_capture_begin: a capture is already open");
   if (ctx->profile) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_capture_begin: switch per-launch profiling off first");
   DeviceGuard g(ctx->device);
@@ -455,11 +451,11 @@ extern "C" int wdc_graph_destroy(wdc_context* ctx, wdc_graph* graph) {
 }
 
 static int report_device_status(wdc_context* ctx) {
-  // status_word_host is refreshed by the download/sync paths below
-  if (ctx->status_word_host[0] != 0) {
-    int code = ctx->status_word_host[0];
-    ctx->status_word_host[0] = 0;
-    cudaMemsetAsync(ctx->status_word, 0, 256, ctx->stream);
+  // (what a kernel wrote is visible here once the host has waited for the kernel)
+  volatile int* word = ctx->status_word_host;
+  const int code = *word;
+  if (code != 0) {
+    *word = 0;
     return wdc_fail(ctx, WDC_ERR_DEVICE_WAIT, "a bounded device-side wait expired (kernel status %d)", code);
   }
   return WDC_OK;
@@ -467,27 +463,16 @@ static int report_device_status(wdc_context* ctx) {
 
 extern "C" int wdc_sync(wdc_context* ctx) {
   if (!ctx) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_sync: null context");
+  WDC_NO_TAPE(ctx);
   DeviceGuard g(ctx->device);
-  WDC_CUDA(ctx, cudaMemcpyAsync(ctx->status_word_host, ctx->status_word, sizeof(int),
-                                cudaMemcpyDeviceToHost, ctx->stream));
   WDC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   return report_device_status(ctx);
-}
-
-extern "C" int wdc_download(wdc_context* ctx, void* host, const void* src, int64_t bytes) {
-  if (!ctx || bytes < 0 || (bytes > 0 && (!host || !src)))
-    return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_download: bad argument");
-  DeviceGuard g(ctx->device);
-  if (bytes > 0) {
-    WDC_CUDA(ctx, cudaMemcpyAsync(host, src, (size_t)bytes, cudaMemcpyDeviceToHost, ctx->stream));
-    ctx->d2h_bytes += bytes;
-  }
-  return wdc_sync(ctx);
 }
 
 extern "C" int wdc_download_async(wdc_context* ctx, void* host, const void* src, int64_t bytes, int64_t* ticket) {
   if (!ctx || !ticket || bytes < 0 || (bytes > 0 && (!host || !src)))
     return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_download_async: bad argument");
+  WDC_NO_TAPE(ctx);
   DeviceGuard g(ctx->device);
   if (!ctx->d2h_stream) {
     WDC_CUDA(ctx, cudaStreamCreateWithFlags(&ctx->d2h_stream, cudaStreamNonBlocking));
@@ -503,9 +488,6 @@ extern "C" int wdc_download_async(wdc_context* ctx, void* host, const void* src,
   WDC_CUDA(ctx, cudaStreamWaitEvent(ctx->d2h_stream, ctx->d2h_fence, 0));
   if (bytes > 0)
     WDC_CUDA(ctx, cudaMemcpyAsync(host, src, (size_t)bytes, cudaMemcpyDeviceToHost, ctx->d2h_stream));
-  // the device status word travels with it, so that wdc_wait_download can report an expired device wait
-  WDC_CUDA(ctx, cudaMemcpyAsync(ctx->status_word_host, ctx->status_word, sizeof(int), cudaMemcpyDeviceToHost,
-                                ctx->d2h_stream));
   const int64_t t = ctx->download_seq++;
   WDC_CUDA(ctx, cudaEventRecord(ctx->download_done[t % wdc_context::kDownloadTickets], ctx->d2h_stream));
   ctx->d2h_bytes += bytes;
@@ -515,6 +497,7 @@ extern "C" int wdc_download_async(wdc_context* ctx, void* host, const void* src,
 
 extern "C" int wdc_wait_download(wdc_context* ctx, int64_t ticket) {
   if (!ctx) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_wait_download: null context");
+  WDC_NO_TAPE(ctx);
   if (ticket < 0 || ticket >= ctx->download_seq)
     return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_wait_download: unknown ticket %lld", (long long)ticket);
   DeviceGuard g(ctx->device);
@@ -523,13 +506,13 @@ extern "C" int wdc_wait_download(wdc_context* ctx, int64_t ticket) {
   if (ctx->download_seq - ticket > wdc_context::kDownloadTickets) slot = ctx->download_seq - 1;
   WDC_CUDA(ctx, cudaEventSynchronize(ctx->download_done[slot % wdc_context::kDownloadTickets]));
   // a bounded device wait that expired before this point is reported here, like wdc_download does
-  if (*(volatile int*)ctx->status_word_host != 0) return report_device_status(ctx);
-  return WDC_OK;
+  return report_device_status(ctx);
 }
 
 extern "C" int wdc_copy(wdc_context* ctx, void* dst, const void* src, int64_t bytes) {
   if (!ctx || bytes < 0 || (bytes > 0 && (!dst || !src)))
     return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_copy: bad argument");
+  WDC_TAPE(ctx, wdc_copy, dst, src, bytes);
   if (bytes == 0) return WDC_OK;
   DeviceGuard g(ctx->device);
   wdc_tc_evict(ctx, dst, bytes);
@@ -546,6 +529,7 @@ __global__ void fill_u32_kernel(uint32_t* dst, uint32_t v, int64_t n) {
 extern "C" int wdc_fill_u32(wdc_context* ctx, void* dst, uint32_t value, int64_t count) {
   if (!ctx || count < 0 || (count > 0 && !dst))
     return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_fill_u32: bad argument");
+  WDC_TAPE(ctx, wdc_fill_u32, dst, value, count);
   wdc_note_write(ctx, dst, count * 4);
   if (count == 0) return WDC_OK;
   DeviceGuard g(ctx->device);
@@ -555,6 +539,7 @@ extern "C" int wdc_fill_u32(wdc_context* ctx, void* dst, uint32_t value, int64_t
 
 extern "C" int wdc_set_option(wdc_context* ctx, const char* name, int64_t value) {
   if (!ctx || !name) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_set_option: null argument");
+  WDC_NO_TAPE(ctx);
   const std::string n(name);
   if (n == "precision") {
     if (value != 0 && value != 1)

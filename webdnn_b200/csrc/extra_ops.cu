@@ -3,7 +3,7 @@
 // results agree with its cpu backend to the last bit wherever the summation order allows.
 #include <math.h>
 
-#include "common.cuh"
+#include "tape.cuh"
 
 // convtranspose.ts:30-263.  The reference computes, per input pixel, output channel and tap, the
 // channel contraction in double and stores it as float32 (matmul, :218-240), then sums the taps that
@@ -140,6 +140,7 @@ static int conv_transpose_by_gemm(wdc_context* ctx, const wdc_convt_desc* d, con
 extern "C" int wdc_conv_transpose2d(wdc_context* ctx, const wdc_convt_desc* d, const float* x, const float* w,
                                     const float* bias, float* y) {
   if (!ctx) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_conv_transpose2d: null context");
+  WDC_TAPE(ctx, wdc_conv_transpose2d, tape_desc(d), x, w, bias, y);
   wdc_note_write(ctx, y);
   WDC_REQUIRE(ctx, d != nullptr, "wdc_conv_transpose2d: null descriptor");
   WDC_REQUIRE(ctx, d->batch >= 0 && d->ch_in > 0 && d->group > 0 && d->ch_out_per_group > 0 && d->in_h > 0 &&
@@ -204,6 +205,7 @@ __global__ void __launch_bounds__(256) instance_norm_kernel(const float* __restr
 extern "C" int wdc_instance_norm(wdc_context* ctx, const float* x, const float* scale, const float* bias, float* y,
                                  int64_t batch, int64_t ch, int64_t area, double eps) {
   if (!ctx) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_instance_norm: null context");
+  WDC_TAPE(ctx, wdc_instance_norm, x, scale, bias, y, batch, ch, area, eps);
   wdc_note_write(ctx, y);
   WDC_REQUIRE(ctx, batch >= 0 && ch > 0 && area > 0, "wdc_instance_norm: bad shape");
   if (batch == 0) return WDC_OK;

@@ -6,7 +6,7 @@
 // Scratch (P, G, and the running h/c state) comes from the context arena.
 #include <math.h>
 
-#include "common.cuh"
+#include "tape.cuh"
 
 int wdc_simt_gemm(wdc_context* ctx, const wdc_gemm_desc* d, const float* A, const float* B, const float* C,
                   float* Y);
@@ -49,6 +49,7 @@ extern "C" int wdc_lstm(wdc_context* ctx, const float* X, const float* W, const 
                         const float* h0, const float* c0, float* Y, float* Yh, float* Yc, int64_t T,
                         int64_t Bt, int64_t I, int64_t H) {
   if (!ctx) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_lstm: null context");
+  WDC_TAPE(ctx, wdc_lstm, X, W, R, bias, h0, c0, Y, Yh, Yc, T, Bt, I, H);
   wdc_note_write(ctx, Yc);
   wdc_note_write(ctx, Yh);
   wdc_note_write(ctx, Y);
@@ -182,6 +183,7 @@ extern "C" int wdc_lstm_static(wdc_context* ctx, const float* X, const float* W,
                                const float* bias, const float* h0, const float* c0, float* Y, float* Yh,
                                float* Yc, int64_t T, int64_t Bt, int64_t I, int64_t H) {
   if (!ctx) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_lstm_static: null context");
+  WDC_NO_TAPE(ctx);
   wdc_note_write(ctx, Yc);
   wdc_note_write(ctx, Yh);
   wdc_note_write(ctx, Y);

@@ -565,7 +565,10 @@ Plan plan_of(wdc_context* ctx, int64_t Bt, int64_t H, int blocks) {
 // clusters would be resident (nothing has been written but Y's filling); any other non-zero status is an error.
 int wdc_lstm_cluster(wdc_context* ctx, const float* P, const float* R, const float* bias, const float* h0,
                      const float* c0, float* Y, float* Yh, float* Yc, int64_t T, int64_t Bt, int64_t H) {
-  if (T < 1 || T > (1 << 24) || Bt > (1 << 20) || H % 4 != 0 || H > 8 * KC_MAX) return WDC_ERR_UNSUPPORTED;
+  // One to three steps do not pay for filling Y and bringing R into tensor memory, and below 32 units most rows of the
+  // MMA would be empty: the other paths keep those.
+  if (T < 4 || H < UNITS) return WDC_ERR_UNSUPPORTED;
+  if (T > (1 << 24) || Bt > (1 << 20) || H % 4 != 0 || H > 8 * KC_MAX) return WDC_ERR_UNSUPPORTED;
   if ((((uintptr_t)R | (uintptr_t)Y | (uintptr_t)h0) & 15) != 0) return WDC_ERR_UNSUPPORTED;
   ClusterArgs a = {P, R, bias, h0, c0, Y, Yh, Yc, ctx->status_word, (int)T, (int)Bt, (int)H};
   a.blocks = (int)((H + UNITS - 1) / UNITS);

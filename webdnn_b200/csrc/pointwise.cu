@@ -3,7 +3,7 @@
 // the SM count.
 #include <math.h>
 
-#include "common.cuh"
+#include "tape.cuh"
 
 // JS ToInt32 of a double: what a store into an Int32Array does
 // (operators/cpu/operators/standard/binary7.ts writes doubles into typed arrays).
@@ -128,6 +128,7 @@ static int launch_unary(wdc_context* ctx, const float* src, float* dst, int64_t 
 extern "C" int wdc_unary(wdc_context* ctx, int op, int dtype, const void* src, void* dst, int64_t n,
                          float p0, float p1) {
   if (!ctx) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_unary: null context");
+  WDC_TAPE(ctx, wdc_unary, op, dtype, src, dst, n, p0, p1);
   wdc_note_write(ctx, dst);
   WDC_REQUIRE(ctx, n >= 0 && (n == 0 || (src && dst)), "wdc_unary: bad buffer or count");
   if (n == 0) return WDC_OK;
@@ -302,6 +303,8 @@ static int launch_binary_f32(wdc_context* ctx, const float* a, const float* b, f
 extern "C" int wdc_binary(wdc_context* ctx, int op, int dtype, const void* a, const void* b, void* out,
                           int ndim, const int64_t* dims, const int64_t* sa, const int64_t* sb) {
   if (!ctx) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_binary: null context");
+  WDC_TAPE(ctx, wdc_binary, op, dtype, a, b, out, ndim, tape_array(dims, ndim), tape_array(sa, ndim),
+           tape_array(sb, ndim));
   wdc_note_write(ctx, out);
   WDC_REQUIRE(ctx, ndim >= 0 && ndim <= 6, "wdc_binary: rank %d not in 0..6", ndim);
   WDC_REQUIRE(ctx, op >= WDC_B_ADD && op <= WDC_B_MIN, "wdc_binary: unknown op %d", op);
@@ -390,6 +393,7 @@ __global__ void cast_i32_f32_kernel(const int32_t* __restrict__ s, float* __rest
 extern "C" int wdc_cast(wdc_context* ctx, int src_dtype, int dst_dtype, const void* src, void* dst,
                         int64_t n) {
   if (!ctx) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_cast: null context");
+  WDC_TAPE(ctx, wdc_cast, src_dtype, dst_dtype, src, dst, n);
   wdc_note_write(ctx, dst);
   WDC_REQUIRE(ctx, n >= 0 && (n == 0 || (src && dst)), "wdc_cast: bad buffer or count");
   if (n == 0) return WDC_OK;
@@ -459,6 +463,7 @@ extern "C" int wdc_channel_affine(wdc_context* ctx, const float* x, const float*
                                   const float* shift, float* y, int64_t outer, int64_t channels,
                                   int64_t inner, int relu) {
   if (!ctx) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_channel_affine: null context");
+  WDC_TAPE(ctx, wdc_channel_affine, x, scale, shift, y, outer, channels, inner, relu);
   wdc_note_write(ctx, y);
   WDC_REQUIRE(ctx, outer >= 0 && channels > 0 && inner > 0, "wdc_channel_affine: bad shape");
   int64_t n = outer * channels * inner;
@@ -530,6 +535,7 @@ __global__ void __launch_bounds__(256) decode_eightbit_kernel(const uint8_t* __r
 
 extern "C" int wdc_decode_eightbit(wdc_context* ctx, const void* codes, float* out, int64_t n, float scale) {
   if (!ctx) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_decode_eightbit: null context");
+  WDC_NO_TAPE(ctx);
   wdc_note_write(ctx, out);
   WDC_REQUIRE(ctx, n >= 0 && (n == 0 || (codes && out)), "wdc_decode_eightbit: bad buffer or count");
   WDC_REQUIRE(ctx, (((uintptr_t)codes | (uintptr_t)out) & 15) == 0, "wdc_decode_eightbit: buffers must be 16-byte aligned");

@@ -4,7 +4,7 @@
 // 128-bit accesses.
 #include <math.h>
 
-#include "common.cuh"
+#include "tape.cuh"
 
 template <bool IS_MAX, int VEC>
 __global__ void __launch_bounds__(256) pool2d_kernel(wdc_pool_desc d, const float* __restrict__ x,
@@ -156,9 +156,13 @@ static int pool_common(wdc_context* ctx, const wdc_pool_desc* d, const float* x,
 }
 
 extern "C" int wdc_maxpool2d(wdc_context* ctx, const wdc_pool_desc* d, const float* x, float* y) {
+  if (!ctx) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_maxpool2d: null context");
+  WDC_TAPE(ctx, wdc_maxpool2d, tape_desc(d), x, y);
   return pool_common(ctx, d, x, y, true, "wdc_maxpool2d");
 }
 extern "C" int wdc_avgpool2d(wdc_context* ctx, const wdc_pool_desc* d, const float* x, float* y) {
+  if (!ctx) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_avgpool2d: null context");
+  WDC_TAPE(ctx, wdc_avgpool2d, tape_desc(d), x, y);
   return pool_common(ctx, d, x, y, false, "wdc_avgpool2d");
 }
 
@@ -295,6 +299,7 @@ __global__ void __launch_bounds__(GAP_MAPS) gap_dense_kernel(const float* __rest
 extern "C" int wdc_global_avgpool(wdc_context* ctx, const float* x, float* y, int64_t batch, int64_t ch,
                                   int64_t area, int64_t xs_n, int64_t xs_c, int64_t xs_p) {
   if (!ctx) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_global_avgpool: null context");
+  WDC_TAPE(ctx, wdc_global_avgpool, x, y, batch, ch, area, xs_n, xs_c, xs_p);
   wdc_note_write(ctx, y);
   WDC_REQUIRE(ctx, batch >= 0 && ch >= 0 && area > 0, "wdc_global_avgpool: bad shape");
   if (batch * ch == 0) return WDC_OK;

@@ -3,7 +3,7 @@
 // read from HBM exactly once) or by one CTA (longer rows, re-read through L2).
 #include <math.h>
 
-#include "common.cuh"
+#include "tape.cuh"
 
 __device__ __forceinline__ float warp_max(float v) {
 #pragma unroll
@@ -149,6 +149,7 @@ __global__ void __launch_bounds__(256) softmax_block_reg_kernel(const float* __r
 
 extern "C" int wdc_softmax(wdc_context* ctx, const float* x, float* y, int64_t outer, int64_t len) {
   if (!ctx) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_softmax: null context");
+  WDC_TAPE(ctx, wdc_softmax, x, y, outer, len);
   wdc_note_write(ctx, y);
   WDC_REQUIRE(ctx, outer >= 0 && len >= 0, "wdc_softmax: negative shape");
   if (outer == 0 || len == 0) return WDC_OK;
@@ -264,6 +265,7 @@ __global__ void __launch_bounds__(256) reduce_cols_kernel(int kind, int final, c
 extern "C" int wdc_reduce_axis(wdc_context* ctx, int kind, int final, const float* x, float* y,
                                int64_t outer, int64_t red, int64_t inner, int64_t total) {
   if (!ctx) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_reduce_axis: null context");
+  WDC_TAPE(ctx, wdc_reduce_axis, kind, final, x, y, outer, red, inner, total);
   wdc_note_write(ctx, y);
   WDC_REQUIRE(ctx, kind >= R_SUM && kind <= R_SUMSQUARE, "wdc_reduce_axis: unknown kind %d", kind);
   WDC_REQUIRE(ctx, outer >= 0 && red >= 0 && inner >= 0, "wdc_reduce_axis: bad shape");
@@ -430,6 +432,7 @@ __global__ void __launch_bounds__(256) layernorm_block_reg_kernel(const float* _
 extern "C" int wdc_layernorm(wdc_context* ctx, const float* x, const float* gamma, const float* beta,
                              float* y, int64_t outer, int64_t len, float eps) {
   if (!ctx) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_layernorm: null context");
+  WDC_TAPE(ctx, wdc_layernorm, x, gamma, beta, y, outer, len, eps);
   wdc_note_write(ctx, y);
   WDC_REQUIRE(ctx, outer >= 0 && len > 0, "wdc_layernorm: bad shape");
   if (outer == 0) return WDC_OK;
@@ -495,6 +498,7 @@ __global__ void __launch_bounds__(256) argmax_kernel(const float* __restrict__ x
 extern "C" int wdc_argmax(wdc_context* ctx, const float* x, int32_t* y, int64_t outer, int64_t len,
                           int select_last) {
   if (!ctx) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_argmax: null context");
+  WDC_TAPE(ctx, wdc_argmax, x, y, outer, len, select_last);
   wdc_note_write(ctx, y);
   WDC_REQUIRE(ctx, outer >= 0 && len > 0, "wdc_argmax: bad shape");
   if (outer == 0) return WDC_OK;

@@ -1,0 +1,138 @@
+// Recording and repeating the calls of a run (see tape.cuh), and a captured graph's run with its host transfers.
+#include "tape.cuh"
+
+thread_local wdc_tape* wdc_thread_tape = nullptr;
+
+extern "C" int wdc_tape_begin(wdc_context* ctx, int n_in, void* const* in, const int64_t* bytes) {
+  if (!ctx || n_in < 0 || (n_in > 0 && (!in || !bytes)))
+    return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_tape_begin: bad argument");
+  if (wdc_thread_tape) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_tape_begin: this thread is already recording a tape");
+  if (ctx->capture_arena) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_tape_begin: a capture is open");
+  wdc_tape* t = new wdc_tape();
+  t->ctx = ctx;
+  t->n_in = t->n_slots = n_in;
+  for (int i = 0; i < n_in; i++) {
+    t->in_bytes.push_back(bytes[i]);
+    // (an input passed twice, or an empty one, could not be told from its twin)
+    if (in[i] && bytes[i] > 0) t->valid &= t->live.insert({(char*)in[i], {i, bytes[i]}}).second;
+  }
+  wdc_thread_tape = t;
+  return WDC_OK;
+}
+
+extern "C" int wdc_tape_end(wdc_context* ctx, int n_out, void* const* out, wdc_tape** tape) {
+  if (!ctx || !tape || (n_out > 0 && !out)) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_tape_end: bad argument");
+  *tape = nullptr;
+  wdc_tape* t = wdc_thread_tape;
+  if (!t || t->ctx != ctx) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_tape_end: no tape is being recorded");
+  wdc_thread_tape = nullptr;
+  // every result is a buffer of its own that the run allocated, and nothing else it allocated is left
+  size_t left = 0;
+  for (auto& kv : t->live)
+    if (kv.second.first >= t->n_in) left++;
+  std::vector<bool> taken((size_t)t->n_slots, false);
+  for (int i = 0; i < n_out && t->valid; i++) {
+    const wdc_tape::Ref r = t->ref(out[i]);
+    t->valid = r.slot >= t->n_in && r.offset == 0 && !taken[(size_t)r.slot];
+    if (t->valid) {
+      taken[(size_t)r.slot] = true;
+      t->outs.push_back(r.slot);
+    }
+  }
+  if (n_out < 0 || left != (size_t)n_out) t->valid = false;
+  t->live.clear();
+  if (!t->valid) {
+    delete t;
+    return WDC_OK;
+  }
+  *tape = t;
+  return WDC_OK;
+}
+
+extern "C" int wdc_tape_destroy(wdc_context* ctx, wdc_tape* tape) {
+  if (!ctx) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_tape_destroy: null context");
+  delete tape;
+  return WDC_OK;
+}
+
+// What wdc_alloc and wdc_free note about themselves.
+void wdc_tape_note_alloc(wdc_tape* t, void* p, int64_t bytes) {
+  const int slot = t->n_slots++;
+  t->live[(char*)p] = {slot, bytes > 0 ? bytes : 1};
+  t->ops.push_back([slot, bytes](wdc_context* ctx, char** slots) {
+    return wdc_alloc(ctx, bytes, (void**)&slots[slot]);
+  });
+}
+void wdc_tape_note_free(wdc_tape* t, void* p) {
+  auto it = t->live.find((char*)p);
+  if (it == t->live.end() || it->second.first < t->n_in) {   // not the run's own buffer
+    t->valid = false;
+    return;
+  }
+  const int slot = it->second.first;
+  t->live.erase(it);
+  t->ops.push_back([slot](wdc_context* ctx, char** slots) {
+    void* q = slots[slot];
+    slots[slot] = nullptr;
+    return wdc_free(ctx, q);
+  });
+}
+
+extern "C" int wdc_tape_run(wdc_context* ctx, wdc_tape* tape, const void* const* in, const int32_t* in_on_host,
+                            void** out, void* const* out_host, const int64_t* out_bytes) {
+  if (!ctx || !tape || (tape->n_in > 0 && (!in || !in_on_host)) || (!tape->outs.empty() && !out))
+    return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_tape_run: bad argument");
+  WDC_NO_TAPE(ctx);
+  DeviceGuard g(ctx->device);
+  std::vector<char*> slots((size_t)tape->n_slots, nullptr);
+  int s = WDC_OK;
+  for (int i = 0; i < tape->n_in && s == WDC_OK; i++) {
+    if (!in_on_host[i]) {
+      slots[(size_t)i] = (char*)in[i];
+      continue;
+    }
+    s = wdc_alloc(ctx, tape->in_bytes[(size_t)i], (void**)&slots[(size_t)i]);
+    if (s == WDC_OK && tape->in_bytes[(size_t)i] > 0)
+      s = wdc_stage_in(ctx, slots[(size_t)i], in[i], tape->in_bytes[(size_t)i]);
+  }
+  for (size_t k = 0; k < tape->ops.size() && s == WDC_OK; k++) s = tape->ops[k](ctx, slots.data());
+  for (int i = 0; i < tape->n_in; i++)   // stream-ordered: reused only by work queued after this run
+    if (in_on_host[i] && slots[(size_t)i]) {
+      wdc_free(ctx, slots[(size_t)i]);
+      slots[(size_t)i] = nullptr;
+    }
+  const int n_out = (int)tape->outs.size();
+  if (s == WDC_OK) {
+    for (int i = 0; i < n_out; i++) out[i] = slots[(size_t)tape->outs[(size_t)i]];
+    if (!out_host) return WDC_OK;
+    s = wdc_stage_out(ctx, n_out, out_host, (const void* const*)out, out_bytes);
+  }
+  // results have been read, or a call failed: nothing of the run stays allocated
+  for (int i = tape->n_in; i < tape->n_slots; i++)
+    if (slots[(size_t)i]) wdc_free(ctx, slots[(size_t)i]);
+  for (int i = 0; i < n_out; i++) out[i] = nullptr;
+  return s;
+}
+
+extern "C" int wdc_graph_run(wdc_context* ctx, wdc_graph* graph, int n_in, void* const* dst, const void* const* src,
+                             const int64_t* in_bytes, const int32_t* in_on_host, int n_out, void* const* host,
+                             const void* const* out, const int64_t* out_bytes) {
+  if (!ctx || !graph || n_in < 0 || n_out < 0 || (n_in > 0 && (!dst || !src || !in_bytes || !in_on_host)) ||
+      (n_out > 0 && (!host || !out || !out_bytes)))
+    return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_graph_run: bad argument");
+  WDC_NO_TAPE(ctx);
+  DeviceGuard g(ctx->device);
+  for (int i = 0; i < n_in; i++) {
+    if (in_bytes[i] <= 0) continue;
+    wdc_tc_evict(ctx, dst[i], in_bytes[i]);
+    if (in_on_host[i]) {
+      const int s = wdc_stage_in(ctx, dst[i], src[i], in_bytes[i]);
+      if (s != WDC_OK) return s;
+    } else {
+      WDC_CUDA(ctx, cudaMemcpyAsync(dst[i], src[i], (size_t)in_bytes[i], cudaMemcpyDeviceToDevice, ctx->stream));
+    }
+  }
+  const int s = wdc_graph_launch(ctx, graph);
+  if (s != WDC_OK) return s;
+  return n_out > 0 ? wdc_stage_out(ctx, n_out, host, out, out_bytes) : WDC_OK;
+}

@@ -1,0 +1,285 @@
+// Transfers between host and device memory on the compute stream.
+//
+// The driver moves pageable memory through its own staging buffers with one thread: 11 us for 4 KB before anything
+// else can be queued, 12.7 GB/s for megabytes (605 us for an 800x800 image), where the link takes 50 GB/s from
+// page-locked memory.  Here the context keeps a ring of page-locked chunks: a transfer is cut into chunks, each is
+// copied by a few threads and sent (or received and copied) while its neighbours are on the link.  Page-locked
+// buffers of the caller's go straight to the link.
+#include <string.h>
+
+#include <atomic>
+#include <condition_variable>
+#include <thread>
+
+#include "tape.cuh"
+
+namespace {
+
+constexpr int64_t CHUNK = 512 << 10;    // long enough to hide an event and a copy call (a few us) behind 10 us of link
+constexpr int CHUNKS = 16;
+constexpr int64_t PIECE = 64 << 10;     // what a thread takes at a time
+constexpr int64_t ALONE = 256 << 10;    // below this the other threads would only be woken up
+constexpr int64_t PINNED_CHECK = 256 << 10;   // asking the driver what a pointer is costs about a microsecond
+constexpr int MAX_HELPERS = 3;
+
+// memcpy by the caller and up to MAX_HELPERS threads that take pieces from a common counter: a helper that is still
+// asleep costs nothing, the caller takes its pieces.  Helpers poll for a while after a job, then sleep.
+class CopyTeam {
+ public:
+  ~CopyTeam() {
+    {
+      std::lock_guard<std::mutex> lk(mu_);
+      stop_ = true;
+    }
+    cv_.notify_all();
+    for (auto& t : helpers_) t.join();
+  }
+  void copy(char* dst, const char* src, int64_t bytes) {
+    if (bytes < ALONE) {
+      memcpy(dst, src, (size_t)bytes);
+      return;
+    }
+    if (helpers_.empty()) start();
+    Job job;
+    job.dst = dst;
+    job.src = src;
+    job.bytes = bytes;
+    job.pieces = (int)((bytes + PIECE - 1) / PIECE);
+    {
+      std::lock_guard<std::mutex> lk(mu_);
+      job_ = &job;
+      seq_.fetch_add(1, std::memory_order_release);
+    }
+    if (asleep_.load() > 0) cv_.notify_all();
+    work(job);
+    {
+      std::lock_guard<std::mutex> lk(mu_);   // no helper picks the job up any more ...
+      job_ = nullptr;
+    }
+    while (job.users.load(std::memory_order_acquire) > 0) pause();   // ... and those who did have left it
+  }
+
+ private:
+  struct Job {
+    char* dst;
+    const char* src;
+    int64_t bytes;
+    int pieces;
+    std::atomic<int> next{0}, users{0};
+  };
+  static void pause() {
+#if defined(__x86_64__)
+    __builtin_ia32_pause();
+#else
+    std::this_thread::yield();
+#endif
+  }
+  static void work(Job& j) {
+    for (int i; (i = j.next.fetch_add(1, std::memory_order_relaxed)) < j.pieces;) {
+      const int64_t off = (int64_t)i * PIECE, n = j.bytes - off < PIECE ? j.bytes - off : PIECE;
+      memcpy(j.dst + off, j.src + off, (size_t)n);
+    }
+  }
+  void start() {
+    const unsigned cpus = std::thread::hardware_concurrency();
+    const int n = cpus > MAX_HELPERS ? MAX_HELPERS : cpus > 1 ? (int)cpus - 1 : 0;
+    for (int i = 0; i < n; i++) helpers_.emplace_back([this] { run(); });
+  }
+  void run() {
+    uint64_t seen = 0;
+    for (;;) {
+      int polls = 0;
+      while (seq_.load(std::memory_order_acquire) == seen && polls < 20000) {   // some 0.5 ms
+        pause();
+        polls++;
+      }
+      Job* job = nullptr;
+      {
+        std::unique_lock<std::mutex> lk(mu_);
+        if (seq_.load() == seen) {
+          asleep_++;
+          cv_.wait(lk, [&] { return stop_ || seq_.load() != seen; });
+          asleep_--;
+        }
+        if (stop_) return;
+        seen = seq_.load();
+        job = job_;
+        if (job) job->users.fetch_add(1, std::memory_order_relaxed);
+      }
+      if (job) {
+        work(*job);
+        job->users.fetch_sub(1, std::memory_order_release);
+      }
+    }
+  }
+  std::vector<std::thread> helpers_;
+  std::mutex mu_;
+  std::condition_variable cv_;
+  std::atomic<uint64_t> seq_{0};
+  std::atomic<int> asleep_{0};
+  Job* job_ = nullptr;
+  bool stop_ = false;
+};
+
+}  // namespace
+
+struct wdc_stager {
+  std::mutex mu;             // one transfer at a time uses the ring
+  char* ring = nullptr;
+  cudaEvent_t done[CHUNKS] = {};
+  bool busy[CHUNKS] = {};    // a transfer recorded done[i] and nobody has waited for it yet
+  int next = 0;
+  CopyTeam team;
+};
+
+namespace {
+
+int stager_of(wdc_context* ctx, wdc_stager** out) {
+  std::lock_guard<std::mutex> lk(ctx->mu);
+  if (!ctx->stager) {
+    wdc_stager* s = new wdc_stager();
+    cudaError_t e = cudaMallocHost((void**)&s->ring, (size_t)(CHUNKS * CHUNK));
+    for (auto& ev : s->done)
+      if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+    ctx->stager = s;
+    if (e != cudaSuccess) return wdc_check_cuda(ctx, e, "page-locked staging memory");
+  }
+  *out = ctx->stager;
+  return WDC_OK;
+}
+
+// The next chunk of the ring, free for use.
+int take_chunk(wdc_context* ctx, wdc_stager* s, int* index) {
+  const int i = s->next;
+  s->next = (i + 1) % CHUNKS;
+  if (s->busy[i]) {
+    WDC_CUDA(ctx, cudaEventSynchronize(s->done[i]));
+    s->busy[i] = false;
+  }
+  *index = i;
+  return WDC_OK;
+}
+
+bool page_locked(const void* p, int64_t bytes) {
+  if (bytes < PINNED_CHECK) return false;
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeHost;
+}
+
+}  // namespace
+
+void wdc_stager_destroy(wdc_context* ctx) {
+  wdc_stager* s = ctx->stager;
+  if (!s) return;
+  for (auto& ev : s->done)
+    if (ev) cudaEventDestroy(ev);
+  if (s->ring) cudaFreeHost(s->ring);
+  delete s;
+  ctx->stager = nullptr;
+}
+
+// host -> device, ordered with the compute stream; pageable sources may be released when the call returns.
+int wdc_stage_in(wdc_context* ctx, void* dst, const void* host, int64_t bytes) {
+  if (ctx->capture_arena)
+    return wdc_fail(ctx, WDC_ERR_INVALID, "a transfer from host memory cannot be part of a captured run");
+  ctx->h2d_bytes += bytes;
+  if (page_locked(host, bytes)) {
+    WDC_CUDA(ctx, cudaMemcpyAsync(dst, host, (size_t)bytes, cudaMemcpyHostToDevice, ctx->stream));
+    return WDC_OK;
+  }
+  wdc_stager* s = nullptr;
+  int st = stager_of(ctx, &s);
+  if (st != WDC_OK) return st;
+  std::lock_guard<std::mutex> lk(s->mu);
+  for (int64_t off = 0; off < bytes; off += CHUNK) {
+    const int64_t n = bytes - off < CHUNK ? bytes - off : CHUNK;
+    int i;
+    st = take_chunk(ctx, s, &i);
+    if (st != WDC_OK) return st;
+    char* chunk = s->ring + i * CHUNK;
+    s->team.copy(chunk, (const char*)host + off, n);
+    WDC_CUDA(ctx, cudaMemcpyAsync((char*)dst + off, chunk, (size_t)n, cudaMemcpyHostToDevice, ctx->stream));
+    WDC_CUDA(ctx, cudaEventRecord(s->done[i], ctx->stream));
+    s->busy[i] = true;
+  }
+  return WDC_OK;
+}
+
+// device -> host for several buffers; waits for the compute stream.
+int wdc_stage_out(wdc_context* ctx, int count, void* const* host, const void* const* src, const int64_t* bytes) {
+  if (ctx->capture_arena)
+    return wdc_fail(ctx, WDC_ERR_INVALID, "a transfer to host memory cannot be part of a captured run");
+  wdc_stager* s = nullptr;
+  int st = stager_of(ctx, &s);
+  if (st != WDC_OK) return st;
+  {
+    std::lock_guard<std::mutex> lk(s->mu);
+    struct Part {
+      char* to;
+      int64_t n;
+      int chunk;
+    };
+    Part queue[CHUNKS];
+    int head = 0, queued = 0;
+    auto finish_one = [&]() -> int {
+      Part& p = queue[head];
+      head = (head + 1) % CHUNKS;
+      queued--;
+      WDC_CUDA(ctx, cudaEventSynchronize(s->done[p.chunk]));
+      s->busy[p.chunk] = false;
+      s->team.copy(p.to, s->ring + p.chunk * CHUNK, p.n);
+      return WDC_OK;
+    };
+    for (int b = 0; b < count; b++) {
+      if (bytes[b] <= 0) continue;
+      ctx->d2h_bytes += bytes[b];
+      if (page_locked(host[b], bytes[b])) {
+        WDC_CUDA(ctx, cudaMemcpyAsync(host[b], src[b], (size_t)bytes[b], cudaMemcpyDeviceToHost, ctx->stream));
+        continue;
+      }
+      for (int64_t off = 0; off < bytes[b]; off += CHUNK) {
+        const int64_t n = bytes[b] - off < CHUNK ? bytes[b] - off : CHUNK;
+        if (queued == CHUNKS) {
+          st = finish_one();
+          if (st != WDC_OK) return st;
+        }
+        int i;
+        st = take_chunk(ctx, s, &i);
+        if (st != WDC_OK) return st;
+        WDC_CUDA(ctx, cudaMemcpyAsync(s->ring + i * CHUNK, (const char*)src[b] + off, (size_t)n, cudaMemcpyDeviceToHost,
+                                      ctx->stream));
+        WDC_CUDA(ctx, cudaEventRecord(s->done[i], ctx->stream));
+        s->busy[i] = true;
+        queue[(head + queued) % CHUNKS] = {(char*)host[b] + off, n, i};
+        queued++;
+      }
+    }
+    while (queued) {
+      st = finish_one();
+      if (st != WDC_OK) return st;
+    }
+  }
+  return wdc_sync(ctx);
+}
+
+extern "C" int wdc_upload(wdc_context* ctx, void* dst, const void* host, int64_t bytes) {
+  if (!ctx || bytes < 0 || (bytes > 0 && (!dst || !host)))
+    return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_upload: bad argument");
+  WDC_NO_TAPE(ctx);
+  if (bytes == 0) return WDC_OK;
+  DeviceGuard g(ctx->device);
+  wdc_tc_evict(ctx, dst, bytes);
+  return wdc_stage_in(ctx, dst, host, bytes);
+}
+
+extern "C" int wdc_download(wdc_context* ctx, void* host, const void* src, int64_t bytes) {
+  if (!ctx || bytes < 0 || (bytes > 0 && (!host || !src)))
+    return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_download: bad argument");
+  WDC_NO_TAPE(ctx);
+  DeviceGuard g(ctx->device);
+  return wdc_stage_out(ctx, 1, &host, &src, &bytes);
+}

@@ -91,6 +91,11 @@ SIGNATURES = {
     "wdc_capture_end": (c_int, [c_void_p, POINTER(c_void_p)]),
     "wdc_graph_launch": (c_int, [c_void_p, c_void_p]),
     "wdc_graph_destroy": (c_int, [c_void_p, c_void_p]),
+    "wdc_graph_run": (c_int, [c_void_p, c_void_p, c_int] + [c_void_p] * 4 + [c_int] + [c_void_p] * 3),
+    "wdc_tape_begin": (c_int, [c_void_p, c_int, c_void_p, c_void_p]),
+    "wdc_tape_end": (c_int, [c_void_p, c_int, c_void_p, POINTER(c_void_p)]),
+    "wdc_tape_run": (c_int, [c_void_p, c_void_p] + [c_void_p] * 5),
+    "wdc_tape_destroy": (c_int, [c_void_p, c_void_p]),
     "wdc_upload_async": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, POINTER(c_int64)]),
     "wdc_upload_fresh_async": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, POINTER(c_int64)]),
     "wdc_wait_upload": (c_int, [c_void_p, c_int64]),

@@ -27,7 +27,8 @@ from typing import Dict, List, Optional, Sequence, Union
 import numpy as np
 
 from . import onnx_io, tensor_loader
-from .backend import CPUTensor, EightbitCPUTensor, WebDNNCPUContext, WebDNNCudaContext
+from .backend import (NP_DTYPE, CPUTensor, CudaTensor, EightbitCPUTensor, WebDNNCPUContext, WebDNNCudaContext,
+                      like_cpu_tensor)
 from .model_transform import find_tensor_release_timing, model_transform
 from .onnx_io import FLOAT, INT32, INT64, Model, clip_long
 from .tensor_loader import TensorLoader
@@ -76,8 +77,17 @@ class Runner:
         self._captured: Dict[tuple, "CapturedRun"] = {}
         self._seen: Dict[tuple, int] = {}
         self._uncapturable = False
+        # runs that are not replayed as a graph: from its second use on, a signature's calls are taped, and later runs
+        # repeat the tape with one call of the library.  None: this signature cannot be taped.
+        self._tapes: Dict[tuple, Optional["TapedRun"]] = {}
+        self._untapeable = set()                  # signatures whose first run used the cpu backend
     MAX_CAPTURED_SIGNATURES = 4                   # each recorded run keeps its own activation memory
+    MAX_TAPES = 64                                # a tape is a list of calls on the host: some 20 KB for ResNet-50
     GRAPH_REPLAY_AUTO_BATCH = 32
+
+    @staticmethod
+    def _signature(inputs) -> tuple:
+        return tuple([(tuple(t.dims), t.data_type, getattr(t, "layout", "nchw")) for t in inputs])
 
     def _replay_wanted(self, inputs) -> bool:
         if self.graph_replay:
@@ -116,6 +126,7 @@ class Runner:
                     model.graph.initializer[own[rec.name]] = t
                 else:
                     model.graph.initializer.append(t)
+        self._drop_tapes()
         model_transform(model, self.backend_order)
         if not model.opset_import:
             raise ValueError("opsetImport is empty")
@@ -151,7 +162,7 @@ class Runner:
                 raise ValueError(f"Unsupported initializer dataType {t.data_type}")
         return tensors
 
-    def capture(self, inputs: Sequence[CPUTensor]) -> CapturedRun:
+    def capture(self, inputs: Sequence[CPUTensor]) -> "CapturedRun":
         """Records ``run(inputs)`` on the cuda backend as a CUDA graph.  The run is executed once
         normally first (constants are moved, packed and split then), and the recorded run must stay on
         the device: a node placed on the cpu backend, or an operator that uploads host data while it
@@ -168,7 +179,7 @@ class Runner:
                 own = ctx.empty_tensor(t.dims, t.data_type)
                 ctx._call("wdc_copy", ctypes.c_void_p(own.ptr), ctypes.c_void_p(t.ptr), own.length * 4)
                 dev_in.append(own)
-        for o in self.run(dev_in, outputs_on_device=True):
+        for o in self._run_nodes(dev_in, outputs_on_device=True):
             o.dispose()
         if self.nodes_on("cpu"):
             for t in dev_in:
@@ -177,7 +188,7 @@ class Runner:
         ctx.sync()
         ctx.capture_begin()
         try:
-            outs = self.run(dev_in, outputs_on_device=True)
+            outs = self._canonical_outputs(self._run_nodes(dev_in, outputs_on_device=True))
         except Exception:
             try:
                 ctx.capture_end()
@@ -209,11 +220,13 @@ class Runner:
             raise RuntimeError("not initialized")
         if not wait:
             return self._run_pending(inputs)
-        if (self._replay_wanted(inputs) and not measure_performance and not outputs_on_device
-                and len(inputs) == len(self.inputs_without_initializer)
+        ctx = self.backend_contexts.get("cuda")
+        if (ctx is None or measure_performance or ctx.profile or len(inputs) != len(self.inputs_without_initializer)):
+            return self._run_nodes(inputs, measure_performance, outputs_on_device)
+        sig = self._signature(inputs)
+        if (not outputs_on_device and self._replay_wanted(inputs)
                 and all(t.backend == "cpu" or (t.backend == "cuda" and getattr(t, "layout", "nchw") == "nchw")
                         for t in inputs)):
-            sig = tuple((tuple(t.dims), t.data_type) for t in inputs)
             cap = self._captured.get(sig)
             if cap is None and not self._uncapturable and self._seen.get(sig, 0) >= 1 \
                     and len(self._captured) < self.MAX_CAPTURED_SIGNATURES:
@@ -225,7 +238,85 @@ class Runner:
             if cap is not None:
                 self.graph_replays += 1
                 return cap.run(inputs)
-            self._seen[sig] = self._seen.get(sig, 0) + 1
+        key = (outputs_on_device, sig)
+        tape = self._tapes.get(key)
+        if tape is not None:
+            self.node_backends = tape.node_backends
+            return tape.run(inputs)
+        seen = self._seen.get(sig, 0)
+        self._seen[sig] = seen + 1
+        if seen >= 1 and key not in self._tapes and sig not in self._untapeable:
+            return self._run_taping(inputs, key)
+        results = self._run_nodes(inputs, False, outputs_on_device)
+        if seen == 0 and self.nodes_on("cpu"):
+            self._untapeable.add(sig)
+        return results
+
+    @staticmethod
+    def _canonical_outputs(outs) -> list:
+        """Results in the row-major order a host reads, converted on the device where they are stored otherwise."""
+        canon = []
+        for o in outs:
+            c = o.context.canonical(o) if isinstance(o, CudaTensor) else o
+            if c is not o:
+                o.dispose()
+            canon.append(c)
+        return canon
+
+    def _run_taping(self, inputs, key):
+        """An ordinary run whose calls are noted (all nodes are on the cuda backend: the signature's first run showed
+        it).  Runs that cannot be repeated go node by node from then on."""
+        outputs_on_device = key[0]
+        ctx = self.backend_contexts["cuda"]
+        moved = []
+        dev_in = []
+        for t in inputs:
+            if t.backend == "cpu":
+                t = ctx.move_tensor(t)
+                moved.append(t)
+            else:
+                ctx.asserts_cuda_tensor(t)
+                ctx.wait_upload(t)
+            dev_in.append(t)
+        tape = None
+        ctx.tape_begin(dev_in)
+        try:
+            outs = self._run_nodes(dev_in, outputs_on_device=True)
+            if not outputs_on_device:
+                outs = self._canonical_outputs(outs)
+        except Exception:
+            ctx.tape_end(None)
+            for t in moved:
+                t.dispose()
+            raise
+        if all(isinstance(o, CudaTensor) for o in outs) and not self.nodes_on("cpu"):
+            tape = ctx.tape_end(outs)
+        else:
+            ctx.tape_end(None)
+        while len(self._tapes) >= self.MAX_TAPES:
+            old = self._tapes.pop(next(iter(self._tapes)))
+            if old is not None:
+                old.dispose()
+        self._tapes[key] = TapedRun(ctx, tape, outs, outputs_on_device, self.node_backends) if tape else None
+        if not outputs_on_device:
+            results = []
+            for o in outs:
+                results.append(o if o.backend == "cpu" else self.backend_contexts["cpu"].move_tensor(o, {}))
+                o.dispose()
+            outs = results
+        for t in moved:
+            t.dispose()
+        return outs
+
+    def _drop_tapes(self) -> None:
+        for tape in self._tapes.values():
+            if tape is not None:
+                tape.dispose()
+        self._tapes.clear()
+        self._untapeable.clear()
+
+    def _run_nodes(self, inputs, measure_performance: bool = False, outputs_on_device: bool = False):
+        """The run node by node."""
         graph = self.model.graph
         tensors_for_backends: Dict[str, Dict[str, object]] = {b: {} for b in BACKENDS}
         for name, tensor in self.initializer_tensors.items():
@@ -350,7 +441,7 @@ class Runner:
         cap = None
         replay = self._replay_wanted(inputs)
         if replay and len(inputs) == len(self.inputs_without_initializer):
-            cap = self._captured.get(tuple((tuple(t.dims), t.data_type) for t in inputs))
+            cap = self._captured.get(self._signature(inputs))
         if cap is not None:
             self.graph_replays += 1
             cap.load_inputs(inputs)
@@ -379,6 +470,7 @@ class Runner:
         for cap in self._captured.values():
             cap.dispose()
         self._captured.clear()
+        self._drop_tapes()
         for kv in self.copied_initializer_tensors.values():
             for t in kv.values():
                 t.dispose()
@@ -406,6 +498,59 @@ class PendingRun:
         return outs
 
 
+def _host_array(t) -> np.ndarray:
+    """A cpu tensor's data as the library takes it: contiguous, of the dtype's width."""
+    return np.ascontiguousarray(t.get_data(), dtype=NP_DTYPE[t.data_type])
+
+
+class TapedRun:
+    """One ``Runner.run`` as a tape of library calls (``wdc_tape_*``): a later run with inputs of the same dims, dtypes
+    and layouts is one call, without the interpreter's work per node.  Buffers are allocated anew by every run."""
+
+    def __init__(self, context: WebDNNCudaContext, tape: int, outputs: List[CudaTensor], on_device: bool, node_backends):
+        self.context, self.tape, self.on_device, self.node_backends = context, tape, on_device, node_backends
+        self.outputs = [CudaTensor.adopt(o, 0) for o in outputs]     # dims, dtype and layout of the results
+        for o in self.outputs:
+            o.disposed = True
+        n = len(outputs)
+        self._ptrs = ctypes.c_void_p * max(n, 1)
+        self._bytes = (ctypes.c_int64 * max(n, 1))(*(o.length * 4 for o in outputs))
+        self._run = context._L.lib.wdc_tape_run
+
+    def run(self, inputs):
+        ctx = self.context
+        n = len(inputs)
+        src, on_host, keep = (ctypes.c_void_p * n)(), (ctypes.c_int32 * n)(), []
+        for i, t in enumerate(inputs):
+            if t.backend == "cpu":
+                a = _host_array(t)
+                keep.append(a)
+                src[i] = a.__array_interface__["data"][0]
+                on_host[i] = 1
+            else:
+                ctx.asserts_cuda_tensor(t)
+                if t.upload_ticket is not None:
+                    ctx.wait_upload(t)
+                src[i] = t.ptr
+        out = self._ptrs()
+        if self.on_device:
+            host = None
+        else:
+            data = [np.empty(o.length, NP_DTYPE[o.data_type]) for o in self.outputs]
+            host = self._ptrs(*[a.__array_interface__["data"][0] for a in data])
+        st = self._run(ctx.handle, self.tape, src, on_host, out, host, self._bytes)
+        if st != 0:
+            ctx._L.check(ctx.handle, st)
+        if self.on_device:
+            return [CudaTensor.adopt(o, p) for o, p in zip(self.outputs, out)]
+        return [like_cpu_tensor(o, a) for o, a in zip(self.outputs, data)]
+
+    def dispose(self) -> None:
+        if self.tape is not None:
+            self.context.tape_destroy(self.tape)
+            self.tape = None
+
+
 class CapturedRun:
     """One ``Runner.run`` recorded as a CUDA graph (``Runner.capture``): every later ``run`` copies the
     inputs into the recorded input buffers, replays all launches with one call and reads the outputs
@@ -414,24 +559,47 @@ class CapturedRun:
 
     def __init__(self, context: WebDNNCudaContext, graph: int, inputs: List, outputs: List):
         self.context, self.graph, self.inputs, self.outputs = context, graph, inputs, outputs
+        n, m = len(inputs), len(outputs)
+        self._dst = (ctypes.c_void_p * max(n, 1))(*(t.ptr for t in inputs))
+        self._in_bytes = (ctypes.c_int64 * max(n, 1))(*(t.length * 4 for t in inputs))
+        self._out = (ctypes.c_void_p * max(m, 1))(*(t.ptr for t in outputs))
+        self._out_bytes = (ctypes.c_int64 * max(m, 1))(*(t.length * 4 for t in outputs))
 
     def launch(self) -> None:
         """Replay on the inputs currently in the recorded input buffers; results stay on the device."""
         self.context.graph_launch(self.graph)
 
     def run(self, inputs: Sequence[CPUTensor]) -> List[CPUTensor]:
-        if len(inputs) != len(self.inputs):
-            raise ValueError("length of inputs mismatch")
-        self.load_inputs(inputs)
-        self.launch()
-        return [self.context.cpu_context.empty_tensor(o.dims, o.data_type, o.get_data()) for o in self.outputs]
+        self._check_inputs(inputs)
+        ctx = self.context
+        n, m = len(inputs), len(self.outputs)
+        src, on_host, keep = (ctypes.c_void_p * n)(), (ctypes.c_int32 * n)(), []
+        for i, t in enumerate(inputs):
+            if t.backend == "cpu":
+                a = _host_array(t)
+                keep.append(a)
+                src[i] = a.__array_interface__["data"][0]
+                on_host[i] = 1
+            else:
+                # a batch already on the device (moved there by prefetch_tensor while the previous run computed):
+                # order after its transfer, then a device-to-device copy into the recorded input buffer
+                ctx.wait_upload(t)
+                src[i] = t.ptr
+        data = [np.empty(o.length, NP_DTYPE[o.data_type]) for o in self.outputs]
+        host = (ctypes.c_void_p * max(m, 1))(*[a.__array_interface__["data"][0] for a in data])
+        ctx._call("wdc_graph_run", self.graph, n, self._dst, src, self._in_bytes, on_host, m, host, self._out, self._out_bytes)
+        return [like_cpu_tensor(o, a) for o, a in zip(self.outputs, data)]
 
-    def load_inputs(self, inputs: Sequence[CPUTensor]) -> None:
+    def _check_inputs(self, inputs) -> None:
         if len(inputs) != len(self.inputs):
             raise ValueError("length of inputs mismatch")
         for dst, src in zip(self.inputs, inputs):
-            if list(src.dims) != list(dst.dims) or src.data_type != dst.data_type:
+            if list(src.dims) != dst.dims or src.data_type != dst.data_type:
                 raise ValueError("CapturedRun.run: input shape or dtype differs from the captured one")
+
+    def load_inputs(self, inputs: Sequence[CPUTensor]) -> None:
+        self._check_inputs(inputs)
+        for dst, src in zip(self.inputs, inputs):
             if src.backend == "cpu":
                 dst.set_data(src.get_data())
             else:
