@@ -44,6 +44,11 @@ int wdc_destroy(wdc_context* ctx);
 const char* wdc_last_error(wdc_context* ctx);
 int wdc_alloc(wdc_context* ctx, int64_t bytes, void** dptr);
 int wdc_free(wdc_context* ctx, void* dptr);
+/* Declares a buffer a constant of the model (an initializer, or one re-laid out from it): the caller promises that no
+ * work queued from now on writes it while it is used.  A contraction with such a weight may read it before the work
+ * queued earlier has finished, which is what its low-latency kernel lives on.  Freeing the buffer, or a call that
+ * writes it, ends the declaration. */
+int wdc_declare_constant(wdc_context* ctx, const void* ptr, int64_t bytes);
 /* Pinned host staging memory (page-locked), for callers that want true async H2D. */
 int wdc_host_alloc(wdc_context* ctx, int64_t bytes, void** hptr);
 int wdc_host_free(wdc_context* ctx, void* hptr);

@@ -111,3 +111,47 @@ def test_lstm_recurrence(cuda_context, seq, batch, inp, hidden, state):
             t.dispose()
     for g, w in zip(got, want):
         assert max_err_rel_linf(g, np.asarray(w).reshape(g.shape)) <= 1e-5
+
+
+# edges of the small kernel: rows of a tile and of its shares, columns of both tile widths, K blocks per CTA of a cluster,
+# more segments than accumulators, short last K blocks of a tap, strides and padding; it takes declared constants only
+@pytest.mark.parametrize("n,cin,cout,size,k,stride,pad,res", [
+    (1, 32, 32, (1, 1), 1, 1, 0, False), (1, 64, 36, (1, 127), 1, 1, 0, True), (1, 256, 64, (3, 43), 1, 1, 0, True),
+    (1, 512, 132, (7, 7), 3, 1, 1, True), (2, 100, 68, (9, 9), 3, 2, 1, False), (1, 1024, 256, (14, 14), 1, 1, 0, False),
+    (1, 36, 2048, (10, 10), 1, 1, 0, True), (1, 64, 256, (56, 56), 1, 1, 0, True), (1, 2048, 512, (5, 5), 1, 1, 0, False),
+    (3, 128, 128, (28, 28), 3, 1, 1, False), (1, 2304, 64, (8, 16), 1, 1, 0, False)])
+@pytest.mark.parametrize("precision", ["tf32x3", "tf32x1"])
+def test_small_outputs(cuda_context, n, cin, cout, size, k, stride, pad, res, precision):
+    from oracle import ops
+    from webdnn_b200.backend import CPUTensor
+    from webdnn_b200.lib import ConvDesc
+    ctx = cuda_context
+    rng = np.random.default_rng(cin + cout)
+    x = rng.standard_normal((n, cin, *size)).astype(np.float32)
+    w = (rng.standard_normal((cout, cin, k, k)) * np.sqrt(2.0 / (cin * k * k))).astype(np.float32)
+    scale, shift = rng.uniform(0.5, 1.5, cout).astype(np.float32), rng.uniform(-1, 1, cout).astype(np.float32)
+    oh, ow = ((s + 2 * pad - k) // stride + 1 for s in size)
+    r = rng.standard_normal((n, cout, oh, ow)).astype(np.float32)
+    want = ops.conv2d(x, w, None, (stride, stride), (pad,) * 4).astype(np.float64) * scale[:, None, None] + shift[:, None, None]
+    want = np.maximum(want + r, 0) if res else want
+    put = lambda a: ctx.move_tensor(CPUTensor.from_array(np.ascontiguousarray(a)))  # noqa: E731
+    dx, dr = ctx.channels_last(put(x)), ctx.channels_last(put(r))
+    dw, dsc, dsh = put(w.transpose(0, 2, 3, 1)), put(scale), put(shift)
+    ctx.declare_constant(dw)
+    ctx.declare_constant(dsc)
+    y = ctx.empty_tensor([n, cout, oh, ow], layout="nhwc")
+    d = ConvDesc(batch=n, ch_in=cin, in_h=size[0], in_w=size[1], ch_out=cout, k_h=k, k_w=k, out_h=oh, out_w=ow, stride_h=stride,
+                 stride_w=stride, pad_t=pad, pad_l=pad, dil_h=1, dil_w=1, group=1, relu=int(res))
+    ctx.set_precision(precision)
+    try:
+        for split_k in (1, 0):      # clusters of ranges, and one CTA per tile
+            ctx.set_option("split_k", split_k)
+            for _ in range(2):      # the first call splits the weights; the read waits, so the second loads them early
+                ctx.conv2d(d, dx, dw, dsc, dsh, dr if res else None, y)
+                got = y.get_data().reshape(want.shape)
+                assert max_err_rel_linf(got, want) <= (5e-6 if precision == "tf32x3" else 3e-3)
+    finally:
+        ctx.set_option("split_k", 1)
+        ctx.set_precision("tf32x3")
+    for t in (dx, dr, dw, dsc, dsh, y):
+        t.dispose()

@@ -162,6 +162,7 @@ class CudaTensor(TensorImpl):
         self.layout = layout
         self.aux: Dict[str, "CudaTensor"] = {}  # derived device data that lives and dies with this tensor
         self.upload_ticket: Optional[int] = None  # pending transfer on the copy stream (prefetch_tensor)
+        self.constant = False     # an initializer's copy, or data derived from one (WebDNNCudaContext.declare_constant)
         self.disposed = False
 
     @classmethod
@@ -173,7 +174,7 @@ class CudaTensor(TensorImpl):
         t.dims, t.ndim, t.data_type, t.backend = list(template.dims), template.ndim, template.data_type, "cuda"
         t.strides, t.length = list(template.strides), template.length
         t.context, t.byte_length, t.shared_buffer, t.layout = template.context, template.byte_length, buf, template.layout
-        t.aux, t.upload_ticket, t.disposed = {}, None, False
+        t.aux, t.upload_ticket, t.constant, t.disposed = {}, None, False, False
         return t
 
     @property
@@ -395,6 +396,11 @@ class WebDNNCudaContext:
         dst = CudaTensor(self, tensor.dims, tensor.data_type)
         dst.set_data(tensor.get_data())
         return dst
+
+    def declare_constant(self, t: CudaTensor) -> None:
+        """``t`` holds a constant of the model: nothing queued from now on writes it (``wdc_declare_constant``)."""
+        t.constant = True
+        self._call("wdc_declare_constant", c_void_p(t.ptr), t.length * 4)
 
     def decode_eightbit(self, codes: np.ndarray, scale: float, dims: Sequence[int]) -> CudaTensor:
         """float32 tensor from the 8-bit codes of a WDN2 container: the codes (1 byte per element)

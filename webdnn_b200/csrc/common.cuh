@@ -48,6 +48,8 @@ struct wdc_context {
   wdc_arena* capture_arena = nullptr;
   std::vector<wdc_arena*> graph_arenas;   // arenas owned by finished graphs (and by failed captures)
   std::vector<struct wdc_graph*> live_graphs;   // finished graphs not yet destroyed
+  std::map<const char*, int64_t> constants;   // wdc_declare_constant: start -> bytes
+  int64_t n_waits = 0;                    // times the host has waited for the whole compute stream
   int64_t split_seq = 0;                  // creation counter of the tensor-core path's cached operand splits
   // wdc_set_option
   int opt_precision = 0;                  // 0: tf32x3 (fp32-class accuracy), 1: tf32x1 (one pass, ~1e-3 relative)
@@ -163,8 +165,11 @@ void wdc_tc_evict(wdc_context* ctx, const void* ptr, int64_t bytes);
 // Every entry point that writes device memory reports its output here (the start; the length where it is
 // cheap to know).
 inline void wdc_note_write(wdc_context* ctx, const void* ptr, int64_t bytes = 0) {
-  if (ctx && ptr && ctx->tc_state) wdc_tc_evict(ctx, ptr, bytes);
+  if (ctx && ptr) wdc_tc_evict(ctx, ptr, bytes);
 }
+// Whether p starts a buffer declared constant; drops the declarations that overlap [lo, hi) (context.cu).
+bool wdc_is_constant(wdc_context* ctx, const void* p);
+void wdc_forget_constants(wdc_context* ctx, const char* lo, const char* hi);
 // Extent [*lo, *hi) of the live arena allocation (of any arena of the context) that contains p; false if none.
 bool wdc_arena_extent(wdc_context* ctx, const void* p, const char** lo, const char** hi);
 // A cached split with creation number `born` has been dropped: captured graphs recorded while it existed

@@ -282,6 +282,29 @@ extern "C" int wdc_free(wdc_context* ctx, void* dptr) {
   return WDC_OK;
 }
 
+extern "C" int wdc_declare_constant(wdc_context* ctx, const void* ptr, int64_t bytes) {
+  if (!ctx || !ptr || bytes < 0) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_declare_constant: bad argument");
+  WDC_NO_TAPE(ctx);
+  std::lock_guard<std::mutex> lk(ctx->mu);
+  ctx->constants[(const char*)ptr] = bytes > 0 ? bytes : 1;
+  return WDC_OK;
+}
+
+bool wdc_is_constant(wdc_context* ctx, const void* p) {
+  std::lock_guard<std::mutex> lk(ctx->mu);
+  return ctx->constants.count((const char*)p) != 0;
+}
+
+void wdc_forget_constants(wdc_context* ctx, const char* lo, const char* hi) {
+  std::lock_guard<std::mutex> lk(ctx->mu);
+  auto it = ctx->constants.lower_bound(lo);
+  if (it != ctx->constants.begin()) {
+    auto before = std::prev(it);
+    if (before->first + before->second > lo) it = before;
+  }
+  while (it != ctx->constants.end() && it->first < hi) it = ctx->constants.erase(it);
+}
+
 extern "C" int wdc_host_alloc(wdc_context* ctx, int64_t bytes, void** hptr) {
   if (!ctx || !hptr || bytes < 0) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_host_alloc: bad argument");
   DeviceGuard g(ctx->device);
@@ -466,6 +489,7 @@ extern "C" int wdc_sync(wdc_context* ctx) {
   WDC_NO_TAPE(ctx);
   DeviceGuard g(ctx->device);
   WDC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  ctx->n_waits++;
   return report_device_status(ctx);
 }
 

@@ -57,6 +57,9 @@
 #include <cuda.h>
 
 #include <cstddef>
+#ifdef WDC_TC_DEVELOP
+#include <cstdio>
+#endif
 #include <cstdlib>
 #include <cstring>
 #include <map>
@@ -1267,6 +1270,8 @@ tc_igemm_kernel(const __grid_constant__ TcProblem p, const float* __restrict__ x
   }
 }
 
+#include "conv_tc_small.cuh"
+
 // ---------------------------------------------------------------------------- host side
 // Row r of the weight matrix is multiplied by alpha * scale[r] (scale null = 1) before the split, so
 // that the kernel's epilogue has no per-channel multiply left.
@@ -1451,11 +1456,28 @@ struct WeightEntry {
   int64_t rows = 0, k = 0;
   int64_t src_bytes = 0;  // size of the caller's weight buffer the split was made from
   int64_t born = 0;       // creation number (wdc_context::split_seq), for the staleness of captured graphs
+  // The weight and its scale are declared constants (wdc_declare_constant): tc_small_kernel takes only those, because
+  // it may read them before it waits for earlier grids.  It does so once the split has settled, i.e. is known to have
+  // finished: the host has waited for the stream since (waits = the context's count when the split was queued), or
+  // `done` says so, which is asked from the SETTLE_USES-th use on.  (The choice of the kernel depends on the
+  // declaration alone, so that a run gives the same bits every time.)
+  bool constant = false;
+  bool settled = false;
+  int64_t waits = 0;
+  int uses = 0;
+  cudaEvent_t done = nullptr;
   // tensor maps of the split copies for tile heights of 32, 64 and 128 weight rows (index log2(n / 32)),
   // encoded when a launch first asks for that height
   CUtensorMap map_hi[3], map_lo[3];
   bool has_map[3] = {false, false, false};
 };
+
+constexpr int SETTLE_USES = 4;
+
+void forget_event(WeightEntry& e) {
+  if (e.done) cudaEventDestroy(e.done);
+  e.done = nullptr;
+}
 
 struct TcState {
   EncodeTiledFn encode = nullptr;
@@ -1506,7 +1528,13 @@ int get_weight(wdc_context* ctx, const float* w, const float* scale, float alpha
   memcpy(&key.alpha_bits, &alpha, 4);
   auto it = st->weights.find(key);
   if (it != st->weights.end() && it->second.rows == rows && it->second.k == k) {
-    *out = &it->second;
+    WeightEntry& e = it->second;
+    if (e.constant && !e.settled) {
+      e.settled = ctx->n_waits > e.waits ||
+                  (++e.uses >= SETTLE_USES && !ctx->capture_arena && e.done && cudaEventQuery(e.done) == cudaSuccess);
+      if (e.settled) forget_event(e);
+    }
+    *out = &e;
     return WDC_OK;
   }
   if (ctx->capture_arena)
@@ -1515,6 +1543,7 @@ int get_weight(wdc_context* ctx, const float* w, const float* scale, float alpha
                     "wdc_capture_begin, so that the one-time split is not part of the recorded run");
   if (it != st->weights.end()) {
     WeightEntry old = it->second;
+    forget_event(old);
     st->weights.erase(it);
     wdc_graphs_note_evicted(ctx, old.born);
     wdc_free(ctx, old.hi);
@@ -1546,6 +1575,13 @@ int get_weight(wdc_context* ctx, const float* w, const float* scale, float alpha
     return s;
   }
   e.born = ++ctx->split_seq;
+  e.waits = ctx->n_waits;
+  e.constant = wdc_is_constant(ctx, w) && (!scale || wdc_is_constant(ctx, scale));
+  if (e.constant && (cudaEventCreateWithFlags(&e.done, cudaEventDisableTiming) != cudaSuccess ||
+                     cudaEventRecord(e.done, ctx->stream) != cudaSuccess)) {
+    cudaGetLastError();
+    forget_event(e);
+  }
   auto ins = st->weights.emplace(key, e);
   *out = &ins.first->second;
   return WDC_OK;
@@ -1676,6 +1712,106 @@ void choose_tiling(const wdc_context* ctx, int64_t m, int64_t n, int kblocks, bo
   }
 }
 
+// Tile width and cluster size of tc_small_kernel for an [M, N] output, and whether the launch is likely to be shorter
+// than the persistent kernel's with the tiling given (choose_tiling's).  Microseconds, fitted to the layers of ResNet-50
+// at one image (224 and 800 pixels) and of the DETR-style transformer, each launch behind others in a replayed graph:
+//   small       2.4 (32 columns) or 3.1 (64) + 0.006 per CTA, a K block 0.35 or 0.50, half as much again where two CTAs
+//               share an SM; a cluster adds 0.3 and its exchange, 16 bytes a clock and CTA.  At most two CTAs per SM,
+//               so nothing with more than 296 of them;
+//   persistent  3.6 + 0.03 per column of a tile (set-up, the tile's way out), a K block 0.55 whatever the width; a cut
+//               reduction 4 for the second launch, and the partial sums' way through L2.
+// Some of what it decides, us per launch (persistent -> small): [196, 2304] x 256 13.2 -> 7.2, [49, 512] x 2048 12.8 ->
+// 6.4, [100, 2048] x 256 11.8 -> 6.0, [1280, 1024] x 256 21.2 -> 10.3, [625, 2048] x 512 18.2 -> 15.6.
+bool choose_small(const wdc_context* ctx, const TcProblem& p, int tile_n, int splits, int full_tiles, int* tn, int* cs) {
+  const int64_t tiles_m = ceil_div64(p.M, TILE_M);
+  const int sms = ctx->sm_count;
+  const int rows = p.M < TILE_M ? (int)p.M : TILE_M;
+  double best = 1e30;
+  for (int t = 32; t <= 64; t *= 2) {
+    const int64_t tiles = tiles_m * ceil_div64(p.N, t);
+    for (int c = 1; c <= 8; c *= 2) {
+      const int kbs = (p.kblocks + c - 1) / c;
+      if (tiles * c > 2 * sms || (c - 1) * kbs >= p.kblocks || (c > 1 && !ctx->opt_split_k)) break;
+      double us = (t == 32 ? 2.4 : 3.1) + 0.006 * (double)(tiles * c) + kbs * (t == 32 ? 0.35 : 0.50) * (tiles * c > sms ? 1.45 : 1.0);
+      if (c > 1) us += 0.3 + rows * t * 4.0 * (c - 1) / c / 16 / 1900;
+      if (us < best) {
+        best = us;
+        *tn = t;
+        *cs = c;
+      }
+    }
+  }
+  const int64_t tiles = tiles_m * ceil_div64(p.N, tile_n);
+  double big = 3.6 + 0.03 * tile_n;
+  if (splits == 1) {
+    big += (double)ceil_div64(tiles, sms) * p.kblocks * 0.55;
+  } else {
+    const int64_t rest = tiles - full_tiles;
+    const int kbs = (p.kblocks + splits - 1) / splits;
+    big += ((double)(full_tiles / sms) * p.kblocks + (double)ceil_div64(rest * splits, sms) * kbs) * 0.55;
+    big += 4.0 + 2.0 * (double)(rest * splits) * TILE_M * tile_n * 4 / 6.5e6;
+  }
+  return best < big;
+}
+
+// A launch of tc_small_kernel: p.kblocks, tile counts and geometry are set; `tn` and `cs` chosen by the caller.
+int launch_small(wdc_context* ctx, TcProblem& p, WeightEntry* we, const CUtensorMap& map_a, float* y, int tn, int cs) {
+  typedef void (*Kernel)(const TcProblem, const CUtensorMap, const CUtensorMap, const CUtensorMap, float*, int);
+  static const Kernel kernels[2][4] = {
+      {tc_small_kernel<32, 1>, tc_small_kernel<32, 2>, tc_small_kernel<32, 4>, tc_small_kernel<32, 8>},
+      {tc_small_kernel<64, 1>, tc_small_kernel<64, 2>, tc_small_kernel<64, 4>, tc_small_kernel<64, 8>}};
+  const int wide = tn == 64, ci = cs == 8 ? 3 : cs == 4 ? 2 : cs == 2 ? 1 : 0;
+  const Kernel kernel = kernels[wide][ci];
+  const int smem = wide ? SmallLayout<64>::SMEM : SmallLayout<32>::SMEM;
+  static bool attr_set[64][2][4] = {};
+  if (ctx->device < 0 || ctx->device >= 64) return WDC_ERR_UNSUPPORTED;
+  if (!attr_set[ctx->device][wide][ci]) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
+      cudaGetLastError();
+      return WDC_ERR_UNSUPPORTED;
+    }
+    attr_set[ctx->device][wide][ci] = true;
+  }
+  p.tile_n = tn;
+  p.tiles_m = (int)ceil_div64(p.M, TILE_M);
+  p.tiles_n = (int)ceil_div64(p.N, tn);
+  p.kbs = (p.kblocks + cs - 1) / cs;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)cs;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(p.tiles_m * p.tiles_n * cs));
+  cfg.blockDim = dim3(SM_THREADS);
+  cfg.dynamicSmemBytes = (size_t)smem;
+  cfg.stream = ctx->stream;
+  cfg.attrs = ctx->opt_pdl ? attr : attr + 1;
+  cfg.numAttrs = ctx->opt_pdl ? 2 : 1;
+  const int mi = wide ? 1 : 0;
+  const TcProblem& pc = p;
+  cudaError_t le = cudaLaunchKernelEx(&cfg, kernel, pc, we->map_hi[mi], we->map_lo[mi], map_a, y, we->settled ? 1 : 0);
+  ctx->n_tc_launch++;
+  ctx->n_launch++;
+  int s = wdc_check_cuda(ctx, le, "tc_small_kernel");
+  if (s == WDC_OK) s = wdc_check_cuda(ctx, cudaGetLastError(), "tc_small_kernel");
+  return s;
+}
+
+// Maps of the split weight for tiles of tile_n rows.
+int weight_maps(wdc_context* ctx, WeightEntry* we, int tile_n) {
+  const int mi = tile_n == 128 ? 2 : tile_n == 64 ? 1 : 0;
+  if (we->has_map[mi]) return WDC_OK;
+  const int r1 = encode_map(tc_state(ctx), &we->map_hi[mi], we->hi, we->rows, we->k, tile_n);
+  const int r2 = encode_map(tc_state(ctx), &we->map_lo[mi], we->lo, we->rows, we->k, tile_n);
+  if (r1 || r2)
+    return wdc_fail(ctx, WDC_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d, %d) for a [%lld, %lld] weight", r1, r2,
+                    (long long)we->rows, (long long)we->k);
+  we->has_map[mi] = true;
+  return WDC_OK;
+}
+
 int launch_tc(wdc_context* ctx, TcProblem& p, const float* x, const float* w, float* y, int c4_kw = 0,
               int c4_cin = 0, bool w_k_major = true) {
   WeightEntry* we = nullptr;
@@ -1684,22 +1820,32 @@ int launch_tc(wdc_context* ctx, TcProblem& p, const float* x, const float* w, fl
   p.scale = nullptr;  // folded into the split weights
   p.alpha = 1.f;
   p.kblocks = p.c4 ? p.K / BLOCK_K : p.k_h * p.k_w * p.cblocks;   // K blocks are counted per filter tap
+  p.status = ctx->status_word;
+  p.single_pass = ctx->opt_precision == 1 ? 1 : 0;
   {
     // a split reduction needs the TMA paths on both sides (checked again below) and no first-layer mode
-    const bool may_split = !p.c4 && p.N % 4 == 0 && p.M < (1ll << 27) && tc_state(ctx)->encode_im2col != nullptr &&
-                           (((uintptr_t)p.shift | (uintptr_t)p.residual | (uintptr_t)y) & 15) == 0 &&
-                           (!p.residual || p.res_stride % 4 == 0) && ctx->opt_split_k;
+    const bool may_cut = !p.c4 && p.N % 4 == 0 && p.M < (1ll << 27) && tc_state(ctx)->encode_im2col != nullptr &&
+                         (((uintptr_t)p.shift | (uintptr_t)p.residual | (uintptr_t)y) & 15) == 0 &&
+                         (!p.residual || p.res_stride % 4 == 0);
+    const bool may_split = may_cut && ctx->opt_split_k;
     choose_tiling(ctx, p.M, p.N, p.kblocks, may_split, &p.tile_n, &p.splits, &p.full_tiles);
+    int tn = 0, cs = 0;
+    bool small = may_cut && we->constant && choose_small(ctx, p, p.tile_n, p.splits, p.full_tiles, &tn, &cs);
+#ifdef WDC_TC_DEVELOP
+    if (const char* e = getenv("WDC_TC_SMALL")) {   // "tn,cs" forces the small kernel with that shape, "0,0" the other
+      sscanf(e, "%d,%d", &tn, &cs);
+      small = may_cut && we->constant && tn > 0;
+    }
+#endif
+    CUtensorMap map_a;
+    if (small && encode_a_map(tc_state(ctx), p, x, &map_a)) {
+      s = weight_maps(ctx, we, tn);
+      return s != WDC_OK ? s : launch_small(ctx, p, we, map_a, y, tn, cs);
+    }
   }
   const int mi = p.tile_n == 128 ? 2 : p.tile_n == 64 ? 1 : 0;
-  if (!we->has_map[mi]) {
-    const int r1 = encode_map(tc_state(ctx), &we->map_hi[mi], we->hi, we->rows, we->k, p.tile_n);
-    const int r2 = encode_map(tc_state(ctx), &we->map_lo[mi], we->lo, we->rows, we->k, p.tile_n);
-    if (r1 || r2)
-      return wdc_fail(ctx, WDC_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d, %d) for a [%lld, %lld] weight", r1, r2,
-                      (long long)we->rows, (long long)we->k);
-    we->has_map[mi] = true;
-  }
+  s = weight_maps(ctx, we, p.tile_n);
+  if (s != WDC_OK) return s;
   const CUtensorMap& w_map_hi = we->map_hi[mi];
   const CUtensorMap& w_map_lo = we->map_lo[mi];
   if (ceil_div64(p.M, TILE_M) * ceil_div64(p.N, p.tile_n) >= (1ll << 31) - 65536) return WDC_ERR_UNSUPPORTED;
@@ -1845,9 +1991,8 @@ bool aligned16(const void* p) { return (((uintptr_t)p) & 15) == 0; }
 }  // namespace
 
 void wdc_tc_evict(wdc_context* ctx, const void* ptr, int64_t bytes) {
-  if (!ctx->tc_state) return;
   TcState* st = (TcState*)ctx->tc_state;
-  if (st->weights.empty()) return;
+  if ((!st || st->weights.empty()) && ctx->constants.empty()) return;
   // written extent: the byte range, widened to the arena allocation that contains its start
   const char* lo = (const char*)ptr;
   const char* hi = lo + (bytes > 0 ? bytes : 1);
@@ -1856,6 +2001,8 @@ void wdc_tc_evict(wdc_context* ctx, const void* ptr, int64_t bytes) {
     if (blo < lo) lo = blo;
     if (bhi > hi) hi = bhi;
   }
+  wdc_forget_constants(ctx, lo, hi);
+  if (!st) return;
   // entries whose weight buffer or per-channel scale vector overlaps [lo, hi)
   std::vector<WeightEntry> dropped;
   for (auto it = st->weights.begin(); it != st->weights.end();) {
@@ -1863,6 +2010,7 @@ void wdc_tc_evict(wdc_context* ctx, const void* ptr, int64_t bytes) {
     const char* sc = (const char*)it->first.scale;
     const bool hit = (w < hi && lo < w + it->second.src_bytes) || (sc && sc < hi && lo < sc + it->second.rows * 4);
     if (hit) {
+      forget_event(it->second);
       dropped.push_back(it->second);
       it = st->weights.erase(it);
     } else {
@@ -1878,6 +2026,7 @@ void wdc_tc_evict(wdc_context* ctx, const void* ptr, int64_t bytes) {
 
 void wdc_tc_destroy(wdc_context* ctx) {
   if (!ctx->tc_state) return;
+  for (auto& w : ((TcState*)ctx->tc_state)->weights) forget_event(w.second);
   delete (TcState*)ctx->tc_state;  // the split buffers die with the arena slabs
   ctx->tc_state = nullptr;
 }

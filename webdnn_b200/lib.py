@@ -79,6 +79,7 @@ SIGNATURES = {
     "wdc_last_error": (c_char_p, [c_void_p]),
     "wdc_alloc": (c_int, [c_void_p, c_int64, POINTER(c_void_p)]),
     "wdc_free": (c_int, [c_void_p, c_void_p]),
+    "wdc_declare_constant": (c_int, [c_void_p, c_void_p, c_int64]),
     "wdc_host_alloc": (c_int, [c_void_p, c_int64, POINTER(c_void_p)]),
     "wdc_host_free": (c_int, [c_void_p, c_void_p]),
     "wdc_upload": (c_int, [c_void_p, c_void_p, c_void_p, c_int64]),

@@ -255,6 +255,8 @@ class CudaMatMulBias(OperatorImpl):
             if wt is None:
                 wt = context.empty_tensor([n, k], "float32")
                 context.strided_copy(w, wt, [n, k], [1, n], 0, [k, 1], 0)
+                if w.constant:
+                    context.declare_constant(wt)
                 w.aux["nk"] = wt
             d = ConvDesc(batch=1, ch_in=k, in_h=1, in_w=m, ch_out=n, k_h=1, k_w=1, out_h=1, out_w=m, stride_h=1,
                          stride_w=1, pad_t=0, pad_l=0, dil_h=1, dil_w=1, group=1, relu=int(self.relu), x_nchw=0)
@@ -356,6 +358,8 @@ def _packed_weight(context: WebDNNCudaContext, w: CudaTensor) -> CudaTensor:
         co, cig, kh, kw = w.dims
         pk = context.empty_tensor([co, kh, kw, cig], "float32")
         context._call("wdc_pack_conv_weight", _p(w), _p(pk), co, cig, kh, kw)
+        if w.constant:
+            context.declare_constant(pk)
         w.aux["krsc"] = pk
     return pk
 
@@ -898,6 +902,8 @@ class CudaConvTranspose(OperatorImpl):
                 taps = ks[0] * ks[1]
                 wk = context.empty_tensor([ch_in, ks[0], ks[1], cog], "float32")
                 context.strided_copy(w, wk, [ch_in, taps, cog], [cog * taps, 1, taps], 0, [taps * cog, cog, 1], 0)
+                if w.constant:
+                    context.declare_constant(wk)
                 inputs[1].aux["ckkc"] = wk
             w_layout = 1
         d = ConvTransposeDesc(batch=batch, ch_in=ch_in, in_h=in_h, in_w=in_w, ch_out_per_group=cog, group=self.group,

@@ -372,6 +372,8 @@ class Runner:
                     if other_t is not None:
                         moved = self.backend_contexts[req].move_tensor(
                             other_t, self.tensor_move_options.get(input_name, {}))
+                        if req == "cuda" and input_name in self.initializer_tensors:
+                            self.backend_contexts[req].declare_constant(moved)
                         tensors_for_backends[req][input_name] = moved
                         operator_inputs.append(moved)
                         break
