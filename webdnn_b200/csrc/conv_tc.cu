@@ -341,39 +341,6 @@ __device__ __forceinline__ uint32_t make_idesc(int n) {
   return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(TILE_M >> 4) << 24);
 }
 
-// D[tmem] (+)= A[tmem] * B[smem], the shared-memory descriptor given as its two 32-bit halves (only the low one, which holds the start
-// address, changes from MMA to MMA) and the accumulate flag as a compile-time constant where it is one: the issuing
-// thread is a single lane whose instruction count per K block is part of the kernel's serial path.
-template <bool kAccumulate>
-__device__ __forceinline__ void umma_tf32_ts2(uint32_t tmem_c, uint32_t tmem_a, uint32_t desc_lo, uint32_t desc_hi,
-                                              uint32_t idesc, uint32_t accumulate = 1) {
-  if (kAccumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t.reg .b64 d;\n\t"
-        "mov.b64 d, {%2, %3};\n\t"
-        "setp.eq.b32 p, 0, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], d, %4, p;\n\t}"
-        :
-        : "r"(tmem_c), "r"(tmem_a), "r"(desc_lo), "r"(desc_hi), "r"(idesc)
-        : "memory");
-  } else {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t.reg .b64 d;\n\t"
-        "mov.b64 d, {%2, %3};\n\t"
-        "setp.ne.b32 p, %5, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], d, %4, p;\n\t}"
-        :
-        : "r"(tmem_c), "r"(tmem_a), "r"(desc_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate)
-        : "memory");
-  }
-}
-__device__ __forceinline__ void umma_commit_addr(uint32_t bar_saddr) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_saddr) : "memory");
-}
-__device__ __forceinline__ void umma_commit(unsigned long long* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-               : "memory");
-}
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, unsigned long long* bar,
                                             int x, int y) {
   asm volatile(
@@ -428,6 +395,59 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const float* v) {
       :
       : "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
         "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+
+// Barrier operations on shared-memory addresses: the loops below step through them with additions.
+__device__ __forceinline__ bool try_wait_at(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.b32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ bool test_at(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.b32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ void arrive_at(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void expect_at(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+// tcgen05.mma with A in tensor memory by the lane whose `leader` is 1.  The whole warp runs the issuing loop, so that
+// its addresses are the same in every lane and stay in uniform registers: in a branch of the elected lane alone the
+// arithmetic between two K blocks took longer than their MMAs.
+__device__ __forceinline__ void umma_by(uint32_t leader, uint32_t tmem_c, uint32_t tmem_a, uint32_t desc_lo, uint32_t desc_hi,
+                                        uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, e;\n\t.reg .b64 d;\n\t"
+      "mov.b64 d, {%3, %4};\n\t"
+      "setp.ne.b32 e, %0, 0;\n\t"
+      "setp.ne.b32 p, %6, 0;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::tf32 [%1], [%2], d, %5, p;\n\t}"
+      :
+      : "r"(leader), "r"(tmem_c), "r"(tmem_a), "r"(desc_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void commit_by(uint32_t leader, uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .pred e;\n\t"
+      "setp.ne.b32 e, %0, 0;\n\t"
+      "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%1];\n\t}" ::"r"(leader),
+      "r"(bar)
       : "memory");
 }
 
@@ -864,95 +884,91 @@ tc_igemm_kernel(const __grid_constant__ TcProblem p, const float* __restrict__ x
     }
   } else if (warp == MMA_WARP) {
     // ===================================================================== MMA issuer
-    if (elect_one()) {
-      int stage = 0;
-      uint32_t phase = 0;
-      const uint32_t idesc = make_idesc(p.tile_n);
-      // per-stage operand addresses from a few bases: descriptor low words (start address in 16-byte units) of the
-      // W_hi / W_lo slots, the high word all descriptors share, TMEM column of the stage's A, barrier addresses
-      const uint64_t desc0 = make_smem_desc(smem_u32(w_hi_ptr(0)));
-      const uint32_t desc_hi32 = (uint32_t)(desc0 >> 32);
-      const uint32_t dwh0 = (uint32_t)desc0, dwl0 = (uint32_t)make_smem_desc(smem_u32(w_lo_ptr(0)));
-      const uint32_t dslot = w_slot >> 4;
-      const uint32_t a_col0 = tmem_base + (uint32_t)TMEM_A_COL0;
-      const uint32_t empty0 = smem_u32(&ss->empty_bar[0]);
-      int64_t seg = 0;  // segments issued by this CTA so far
-      bool ok = true;
-      bool f_tok = false;   // answer of the probe made one K block earlier
-      bool s_tok = false;   // the same for the next segment's accumulator
-      PROF_DECL(5);
-      int gk = 0;
-      for (int u = blockIdx.x; u < total_units && ok; u += gridDim.x) {
-        int tile, sp, kb0, kbn;
-        unit_of(p, u, tile, sp, kb0, kbn);
-        uint32_t d_tmem = 0;
-        int buf = 0;
-        int in_seg = 0;
-        for (int kb = 0; kb < kbn; kb++) {
-          const bool seg_last = kb == kbn - 1 || (in_seg == SEG_KBLOCKS - 1 && kbn - (kb + 1) >= SEG_KBLOCKS);
-          PROF_ADD(2);
-          if (in_seg == 0) {
-            buf = (int)(seg % NBUF);
-            if (!s_tok && !mbar_wait(&ss->seg_empty_bar[buf], (uint32_t)((seg / NBUF) & 1) ^ 1, ss, p.status, 31, p.nap_ns)) { ok = false; break; }
-            s_tok = false;
-            PROF_ADD(0);
-            PROF_EV(5, gk);
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            d_tmem = tmem_base + (uint32_t)(buf * 128);
-          }
+    // (all lanes run the loop, one issues: see umma_by)
+    const uint32_t leader = elect_one() ? 1u : 0u;
+    const uint32_t idesc = make_idesc(p.tile_n);
+    // operand addresses step from stage to stage: descriptor low words (start address in 16-byte units) of W_hi, the
+    // high word all descriptors share, the TMEM column of the stage's A, barrier addresses
+    const uint64_t desc0 = make_smem_desc(smem_u32(w_hi_ptr(0)));
+    const uint32_t top = (uint32_t)(desc0 >> 32), w0 = (uint32_t)desc0, dslot = w_slot >> 4;
+    const uint32_t wl_off = (uint32_t)STAGES * dslot;
+    const uint32_t a_col0 = tmem_base + (uint32_t)TMEM_A_COL0;
+    const uint32_t full0 = smem_u32(&ss->full_bar[0]), empty0 = smem_u32(&ss->empty_bar[0]);
+    const uint32_t segf0 = smem_u32(&ss->seg_full_bar[0]), sege0 = smem_u32(&ss->seg_empty_bar[0]);
+    uint32_t wh = w0, a_hi = a_col0, f_bar = full0, e_bar = empty0, phase = 0;
+    int stage = 0;
+    int64_t seg = 0;  // segments issued by this CTA so far
+    bool ok = true;
+    bool f_tok = false;   // answer of the probe made one K block earlier
+    bool s_tok = false;   // the same for the next segment's accumulator
+    PROF_DECL(5);
+    int gk = 0;
+    for (int u = blockIdx.x; u < total_units && ok; u += gridDim.x) {
+      int tile, sp, kb0, kbn;
+      unit_of(p, u, tile, sp, kb0, kbn);
+      const int nseg = segments_of(kbn);
+      for (int si = 0; si < nseg && ok; si++) {
+        const int n = si == nseg - 1 ? kbn - si * SEG_KBLOCKS : SEG_KBLOCKS;
+        const uint32_t buf = (uint32_t)seg & 1u, s_par = (uint32_t)((seg >> 1) & 1) ^ 1u;
+        PROF_ADD(2);
+        if (!s_tok && !mbar_wait(&ss->seg_empty_bar[buf], s_par, ss, p.status, 31, p.nap_ns)) { ok = false; break; }
+        s_tok = false;
+        PROF_ADD(0);
+        PROF_EV(5, gk);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t d_tmem = tmem_base + buf * 128u;
+        for (int i = 0; i < n; i++) {
           PROF_CNT(15, !f_tok);
           if (!f_tok && !mbar_wait(&ss->full_bar[stage], phase, ss, p.status, 32, p.nap_ns)) { ok = false; break; }
           f_tok = false;
           PROF_ADD(1);
           PROF_EV(3, gk);
-          const int stage_n = stage + 1 == STAGES ? 0 : stage + 1;
-          const uint32_t phase_n = stage_n ? phase : phase ^ 1;
+          const bool wrap = stage + 1 == STAGES;
+          const uint32_t f_bar_n = wrap ? full0 : f_bar + 8u, phase_n = wrap ? phase ^ 1u : phase;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t a_hi = a_col0 + (uint32_t)(stage * 64);
-          const uint32_t a_lo = a_hi + 32u;
-          const uint32_t dw_hi = dwh0 + (uint32_t)stage * dslot;
-          const uint32_t dw_lo = dwl0 + (uint32_t)stage * dslot;
+          const uint32_t a_lo = a_hi + 32u, wl = wh + wl_off, first = i ? 1u : 0u;
+          if (p.single_pass) {
 #pragma unroll
-          for (int k = 0; k < BLOCK_K / 8; k++) {
-            const uint32_t adv = (uint32_t)(k * 2);  // 8 tf32 = 32 bytes = 2 x 16-byte units of W
-            const uint32_t acol = (uint32_t)(k * 8); // 8 TMEM columns of A
-            if (TC_DBG(p, 4)) continue;
-            if (p.single_pass) {
-              if (k == 0) umma_tf32_ts2<false>(d_tmem, a_hi, dw_hi, desc_hi32, idesc, in_seg ? 1u : 0u);
-              else umma_tf32_ts2<true>(d_tmem, a_hi + acol, dw_hi + adv, desc_hi32, idesc);
-              continue;
-            }
-            if (k == 0) umma_tf32_ts2<false>(d_tmem, a_lo, dw_hi, desc_hi32, idesc, in_seg ? 1u : 0u);
-            else umma_tf32_ts2<true>(d_tmem, a_lo + acol, dw_hi + adv, desc_hi32, idesc);
-            umma_tf32_ts2<true>(d_tmem, a_hi + acol, dw_lo + adv, desc_hi32, idesc);
-            umma_tf32_ts2<true>(d_tmem, a_hi + acol, dw_hi + adv, desc_hi32, idesc);
-            if (k == PROBE_AFTER_K && !TC_DBG(p, 4096)) {
-              // Probe the next stage's barrier (see the operand splitters) with MMAs of this stage already queued:
-              // the answer takes about 150 cycles, during which this lane issues nothing and the tensor pipe works on
-              // what is queued.  On a segment's last K block also the accumulator the next segment will use.
-              f_tok = mbar_test(&ss->full_bar[stage_n], phase_n);
-              if (seg_last)
-                s_tok = mbar_test(&ss->seg_empty_bar[(int)((seg + 1) % NBUF)], (uint32_t)(((seg + 1) / NBUF) & 1) ^ 1);
+            for (int k = 0; k < BLOCK_K / 8; k++)
+              umma_by(leader, d_tmem, a_hi + (uint32_t)(k * 8), wh + (uint32_t)(k * 2), top, idesc, k ? 1u : first);
+            f_tok = test_at(f_bar_n, phase_n);
+            if (i == n - 1) s_tok = test_at(sege0 + (buf ^ 1u) * 8u, (uint32_t)(((seg + 1) >> 1) & 1) ^ 1u);
+          } else {
+#pragma unroll
+            for (int k = 0; k < BLOCK_K / 8; k++) {
+              const uint32_t adv = (uint32_t)(k * 2);  // 8 tf32 = 32 bytes = 2 x 16-byte units of W
+              const uint32_t acol = (uint32_t)(k * 8); // 8 TMEM columns of A
+              if (TC_DBG(p, 4)) continue;
+              umma_by(leader, d_tmem, a_lo + acol, wh + adv, top, idesc, k ? 1u : first);
+              umma_by(leader, d_tmem, a_hi + acol, wl + adv, top, idesc, 1u);
+              umma_by(leader, d_tmem, a_hi + acol, wh + adv, top, idesc, 1u);
+              if (k == PROBE_AFTER_K && !TC_DBG(p, 4096)) {
+                // Probe the next stage's barrier (see the operand splitters) with MMAs of this stage already queued:
+                // the answer takes about 150 cycles, during which this warp issues nothing and the tensor pipe works on
+                // what is queued.  On a segment's last K block also the accumulator the next segment will use.
+                f_tok = test_at(f_bar_n, phase_n);
+                if (i == n - 1) s_tok = test_at(sege0 + (buf ^ 1u) * 8u, (uint32_t)(((seg + 1) >> 1) & 1) ^ 1u);
+              }
             }
           }
           PROF_ADD(3);
-          umma_commit_addr(empty0 + (uint32_t)stage * 8u);  // stage reusable once these MMAs have read it
-
+          commit_by(leader, e_bar);  // stage reusable once these MMAs have read it
           PROF_ADD(4);
           PROF_EV(4, gk);
           gk++;
-          stage = stage_n; phase = phase_n;
-          if (seg_last) {
-            umma_commit(&ss->seg_full_bar[buf]);  // partial sum of this segment is complete
-            seg++;
-            in_seg = 0;
-          } else {
-            in_seg++;
-          }
+          f_bar = f_bar_n;
+          phase = phase_n;
+          a_hi += 64u;
+          wh += dslot;
+          e_bar += 8u;
+          stage++;
+          if (wrap) { stage = 0; a_hi = a_col0; wh = w0; e_bar = empty0; }
         }
+        commit_by(leader, segf0 + buf * 8u);  // partial sum of this segment is complete
+        seg++;
       }
-      PROF_OUT(6, 5);
     }
+    if (leader) PROF_OUT(6, 5);
   } else if (warp >= EPI_WARP0) {
     // ===================================================================== accumulate + epilogue warps
     const int ew = warp - EPI_WARP0;

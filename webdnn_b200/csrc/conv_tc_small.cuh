@@ -53,35 +53,6 @@ struct SmallShared {
 };
 static_assert(sizeof(SmallShared) <= 256, "SmallLayout::SMEM");
 
-// Barrier operations on shared-memory addresses: the loops below step through them with additions.
-__device__ __forceinline__ bool try_wait_at(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.b32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ bool test_at(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.b32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ void arrive_at(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void expect_at(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
 __device__ __noinline__ bool small_wait_slow(uint32_t bar, uint32_t parity, SmallShared* ss, int* status, int code) {
   const unsigned long long t0 = global_ns();
   for (;;) {
@@ -99,29 +70,6 @@ __device__ __forceinline__ bool small_wait(uint32_t bar, uint32_t parity, SmallS
   for (int i = 0; i < 4096; i++)
     if (try_wait_at(bar, parity)) return true;
   return small_wait_slow(bar, parity, ss, status, code);
-}
-// tcgen05.mma with A in tensor memory by the lane whose `leader` is 1.  The whole warp runs the issuing loop, so that
-// its addresses are the same in every lane and stay in uniform registers: in a branch of the elected lane alone the
-// arithmetic between two K blocks took longer than their MMAs.
-__device__ __forceinline__ void umma_by(uint32_t leader, uint32_t tmem_c, uint32_t tmem_a, uint32_t desc_lo, uint32_t desc_hi,
-                                        uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p, e;\n\t.reg .b64 d;\n\t"
-      "mov.b64 d, {%3, %4};\n\t"
-      "setp.ne.b32 e, %0, 0;\n\t"
-      "setp.ne.b32 p, %6, 0;\n\t"
-      "@e tcgen05.mma.cta_group::1.kind::tf32 [%1], [%2], d, %5, p;\n\t}"
-      :
-      : "r"(leader), "r"(tmem_c), "r"(tmem_a), "r"(desc_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-__device__ __forceinline__ void commit_by(uint32_t leader, uint32_t bar) {
-  asm volatile(
-      "{\n\t.reg .pred e;\n\t"
-      "setp.ne.b32 e, %0, 0;\n\t"
-      "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%1];\n\t}" ::"r"(leader),
-      "r"(bar)
-      : "memory");
 }
 __device__ __forceinline__ uint32_t map_to_rank(uint32_t addr, uint32_t rank) {
   uint32_t r;
