@@ -155,3 +155,28 @@ def test_small_outputs(cuda_context, n, cin, cout, size, k, stride, pad, res, pr
         ctx.set_precision("tf32x3")
     for t in (dx, dr, dw, dsc, dsh, y):
         t.dispose()
+
+
+# maps (32 to a CTA) and pixels (8 warps) around their multiples, and more maps than one round of CTAs
+@pytest.mark.parametrize("batch,ch,area", [(1, 1, 1), (1, 31, 7), (3, 33, 8), (2, 64, 49), (5, 7, 130), (40, 1030, 9)])
+def test_channels_last_average(cuda_context, batch, ch, area):
+    from webdnn_b200.backend import CPUTensor
+    x = np.random.default_rng(ch).standard_normal((batch, area, ch)).astype(np.float32)
+    dx, y = cuda_context.move_tensor(CPUTensor.from_array(x)), cuda_context.empty_tensor([batch, ch])
+    cuda_context._call("wdc_global_avgpool", dx.ptr, y.ptr, batch, ch, area, area * ch, 1, ch)
+    assert max_err_rel_linf(y.get_data().reshape(batch, ch), x.astype(np.float64).mean(axis=1)) <= 1e-6
+    dx.dispose()
+    y.dispose()
+
+
+# the last row of a pair missing, both sizes of CTA, more rows than one round of CTAs, rows held and re-read
+@pytest.mark.parametrize("rows", [1, 2, 625, 4737, 40001])
+@pytest.mark.parametrize("length", [36, 256, 300])
+def test_layernorm_row_counts(cuda_context, rows, length):
+    from oracle import ops
+    rng = np.random.default_rng(rows)
+    x = (rng.standard_normal((rows, length)) * 3 + 1).astype(np.float32)
+    gamma, beta = rng.uniform(0.5, 1.5, length).astype(np.float32), rng.standard_normal(length).astype(np.float32)
+    model = single_op_model("LayerNormalization", {"axis": -1, "epsilon": 1e-5}, [x, gamma, beta], opset=17)
+    (got,) = run_cuda(model, [x, gamma, beta], cuda_context)
+    assert max_err_rel_linf(got, ops.layernorm_chain(x, gamma, beta, 1e-5)) <= 5e-6

@@ -181,6 +181,9 @@ __global__ void __launch_bounds__(256) attn_split_kv_kernel(const float* __restr
                                                             float* __restrict__ vt_hi, float* __restrict__ vt_lo,
                                                             int heads, int tk, int tkp, int64_t k_sb, int64_t k_sh,
                                                             int64_t k_st, int64_t v_sb, int64_t v_sh, int64_t v_st) {
+  pdl_wait();
+  k = pdl_after(k);
+  v = pdl_after(v);
   __shared__ float tile[32][DH + 1];
   const int bh = blockIdx.y, b = bh / heads, h = bh - b * heads;
   const int t0 = blockIdx.x * 32;
@@ -267,8 +270,7 @@ attention_tc_kernel(const AttTcProblem p, const __grid_constant__ CUtensorMap ma
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = sh->tmem_base;
   // the pre-pass (the grid before this one) wrote the split operands this kernel is about to load
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  pdl_wait();
 
   if (warp < 4) {
     // ============================================================================ row threads
@@ -507,8 +509,8 @@ int launch(wdc_context* ctx, const wdc_attention_desc* d, const float* q, const 
     wdc_free(ctx, scratch);
     return WDC_ERR_UNSUPPORTED;
   }
-  attn_split_kv_kernel<DH><<<dim3((unsigned)((tk + 31) / 32), (unsigned)bh), 256, 0, ctx->stream>>>(
-      k, v, k_hi, k_lo, vt_hi, vt_lo, (int)d->heads, tk, tkp, d->k_sb, d->k_sh, d->k_st, d->v_sb, d->v_sh, d->v_st);
+  wdc_launch_pdl(ctx, attn_split_kv_kernel<DH>, dim3((unsigned)((tk + 31) / 32), (unsigned)bh), dim3(256), 0,
+                 k, v, k_hi, k_lo, vt_hi, vt_lo, (int)d->heads, tk, tkp, d->k_sb, d->k_sh, d->k_st, d->v_sb, d->v_sh, d->v_st);
   s = wdc_check_launch(ctx, "attn_split_kv_kernel");
   if (s == WDC_OK) {
     AttTcProblem p;

@@ -126,6 +126,58 @@ struct DeviceGuard {
   }
 };
 
+// Programmatic dependent launch.  A kernel launched with wdc_launch_pdl may start while the grids before it finish: its
+// first statement is pdl_wait(), behind which everything they wrote is visible, and which also lets the next grid start.
+// Pointers that a kernel declares read-only go through pdl_after(), or the compiler might load ahead of the wait.
+#ifdef __CUDACC__
+__device__ __forceinline__ void pdl_grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() {
+  pdl_grid_wait();
+  pdl_let_next_start();
+}
+template <class T>
+__device__ __forceinline__ T* pdl_after(T* p) {
+  size_t g = __cvta_generic_to_global(p);
+  asm volatile("" : "+l"(g)::"memory");
+  return (T*)__cvta_global_to_generic(g);
+}
+template <class... P, class... A>
+void wdc_launch_pdl(wdc_context* ctx, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = ctx->stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = ctx->opt_pdl ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);   // (an error stays for wdc_check_launch)
+}
+#endif
+
+// Buffers that io_copy_kernel (transfer.cu) moves between page-locked host memory and the device.
+struct wdc_io_list {
+  static const int MOST = 8;
+  struct Part {
+    uint32_t* dst;
+    const uint32_t* src;
+    int64_t words;
+  };
+  int n;
+  Part part[MOST];
+  bool operator==(const wdc_io_list& o) const {
+    bool same = n == o.n;
+    for (int i = 0; i < n && same; i++)
+      same = part[i].dst == o.part[i].dst && part[i].src == o.part[i].src && part[i].words == o.part[i].words;
+    return same;
+  }
+};
+dim3 wdc_io_grid(const wdc_io_list& list);
+void* wdc_io_kernel();
+
 static inline int64_t ceil_div64(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 // Grid size for a grid-stride kernel: enough CTAs to fill the SMs a few times over.

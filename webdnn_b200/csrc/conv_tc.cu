@@ -299,8 +299,6 @@ __device__ __forceinline__ void unit_of(const TcProblem& p, int u, int& tile, in
 
 // Programmatic dependent launch.  wait: everything the grids before this one wrote is visible afterwards (a no-op
 // for a launch without the attribute).  launch_dependents: the next grid of the stream may start its own set-up.
-__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred;
@@ -558,8 +556,8 @@ tc_igemm_kernel(const __grid_constant__ TcProblem p, const float* __restrict__ x
   // earlier grids wrote (activations, the residual) and writes memory they may still be reading (the arena reuses
   // freed blocks in stream order): wait for them.  The next grid may begin its own set-up right away; its CTAs
   // become resident as this grid's CTAs exit, and it waits for this grid's completion at the same point.
-  grid_dependency_wait();
-  grid_launch_dependents();
+  pdl_grid_wait();
+  pdl_let_next_start();
   // (the table of per-column addends is filled by the epilogue warps themselves, after this wait: the addends may
   // have been produced by an earlier grid, and the producer warps need not wait for the table)
   // Each CTA walks the K blocks of a full tile from a different starting point so that the CTAs, which all need
@@ -1341,7 +1339,7 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restr
                                                             const float* __restrict__ residual, int64_t res_stride,
                                                             float res_mul, int relu, int64_t M, int N, int tile_n,
                                                             int tiles_n, int full_tiles, int rest_tiles, int splits) {
-  grid_dependency_wait();   // launched as a programmatic dependent of the contraction kernel
+  pdl_grid_wait();   // launched as a programmatic dependent of the contraction kernel
   const int tv = tile_n / 4;                       // float4 cells per tile row
   const int64_t total = (int64_t)rest_tiles * TILE_M * tv;
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1386,16 +1384,18 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restr
 // `plane` = 0: x is NHWC (a pixel's channels are adjacent); > 0: x is NCHW with `plane` pixels per channel plane.
 __global__ void pad_channels4_kernel(const float* __restrict__ x, float* __restrict__ x4, int64_t pixels, int cin,
                                      int64_t plane) {
+  pdl_wait();
+  x = pdl_after(x);
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t step = (int64_t)gridDim.x * blockDim.x;
   for (; i < pixels; i += step) {
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     const float* s = plane ? x + (i / plane) * plane * cin + i % plane : x + i * cin;
     const int64_t cs = plane ? plane : 1;
-    v.x = s[0];
-    if (cin > 1) v.y = s[cs];
-    if (cin > 2) v.z = s[2 * cs];
-    if (cin > 3) v.w = s[3 * cs];
+    v.x = __ldg(s);
+    if (cin > 1) v.y = __ldg(s + cs);
+    if (cin > 2) v.z = __ldg(s + 2 * cs);
+    if (cin > 3) v.w = __ldg(s + 3 * cs);
     reinterpret_cast<float4*>(x4)[i] = v;
   }
 }
@@ -1404,6 +1404,8 @@ __global__ void pad_channels4_kernel(const float* __restrict__ x, float* __restr
 // With hp > h the images are padded vertically too: pad_t zero rows above, hp - pad_t - h below.
 __global__ void pad_channels4_rows_kernel(const float* __restrict__ x, float* __restrict__ x4, int64_t images, int h,
                                           int hp, int pad_t, int w, int wp, int pad_l, int cin, int nchw) {
+  pdl_wait();
+  x = pdl_after(x);
   int64_t total = images * hp * wp;
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t step = (int64_t)gridDim.x * blockDim.x;
@@ -1418,10 +1420,10 @@ __global__ void pad_channels4_rows_kernel(const float* __restrict__ x, float* __
       const int64_t plane = (int64_t)h * w;
       const float* s = nchw ? x + img * plane * cin + (int64_t)yy * w + px : x + ((img * h + yy) * w + px) * cin;
       const int64_t cs = nchw ? plane : 1;
-      v.x = s[0];
-      if (cin > 1) v.y = s[cs];
-      if (cin > 2) v.z = s[2 * cs];
-      if (cin > 3) v.w = s[3 * cs];
+      v.x = __ldg(s);
+      if (cin > 1) v.y = __ldg(s + cs);
+      if (cin > 2) v.z = __ldg(s + 2 * cs);
+      if (cin > 3) v.w = __ldg(s + 3 * cs);
     }
     reinterpret_cast<float4*>(x4)[i] = v;
   }
@@ -2079,11 +2081,11 @@ int wdc_tc_conv2d(wdc_context* ctx, const wdc_conv_desc* d, const float* x, cons
   int s = wdc_alloc(ctx, pixels * 16, (void**)&x4);
   if (s != WDC_OK) return s;
   if (pairs)
-    pad_channels4_rows_kernel<<<grid_for(ctx, pixels, 256, 8), 256, 0, ctx->stream>>>(
+    wdc_launch_pdl(ctx, pad_channels4_rows_kernel, dim3(grid_for(ctx, pixels, 256, 8)), dim3(256), 0, 
         x, x4, d->batch, (int)d->in_h, hp, 0, (int)d->in_w, wp, (int)d->pad_l, (int)d->ch_in,
         d->x_nchw ? 1 : 0);
   else
-    pad_channels4_kernel<<<grid_for(ctx, pixels, 256, 8), 256, 0, ctx->stream>>>(x, x4, pixels, (int)d->ch_in,
+    wdc_launch_pdl(ctx, pad_channels4_kernel, dim3(grid_for(ctx, pixels, 256, 8)), dim3(256), 0, x, x4, pixels, (int)d->ch_in,
                                                                                  d->x_nchw ? d->in_h * d->in_w : 0);
   s = wdc_check_launch(ctx, "pad_channels4_kernel");
   if (s == WDC_OK) {

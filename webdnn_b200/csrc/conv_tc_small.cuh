@@ -190,7 +190,7 @@ tc_small_kernel(const __grid_constant__ TcProblem p, const __grid_constant__ CUt
       if (lane == 0) arrive_at(smem_u32(&ss->seg_empty[buf]));
       drained++;
     };
-    grid_dependency_wait();   // (before the residual and the output are touched; the tiles come after it anyway)
+    pdl_grid_wait();   // (before the residual and the output are touched; the tiles come after it anyway)
     const uint32_t full0 = smem_u32(&ss->full[0]), empty0 = smem_u32(&ss->empty[0]), tfull0 = smem_u32(&ss->t_full[0]);
     // stage and tensor-memory stage of K block kb; `old` = those of kb - T_ST, whose commit frees the latter
     int st = half, ts = half;
@@ -246,7 +246,7 @@ tc_small_kernel(const __grid_constant__ TcProblem p, const __grid_constant__ CUt
       const uint32_t w_bytes = (p.single_pass ? 1u : 2u) * (uint32_t)L::W_BYTES;
       // A constant weight whose split is known to be finished is no output of a grid still running: its first tiles
       // come in while the grids before this one finish.
-      if (!w_early) grid_dependency_wait();
+      if (!w_early) pdl_grid_wait();
       const int tap0 = kb0 / p.cblocks;
       int cb = kb0 - tap0 * p.cblocks, kx0 = tap0 * p.ch_in + cb * BLOCK_K;   // a tap's last block may be short
       uint32_t bar = smem_u32(&ss->full[0]), dst = smem_u32(smem) + (uint32_t)A_TILE_BYTES, par = 1;
@@ -283,8 +283,8 @@ tc_small_kernel(const __grid_constant__ TcProblem p, const __grid_constant__ CUt
       const int cw = ox * p.stride_w - p.pad_l, ch = oy * p.stride_h - p.pad_t;
       const int tap0 = kb0 / p.cblocks;
       int c0 = (kb0 - tap0 * p.cblocks) * BLOCK_K, ky = tap0 / p.k_w, kx = tap0 - ky * p.k_w;
-      grid_dependency_wait();
-      grid_launch_dependents();
+      pdl_grid_wait();
+      pdl_let_next_start();
       uint32_t bar = smem_u32(&ss->full[0]), dst = smem_u32(smem), par = 1;
       constexpr uint32_t to_empty = (uint32_t)(offsetof(SmallShared, empty) - offsetof(SmallShared, full));
       int st = 0, dx = kx * p.dil_w, dy = ky * p.dil_h;

@@ -32,7 +32,7 @@ struct SkinnyArgs {
 
 __device__ __forceinline__ void store_out(const SkinnyArgs& a, int64_t bz, int64_t m, int64_t n, float v) {
   v *= a.alpha;
-  if (a.C) v += __ldg(a.C + m * a.sc0 + n * a.sc1) * a.beta;
+  if (a.C) v += __ldg(pdl_after(a.C) + m * a.sc0 + n * a.sc1) * a.beta;
   if (a.relu) v = v > 0.f ? v : (v == v ? 0.f : v);
   a.Y[(bz * a.m + m) * a.n + n] = v;
 }
@@ -64,13 +64,14 @@ __device__ __forceinline__ int spread_index(int lane) { return lane / (32 / COUN
 // B stored [n][k].  grid: (ceil(n / (NC * ROW_WARPS / wk)), ceil(m / MT), batch); wk warps split K.
 template <int MT, int VEC>
 __global__ void __launch_bounds__(ROW_WARPS * 32) skinny_rows_kernel(const SkinnyArgs a, int wk) {
+  pdl_wait();
   __shared__ float red[ROW_WARPS][MT * NC];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int kw = warp % wk, group = warp / wk, groups = ROW_WARPS / wk;
   const int64_t n0 = ((int64_t)blockIdx.x * groups + group) * NC;
   const int64_t m0 = (int64_t)blockIdx.y * MT, bz = blockIdx.z;
-  const float* A = a.A + bz * a.sab + m0 * a.sa0;
-  const float* B = a.B + bz * a.sbb;
+  const float* A = pdl_after(a.A) + bz * a.sab + m0 * a.sa0;
+  const float* B = pdl_after(a.B) + bz * a.sbb;
   // columns and rows past the edge repeat the last valid one and are not stored
   const float* bp[NC];
 #pragma unroll
@@ -126,12 +127,13 @@ __global__ void __launch_bounds__(ROW_WARPS * 32) skinny_rows_kernel(const Skinn
 // B stored [k][n].  grid: (ceil(n / 32), ceil(m / MT), batch); the warps take rows w, w + 16, ... of B.
 template <int MT>
 __global__ void __launch_bounds__(COL_WARPS * 32) skinny_cols_kernel(const SkinnyArgs a) {
+  pdl_wait();
   __shared__ float red[COL_WARPS][MT][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t n = (int64_t)blockIdx.x * 32 + lane;
   const int64_t m0 = (int64_t)blockIdx.y * MT, bz = blockIdx.z;
-  const float* A = a.A + bz * a.sab + m0 * a.sa0;
-  const float* bp = a.B + bz * a.sbb + (n < a.n ? n : a.n - 1);
+  const float* A = pdl_after(a.A) + bz * a.sab + m0 * a.sa0;
+  const float* bp = pdl_after(a.B) + bz * a.sbb + (n < a.n ? n : a.n - 1);
   const int rows = a.m - m0 < MT ? (int)(a.m - m0) : MT;
   float acc[MT];
 #pragma unroll
@@ -167,9 +169,9 @@ __global__ void __launch_bounds__(COL_WARPS * 32) skinny_cols_kernel(const Skinn
 }
 
 template <int MT>
-void launch_rows(const SkinnyArgs& a, dim3 grid, int wk, bool vec, cudaStream_t stream) {
-  if (vec) skinny_rows_kernel<MT, 4><<<grid, ROW_WARPS * 32, 0, stream>>>(a, wk);
-  else skinny_rows_kernel<MT, 1><<<grid, ROW_WARPS * 32, 0, stream>>>(a, wk);
+void launch_rows(wdc_context* ctx, const SkinnyArgs& a, dim3 grid, int wk, bool vec) {
+  if (vec) wdc_launch_pdl(ctx, skinny_rows_kernel<MT, 4>, grid, dim3(ROW_WARPS * 32), 0, a, wk);
+  else wdc_launch_pdl(ctx, skinny_rows_kernel<MT, 1>, grid, dim3(ROW_WARPS * 32), 0, a, wk);
 }
 
 }  // namespace
@@ -191,16 +193,16 @@ int wdc_skinny_gemm(wdc_context* ctx, const wdc_gemm_desc* d, const float* A, co
     int wk = 1;
     while (wk < ROW_WARPS && (int64_t)wk * 32 * (vec ? 4 : 1) < d->k) wk *= 2;
     const dim3 grid((unsigned)ceil_div64(d->n, NC * (ROW_WARPS / wk)), gy, gz);
-    if (mt == 8) launch_rows<8>(a, grid, wk, vec, ctx->stream);
-    else if (mt == 4) launch_rows<4>(a, grid, wk, vec, ctx->stream);
-    else if (mt == 2) launch_rows<2>(a, grid, wk, vec, ctx->stream);
-    else launch_rows<1>(a, grid, wk, vec, ctx->stream);
+    if (mt == 8) launch_rows<8>(ctx, a, grid, wk, vec);
+    else if (mt == 4) launch_rows<4>(ctx, a, grid, wk, vec);
+    else if (mt == 2) launch_rows<2>(ctx, a, grid, wk, vec);
+    else launch_rows<1>(ctx, a, grid, wk, vec);
     return wdc_check_launch(ctx, "skinny_rows_kernel");
   }
   const dim3 grid((unsigned)ceil_div64(d->n, 32), gy, gz);
-  if (mt == 8) skinny_cols_kernel<8><<<grid, COL_WARPS * 32, 0, ctx->stream>>>(a);
-  else if (mt == 4) skinny_cols_kernel<4><<<grid, COL_WARPS * 32, 0, ctx->stream>>>(a);
-  else if (mt == 2) skinny_cols_kernel<2><<<grid, COL_WARPS * 32, 0, ctx->stream>>>(a);
-  else skinny_cols_kernel<1><<<grid, COL_WARPS * 32, 0, ctx->stream>>>(a);
+  if (mt == 8) wdc_launch_pdl(ctx, skinny_cols_kernel<8>, grid, dim3(COL_WARPS * 32), 0, a);
+  else if (mt == 4) wdc_launch_pdl(ctx, skinny_cols_kernel<4>, grid, dim3(COL_WARPS * 32), 0, a);
+  else if (mt == 2) wdc_launch_pdl(ctx, skinny_cols_kernel<2>, grid, dim3(COL_WARPS * 32), 0, a);
+  else wdc_launch_pdl(ctx, skinny_cols_kernel<1>, grid, dim3(COL_WARPS * 32), 0, a);
   return wdc_check_launch(ctx, "skinny_cols_kernel");
 }

@@ -208,8 +208,6 @@ __global__ void __launch_bounds__(THREADS, kLong && TN == 128 ? 1 : 2) gemm_tc_d
   __shared__ DirectShared sh;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n0 = blockIdx.x * TN, m0 = blockIdx.y * TM;
-  const float* A = a.A + blockIdx.z * a.sab + (int64_t)m0 * a.sa_row;
-  const float* B = a.B + blockIdx.z * a.sbb + (int64_t)n0 * a.sb_row;
   const int rows_a = a.m - m0 < TM ? a.m - m0 : TM, rows_b = a.n - n0 < TN ? a.n - n0 : TN;
   const int kblocks = (a.k + KB - 1) / KB;
 
@@ -224,12 +222,17 @@ __global__ void __launch_bounds__(THREADS, kLong && TN == 128 ? 1 : 2) gemm_tc_d
                  "r"(TMEM_COLS));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
+  pdl_grid_wait();
+  const float* C = pdl_after(a.C);
+  const float* A = pdl_after(a.A) + blockIdx.z * a.sab + (int64_t)m0 * a.sa_row;
+  const float* B = pdl_after(a.B) + blockIdx.z * a.sbb + (int64_t)n0 * a.sb_row;
   float va[TM / 8], vb[TN / 8];
   load_block<TM>(va, A, a.sa_row, a.sa_k, rows_a, 0, a.k, a.mode_a);
   load_block<TN>(vb, B, a.sb_row, a.sb_k, rows_b, 0, a.k, a.mode_b);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  pdl_let_next_start();   // not before this CTA has its tensor memory: a CTA of the next grid might take it and wait for this one
   const uint32_t tmem_base = sh.tmem_base;
   // D = f32, A = B = tf32, both K-major, M = 128, N = TN
   const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
@@ -330,7 +333,7 @@ __global__ void __launch_bounds__(THREADS, kLong && TN == 128 ? 1 : 2) gemm_tc_d
       for (int c = lane; c < COLS; c += 32) {
         if (col0 + c < a.n) {
           float v = stg[r * (COLS + 1) + c] * a.alpha;
-          if (a.C) v += __ldg(a.C + (int64_t)(row0 + r) * a.sc0 + (int64_t)(col0 + c) * a.sc1) * a.beta;
+          if (C) v += __ldg(C + (int64_t)(row0 + r) * a.sc0 + (int64_t)(col0 + c) * a.sc1) * a.beta;
           if (a.relu) v = v > 0.f ? v : (v == v ? 0.f : v);
           Y[(int64_t)(row0 + r) * a.n + col0 + c] = v;
         }
@@ -363,7 +366,7 @@ int launch(wdc_context* ctx, const DirectArgs& a, int batch) {
     attr_set[ctx->device] = true;
   }
   const dim3 grid((unsigned)((a.n + TN - 1) / TN), (unsigned)((a.m + TM - 1) / TM), (unsigned)batch);
-  gemm_tc_direct_kernel<TN, kLong><<<grid, THREADS, smem, ctx->stream>>>(a);
+  wdc_launch_pdl(ctx, gemm_tc_direct_kernel<TN, kLong>, dim3(grid), dim3(THREADS), smem, a);
   ctx->n_tc_launch++;
   return wdc_check_launch(ctx, "gemm_tc_direct_kernel");
 }

@@ -14,6 +14,8 @@ struct CopyShape {
 template <typename T, int M, typename I>
 __global__ void __launch_bounds__(256) strided_copy_kernel(const T* __restrict__ src, T* __restrict__ dst, int64_t n,
                                                            CopyShape sh) {
+  pdl_wait();
+  src = pdl_after(src);
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t step = (int64_t)gridDim.x * blockDim.x;
   I dims[M];
@@ -32,7 +34,7 @@ __global__ void __launch_bounds__(256) strided_copy_kernel(const T* __restrict__
     }
     is += (int64_t)rem * sh.sstr[6 - M];
     id += (int64_t)rem * sh.dstr[6 - M];
-    dst[id] = src[is];
+    dst[id] = __ldg(src + is);
   }
 }
 
@@ -42,8 +44,8 @@ static void launch_strided_copy(wdc_context* ctx, const T* s, T* d, int64_t n, c
   const bool small = n < (1ll << 31);
 #define WDC_COPY_CASE(MM)                                                                                   \
   case MM:                                                                                                  \
-    if (small) strided_copy_kernel<T, MM, uint32_t><<<grid, 256, 0, ctx->stream>>>(s, d, n, sh);            \
-    else strided_copy_kernel<T, MM, int64_t><<<grid, 256, 0, ctx->stream>>>(s, d, n, sh);                   \
+    if (small) wdc_launch_pdl(ctx, strided_copy_kernel<T, MM, uint32_t>, dim3(grid), dim3(256), 0, s, d, n, sh);            \
+    else wdc_launch_pdl(ctx, strided_copy_kernel<T, MM, int64_t>, dim3(grid), dim3(256), 0, s, d, n, sh);                   \
     break;
   switch (m < 1 ? 1 : m) {
     WDC_COPY_CASE(1)
@@ -62,6 +64,8 @@ static void launch_strided_copy(wdc_context* ctx, const T* s, T* d, int64_t n, c
 __global__ void __launch_bounds__(256) transpose_tile_kernel(const uint32_t* __restrict__ src,
                                                              uint32_t* __restrict__ dst, int64_t batch,
                                                              int64_t rows, int64_t cols) {
+  pdl_wait();
+  src = pdl_after(src);
   __shared__ uint32_t tile[32][33];
   int64_t tiles_r = (rows + 31) / 32, tiles_c = (cols + 31) / 32;
   int64_t ntiles = batch * tiles_r * tiles_c;
@@ -93,6 +97,8 @@ __global__ void __launch_bounds__(256) transpose_tile_kernel(const uint32_t* __r
 // scalar with a pitch of 65 words: at most two-way bank conflicts on either side.
 __global__ void __launch_bounds__(256) transpose_tile64_kernel(const float* __restrict__ src, float* __restrict__ dst,
                                                                int64_t batch, int64_t rows, int64_t cols) {
+  pdl_wait();
+  src = pdl_after(src);
   __shared__ float tile[64][65];   // [c][r]
   const int64_t tiles_r = (rows + 63) / 64, tiles_c = (cols + 63) / 64;
   const int64_t ntiles = batch * tiles_r * tiles_c;
@@ -135,6 +141,8 @@ __global__ void __launch_bounds__(256) transpose_tile64_kernel(const float* __re
 __global__ void __launch_bounds__(256) transpose_narrow_cols_kernel(const uint32_t* __restrict__ src,
                                                                     uint32_t* __restrict__ dst, int64_t batch,
                                                                     int64_t rows, int cols) {
+  pdl_wait();
+  src = pdl_after(src);
   int64_t n = batch * rows;
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t step = (int64_t)gridDim.x * blockDim.x;
@@ -148,6 +156,8 @@ __global__ void __launch_bounds__(256) transpose_narrow_cols_kernel(const uint32
 __global__ void __launch_bounds__(256) transpose_narrow_rows_kernel(const uint32_t* __restrict__ src,
                                                                     uint32_t* __restrict__ dst, int64_t batch,
                                                                     int rows, int64_t cols) {
+  pdl_wait();
+  src = pdl_after(src);
   int64_t n = batch * cols;
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t step = (int64_t)gridDim.x * blockDim.x;
@@ -199,26 +209,26 @@ extern "C" int wdc_strided_copy(wdc_context* ctx, const void* src, void* dst, in
       ms[m - 1] == md[m - 2] && (m == 2 || (mt[0] == md[1] * md[2] && ms[0] == md[1] * md[2]))) {
     int64_t batch = m == 3 ? md[0] : 1, rows = md[m - 2], cols = md[m - 1];
     if (cols < 8) {
-      transpose_narrow_cols_kernel<<<grid_for(ctx, batch * rows, 256, 8), 256, 0, ctx->stream>>>(s, d, batch, rows,
+      wdc_launch_pdl(ctx, transpose_narrow_cols_kernel, dim3(grid_for(ctx, batch * rows, 256, 8)), dim3(256), 0, s, d, batch, rows,
                                                                                                  (int)cols);
       return wdc_check_launch(ctx, "transpose_narrow_cols_kernel");
     }
     if (rows < 8) {
-      transpose_narrow_rows_kernel<<<grid_for(ctx, batch * cols, 256, 8), 256, 0, ctx->stream>>>(s, d, batch,
+      wdc_launch_pdl(ctx, transpose_narrow_rows_kernel, dim3(grid_for(ctx, batch * cols, 256, 8)), dim3(256), 0, s, d, batch,
                                                                                                  (int)rows, cols);
       return wdc_check_launch(ctx, "transpose_narrow_rows_kernel");
     }
     if (rows % 4 == 0 && cols % 4 == 0 && rows >= 32 && cols >= 32 && (((uintptr_t)s | (uintptr_t)d) & 15) == 0) {
       const int64_t nt = batch * ((rows + 63) / 64) * ((cols + 63) / 64);
       const int64_t cap64 = (int64_t)ctx->sm_count * 8;
-      transpose_tile64_kernel<<<(int)(nt < cap64 ? nt : cap64), 256, 0, ctx->stream>>>(
+      wdc_launch_pdl(ctx, transpose_tile64_kernel, dim3((int)(nt < cap64 ? nt : cap64)), dim3(256), 0, 
           reinterpret_cast<const float*>(s), reinterpret_cast<float*>(d), batch, rows, cols);
       return wdc_check_launch(ctx, "transpose_tile64_kernel");
     }
     int64_t ntiles = batch * ((rows + 31) / 32) * ((cols + 31) / 32);
     int64_t cap = (int64_t)ctx->sm_count * 16;
     int grid = (int)(ntiles < cap ? ntiles : cap);
-    transpose_tile_kernel<<<grid, 256, 0, ctx->stream>>>(s, d, batch, rows, cols);
+    wdc_launch_pdl(ctx, transpose_tile_kernel, dim3(grid), dim3(256), 0, s, d, batch, rows, cols);
     return wdc_check_launch(ctx, "transpose_tile_kernel");
   }
   CopyShape sh;
@@ -253,16 +263,19 @@ __global__ void __launch_bounds__(256) gather_kernel(const uint32_t* __restrict_
                                                      const int32_t* __restrict__ idx,
                                                      uint32_t* __restrict__ out, int64_t outer,
                                                      int64_t axis_len, int64_t inner, int64_t n_idx) {
+  pdl_wait();
+  data = pdl_after(data);
+  idx = pdl_after(idx);
   int64_t n = outer * n_idx * inner;
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t step = (int64_t)gridDim.x * blockDim.x;
   for (; i < n; i += step) {
     int64_t in = i % inner, k = (i / inner) % n_idx, o = i / (inner * n_idx);
-    int64_t j = idx[k];
+    int64_t j = __ldg(idx + k);
     if (j < 0) j += axis_len;
     // out-of-range indices are clamped instead of read out of bounds
     j = j < 0 ? 0 : (j >= axis_len ? axis_len - 1 : j);
-    out[i] = data[(o * axis_len + j) * inner + in];
+    out[i] = __ldg(data + (o * axis_len + j) * inner + in);
   }
 }
 
@@ -276,7 +289,7 @@ extern "C" int wdc_gather(wdc_context* ctx, const void* data, const int32_t* idx
   if (n == 0) return WDC_OK;
   WDC_REQUIRE(ctx, data && idx && out, "wdc_gather: null buffer");
   DeviceGuard g(ctx->device);
-  gather_kernel<<<grid_for(ctx, n, 256, 8), 256, 0, ctx->stream>>>((const uint32_t*)data, idx,
+  wdc_launch_pdl(ctx, gather_kernel, dim3(grid_for(ctx, n, 256, 8)), dim3(256), 0, (const uint32_t*)data, idx,
                                                                   (uint32_t*)out, outer, axis_len, inner, n_idx);
   return wdc_check_launch(ctx, "gather_kernel");
 }

@@ -79,6 +79,8 @@ template <int OP>
 __global__ void __launch_bounds__(256) unary_f32_kernel(const float* __restrict__ src,
                                                         float* __restrict__ dst, int64_t n,
                                                         float p0, float p1, int vec_ok) {
+  pdl_wait();
+  src = pdl_after(src);
   int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t step = (int64_t)gridDim.x * blockDim.x;
   if (vec_ok) {
@@ -93,18 +95,20 @@ __global__ void __launch_bounds__(256) unary_f32_kernel(const float* __restrict_
       v.w = unary_f32<OP>(v.w, p0, p1);
       d4[i] = v;
     }
-    for (int64_t i = (n4 << 2) + tid; i < n; i += step) dst[i] = unary_f32<OP>(src[i], p0, p1);
+    for (int64_t i = (n4 << 2) + tid; i < n; i += step) dst[i] = unary_f32<OP>(__ldg(src + i), p0, p1);
   } else {
-    for (int64_t i = tid; i < n; i += step) dst[i] = unary_f32<OP>(src[i], p0, p1);
+    for (int64_t i = tid; i < n; i += step) dst[i] = unary_f32<OP>(__ldg(src + i), p0, p1);
   }
 }
 
 __global__ void unary_i32_kernel(int op, const int32_t* __restrict__ src, int32_t* __restrict__ dst,
                                  int64_t n) {
+  pdl_wait();
+  src = pdl_after(src);
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t step = (int64_t)gridDim.x * blockDim.x;
   for (; i < n; i += step) {
-    int32_t v = src[i];
+    int32_t v = __ldg(src + i);
     int32_t r;
     switch (op) {
       case WDC_U_ABS: r = v < 0 ? (int32_t)(0u - (uint32_t)v) : v; break;  // |INT_MIN| wraps
@@ -121,7 +125,7 @@ template <int OP>
 static int launch_unary(wdc_context* ctx, const float* src, float* dst, int64_t n, float p0, float p1) {
   int vec_ok = ((((uintptr_t)src | (uintptr_t)dst) & 15) == 0) ? 1 : 0;
   int64_t items = vec_ok ? (n + 3) / 4 : n;
-  unary_f32_kernel<OP><<<grid_for(ctx, items, 256), 256, 0, ctx->stream>>>(src, dst, n, p0, p1, vec_ok);
+  wdc_launch_pdl(ctx, unary_f32_kernel<OP>, dim3(grid_for(ctx, items, 256)), dim3(256), 0, src, dst, n, p0, p1, vec_ok);
   return wdc_check_launch(ctx, "unary_f32_kernel");
 }
 
@@ -137,7 +141,7 @@ extern "C" int wdc_unary(wdc_context* ctx, int op, int dtype, const void* src, v
     WDC_REQUIRE(ctx, op == WDC_U_ABS || op == WDC_U_NEG || op == WDC_U_RELU || op == WDC_U_SIGN ||
                          op == WDC_U_IDENTITY,
                 "wdc_unary: op %d does not accept int32", op);
-    unary_i32_kernel<<<grid_for(ctx, n, 256), 256, 0, ctx->stream>>>(op, (const int32_t*)src,
+    wdc_launch_pdl(ctx, unary_i32_kernel, dim3(grid_for(ctx, n, 256)), dim3(256), 0, op, (const int32_t*)src,
                                                                     (int32_t*)dst, n);
     return wdc_check_launch(ctx, "unary_i32_kernel");
   }
@@ -220,6 +224,9 @@ __global__ void __launch_bounds__(256) binary_f32_fast_kernel(const float* __res
                                                               const float* __restrict__ b,
                                                               float* __restrict__ out, int64_t n,
                                                               int mode, int64_t period, int vec_ok) {
+  pdl_wait();
+  a = pdl_after(a);
+  b = pdl_after(b);
   int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t step = (int64_t)gridDim.x * blockDim.x;
   if (vec_ok) {
@@ -242,8 +249,8 @@ __global__ void __launch_bounds__(256) binary_f32_fast_kernel(const float* __res
     tid += n4 << 2;
   }
   for (int64_t i = tid; i < n; i += step) {
-    float x = mode == 2 ? a[0] : a[i];
-    float y = mode == 1 ? b[0] : (mode == 3 ? b[i % period] : b[i]);
+    float x = __ldg(a + (mode == 2 ? 0 : i));
+    float y = __ldg(b + (mode == 1 ? 0 : mode == 3 ? i % period : i));
     out[i] = binary_f32<OP>(x, y);
   }
 }
@@ -253,6 +260,9 @@ __global__ void __launch_bounds__(256) binary_f32_general_kernel(const float* __
                                                                  const float* __restrict__ b,
                                                                  float* __restrict__ out, int64_t n,
                                                                  BinaryShape sh) {
+  pdl_wait();
+  a = pdl_after(a);
+  b = pdl_after(b);
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t step = (int64_t)gridDim.x * blockDim.x;
   for (; i < n; i += step) {
@@ -264,12 +274,15 @@ __global__ void __launch_bounds__(256) binary_f32_general_kernel(const float* __
       ia += c * sh.sa[d];
       ib += c * sh.sb[d];
     }
-    out[i] = binary_f32<OP>(a[ia], b[ib]);
+    out[i] = binary_f32<OP>(__ldg(a + ia), __ldg(b + ib));
   }
 }
 
 __global__ void binary_i32_kernel(int op, const int32_t* __restrict__ a, const int32_t* __restrict__ b,
                                   int32_t* __restrict__ out, int64_t n, BinaryShape sh) {
+  pdl_wait();
+  a = pdl_after(a);
+  b = pdl_after(b);
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t step = (int64_t)gridDim.x * blockDim.x;
   for (; i < n; i += step) {
@@ -281,7 +294,7 @@ __global__ void binary_i32_kernel(int op, const int32_t* __restrict__ a, const i
       ia += c * sh.sa[d];
       ib += c * sh.sb[d];
     }
-    out[i] = binary_i32(op, a[ia], b[ib]);
+    out[i] = binary_i32(op, __ldg(a + ia), __ldg(b + ib));
   }
 }
 
@@ -292,11 +305,11 @@ static int launch_binary_f32(wdc_context* ctx, const float* a, const float* b, f
     int vec_ok = ((((uintptr_t)a | (uintptr_t)b | (uintptr_t)out) & 15) == 0) &&
                  (mode != 3 || (period % 4) == 0);
     int64_t items = vec_ok ? (n + 3) / 4 : n;
-    binary_f32_fast_kernel<OP><<<grid_for(ctx, items, 256), 256, 0, ctx->stream>>>(a, b, out, n, mode,
+    wdc_launch_pdl(ctx, binary_f32_fast_kernel<OP>, dim3(grid_for(ctx, items, 256)), dim3(256), 0, a, b, out, n, mode,
                                                                                   period, vec_ok);
     return wdc_check_launch(ctx, "binary_f32_fast_kernel");
   }
-  binary_f32_general_kernel<OP><<<grid_for(ctx, n, 256), 256, 0, ctx->stream>>>(a, b, out, n, sh);
+  wdc_launch_pdl(ctx, binary_f32_general_kernel<OP>, dim3(grid_for(ctx, n, 256)), dim3(256), 0, a, b, out, n, sh);
   return wdc_check_launch(ctx, "binary_f32_general_kernel");
 }
 
@@ -327,7 +340,7 @@ extern "C" int wdc_binary(wdc_context* ctx, int op, int dtype, const void* a, co
   WDC_REQUIRE(ctx, a && b && out, "wdc_binary: null buffer");
   DeviceGuard g(ctx->device);
   if (dtype == 1) {
-    binary_i32_kernel<<<grid_for(ctx, n, 256), 256, 0, ctx->stream>>>(op, (const int32_t*)a,
+    wdc_launch_pdl(ctx, binary_i32_kernel, dim3(grid_for(ctx, n, 256)), dim3(256), 0, op, (const int32_t*)a,
                                                                      (const int32_t*)b, (int32_t*)out, n, sh);
     return wdc_check_launch(ctx, "binary_i32_kernel");
   }
@@ -380,14 +393,18 @@ extern "C" int wdc_binary(wdc_context* ctx, int op, int dtype, const void* a, co
 
 // --------------------------------------------------------------------------------- cast
 __global__ void cast_f32_i32_kernel(const float* __restrict__ s, int32_t* __restrict__ d, int64_t n) {
+  pdl_wait();
+  s = pdl_after(s);
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t step = (int64_t)gridDim.x * blockDim.x;
-  for (; i < n; i += step) d[i] = to_int32((double)s[i]);
+  for (; i < n; i += step) d[i] = to_int32((double)__ldg(s + i));
 }
 __global__ void cast_i32_f32_kernel(const int32_t* __restrict__ s, float* __restrict__ d, int64_t n) {
+  pdl_wait();
+  s = pdl_after(s);
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t step = (int64_t)gridDim.x * blockDim.x;
-  for (; i < n; i += step) d[i] = (float)s[i];
+  for (; i < n; i += step) d[i] = (float)__ldg(s + i);
 }
 
 extern "C" int wdc_cast(wdc_context* ctx, int src_dtype, int dst_dtype, const void* src, void* dst,
@@ -400,11 +417,11 @@ extern "C" int wdc_cast(wdc_context* ctx, int src_dtype, int dst_dtype, const vo
   DeviceGuard g(ctx->device);
   if (src_dtype == dst_dtype && (src_dtype == 0 || src_dtype == 1)) return wdc_copy(ctx, dst, src, n * 4);
   if (src_dtype == 0 && dst_dtype == 1) {
-    cast_f32_i32_kernel<<<grid_for(ctx, n, 256), 256, 0, ctx->stream>>>((const float*)src, (int32_t*)dst, n);
+    wdc_launch_pdl(ctx, cast_f32_i32_kernel, dim3(grid_for(ctx, n, 256)), dim3(256), 0, (const float*)src, (int32_t*)dst, n);
     return wdc_check_launch(ctx, "cast_f32_i32_kernel");
   }
   if (src_dtype == 1 && dst_dtype == 0) {
-    cast_i32_f32_kernel<<<grid_for(ctx, n, 256), 256, 0, ctx->stream>>>((const int32_t*)src, (float*)dst, n);
+    wdc_launch_pdl(ctx, cast_i32_f32_kernel, dim3(grid_for(ctx, n, 256)), dim3(256), 0, (const int32_t*)src, (float*)dst, n);
     return wdc_check_launch(ctx, "cast_i32_f32_kernel");
   }
   return wdc_fail(ctx, WDC_ERR_UNSUPPORTED, "wdc_cast: %d -> %d not supported", src_dtype, dst_dtype);
@@ -417,6 +434,10 @@ __global__ void __launch_bounds__(256) channel_affine_kernel(const float* __rest
                                                              float* __restrict__ y, int64_t n,
                                                              int64_t channels, int64_t inner, int relu,
                                                              int vec_ok) {
+  pdl_wait();
+  x = pdl_after(x);
+  scale = pdl_after(scale);
+  shift = pdl_after(shift);
   int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t step = (int64_t)gridDim.x * blockDim.x;
   if (vec_ok) {  // inner == 1 (channels innermost, multiple of 4) or inner % 4 == 0
@@ -474,7 +495,7 @@ extern "C" int wdc_channel_affine(wdc_context* ctx, const float* x, const float*
   int vec_ok = aligned && (n % 4 == 0) &&
                ((inner == 1 && channels % 4 == 0) || (inner > 1 && inner % 4 == 0));
   int64_t items = vec_ok ? n / 4 : n;
-  channel_affine_kernel<<<grid_for(ctx, items, 256), 256, 0, ctx->stream>>>(x, scale, shift, y, n,
+  wdc_launch_pdl(ctx, channel_affine_kernel, dim3(grid_for(ctx, items, 256)), dim3(256), 0, x, scale, shift, y, n,
                                                                            channels, inner, relu, vec_ok);
   return wdc_check_launch(ctx, "channel_affine_kernel");
 }
@@ -509,6 +530,8 @@ __constant__ double kEightbitLevels[128] = {
 
 __global__ void __launch_bounds__(256) decode_eightbit_kernel(const uint8_t* __restrict__ codes,
                                                               float* __restrict__ out, int64_t n, float scale) {
+  pdl_wait();
+  codes = pdl_after(codes);
   __shared__ float table[256];
   {
     const int i = threadIdx.x;
@@ -530,7 +553,7 @@ __global__ void __launch_bounds__(256) decode_eightbit_kernel(const uint8_t* __r
   }
   // tail of fewer than 16 codes
   for (int64_t i = groups * 16 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += step)
-    out[i] = table[codes[i]];
+    out[i] = table[__ldg(codes + i)];
 }
 
 extern "C" int wdc_decode_eightbit(wdc_context* ctx, const void* codes, float* out, int64_t n, float scale) {
@@ -541,7 +564,7 @@ extern "C" int wdc_decode_eightbit(wdc_context* ctx, const void* codes, float* o
   WDC_REQUIRE(ctx, (((uintptr_t)codes | (uintptr_t)out) & 15) == 0, "wdc_decode_eightbit: buffers must be 16-byte aligned");
   if (n == 0) return WDC_OK;
   DeviceGuard g(ctx->device);
-  decode_eightbit_kernel<<<grid_for(ctx, (n + 15) / 16, 256, 8), 256, 0, ctx->stream>>>((const uint8_t*)codes, out, n,
+  wdc_launch_pdl(ctx, decode_eightbit_kernel, dim3(grid_for(ctx, (n + 15) / 16, 256, 8)), dim3(256), 0, (const uint8_t*)codes, out, n,
                                                                                       scale);
   return wdc_check_launch(ctx, "decode_eightbit_kernel");
 }

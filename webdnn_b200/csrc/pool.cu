@@ -9,6 +9,8 @@
 template <bool IS_MAX, int VEC>
 __global__ void __launch_bounds__(256) pool2d_kernel(wdc_pool_desc d, const float* __restrict__ x,
                                                      float* __restrict__ y, int c_fastest) {
+  pdl_wait();
+  x = pdl_after(x);
   int64_t chv = d.ch / VEC;
   int64_t n = d.batch * chv * d.out_h * d.out_w;
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -79,6 +81,8 @@ __global__ void __launch_bounds__(256) maxpool_cl_small_kernel(const float4* __r
                                                                int n_out, int chv, int in_h, int in_w, int out_h,
                                                                int out_w, int stride_h, int stride_w, int pad_t,
                                                                int pad_l) {
+  pdl_wait();
+  x = pdl_after(x);
   const int step = gridDim.x * blockDim.x;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_out; i += step) {
     int rem = i;
@@ -140,17 +144,17 @@ static int pool_common(wdc_context* ctx, const wdc_pool_desc* d, const float* x,
     float4* y4 = reinterpret_cast<float4*>(y);
 #define WDC_POOL_ARGS (int)items, (int)(d->ch / 4), (int)d->in_h, (int)d->in_w, (int)d->out_h, (int)d->out_w, \
                       (int)d->stride_h, (int)d->stride_w, (int)d->pad_t, (int)d->pad_l
-    if (d->k_h == 3) maxpool_cl_small_kernel<3, 3><<<grid, 256, 0, ctx->stream>>>(x4, y4, WDC_POOL_ARGS);
-    else maxpool_cl_small_kernel<2, 2><<<grid, 256, 0, ctx->stream>>>(x4, y4, WDC_POOL_ARGS);
+    if (d->k_h == 3) wdc_launch_pdl(ctx, maxpool_cl_small_kernel<3, 3>, dim3(grid), dim3(256), 0, x4, y4, WDC_POOL_ARGS);
+    else wdc_launch_pdl(ctx, maxpool_cl_small_kernel<2, 2>, dim3(grid), dim3(256), 0, x4, y4, WDC_POOL_ARGS);
 #undef WDC_POOL_ARGS
     return wdc_check_launch(ctx, "maxpool_cl_small_kernel");
   }
   if (is_max) {
-    if (vec) pool2d_kernel<true, 4><<<grid, 256, 0, ctx->stream>>>(*d, x, y, 1);
-    else pool2d_kernel<true, 1><<<grid, 256, 0, ctx->stream>>>(*d, x, y, cl ? 1 : 0);
+    if (vec) wdc_launch_pdl(ctx, pool2d_kernel<true, 4>, dim3(grid), dim3(256), 0, *d, x, y, 1);
+    else wdc_launch_pdl(ctx, pool2d_kernel<true, 1>, dim3(grid), dim3(256), 0, *d, x, y, cl ? 1 : 0);
   } else {
-    if (vec) pool2d_kernel<false, 4><<<grid, 256, 0, ctx->stream>>>(*d, x, y, 1);
-    else pool2d_kernel<false, 1><<<grid, 256, 0, ctx->stream>>>(*d, x, y, cl ? 1 : 0);
+    if (vec) wdc_launch_pdl(ctx, pool2d_kernel<false, 4>, dim3(grid), dim3(256), 0, *d, x, y, 1);
+    else wdc_launch_pdl(ctx, pool2d_kernel<false, 1>, dim3(grid), dim3(256), 0, *d, x, y, cl ? 1 : 0);
   }
   return wdc_check_launch(ctx, "pool2d_kernel");
 }
@@ -166,25 +170,42 @@ extern "C" int wdc_avgpool2d(wdc_context* ctx, const wdc_pool_desc* d, const flo
   return pool_common(ctx, d, x, y, false, "wdc_avgpool2d");
 }
 
-// Global average pool.  Channels-last: one thread per (b, c), walking pixels with stride xs_p,
-// coalesced across c.  NCHW: one warp per (b, c), lanes stride the pixels.
+// Global average pool.  Channels-last: a warp's lanes are 32 consecutive (b, c), so every pixel it reads is coalesced,
+// and the 8 warps of a CTA share the pixels: one thread walking a 7x7 map alone is 49 dependent additions in double
+// behind a few loads at a time, 7 us for the 2048 channels of one image whatever the GPU has idle.
 __global__ void __launch_bounds__(256) gap_cl_kernel(const float* __restrict__ x, float* __restrict__ y,
-                                                     int64_t batch, int64_t ch, int64_t area,
+                                                     int64_t maps, int64_t ch, int64_t area,
                                                      int64_t xs_n, int64_t xs_p) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  int64_t step = (int64_t)gridDim.x * blockDim.x;
-  for (; i < batch * ch; i += step) {
-    int64_t b = i / ch, c = i % ch;
-    const float* p = x + b * xs_n + c;
+  pdl_wait();
+  x = pdl_after(x);
+  __shared__ double part[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int64_t m0 = (int64_t)blockIdx.x * 32; m0 < maps; m0 += (int64_t)gridDim.x * 32) {
+    const int64_t m = m0 + lane;
     double s = 0;
-    for (int64_t a = 0; a < area; a++) s += (double)__ldg(p + a * xs_p);
-    y[i] = (float)(s / (double)area);
+    if (m < maps) {
+      const int64_t b = m / ch, c = m - b * ch;
+      const float* p = x + b * xs_n + c;
+#pragma unroll 8
+      for (int64_t a = warp; a < area; a += 8) s += (double)__ldg(p + a * xs_p);
+    }
+    part[warp][lane] = s;
+    __syncthreads();
+    if (warp == 0 && m < maps) {
+#pragma unroll
+      for (int w = 1; w < 8; w++) s += part[w][lane];
+      y[m] = (float)(s / (double)area);
+    }
+    __syncthreads();
   }
 }
 
+// NCHW: one warp per (b, c), lanes stride the pixels.
 __global__ void __launch_bounds__(256) gap_warp_kernel(const float* __restrict__ x, float* __restrict__ y,
                                                        int64_t batch, int64_t ch, int64_t area,
                                                        int64_t xs_n, int64_t xs_c, int64_t xs_p) {
+  pdl_wait();
+  x = pdl_after(x);
   int lane = threadIdx.x & 31;
   int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   int64_t rstep = (int64_t)gridDim.x * (blockDim.x >> 5);
@@ -206,6 +227,8 @@ template <int L>
 __global__ void __launch_bounds__(256) gap_group_kernel(const float* __restrict__ x, float* __restrict__ y,
                                                         int64_t rows, int64_t ch, int area, int64_t xs_n,
                                                         int64_t xs_c, int64_t xs_p) {
+  pdl_wait();
+  x = pdl_after(x);
   constexpr int R = 2;                                   // rows per lane group and iteration: twice the loads in flight
   const int gl = threadIdx.x % L;
   const int64_t gid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / L;
@@ -255,6 +278,8 @@ constexpr int GAP_MAPS = 128;
 constexpr int GAP_MAX_AREA = 96;
 __global__ void __launch_bounds__(GAP_MAPS) gap_dense_kernel(const float* __restrict__ x, float* __restrict__ y,
                                                              int64_t rows, int area) {
+  pdl_wait();
+  x = pdl_after(x);
   extern __shared__ __align__(16) float buf[];             // GAP_MAPS * area words: several CTAs per SM
   const double inv_area = 1.0 / (double)area;
   const int64_t chunks = (rows + GAP_MAPS - 1) / GAP_MAPS;
@@ -306,7 +331,8 @@ extern "C" int wdc_global_avgpool(wdc_context* ctx, const float* x, float* y, in
   WDC_REQUIRE(ctx, x && y, "wdc_global_avgpool: null buffer");
   DeviceGuard g(ctx->device);
   if (xs_c == 1) {
-    gap_cl_kernel<<<grid_for(ctx, batch * ch, 256, 8), 256, 0, ctx->stream>>>(x, y, batch, ch, area, xs_n, xs_p);
+    wdc_launch_pdl(ctx, gap_cl_kernel, dim3(grid_for(ctx, batch * ch, 32, 8)), dim3(256), 0, x, y, batch * ch, ch, area,
+                   xs_n, xs_p);
     return wdc_check_launch(ctx, "gap_cl_kernel");
   }
   if (area <= GAP_MAX_AREA && xs_p == 1 && xs_c == area && xs_n == ch * area && (((uintptr_t)x) & 15) == 0) {
@@ -314,18 +340,18 @@ extern "C" int wdc_global_avgpool(wdc_context* ctx, const float* x, float* y, in
     const int64_t chunks = (rows + GAP_MAPS - 1) / GAP_MAPS;
     const size_t smem = (size_t)GAP_MAPS * area * 4;       // 25 KB for 7x7 maps: eight CTAs per SM
     const int64_t cap = (int64_t)ctx->sm_count * 8;
-    gap_dense_kernel<<<(int)(chunks < cap ? chunks : cap), GAP_MAPS, smem, ctx->stream>>>(x, y, rows, (int)area);
+    wdc_launch_pdl(ctx, gap_dense_kernel, dim3((int)(chunks < cap ? chunks : cap)), dim3(GAP_MAPS), smem, x, y, rows, (int)area);
     return wdc_check_launch(ctx, "gap_dense_kernel");
   }
   if (area <= 128 && batch * ch < (1ll << 31) && ch < (1ll << 31)) {
     const int64_t rows = batch * ch;
     const int a = (int)area;
-    if (area <= 32) gap_group_kernel<4><<<grid_for(ctx, rows * 4, 256, 8), 256, 0, ctx->stream>>>(x, y, rows, ch, a, xs_n, xs_c, xs_p);
-    else if (area <= 64) gap_group_kernel<8><<<grid_for(ctx, rows * 8, 256, 8), 256, 0, ctx->stream>>>(x, y, rows, ch, a, xs_n, xs_c, xs_p);
-    else gap_group_kernel<16><<<grid_for(ctx, rows * 16, 256, 8), 256, 0, ctx->stream>>>(x, y, rows, ch, a, xs_n, xs_c, xs_p);
+    if (area <= 32) wdc_launch_pdl(ctx, gap_group_kernel<4>, dim3(grid_for(ctx, rows * 4, 256, 8)), dim3(256), 0, x, y, rows, ch, a, xs_n, xs_c, xs_p);
+    else if (area <= 64) wdc_launch_pdl(ctx, gap_group_kernel<8>, dim3(grid_for(ctx, rows * 8, 256, 8)), dim3(256), 0, x, y, rows, ch, a, xs_n, xs_c, xs_p);
+    else wdc_launch_pdl(ctx, gap_group_kernel<16>, dim3(grid_for(ctx, rows * 16, 256, 8)), dim3(256), 0, x, y, rows, ch, a, xs_n, xs_c, xs_p);
     return wdc_check_launch(ctx, "gap_group_kernel");
   }
-  gap_warp_kernel<<<grid_for(ctx, batch * ch * 32, 256, 8), 256, 0, ctx->stream>>>(x, y, batch, ch, area,
+  wdc_launch_pdl(ctx, gap_warp_kernel, dim3(grid_for(ctx, batch * ch * 32, 256, 8)), dim3(256), 0, x, y, batch, ch, area,
                                                                                   xs_n, xs_c, xs_p);
   return wdc_check_launch(ctx, "gap_warp_kernel");
 }

@@ -20,6 +20,13 @@ __device__ __forceinline__ double warp_sum_d(double v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
+template <int R>
+__device__ __forceinline__ void warp_sum_d(double (&v)[R]) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int r = 0; r < R; r++) v[r] += __shfl_xor_sync(0xffffffffu, v[r], o);
+}
 
 // ------------------------------------------------------------------------------ softmax
 // operators/cpu/operators/standard/softmax.ts:39-57: max, exp(v - max), sum, divide.
@@ -27,6 +34,8 @@ template <int ITEMS>
 __global__ void __launch_bounds__(256) softmax_warp_kernel(const float* __restrict__ x,
                                                            float* __restrict__ y, int64_t outer,
                                                            int len) {
+  pdl_wait();
+  x = pdl_after(x);
   int lane = threadIdx.x & 31;
   int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   int64_t rstep = (int64_t)gridDim.x * (blockDim.x >> 5);
@@ -62,6 +71,8 @@ __global__ void __launch_bounds__(256) softmax_warp_kernel(const float* __restri
 __global__ void __launch_bounds__(512) softmax_block_kernel(const float* __restrict__ x,
                                                             float* __restrict__ y, int64_t outer,
                                                             int64_t len) {
+  pdl_wait();
+  x = pdl_after(x);
   __shared__ float red[32];
   __shared__ float bcast;
   int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -117,6 +128,8 @@ __device__ __forceinline__ float block_reduce_f(float v, float* red, bool is_max
 template <int ITEMS>
 __global__ void __launch_bounds__(256) softmax_block_reg_kernel(const float* __restrict__ x, float* __restrict__ y,
                                                                 int64_t outer, int len) {
+  pdl_wait();
+  x = pdl_after(x);
   __shared__ float red[8];
   for (int64_t row = blockIdx.x; row < outer; row += gridDim.x) {
     const float* xr = x + row * len;
@@ -159,7 +172,7 @@ extern "C" int wdc_softmax(wdc_context* ctx, const float* x, float* y, int64_t o
     int wpb = 8;
     int grid = grid_for(ctx, outer * 32, wpb * 32, 8);
     int l = (int)len;
-#define SM(IT) softmax_warp_kernel<IT><<<grid, wpb * 32, 0, ctx->stream>>>(x, y, outer, l)
+#define SM(IT) wdc_launch_pdl(ctx, softmax_warp_kernel<IT>, dim3(grid), dim3(wpb * 32), 0, x, y, outer, l)
     if (len <= 32) SM(1);
     else if (len <= 128) SM(4);
     else if (len <= 256) SM(8);
@@ -174,13 +187,13 @@ extern "C" int wdc_softmax(wdc_context* ctx, const float* x, float* y, int64_t o
     const int64_t cap = (int64_t)ctx->sm_count * 8;
     const int grid = (int)(outer < cap ? outer : cap);
     const int l = (int)len;
-    if (len <= 256 * 8) softmax_block_reg_kernel<8><<<grid, 256, 0, ctx->stream>>>(x, y, outer, l);
-    else if (len <= 256 * 16) softmax_block_reg_kernel<16><<<grid, 256, 0, ctx->stream>>>(x, y, outer, l);
-    else softmax_block_reg_kernel<32><<<grid, 256, 0, ctx->stream>>>(x, y, outer, l);
+    if (len <= 256 * 8) wdc_launch_pdl(ctx, softmax_block_reg_kernel<8>, dim3(grid), dim3(256), 0, x, y, outer, l);
+    else if (len <= 256 * 16) wdc_launch_pdl(ctx, softmax_block_reg_kernel<16>, dim3(grid), dim3(256), 0, x, y, outer, l);
+    else wdc_launch_pdl(ctx, softmax_block_reg_kernel<32>, dim3(grid), dim3(256), 0, x, y, outer, l);
     return wdc_check_launch(ctx, "softmax_block_reg_kernel");
   }
   int grid = (int)(outer < (int64_t)ctx->sm_count * 4 ? outer : (int64_t)ctx->sm_count * 4);
-  softmax_block_kernel<<<grid, 512, 0, ctx->stream>>>(x, y, outer, len);
+  wdc_launch_pdl(ctx, softmax_block_kernel, dim3(grid), dim3(512), 0, x, y, outer, len);
   return wdc_check_launch(ctx, "softmax_block_kernel");
 }
 
@@ -222,6 +235,8 @@ __device__ __forceinline__ double red_finish(int kind, int final, double s, int6
 __global__ void __launch_bounds__(256) reduce_rows_kernel(int kind, int final, const float* __restrict__ x,
                                                           float* __restrict__ y, int64_t outer,
                                                           int64_t red, int64_t total) {
+  pdl_wait();
+  x = pdl_after(x);
   int lane = threadIdx.x & 31;
   int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   int64_t rstep = (int64_t)gridDim.x * (blockDim.x >> 5);
@@ -240,6 +255,8 @@ __global__ void __launch_bounds__(256) reduce_rows_kernel(int kind, int final, c
 __global__ void __launch_bounds__(256) reduce_cols_kernel(int kind, int final, const float* __restrict__ x,
                                                           float* __restrict__ y, int64_t outer,
                                                           int64_t red, int64_t inner, int64_t total) {
+  pdl_wait();
+  x = pdl_after(x);
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t step = (int64_t)gridDim.x * blockDim.x;
   int64_t n = outer * inner;
@@ -273,11 +290,11 @@ extern "C" int wdc_reduce_axis(wdc_context* ctx, int kind, int final, const floa
   WDC_REQUIRE(ctx, y && (x || red == 0), "wdc_reduce_axis: null buffer");
   DeviceGuard g(ctx->device);
   if (inner == 1 && red >= 64) {
-    reduce_rows_kernel<<<grid_for(ctx, outer * 32, 256, 8), 256, 0, ctx->stream>>>(kind, final, x, y,
+    wdc_launch_pdl(ctx, reduce_rows_kernel, dim3(grid_for(ctx, outer * 32, 256, 8)), dim3(256), 0, kind, final, x, y,
                                                                                   outer, red, total);
     return wdc_check_launch(ctx, "reduce_rows_kernel");
   }
-  reduce_cols_kernel<<<grid_for(ctx, outer * inner, 256, 8), 256, 0, ctx->stream>>>(
+  wdc_launch_pdl(ctx, reduce_cols_kernel, dim3(grid_for(ctx, outer * inner, 256, 8)), dim3(256), 0, 
       kind, final, x, y, outer, red, inner, total);
   return wdc_check_launch(ctx, "reduce_cols_kernel");
 }
@@ -295,30 +312,44 @@ __global__ void __launch_bounds__(256) layernorm_warp_kernel(const float* __rest
                                                              const float* __restrict__ beta,
                                                              float* __restrict__ y, int64_t outer,
                                                              int len, float eps) {
+  pdl_wait();
+  x = pdl_after(x);
+  gamma = pdl_after(gamma);
+  beta = pdl_after(beta);
   constexpr int R = ITEMS <= 8 ? 2 : 1;   // rows per warp iteration
+  constexpr int KEPT = ITEMS <= 8 ? ITEMS : 1;
   const double inv_len = 1.0 / (double)len;   // a double division per row costs more than the rest of the row
   int lane = threadIdx.x & 31;
   int64_t row0 = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * R;
   int64_t rstep = (int64_t)gridDim.x * (blockDim.x >> 5) * R;
+  float gk[KEPT], bk[KEPT];   // short rows: gamma and beta are read while the first row is, not behind its sums
+#pragma unroll
+  for (int i = 0; i < KEPT; i++) {
+    const int c = i * 32 + lane;
+    gk[i] = ITEMS <= 8 && gamma && c < len ? __ldg(gamma + c) : 1.f;
+    bk[i] = ITEMS <= 8 && beta && c < len ? __ldg(beta + c) : 0.f;
+  }
   for (; row0 < outer; row0 += rstep) {
     float v[R][ITEMS];
-    float s[R];
+    double s[R];
 #pragma unroll
     for (int r = 0; r < R; r++) {
       const bool live = row0 + r < outer;
       const float* xr = x + (row0 + r) * len;
-      s[r] = 0.f;
+      float t = 0.f;
 #pragma unroll
       for (int i = 0; i < ITEMS; i++) {
         int c = i * 32 + lane;
-        v[r][i] = (live && c < len) ? xr[c] : 0.f;
-        s[r] += v[r][i];
+        v[r][i] = (live && c < len) ? __ldg(xr + c) : 0.f;
+        t += v[r][i];
       }
+      s[r] = (double)t;
     }
+    // the rows' two chains of sums run side by side: a shuffle and a double addition each are latency, not work
+    warp_sum_d<R>(s);
 #pragma unroll
     for (int r = 0; r < R; r++) {
-      if (row0 + r >= outer) continue;   // warp-uniform
-      float mean = (float)(warp_sum_d((double)s[r]) * inv_len);
+      const float mean = (float)(s[r] * inv_len);
       float q = 0.f;
 #pragma unroll
       for (int i = 0; i < ITEMS; i++) {
@@ -327,16 +358,21 @@ __global__ void __launch_bounds__(256) layernorm_warp_kernel(const float* __rest
         float sq = v[r][i] * v[r][i];            // Mul / Pow 2
         q += c < len ? sq : 0.f;
       }
-      float var = (float)(warp_sum_d((double)q) * inv_len);  // ReduceMean
-      float rden = 1.f / sqrtf(var + eps);                // Add, Sqrt; the Div as a multiplication (within an ulp)
+      s[r] = (double)q;
+    }
+    warp_sum_d<R>(s);
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+      const float var = (float)(s[r] * inv_len);          // ReduceMean
+      const float rden = 1.f / sqrtf(var + eps);          // Add, Sqrt; the Div as a multiplication (within an ulp)
       float* yr = y + (row0 + r) * len;
 #pragma unroll
       for (int i = 0; i < ITEMS; i++) {
         int c = i * 32 + lane;
-        if (c < len) {
-          float o = v[r][i] * rden;              // Div
-          if (gamma) o = o * gamma[c];           // Mul
-          if (beta) o = o + beta[c];             // Add
+        if (row0 + r < outer && c < len) {
+          float o = v[r][i] * rden;                                                        // Div
+          if (gamma) o = o * (ITEMS <= 8 ? gk[i % KEPT] : __ldg(gamma + c));                // Mul
+          if (beta) o = o + (ITEMS <= 8 ? bk[i % KEPT] : __ldg(beta + c));                  // Add
           yr[c] = o;
         }
       }
@@ -361,6 +397,10 @@ __global__ void __launch_bounds__(256) layernorm_block_kernel(const float* __res
                                                               const float* __restrict__ beta,
                                                               float* __restrict__ y, int64_t outer, int64_t len,
                                                               float eps) {
+  pdl_wait();
+  x = pdl_after(x);
+  gamma = pdl_after(gamma);
+  beta = pdl_after(beta);
   __shared__ double scratch[8];
   for (int64_t row = blockIdx.x; row < outer; row += gridDim.x) {
     const float* xr = x + row * len;
@@ -392,6 +432,10 @@ __global__ void __launch_bounds__(256) layernorm_block_reg_kernel(const float* _
                                                                   const float* __restrict__ beta,
                                                                   float* __restrict__ y, int64_t outer, int len,
                                                                   float eps) {
+  pdl_wait();
+  x = pdl_after(x);
+  gamma = pdl_after(gamma);
+  beta = pdl_after(beta);
   __shared__ double scratch[8];
   const double inv_len = 1.0 / (double)len;
   for (int64_t row = blockIdx.x; row < outer; row += gridDim.x) {
@@ -442,19 +486,23 @@ extern "C" int wdc_layernorm(wdc_context* ctx, const float* x, const float* gamm
     const int64_t cap = (int64_t)ctx->sm_count * 8;
     const int grid = (int)(outer < cap ? outer : cap);
     const int l = (int)len;
-    if (len <= 256 * 8) layernorm_block_reg_kernel<8><<<grid, 256, 0, ctx->stream>>>(x, gamma, beta, y, outer, l, eps);
-    else if (len <= 256 * 16) layernorm_block_reg_kernel<16><<<grid, 256, 0, ctx->stream>>>(x, gamma, beta, y, outer, l, eps);
-    else layernorm_block_reg_kernel<32><<<grid, 256, 0, ctx->stream>>>(x, gamma, beta, y, outer, l, eps);
+    if (len <= 256 * 8) wdc_launch_pdl(ctx, layernorm_block_reg_kernel<8>, dim3(grid), dim3(256), 0, x, gamma, beta, y, outer, l, eps);
+    else if (len <= 256 * 16) wdc_launch_pdl(ctx, layernorm_block_reg_kernel<16>, dim3(grid), dim3(256), 0, x, gamma, beta, y, outer, l, eps);
+    else wdc_launch_pdl(ctx, layernorm_block_reg_kernel<32>, dim3(grid), dim3(256), 0, x, gamma, beta, y, outer, l, eps);
     return wdc_check_launch(ctx, "layernorm_block_reg_kernel");
   }
   if (len > 1024) {
     const int64_t cap = (int64_t)ctx->sm_count * 8;
-    layernorm_block_kernel<<<(int)(outer < cap ? outer : cap), 256, 0, ctx->stream>>>(x, gamma, beta, y, outer, len, eps);
+    wdc_launch_pdl(ctx, layernorm_block_kernel, dim3((int)(outer < cap ? outer : cap)), dim3(256), 0, x, gamma, beta, y, outer, len, eps);
     return wdc_check_launch(ctx, "layernorm_block_kernel");
   }
-  int grid = grid_for(ctx, outer * 32, 256, 8);
+  // rows for fewer than two CTAs of 8 warps per SM: CTAs of 2 warps, or 625 rows of 256 would use 40 of the 148 SMs
+  const int per_warp = len <= 256 ? 2 : 1;
+  const int threads = outer < (int64_t)ctx->sm_count * 16 * per_warp ? 64 : 256;
+  int grid = grid_for(ctx, ceil_div64(outer, per_warp) * 32, threads, 8);
   int l = (int)len;
-#define LN(IT) layernorm_warp_kernel<IT><<<grid, 256, 0, ctx->stream>>>(x, gamma, beta, y, outer, l, eps)
+#define LN(IT) \
+  wdc_launch_pdl(ctx, layernorm_warp_kernel<IT>, dim3(grid), dim3(threads), 0, x, gamma, beta, y, outer, l, eps)
   if (len <= 32) LN(1);
   else if (len <= 128) LN(4);
   else if (len <= 256) LN(8);
@@ -467,6 +515,8 @@ extern "C" int wdc_layernorm(wdc_context* ctx, const float* x, const float* gamm
 // ------------------------------------------------------------------------------- argmax
 __global__ void __launch_bounds__(256) argmax_kernel(const float* __restrict__ x, int32_t* __restrict__ y,
                                                      int64_t outer, int64_t len, int select_last) {
+  pdl_wait();
+  x = pdl_after(x);
   int lane = threadIdx.x & 31;
   int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   int64_t rstep = (int64_t)gridDim.x * (blockDim.x >> 5);
@@ -504,6 +554,6 @@ extern "C" int wdc_argmax(wdc_context* ctx, const float* x, int32_t* y, int64_t 
   if (outer == 0) return WDC_OK;
   WDC_REQUIRE(ctx, x && y, "wdc_argmax: null buffer");
   DeviceGuard g(ctx->device);
-  argmax_kernel<<<grid_for(ctx, outer * 32, 256, 8), 256, 0, ctx->stream>>>(x, y, outer, len, select_last);
+  wdc_launch_pdl(ctx, argmax_kernel, dim3(grid_for(ctx, outer * 32, 256, 8)), dim3(256), 0, x, y, outer, len, select_last);
   return wdc_check_launch(ctx, "argmax_kernel");
 }
