@@ -375,17 +375,6 @@ extern "C" int wdc_wait_upload(wdc_context* ctx, int64_t ticket) {
 }
 
 // ---- capture of one run into a CUDA graph ------------------------------------------------------
-struct wdc_graph {
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
-  wdc_arena* arena = nullptr;  // owns every buffer the captured launches touch that was allocated while capturing
-  // The recorded launches hold the addresses of the tensor-core path's cached operand splits (hi/lo copies of
-  // the weights).  split_seq = the context's split counter when the capture ended: if a split that is that old
-  // is dropped later (its weight was rewritten or freed), the graph would read freed memory, so it goes stale.
-  int64_t split_seq = 0;
-  bool stale = false;
-};
-
 void wdc_graphs_note_evicted(wdc_context* ctx, int64_t born) {
   for (wdc_graph* g : ctx->live_graphs)
     if (born <= g->split_seq) g->stale = true;
@@ -460,6 +449,9 @@ extern "C" int wdc_graph_destroy(wdc_context* ctx, wdc_graph* graph) {
   for (size_t i = 0; i < ctx->live_graphs.size(); i++)
     if (ctx->live_graphs[i] == graph) ctx->live_graphs.erase(ctx->live_graphs.begin() + i--);
   if (graph->exec) cudaGraphExecDestroy(graph->exec);
+  for (cudaGraphExec_t e : graph->io_exec)
+    if (e) cudaGraphExecDestroy(e);
+  if (graph->io_host) cudaFreeHost(graph->io_host);
   if (graph->graph) cudaGraphDestroy(graph->graph);
   if (graph->arena) {
     if (!graph->arena->live.empty())
@@ -545,6 +537,7 @@ extern "C" int wdc_copy(wdc_context* ctx, void* dst, const void* src, int64_t by
 }
 
 __global__ void fill_u32_kernel(uint32_t* dst, uint32_t v, int64_t n) {
+  pdl_wait();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t step = (int64_t)gridDim.x * blockDim.x;
   for (; i < n; i += step) dst[i] = v;
@@ -557,7 +550,7 @@ extern "C" int wdc_fill_u32(wdc_context* ctx, void* dst, uint32_t value, int64_t
   wdc_note_write(ctx, dst, count * 4);
   if (count == 0) return WDC_OK;
   DeviceGuard g(ctx->device);
-  fill_u32_kernel<<<grid_for(ctx, count, 256), 256, 0, ctx->stream>>>((uint32_t*)dst, value, count);
+  wdc_launch_pdl(ctx, fill_u32_kernel, dim3(grid_for(ctx, count, 256)), dim3(256), 0, (uint32_t*)dst, value, count);
   return wdc_check_launch(ctx, "fill_u32_kernel");
 }
 

@@ -1,4 +1,6 @@
 // Recording and repeating the calls of a run (see tape.cuh), and a captured graph's run with its host transfers.
+#include <string.h>
+
 #include "tape.cuh"
 
 thread_local wdc_tape* wdc_thread_tape = nullptr;
@@ -114,6 +116,125 @@ extern "C" int wdc_tape_run(wdc_context* ctx, wdc_tape* tape, const void* const*
   return s;
 }
 
+namespace {
+
+constexpr int64_t IO_LIMIT = 128 << 10;   // transfers that a kernel makes (see transfer.cu)
+
+int64_t padded(int64_t bytes) { return bytes > 0 ? (bytes + 15) / 16 * 16 : 0; }
+
+// The graph with its transfers as kernels at both ends (`with_in`: inputs too).  Null when it could not be made.
+cudaGraphExec_t io_graph(wdc_graph* g, bool with_in, const wdc_io_list& in, const wdc_io_list& out) {
+  if (g->io_exec[with_in])   // (made for other buffers: the caller goes the general way)
+    return g->io_in[with_in] == in && g->io_out == out ? g->io_exec[with_in] : nullptr;
+  if (g->io_failed || (g->io_exec[!with_in] && !(g->io_out == out))) return nullptr;
+  cudaGraph_t whole = nullptr;
+  cudaGraphNode_t first = nullptr, body = nullptr, last = nullptr;
+  auto kernel_node = [](const wdc_io_list& list, void** args) {
+    cudaKernelNodeParams k = {};
+    k.func = wdc_io_kernel();
+    k.gridDim = wdc_io_grid(list);
+    k.blockDim = dim3(256);
+    k.kernelParams = args;
+    return k;
+  };
+  wdc_io_list in_copy = in, out_copy = out;
+  void* in_args[] = {&in_copy};
+  void* out_args[] = {&out_copy};
+  cudaError_t e = cudaGraphCreate(&whole, 0);
+  if (e == cudaSuccess && with_in) {
+    const cudaKernelNodeParams k = kernel_node(in, in_args);
+    e = cudaGraphAddKernelNode(&first, whole, nullptr, 0, &k);
+  }
+  if (e == cudaSuccess) e = cudaGraphAddChildGraphNode(&body, whole, first ? &first : nullptr, first ? 1 : 0, g->graph);
+  if (e == cudaSuccess) {
+    const cudaKernelNodeParams k = kernel_node(out, out_args);
+    e = cudaGraphAddKernelNode(&last, whole, &body, 1, &k);
+  }
+  if (e == cudaSuccess) e = cudaGraphInstantiate(&g->io_exec[with_in], whole, 0);
+  if (whole) cudaGraphDestroy(whole);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    g->io_failed = true;
+    g->io_exec[with_in] = nullptr;
+  }
+  g->io_in[with_in] = in;
+  g->io_out = out;
+  return g->io_exec[with_in];
+}
+
+// A run whose outputs (and, when they come from the host, inputs) are small.  False: not taken, nothing happened.
+bool run_small(wdc_context* ctx, wdc_graph* g, int n_in, void* const* dst, const void* const* src, const int64_t* in_bytes,
+               const int32_t* in_on_host, int n_out, void* const* host, const void* const* out, const int64_t* out_bytes,
+               int* status) {
+  int64_t in_total = 0, out_total = 0;
+  bool from_host = n_in > 0, words = true;
+  for (int i = 0; i < n_in; i++) {
+    in_total += padded(in_bytes[i]);
+    from_host &= in_on_host[i] != 0;
+    words &= in_bytes[i] % 4 == 0;
+  }
+  for (int i = 0; i < n_out; i++) {
+    out_total += padded(out_bytes[i]);
+    words &= out_bytes[i] % 4 == 0;
+  }
+  if (g->stale || g->io_failed || ctx->capture_arena || !words || n_out < 1 || n_out > wdc_io_list::MOST ||
+      n_in > wdc_io_list::MOST || out_total > IO_LIMIT || out_total == 0)
+    return false;
+  const bool with_in = from_host && in_total > 0 && in_total <= IO_LIMIT;
+  std::lock_guard<std::mutex> lk(g->io_mu);
+  if (!g->io_host) {   // (sized by the first run; the buffers of a captured run do not change)
+    g->io_bytes = (in_total <= IO_LIMIT ? in_total : 0) + out_total;
+    g->io_in_bytes = in_total <= IO_LIMIT ? in_total : 0;
+    if (cudaMallocHost((void**)&g->io_host, (size_t)g->io_bytes) != cudaSuccess) {
+      cudaGetLastError();
+      g->io_failed = true;
+      return false;
+    }
+  }
+  if ((with_in && in_total != g->io_in_bytes) || g->io_in_bytes + out_total > g->io_bytes) return false;
+  wdc_io_list ins = {}, outs = {};
+  int64_t at = 0;
+  for (int i = 0; with_in && i < n_in; i++) {
+    if (in_bytes[i] <= 0) continue;
+    memcpy(g->io_host + at, src[i], (size_t)in_bytes[i]);
+    ins.part[ins.n++] = {(uint32_t*)dst[i], (const uint32_t*)(g->io_host + at), in_bytes[i] / 4};
+    at += padded(in_bytes[i]);
+  }
+  at = g->io_in_bytes;
+  for (int i = 0; i < n_out; i++) {
+    if (out_bytes[i] <= 0) continue;
+    outs.part[outs.n++] = {(uint32_t*)(g->io_host + at), (const uint32_t*)out[i], out_bytes[i] / 4};
+    at += padded(out_bytes[i]);
+  }
+  cudaGraphExec_t exec = io_graph(g, with_in, ins, outs);
+  if (!exec) return false;
+  int s = WDC_OK;
+  for (int i = 0; i < n_in && s == WDC_OK; i++) {
+    if (in_bytes[i] <= 0) continue;
+    wdc_tc_evict(ctx, dst[i], in_bytes[i]);
+    if (with_in) ctx->h2d_bytes += in_bytes[i];
+    else if (in_on_host[i]) s = wdc_stage_in(ctx, dst[i], src[i], in_bytes[i]);
+    else
+      s = wdc_check_cuda(ctx, cudaMemcpyAsync(dst[i], src[i], (size_t)in_bytes[i], cudaMemcpyDeviceToDevice, ctx->stream),
+                         "copy of an input");
+  }
+  if (s == WDC_OK && g->stale) s = wdc_graph_launch(ctx, g);   // (gone stale just now: the error it gives)
+  else if (s == WDC_OK) {
+    s = wdc_check_cuda(ctx, cudaGraphLaunch(exec, ctx->stream), "cudaGraphLaunch");
+    ctx->n_launch++;
+  }
+  if (s == WDC_OK) s = wdc_sync(ctx);
+  for (int i = 0, k = 0; i < n_out && s == WDC_OK; i++) {
+    if (out_bytes[i] <= 0) continue;
+    memcpy(host[i], outs.part[k++].dst, (size_t)out_bytes[i]);
+    ctx->d2h_bytes += out_bytes[i];
+  }
+  *status = s;
+  return true;
+}
+
+}  // namespace
+
 extern "C" int wdc_graph_run(wdc_context* ctx, wdc_graph* graph, int n_in, void* const* dst, const void* const* src,
                              const int64_t* in_bytes, const int32_t* in_on_host, int n_out, void* const* host,
                              const void* const* out, const int64_t* out_bytes) {
@@ -122,6 +243,8 @@ extern "C" int wdc_graph_run(wdc_context* ctx, wdc_graph* graph, int n_in, void*
     return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_graph_run: bad argument");
   WDC_NO_TAPE(ctx);
   DeviceGuard g(ctx->device);
+  int small = WDC_OK;
+  if (run_small(ctx, graph, n_in, dst, src, in_bytes, in_on_host, n_out, host, out, out_bytes, &small)) return small;
   for (int i = 0; i < n_in; i++) {
     if (in_bytes[i] <= 0) continue;
     wdc_tc_evict(ctx, dst[i], in_bytes[i]);

@@ -130,3 +130,23 @@ void tape_note(wdc_tape* t, F fn, A... args) {
 #define WDC_NO_TAPE(ctx)       \
   TapeScope tape_scope_(ctx);  \
   if (tape_scope_.tape) tape_scope_.tape->valid = false
+
+// A captured run (context.cu).
+struct wdc_graph {
+  cudaGraph_t graph = nullptr;
+  cudaGraphExec_t exec = nullptr;
+  wdc_arena* arena = nullptr;  // owns every buffer the captured launches touch that was allocated while capturing
+  // The recorded launches hold the addresses of the tensor-core path's cached operand splits (hi/lo copies of
+  // the weights).  split_seq = the context's split counter when the capture ended: if a split that is that old
+  // is dropped later (its weight was rewritten or freed), the graph would read freed memory, so it goes stale.
+  int64_t split_seq = 0;
+  bool stale = false;
+  // wdc_graph_run with small transfers: the graph between one kernel that brings the inputs in from page-locked memory
+  // (index 1; index 0 leaves that out) and one that takes the outputs there, so that a run is one launch and one wait
+  cudaGraphExec_t io_exec[2] = {nullptr, nullptr};
+  bool io_failed = false;
+  char* io_host = nullptr;          // page-locked: inputs, then outputs
+  int64_t io_in_bytes = 0, io_bytes = 0;
+  wdc_io_list io_in[2] = {}, io_out = {};   // what the kernels were made with
+  std::mutex io_mu;                 // a run owns the staging memory from its inputs to its outputs
+};

@@ -4,7 +4,8 @@
 // else can be queued, 12.7 GB/s for megabytes (605 us for an 800x800 image), where the link takes 50 GB/s from
 // page-locked memory.  Here the context keeps a ring of page-locked chunks: a transfer is cut into chunks, each is
 // copied by a few threads and sent (or received and copied) while its neighbours are on the link.  Page-locked
-// buffers of the caller's go straight to the link.
+// buffers of the caller's go straight to the link.  Small transfers leave the copy engines out: a kernel of the compute
+// stream reads or writes the page-locked memory, which saves the switch between the two.
 #include <string.h>
 
 #include <atomic>
@@ -16,11 +17,12 @@
 namespace {
 
 constexpr int64_t CHUNK = 512 << 10;    // long enough to hide an event and a copy call (a few us) behind 10 us of link
-constexpr int CHUNKS = 16;
+constexpr int CHUNKS = 32;
 constexpr int64_t PIECE = 64 << 10;     // what a thread takes at a time
 constexpr int64_t ALONE = 256 << 10;    // below this the other threads would only be woken up
 constexpr int64_t PINNED_CHECK = 256 << 10;   // asking the driver what a pointer is costs about a microsecond
-constexpr int MAX_HELPERS = 3;
+constexpr int64_t BY_KERNEL = 128 << 10;      // up to here the link's latency, not its rate, is the time
+constexpr int MAX_HELPERS = 5;
 
 // memcpy by the caller and up to MAX_HELPERS threads that take pieces from a common counter: a helper that is still
 // asleep costs nothing, the caller takes its pieces.  Helpers poll for a while after a job, then sleep.
@@ -34,9 +36,13 @@ class CopyTeam {
     cv_.notify_all();
     for (auto& t : helpers_) t.join();
   }
-  void copy(char* dst, const char* src, int64_t bytes) {
+  // dst[c] <- src in chunks of CHUNK bytes; sent(c) is called by the caller's thread, in order, as chunks are complete.
+  template <class F>
+  void copy(char* const* dst, const char* src, int64_t bytes, F sent) {
+    const int chunks = (int)((bytes + CHUNK - 1) / CHUNK);
     if (bytes < ALONE) {
-      memcpy(dst, src, (size_t)bytes);
+      memcpy(dst[0], src, (size_t)bytes);
+      sent(0);
       return;
     }
     if (helpers_.empty()) start();
@@ -51,21 +57,29 @@ class CopyTeam {
       seq_.fetch_add(1, std::memory_order_release);
     }
     if (asleep_.load() > 0) cv_.notify_all();
-    work(job);
+    for (int c = 0; c < chunks;) {
+      const int64_t n = bytes - (int64_t)c * CHUNK < CHUNK ? bytes - (int64_t)c * CHUNK : CHUNK;
+      if (job.done[c].load(std::memory_order_acquire) == (int)((n + PIECE - 1) / PIECE)) sent(c++);
+      else if (!take(job)) pause();
+    }
     {
       std::lock_guard<std::mutex> lk(mu_);   // no helper picks the job up any more ...
       job_ = nullptr;
     }
     while (job.users.load(std::memory_order_acquire) > 0) pause();   // ... and those who did have left it
   }
+  void copy(char* dst, const char* src, int64_t bytes) {   // at most one chunk
+    copy(&dst, src, bytes, [](int) {});
+  }
 
  private:
   struct Job {
-    char* dst;
+    char* const* dst;
     const char* src;
     int64_t bytes;
     int pieces;
     std::atomic<int> next{0}, users{0};
+    std::atomic<int> done[CHUNKS] = {};   // pieces of a chunk that have been copied
   };
   static void pause() {
 #if defined(__x86_64__)
@@ -74,11 +88,14 @@ class CopyTeam {
     std::this_thread::yield();
 #endif
   }
-  static void work(Job& j) {
-    for (int i; (i = j.next.fetch_add(1, std::memory_order_relaxed)) < j.pieces;) {
-      const int64_t off = (int64_t)i * PIECE, n = j.bytes - off < PIECE ? j.bytes - off : PIECE;
-      memcpy(j.dst + off, j.src + off, (size_t)n);
-    }
+  // Copies the next piece; false when none is left.
+  static bool take(Job& j) {
+    const int i = j.next.fetch_add(1, std::memory_order_relaxed);
+    if (i >= j.pieces) return false;
+    const int64_t off = (int64_t)i * PIECE, n = j.bytes - off < PIECE ? j.bytes - off : PIECE;
+    memcpy(j.dst[off / CHUNK] + off % CHUNK, j.src + off, (size_t)n);
+    j.done[off / CHUNK].fetch_add(1, std::memory_order_release);
+    return true;
   }
   void start() {
     const unsigned cpus = std::thread::hardware_concurrency();
@@ -107,7 +124,7 @@ class CopyTeam {
         if (job) job->users.fetch_add(1, std::memory_order_relaxed);
       }
       if (job) {
-        work(*job);
+        while (take(*job)) {}
         job->users.fetch_sub(1, std::memory_order_release);
       }
     }
@@ -170,7 +187,28 @@ bool page_locked(const void* p, int64_t bytes) {
   return a.type == cudaMemoryTypeHost;
 }
 
+// Words of several buffers, copied by one launch.  Page-locked host memory on one side.
+__global__ void __launch_bounds__(256) io_copy_kernel(const wdc_io_list list) {
+  pdl_wait();
+  for (int s = 0; s < list.n; s++) {
+    const wdc_io_list::Part p = list.part[s];
+    const int64_t vec = (((uintptr_t)p.dst | (uintptr_t)p.src) & 15) == 0 ? p.words / 4 : 0;
+    const int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i = first; i < vec; i += step)
+      reinterpret_cast<uint4*>(p.dst)[i] = __ldcv(reinterpret_cast<const uint4*>(p.src) + i);
+    for (int64_t i = vec * 4 + first; i < p.words; i += step) p.dst[i] = __ldcv(p.src + i);
+  }
+}
+
 }  // namespace
+
+dim3 wdc_io_grid(const wdc_io_list& list) {
+  int64_t most = 0;
+  for (int i = 0; i < list.n; i++) most = list.part[i].words > most ? list.part[i].words : most;
+  const int64_t blocks = ceil_div64(most, 4 * 256);
+  return dim3((unsigned)(blocks < 1 ? 1 : blocks < 64 ? blocks : 64));
+}
+void* wdc_io_kernel() { return (void*)io_copy_kernel; }
 
 void wdc_stager_destroy(wdc_context* ctx) {
   wdc_stager* s = ctx->stager;
@@ -195,16 +233,39 @@ int wdc_stage_in(wdc_context* ctx, void* dst, const void* host, int64_t bytes) {
   int st = stager_of(ctx, &s);
   if (st != WDC_OK) return st;
   std::lock_guard<std::mutex> lk(s->mu);
-  for (int64_t off = 0; off < bytes; off += CHUNK) {
-    const int64_t n = bytes - off < CHUNK ? bytes - off : CHUNK;
+  if (bytes <= BY_KERNEL && bytes % 4 == 0) {
     int i;
     st = take_chunk(ctx, s, &i);
     if (st != WDC_OK) return st;
-    char* chunk = s->ring + i * CHUNK;
-    s->team.copy(chunk, (const char*)host + off, n);
-    WDC_CUDA(ctx, cudaMemcpyAsync((char*)dst + off, chunk, (size_t)n, cudaMemcpyHostToDevice, ctx->stream));
+    memcpy(s->ring + i * CHUNK, host, (size_t)bytes);
+    wdc_io_list list = {};
+    list.n = 1;
+    list.part[0] = {(uint32_t*)dst, (const uint32_t*)(s->ring + i * CHUNK), bytes / 4};
+    wdc_launch_pdl(ctx, io_copy_kernel, wdc_io_grid(list), dim3(256), 0, list);
+    WDC_CUDA(ctx, cudaGetLastError());
     WDC_CUDA(ctx, cudaEventRecord(s->done[i], ctx->stream));
     s->busy[i] = true;
+    return WDC_OK;
+  }
+  for (int64_t base = 0; base < bytes; base += CHUNKS * CHUNK) {   // a ring's worth at a time
+    const int64_t part = bytes - base < CHUNKS * CHUNK ? bytes - base : CHUNKS * CHUNK;
+    int index[CHUNKS];
+    char* chunk[CHUNKS];
+    for (int64_t off = 0; off < part; off += CHUNK) {
+      const int c = (int)(off / CHUNK);
+      st = take_chunk(ctx, s, &index[c]);
+      if (st != WDC_OK) return st;
+      chunk[c] = s->ring + index[c] * CHUNK;
+    }
+    cudaError_t e = cudaSuccess;
+    s->team.copy(chunk, (const char*)host + base, part, [&](int c) {
+      const int64_t off = (int64_t)c * CHUNK, n = part - off < CHUNK ? part - off : CHUNK;
+      if (e == cudaSuccess)
+        e = cudaMemcpyAsync((char*)dst + base + off, chunk[c], (size_t)n, cudaMemcpyHostToDevice, ctx->stream);
+      if (e == cudaSuccess) e = cudaEventRecord(s->done[index[c]], ctx->stream);
+      if (e == cudaSuccess) s->busy[index[c]] = true;
+    });
+    if (e != cudaSuccess) return wdc_check_cuda(ctx, e, "transfer to the device");
   }
   return WDC_OK;
 }
@@ -216,6 +277,33 @@ int wdc_stage_out(wdc_context* ctx, int count, void* const* host, const void* co
   wdc_stager* s = nullptr;
   int st = stager_of(ctx, &s);
   if (st != WDC_OK) return st;
+  int64_t total = 0;
+  bool words = true;
+  for (int b = 0; b < count; b++) {
+    total += bytes[b] > 0 ? (bytes[b] + 15) / 16 * 16 : 0;
+    words &= bytes[b] % 4 == 0;
+  }
+  if (total > 0 && total <= BY_KERNEL && words && count <= wdc_io_list::MOST) {
+    std::lock_guard<std::mutex> lk(s->mu);
+    int i;
+    st = take_chunk(ctx, s, &i);
+    if (st != WDC_OK) return st;
+    char* at = s->ring + i * CHUNK;
+    wdc_io_list list = {};
+    for (int b = 0; b < count; b++) {
+      if (bytes[b] <= 0) continue;
+      ctx->d2h_bytes += bytes[b];
+      list.part[list.n++] = {(uint32_t*)at, (const uint32_t*)src[b], bytes[b] / 4};
+      at += (bytes[b] + 15) / 16 * 16;
+    }
+    wdc_launch_pdl(ctx, io_copy_kernel, wdc_io_grid(list), dim3(256), 0, list);
+    WDC_CUDA(ctx, cudaGetLastError());
+    st = wdc_sync(ctx);
+    if (st != WDC_OK) return st;
+    for (int b = 0, k = 0; b < count; b++)
+      if (bytes[b] > 0) memcpy(host[b], list.part[k++].dst, (size_t)bytes[b]);
+    return WDC_OK;
+  }
   {
     std::lock_guard<std::mutex> lk(s->mu);
     struct Part {
