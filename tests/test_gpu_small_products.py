@@ -180,3 +180,28 @@ def test_layernorm_row_counts(cuda_context, rows, length):
     model = single_op_model("LayerNormalization", {"axis": -1, "epsilon": 1e-5}, [x, gamma, beta], opset=17)
     (got,) = run_cuda(model, [x, gamma, beta], cuda_context)
     assert max_err_rel_linf(got, ops.layernorm_chain(x, gamma, beta, 1e-5)) <= 5e-6
+
+
+# clusters of 2, 4 and 8 CTAs per query tile: ranges of chunks of unequal length, a ragged last chunk and last rows
+@pytest.mark.parametrize("batch,heads,tq,tk,dh", [(1, 3, 130, 257, 32), (1, 8, 625, 625, 32), (1, 8, 100, 625, 32),
+                                                  (3, 1, 17, 256, 32), (1, 4, 300, 450, 64), (1, 2, 100, 640, 64)])
+def test_attention_shared_by_a_cluster(cuda_context, batch, heads, tq, tk, dh):
+    from ctypes import c_void_p
+
+    from webdnn_b200.backend import CPUTensor
+    from webdnn_b200.lib import AttentionDesc
+    rng = np.random.default_rng(tq + tk)
+    w = heads * dh
+    q, k, v = (2 * rng.standard_normal((batch, t, w)).astype(np.float32) for t in (tq, tk, tk))
+    qh, kh, vh = (x.reshape(batch, -1, heads, dh).transpose(0, 2, 1, 3).astype(np.float64) for x in (q, k, v))
+    s = qh @ kh.transpose(0, 1, 3, 2) * dh ** -0.5
+    p = np.exp(s - s.max(-1, keepdims=True))
+    want = (p / p.sum(-1, keepdims=True) @ vh).transpose(0, 2, 1, 3).reshape(batch, tq, w)
+    put = lambda a: cuda_context.move_tensor(CPUTensor.from_array(a))  # noqa: E731
+    dq, dk, dv, y = put(q), put(k), put(v), cuda_context.empty_tensor([batch, tq, w])
+    d = AttentionDesc(batch=batch, heads=heads, tq=tq, tk=tk, dh=dh, q_sb=tq * w, q_sh=dh, q_st=w, k_sb=tk * w, k_sh=dh,
+                      k_st=w, v_sb=tk * w, v_sh=dh, v_st=w, y_sb=tq * w, y_sh=dh, y_st=w, scale=dh ** -0.5)
+    cuda_context._call("wdc_attention", byref(d), *(c_void_p(t.ptr) for t in (dq, dk, dv, y)))
+    assert max_err_rel_linf(y.get_data().reshape(want.shape), want) <= 1e-5
+    for t in (dq, dk, dv, y):
+        t.dispose()

@@ -20,10 +20,14 @@
 // 128B-swizzled shared memory, two stages deep.  Keys past tk read as zero or as the next head's rows; their
 // scores are replaced by -inf before the maximum, so they contribute nothing.
 //
-// Warps: 0-3 row threads, 4 TMA producer, 5 MMA issuer (one elected lane each).  With a head size of 32 a CTA needs
-// 256 TMEM columns and 64 KB of shared memory, so two CTAs share an SM and one's softmax overlaps the other's MMAs.
-// Every mbarrier wait is bounded (2 s): on expiry the CTA records a status code, raises its abort flag, frees its
-// TMEM and returns.  No cluster, no multicast.
+// A chunk is a serial chain (S, softmax, P V) of about 2 us, so one image's 40 query tiles used 40 SMs for ten chunks
+// while the others idled.  Where CTAs are few, a cluster of 2, 4 or 8 shares a query tile: each takes a range of the
+// chunks, and the partial results (row maximum, row sum, unnormalised row) are combined through distributed shared
+// memory, each CTA finishing its part of the rows (choose_cluster).
+//
+// Warps: 0-3 row threads, 4 TMA producer (one elected lane), 5 MMA issuer.  With a head size of 32 a CTA needs 256 TMEM columns and 64 KB of shared memory, so two CTAs share an SM and
+// one's softmax overlaps the other's MMAs.  Every mbarrier wait is bounded (2 s): on expiry the CTA records a status
+// code, raises its abort flag, still meets its cluster, frees its TMEM and returns.  No multicast.
 #include <cuda.h>
 
 #include <math.h>
@@ -36,6 +40,7 @@ constexpr int BQ = 128;           // query rows per CTA = TMEM lanes
 constexpr int BK = 64;            // keys per chunk
 constexpr int ATT_THREADS = 192;
 constexpr int STAGES = 2;
+constexpr int PARTS_OFFSET = 256;  // behind the stages: AttShared, then a cluster's partial results
 constexpr unsigned long long WAIT_LIMIT_NS = 2000000000ull;
 
 struct AttTcProblem {
@@ -43,6 +48,7 @@ struct AttTcProblem {
   float* y;
   int64_t q_sb, q_sh, q_st, y_sb, y_sh, y_st;
   int heads, tq, tk;
+  int cs;             // CTAs per query tile (a cluster)
   float scale_log2;   // scale * log2(e): the softmax runs on exp2
   int* status;
 };
@@ -53,6 +59,8 @@ struct AttShared {
   unsigned int tmem_base;
   volatile int abort_flag;
 };
+
+static_assert(sizeof(AttShared) <= PARTS_OFFSET, "AttShared's place");
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(unsigned long long* bar, int count) {
@@ -124,19 +132,47 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr) {
 __device__ __forceinline__ uint32_t make_idesc(int n) {
   return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(BQ >> 4) << 24);
 }
-__device__ __forceinline__ void umma_tf32_ts(uint32_t tmem_c, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc,
-                                             uint32_t accumulate) {
+// kAll: the whole warp runs the issuing loop, so that its addresses stay in uniform registers, and the lane whose `leader`
+// is 1 issues; else the calling lane does.
+template <bool kAll>
+__device__ __forceinline__ void umma_by(uint32_t leader, uint32_t tmem_c, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc,
+                                        uint32_t accumulate) {
+  if (kAll)
+    asm volatile(
+        "{\n\t.reg .pred p, e;\n\t"
+        "setp.ne.b32 e, %0, 0;\n\t"
+        "setp.ne.b32 p, %5, 0;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::tf32 [%1], [%2], %3, %4, p;\n\t}"
+        :
+        : "r"(leader), "r"(tmem_c), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}"
+        :
+        : "r"(tmem_c), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void commit_by(uint32_t leader, unsigned long long* bar) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}"
-      :
-      : "r"(tmem_c), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      "{\n\t.reg .pred e;\n\t"
+      "setp.ne.b32 e, %0, 0;\n\t"
+      "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%1];\n\t}" ::"r"(leader),
+      "r"(smem_u32(bar))
       : "memory");
 }
-__device__ __forceinline__ void umma_commit(unsigned long long* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-               : "memory");
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+// Stores to CTA `rank`'s shared memory, at the address the word has in this CTA's.
+__device__ __forceinline__ uint32_t cluster_at(const float* p, int rank) {
+  uint32_t at;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(smem_u32(p)), "r"(rank));
+  return at;
+}
+__device__ __forceinline__ void cluster_st(uint32_t at, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(at), "f"(v) : "memory");
 }
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, unsigned long long* bar, int x, int y) {
   asm volatile(
@@ -226,9 +262,11 @@ struct AttLayout {
   // tensor-memory columns
   static constexpr int Q_HI = 0, Q_LO = DH, S = 2 * DH, P_LO = S + BK, O = P_LO + BK;
   static constexpr int TMEM_COLS = DH == 32 ? 256 : 512;   // 224 or 320 used; a power of two must be allocated
+  static constexpr int PARTS = (DH + 2) * BQ * 4;          // clusters: partial results of the rows a CTA finishes
 };
 
-template <int DH>
+// kCluster: p.cs > 1 CTAs share a query tile.
+template <int DH, bool kCluster>
 __global__ void __launch_bounds__(ATT_THREADS, DH == 32 ? 2 : 1)
 attention_tc_kernel(const AttTcProblem p, const __grid_constant__ CUtensorMap map_k_hi,
                     const __grid_constant__ CUtensorMap map_k_lo, const __grid_constant__ CUtensorMap map_vt_hi,
@@ -239,8 +277,11 @@ attention_tc_kernel(const AttTcProblem p, const __grid_constant__ CUtensorMap ma
   AttShared* sh = reinterpret_cast<AttShared*>(stage_base + STAGES * L::STAGE_BYTES);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int bh = blockIdx.y, b = bh / p.heads, h = bh - b * p.heads;
-  const int q0 = blockIdx.x * BQ;
-  const int nck = (p.tk + BK - 1) / BK;
+  const int cs = kCluster ? p.cs : 1, rank = (int)blockIdx.x % cs;   // (clusters are cs consecutive CTAs)
+  const int q0 = (int)blockIdx.x / cs * BQ;
+  const int chunks = (p.tk + BK - 1) / BK;
+  const int first = kCluster ? (int)((int64_t)rank * chunks / cs) : 0;   // this CTA's chunks
+  const int nck = (kCluster ? (int)((int64_t)(rank + 1) * chunks / cs) : chunks) - first;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; s++) {
@@ -269,9 +310,12 @@ attention_tc_kernel(const AttTcProblem p, const __grid_constant__ CUtensorMap ma
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = sh->tmem_base;
+  if (kCluster) cluster_arrive();   // this CTA has begun: its peers may write to its shared memory (waited for below)
   // the pre-pass (the grid before this one) wrote the split operands this kernel is about to load
   pdl_wait();
 
+  bool ok = true;
+  float o[DH], m = -INFINITY, l = 0.f;                      // row threads: unnormalised row, its maximum and sum
   if (warp < 4) {
     // ============================================================================ row threads
     const int r = threadIdx.x;                              // query row inside the tile = TMEM lane
@@ -279,7 +323,7 @@ attention_tc_kernel(const AttTcProblem p, const __grid_constant__ CUtensorMap ma
     const int qrow = q0 + r;
     {
       // Q row -> tensor memory: high part raw (the tensor core truncates), low part x - truncate(x)
-      const float* qp = p.q + (int64_t)b * p.q_sb + (int64_t)h * p.q_sh + (int64_t)qrow * p.q_st;
+      const float* qp = pdl_after(p.q) + (int64_t)b * p.q_sb + (int64_t)h * p.q_sh + (int64_t)qrow * p.q_st;
 #pragma unroll
       for (int c0 = 0; c0 < DH; c0 += 16) {
         float hi[16], lo[16];
@@ -298,11 +342,8 @@ attention_tc_kernel(const AttTcProblem p, const __grid_constant__ CUtensorMap ma
       __syncwarp();
       if (lane == 0) mbar_arrive(&sh->q_ready);
     }
-    float o[DH];
 #pragma unroll
     for (int c = 0; c < DH; c++) o[c] = 0.f;
-    float m = -INFINITY, l = 0.f;
-    bool ok = true;
     for (int j = 0; j < nck && ok; j++) {
       const uint32_t ph = (uint32_t)(j & 1);
       ok = mbar_wait(&sh->s_full, ph, sh, p.status, 71);
@@ -312,8 +353,8 @@ attention_tc_kernel(const AttTcProblem p, const __grid_constant__ CUtensorMap ma
 #pragma unroll
       for (int c0 = 0; c0 < BK; c0 += 16) tmem_ld16(lane_base + (uint32_t)(L::S + c0), s + c0);
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      const int valid = p.tk - j * BK;                      // columns of this chunk that are real keys
-      float mc = -INFINITY;
+      const int valid = p.tk - (first + j) * BK;            // columns of this chunk that are real keys
+      float mc = -INFINITY, sum = 0.f;
 #pragma unroll
       for (int c = 0; c < BK; c++) {
         s[c] = c < valid ? s[c] * p.scale_log2 : -INFINITY;
@@ -321,7 +362,6 @@ attention_tc_kernel(const AttTcProblem p, const __grid_constant__ CUtensorMap ma
       }
       const float m_new = fmaxf(m, mc);
       const float alpha = exp2f(m - m_new);                 // 0 for the first chunk (m = -inf)
-      float sum = 0.f;
 #pragma unroll
       for (int c = 0; c < BK; c++) {
         s[c] = exp2f(s[c] - m_new);
@@ -356,7 +396,7 @@ attention_tc_kernel(const AttTcProblem p, const __grid_constant__ CUtensorMap ma
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     }
-    if (ok && qrow < p.tq) {
+    if (!kCluster && ok && qrow < p.tq) {
       const float inv = 1.f / l;
       float* yp = p.y + (int64_t)b * p.y_sb + (int64_t)h * p.y_sh + (int64_t)qrow * p.y_st;
 #pragma unroll
@@ -366,7 +406,6 @@ attention_tc_kernel(const AttTcProblem p, const __grid_constant__ CUtensorMap ma
   } else if (warp == 4) {
     // ============================================================================ TMA producer
     if (elect_one()) {
-      bool ok = true;
       for (int j = 0; j < nck && ok; j++) {
         const int st = j % STAGES;
         const uint32_t ph = (uint32_t)((j / STAGES) & 1);
@@ -374,7 +413,7 @@ attention_tc_kernel(const AttTcProblem p, const __grid_constant__ CUtensorMap ma
         if (!ok) break;
         unsigned char* sb = stage_base + st * L::STAGE_BYTES;
         mbar_arrive_expect_tx(&sh->kv_full[st], (uint32_t)L::STAGE_BYTES);
-        const int krow = bh * p.tk + j * BK;
+        const int t0 = (first + j) * BK, krow = bh * p.tk + t0;
 #pragma unroll
         for (int kb = 0; kb < L::KB; kb++) {
           tma_load_2d(sb + L::K_HI + kb * L::K_TILE, &map_k_hi, &sh->kv_full[st], kb * 32, krow);
@@ -382,22 +421,25 @@ attention_tc_kernel(const AttTcProblem p, const __grid_constant__ CUtensorMap ma
         }
 #pragma unroll
         for (int blk = 0; blk < 2; blk++) {
-          tma_load_2d(sb + L::V_HI + blk * L::V_TILE, &map_vt_hi, &sh->kv_full[st], j * BK + blk * 32, bh * DH);
-          tma_load_2d(sb + L::V_LO + blk * L::V_TILE, &map_vt_lo, &sh->kv_full[st], j * BK + blk * 32, bh * DH);
+          tma_load_2d(sb + L::V_HI + blk * L::V_TILE, &map_vt_hi, &sh->kv_full[st], t0 + blk * 32, bh * DH);
+          tma_load_2d(sb + L::V_LO + blk * L::V_TILE, &map_vt_lo, &sh->kv_full[st], t0 + blk * 32, bh * DH);
         }
       }
     }
   } else {
     // ============================================================================ MMA issuer
-    if (elect_one()) {
+    // (where CTAs fill the GPU, one lane alone: the row threads lose more to a warp that polls than the issue loop gains)
+    const bool elected = elect_one();
+    const uint32_t leader = elected ? 1u : 0u;
+    if (kCluster || elected) {
       const uint32_t idesc_s = make_idesc(BK), idesc_o = make_idesc(DH);
       const uint32_t t_qhi = tmem_base + L::Q_HI, t_qlo = tmem_base + L::Q_LO, t_s = tmem_base + L::S,
                      t_plo = tmem_base + L::P_LO, t_o = tmem_base + L::O;
-      bool ok = mbar_wait(&sh->q_ready, 0, sh, p.status, 74);
+      ok = mbar_wait(&sh->q_ready, 0, sh, p.status, 74);
       for (int j = 0; j < nck && ok; j++) {
         const int st = j % STAGES;
-        const uint32_t ph = (uint32_t)(j & 1);
-        ok = mbar_wait(&sh->kv_full[st], (uint32_t)((j / STAGES) & 1), sh, p.status, 75);
+        const uint32_t ph = (uint32_t)(j & 1), sph = (uint32_t)((j / STAGES) & 1);
+        ok = mbar_wait(&sh->kv_full[st], sph, sh, p.status, 75);
         if (!ok) break;
         // S shares its columns with the previous chunk's P: wait until that chunk's P V has completed (its O has
         // been produced), which the o_full barrier of the previous chunk says
@@ -415,12 +457,12 @@ attention_tc_kernel(const AttTcProblem p, const __grid_constant__ CUtensorMap ma
           for (int k8 = 0; k8 < 4; k8++) {
             const uint32_t acol = (uint32_t)(kb * 32 + k8 * 8);
             const uint64_t adv = (uint64_t)(k8 * 2);
-            umma_tf32_ts(t_s, t_qlo + acol, d_hi + adv, idesc_s, (kb | k8) ? 1u : 0u);
-            umma_tf32_ts(t_s, t_qhi + acol, d_lo + adv, idesc_s, 1u);
-            umma_tf32_ts(t_s, t_qhi + acol, d_hi + adv, idesc_s, 1u);
+            umma_by<kCluster>(leader, t_s, t_qlo + acol, d_hi + adv, idesc_s, (kb | k8) ? 1u : 0u);
+            umma_by<kCluster>(leader, t_s, t_qhi + acol, d_lo + adv, idesc_s, 1u);
+            umma_by<kCluster>(leader, t_s, t_qhi + acol, d_hi + adv, idesc_s, 1u);
           }
         }
-        umma_commit(&sh->s_full);
+        commit_by(leader, &sh->s_full);
         ok = mbar_wait(&sh->p_ready, ph, sh, p.status, 77);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -432,13 +474,13 @@ attention_tc_kernel(const AttTcProblem p, const __grid_constant__ CUtensorMap ma
           for (int k8 = 0; k8 < 4; k8++) {
             const uint32_t acol = (uint32_t)(blk * 32 + k8 * 8);
             const uint64_t adv = (uint64_t)(k8 * 2);
-            umma_tf32_ts(t_o, t_plo + acol, d_hi + adv, idesc_o, (blk | k8) ? 1u : 0u);
-            umma_tf32_ts(t_o, t_s + acol, d_lo + adv, idesc_o, 1u);
-            umma_tf32_ts(t_o, t_s + acol, d_hi + adv, idesc_o, 1u);
+            umma_by<kCluster>(leader, t_o, t_plo + acol, d_hi + adv, idesc_o, (blk | k8) ? 1u : 0u);
+            umma_by<kCluster>(leader, t_o, t_s + acol, d_lo + adv, idesc_o, 1u);
+            umma_by<kCluster>(leader, t_o, t_s + acol, d_hi + adv, idesc_o, 1u);
           }
         }
-        umma_commit(&sh->kv_empty[st]);   // the stage's tiles have been read
-        umma_commit(&sh->o_full);
+        commit_by(leader, &sh->kv_empty[st]);   // the stage's tiles have been read
+        commit_by(leader, &sh->o_full);
       }
     }
   }
@@ -448,6 +490,54 @@ attention_tc_kernel(const AttTcProblem p, const __grid_constant__ CUtensorMap ma
   if (warp == 5) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(L::TMEM_COLS));
+  }
+  if (!kCluster) return;
+
+  // ============================================================================== the cluster's partial results
+  // This CTA finishes rows rank * rows ..; peer i's part of them arrives at parts[i]: [channel][row], maxima, sums.
+  const int rows = BQ / cs, set = (DH + 2) * rows;
+  float* parts = reinterpret_cast<float*>(stage_base + STAGES * L::STAGE_BYTES + PARTS_OFFSET);
+  cluster_wait();
+  if (warp < 4) {
+    const int r = threadIdx.x;
+    const uint32_t at = cluster_at(parts + rank * set + r % rows, r / rows);
+#pragma unroll
+    for (int c = 0; c < DH; c++) cluster_st(at + (uint32_t)(c * rows * 4), o[c]);
+    cluster_st(at + (uint32_t)(DH * rows * 4), m);
+    cluster_st(at + (uint32_t)((DH + 1) * rows * 4), l);
+  }
+  cluster_arrive();
+  cluster_wait();
+  if (warp < 4 && ok) {
+    // cs threads per row, DH / cs channels each
+    const int r = (int)threadIdx.x % rows, c0 = (int)threadIdx.x / rows * (DH / cs);
+    const float* mine = parts + r;
+    float wp[8], top = -INFINITY, total = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      wp[i] = i < cs ? mine[i * set + DH * rows] : -INFINITY;
+      top = fmaxf(top, wp[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      if (i < cs) {
+        wp[i] = exp2f(wp[i] - top);
+        total = fmaf(mine[i * set + (DH + 1) * rows], wp[i], total);
+      }
+    }
+    const float inv = 1.f / total;
+    const int qrow = q0 + rank * rows + r;
+    float* yp = p.y + (int64_t)b * p.y_sb + (int64_t)h * p.y_sh + (int64_t)qrow * p.y_st;
+    for (int c = c0; c < c0 + DH / cs; c += 4) {
+      float out[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int i = 0; i < 8; i++)
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+          if (i < cs) out[e] = fmaf(mine[i * set + (c + e) * rows], wp[i], out[e]);
+      if (qrow < p.tq)
+        *reinterpret_cast<float4*>(yp + c) = make_float4(out[0] * inv, out[1] * inv, out[2] * inv, out[3] * inv);
+    }
   }
 }
 
@@ -482,16 +572,37 @@ bool encode_2d(CUtensorMap* map, const float* base, int64_t rows, int64_t cols, 
                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// CTAs per query tile.  In units of a chunk's time (about 1.7 us), a CTA costs 1.5 and its chunks, a cluster CLUSTER for
+// its barriers and the exchange; CTAs run in rounds of as many as the GPU holds.  Measured, us per call with the pre-pass,
+// 8 heads of 32 (one CTA -> what this chooses): 625 x 625 at batch 1 27.1 -> 21.4 (4 CTAs), 100 x 625 at batch 1 26.7 ->
+// 16.4 (8), at batch 8 32.6 -> 25.2 (4); two chunks lose to a cluster (13.9 -> 15.5).
+constexpr double CLUSTER = 2.0;
+int choose_cluster(const wdc_context* ctx, int64_t tiles, int64_t tk, int per_sm) {
+  const int64_t chunks = ceil_div64(tk, BK), slots = (int64_t)ctx->sm_count * per_sm;
+  int best = 1;
+  double best_t = 1e300;
+  for (int cs = 1; cs <= 8 && cs <= chunks; cs *= 2) {
+    const double t = (double)ceil_div64(tiles * cs, slots) * ((double)ceil_div64(chunks, cs) + (cs > 1 ? 1.5 + CLUSTER : 1.5));
+    if (t < best_t - 1e-9) {
+      best_t = t;
+      best = cs;
+    }
+  }
+  return best;
+}
+
 template <int DH>
 int launch(wdc_context* ctx, const wdc_attention_desc* d, const float* q, const float* k, const float* v, float* y) {
   using L = AttLayout<DH>;
   const int64_t bh = d->batch * d->heads;
   const int tk = (int)d->tk, tkp = (tk + 3) & ~3;
   static bool attr_set[64] = {};
-  const int smem = STAGES * L::STAGE_BYTES + (int)sizeof(AttShared) + 1024;
+  const int smem = STAGES * L::STAGE_BYTES + PARTS_OFFSET + L::PARTS + 1024;
   if (ctx->device < 0 || ctx->device >= 64) return WDC_ERR_UNSUPPORTED;
   if (!attr_set[ctx->device]) {
-    if (cudaFuncSetAttribute(attention_tc_kernel<DH>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
+    const cudaFuncAttribute what = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    if (cudaFuncSetAttribute(attention_tc_kernel<DH, false>, what, smem - L::PARTS) != cudaSuccess ||
+        cudaFuncSetAttribute(attention_tc_kernel<DH, true>, what, smem) != cudaSuccess) {
       cudaGetLastError();
       return WDC_ERR_UNSUPPORTED;
     }
@@ -520,18 +631,30 @@ int launch(wdc_context* ctx, const wdc_attention_desc* d, const float* q, const 
     p.heads = (int)d->heads; p.tq = (int)d->tq; p.tk = tk;
     p.scale_log2 = d->scale * 1.4426950408889634f;
     p.status = ctx->status_word;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    p.cs = choose_cluster(ctx, ceil_div64(d->tq, BQ) * bh, tk, DH == 32 ? 2 : 1);
+    cudaLaunchAttribute attr[2];
+    int n_attr = 0;
+    if (p.cs > 1) {
+      attr[n_attr].id = cudaLaunchAttributeClusterDimension;
+      attr[n_attr].val.clusterDim.x = (unsigned)p.cs;
+      attr[n_attr].val.clusterDim.y = attr[n_attr].val.clusterDim.z = 1;
+      n_attr++;
+    }
+    if (ctx->opt_pdl) {
+      attr[n_attr].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr[n_attr].val.programmaticStreamSerializationAllowed = 1;
+      n_attr++;
+    }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)((d->tq + BQ - 1) / BQ), (unsigned)bh);
+    cfg.gridDim = dim3((unsigned)(ceil_div64(d->tq, BQ) * p.cs), (unsigned)bh);
     cfg.blockDim = dim3(ATT_THREADS);
-    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.dynamicSmemBytes = (size_t)(p.cs > 1 ? smem : smem - L::PARTS);
     cfg.stream = ctx->stream;
     cfg.attrs = attr;
-    cfg.numAttrs = ctx->opt_pdl ? 1 : 0;
+    cfg.numAttrs = (unsigned)n_attr;
     const AttTcProblem& pc = p;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, attention_tc_kernel<DH>, pc, m_k_hi, m_k_lo, m_vt_hi, m_vt_lo);
+    cudaError_t e = p.cs > 1 ? cudaLaunchKernelEx(&cfg, attention_tc_kernel<DH, true>, pc, m_k_hi, m_k_lo, m_vt_hi, m_vt_lo)
+                             : cudaLaunchKernelEx(&cfg, attention_tc_kernel<DH, false>, pc, m_k_hi, m_k_lo, m_vt_hi, m_vt_lo);
     ctx->n_launch++;
     ctx->n_tc_launch++;
     s = wdc_check_cuda(ctx, e, "attention_tc_kernel");
