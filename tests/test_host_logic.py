@@ -283,3 +283,30 @@ def test_bench_reference_arm_prints_the_contract_line():
     assert d["cpu_baseline"]["kind"] == "port" and d["cpu_baseline"]["cores"] >= 1 and d["cpu_baseline"]["value"] == d["value"]
     assert d["e2e"] == {"value": d["value"], "unit": "images/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0}
     assert "workload" in d["config"]
+
+
+def test_projections_of_one_tensor_for_attention_lie_side_by_side():
+    dec = 3
+    m = zoo.detr(batch=2, size=64, d=64, heads=2, enc_layers=1, dec_layers=dec, ffn=64, queries=5, classes=7, width=8,
+                 blocks=(1, 1, 1, 1))
+    model_transform(m, ["cuda", "cpu"])
+    shapes = {t.name: t.dims for t in m.graph.initializer}
+    wide = {n.output[0]: shapes[n.input[1]][1] for n in m.graph.node
+            if n.op_type == "CudaMatMulBias" and n.name.endswith("__cuda_side_by_side")}
+    # q and k of every self-attention; k, and v, of all the decoder's attentions over the encoder's result
+    assert sorted(wide.values()) == [128] * (1 + dec) + [64 * dec] * 2
+    seen = []
+    for n in m.graph.node:
+        if n.op_type == "CudaAttention":
+            att = {a.name: a.i for a in n.attribute}
+            for i, key in enumerate(("q", "k", "v")):
+                if n.input[i] in wide:
+                    assert att[key + "_width"] == wide[n.input[i]]
+                    seen.append((n.input[i], att[key + "_column"]))
+                else:
+                    assert key + "_width" not in att
+    assert len(seen) == len(set(seen)) == 2 * (1 + dec) + 2 * dec
+    known = {vi.name for vi in m.graph.input} | set(shapes)
+    for n in m.graph.node:
+        assert all(i in known for i in n.input), (n.op_type, n.name)
+        known.update(n.output)

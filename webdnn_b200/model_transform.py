@@ -17,6 +17,8 @@ unchanged:
   axis -> ``MatMul``(., v) on rank-3 tensors -> ``CudaAttention``; the head split in front of q, k, v
   (``Reshape`` [b, t, h, c] -> ``Transpose`` 0,2,1,3 -> ``Reshape`` [b*h, t, c]) and the head merge behind the
   result are absorbed as strides when their shapes are constants.
+* several ``CudaMatMulBias`` nodes that project one tensor for such attention nodes (q and k of a layer, the k or v of
+  all decoder layers) -> one with their weights side by side; the attention reads its columns.
 
 The private op types are registered like a custom operator (``example/custom_operator/twice.ts``),
 the same way the offline WebGL passes rename ``op_type`` to ``ConvReshapeWebGL`` / ``MatMulNT141``.
@@ -412,7 +414,75 @@ def _fuse_cuda(model: Model) -> None:
     g.initializer = [t for t in g.initializer if t.name in used]
 
 
+def _merge_projections(model: Model) -> None:
+    """Linear layers of one tensor whose results only attention nodes read become one linear layer.
+
+    A projection of 625 rows to 256 columns is a launch of 20 tiles, mostly latency: two cost twice one.  Side by side
+    they are one launch that fills the GPU better; the columns keep their own sums, so results do not change."""
+    g = model.graph
+    if model.metadata_props.get("WebDNN2.WeightPaths"):
+        return   # weights outside the graph may still be on their way
+    inits = {t.name: t for t in g.initializer}
+    graph_outputs = {vi.name for vi in g.output}
+    readers: Dict[str, List[Node]] = {}
+    for n in g.node:
+        for i in n.input:
+            readers.setdefault(i, []).append(n)
+
+    def mergeable(n: Node) -> bool:
+        attrs = {a.name: a.i for a in n.attribute}
+        if n.op_type != "CudaMatMulBias" or attrs["relu"] or attrs["has_residual"] or len(n.input) != 3:
+            return False
+        w, b, out = inits.get(n.input[1]), inits.get(n.input[2]), n.output[0]
+        if w is None or b is None or w.data_type != FLOAT or b.data_type != FLOAT or w.dims[1] % 4 or out in graph_outputs:
+            return False
+        users = readers.get(out, [])
+        return bool(users) and all(u.op_type == "CudaAttention" and
+                                   {a.name: a.i for a in u.attribute}["heads"] > 0 for u in users)
+
+    groups: Dict[str, List[Node]] = {}
+    for n in g.node:
+        if mergeable(n):
+            groups.setdefault(n.input[0], []).append(n)
+    place: Dict[str, tuple] = {}   # old result -> (merged result, first column, columns of the merged result)
+    replace_at: Dict[int, Node] = {}
+    removed = set()
+    for x, nodes in groups.items():
+        if len(nodes) < 2:
+            continue
+        ws = [np.asarray(inits[n.input[1]].array).reshape(inits[n.input[1]].dims) for n in nodes]
+        bs = [np.asarray(inits[n.input[2]].array).reshape(-1) for n in nodes]
+        base = f"{nodes[0].name or nodes[0].output[0]}__cuda_side_by_side"
+        g.initializer.append(make_tensor(base + "_w", np.ascontiguousarray(np.concatenate(ws, axis=1), np.float32)))
+        g.initializer.append(make_tensor(base + "_b", np.ascontiguousarray(np.concatenate(bs), np.float32)))
+        width = sum(w.shape[1] for w in ws)
+        col = 0
+        for n, w in zip(nodes, ws):
+            place[n.output[0]] = (base, col, width)
+            col += w.shape[1]
+            removed.add(id(n))
+        replace_at[id(nodes[0])] = Node("CudaMatMulBias", [x, base + "_w", base + "_b"], [base], base,
+                                        [make_attr("relu", 0), make_attr("has_residual", 0)])
+    if not place:
+        return
+    new_nodes = []
+    for n in g.node:
+        if id(n) in replace_at:
+            new_nodes.append(replace_at[id(n)])
+        elif id(n) not in removed:
+            if n.op_type == "CudaAttention":
+                for i, key in enumerate(("q", "k", "v")):
+                    if n.input[i] in place:
+                        n.input[i], first, width = place[n.input[i]]
+                        n.attribute += [make_attr(f"{key}_column", first), make_attr(f"{key}_width", width)]
+            new_nodes.append(n)
+    g.node = new_nodes
+    used = {i for n in g.node for i in n.input} | graph_outputs
+    g.initializer = [t for t in g.initializer if t.name in used]
+
+
 def model_transform(model: Model, backend_order) -> None:
     if "cuda" in backend_order:
         _fuse_cuda(model)
+        _merge_projections(model)
     rename_duplicated_node(model)

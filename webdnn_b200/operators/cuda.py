@@ -282,7 +282,8 @@ class CudaAttention(OperatorImpl):
 
     Inputs are either rank-3 [batch*heads, tokens, c] tensors (``heads`` attribute 0), or the tensors
     in front of the head split, [batch, tokens, heads*c] in memory, read through strides.  With
-    ``merge_heads`` the result is written as [batch, tq, heads*c], else as [batch*heads, tq, c]."""
+    ``merge_heads`` the result is written as [batch, tq, heads*c], else as [batch*heads, tq, c].  An operand with a
+    ``width`` attribute is columns ``column`` .. of a tensor with rows of that many."""
 
     def __init__(self):
         super().__init__("cuda")
@@ -293,6 +294,8 @@ class CudaAttention(OperatorImpl):
         self.heads = get_attr_int(attribute, "heads", 0)
         self.head_size = get_attr_int(attribute, "head_size", 0)
         self.merge = get_attr_int(attribute, "merge_heads", 0) != 0
+        self.columns = [(get_attr_int(attribute, f"{key}_column", 0), get_attr_int(attribute, f"{key}_width", 0))
+                        for key in ("q", "k", "v")]
 
     def run(self, context, inputs, n_outputs):
         context.asserts_cuda_tensor_array(inputs)
@@ -301,15 +304,14 @@ class CudaAttention(OperatorImpl):
         if any(t.data_type != "float32" for t in (q, k, v)):
             raise TypeError("only float32 is supported")
         if self.heads:
-            b, h = self.batch, self.heads
-            if k.length != v.length:
+            b, h, c = self.batch, self.heads, self.head_size
+            width = [w or h * c for _, w in self.columns]
+            if c <= 0 or any(t.length % (b * w) for t, w in zip((q, k, v), width)):
                 raise ValueError("CudaAttention: operand sizes do not match the head split")
-            c = self.head_size
-            if c <= 0 or q.length % (b * h * c) or k.length % (b * h * c):
+            tq, tk, tv = (t.length // (b * w) for t, w in zip((q, k, v), width))
+            if tk != tv:
                 raise ValueError("CudaAttention: operand sizes do not match the head split")
-            tq, tk = q.length // (b * h * c), k.length // (b * h * c)
-            sq = (tq * h * c, c, h * c)
-            sk = (tk * h * c, c, h * c)
+            sq, sk, sv = ((t * w, c, w) for t, w in zip((tq, tk, tk), width))
         else:
             if q.ndim != 3 or k.ndim != 3 or v.ndim != 3:
                 raise ValueError("CudaAttention: operands must have rank 3")
@@ -319,7 +321,7 @@ class CudaAttention(OperatorImpl):
             if k.dims != [b, tk, c] or v.dims != [b, tk, c]:
                 raise ValueError("CudaAttention: operand shapes do not match")
             sq = (tq * c, 0, c)
-            sk = (tk * c, 0, c)
+            sk = sv = (tk * c, 0, c)
         if self.merge:
             y = context.empty_tensor([b, tq, h * c], "float32")
             sy = (tq * h * c, c, h * c)
@@ -330,9 +332,10 @@ class CudaAttention(OperatorImpl):
             if c in (32, 64):
                 d = AttentionDesc(batch=b, heads=h, tq=tq, tk=tk, dh=c,
                                   q_sb=sq[0], q_sh=sq[1], q_st=sq[2], k_sb=sk[0], k_sh=sk[1], k_st=sk[2],
-                                  v_sb=sk[0], v_sh=sk[1], v_st=sk[2], y_sb=sy[0], y_sh=sy[1], y_st=sy[2],
+                                  v_sb=sv[0], v_sh=sv[1], v_st=sv[2], y_sb=sy[0], y_sh=sy[1], y_st=sy[2],
                                   scale=self.scale)
-                context._call("wdc_attention", byref(d), _p(q), _p(k), _p(v), _p(y))
+                at = [c_void_p(t.ptr + 4 * first) for t, (first, _) in zip((q, k, v), self.columns)]
+                context._call("wdc_attention", byref(d), *at, _p(y))
             elif self.heads:
                 raise ValueError("CudaAttention: a head split is only absorbed for head sizes 32 and 64")
             else:
