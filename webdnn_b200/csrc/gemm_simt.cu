@@ -1,6 +1,6 @@
 // CUDA-core fp32 contraction kernel: strided/batched GEMM and implicit-GEMM convolution with the
-// fused epilogues.  It is the path for shapes the tcgen05 kernel does not take (grouped or dilated
-// convolutions, channel counts that are not a multiple of 32, tiny or oddly strided matrices).
+// fused epilogues.  It is the path for what the other contraction kernels do not take: grouped convolutions, channel
+// counts that are not a multiple of 4, and a Gemm that accumulates into its output.
 // 64x64 output tile per CTA, K step 16, 256 threads, 4x4 accumulators per thread, fp32 FMA.
 #include "tape.cuh"
 

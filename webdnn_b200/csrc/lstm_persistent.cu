@@ -1,4 +1,5 @@
-// ONNX LSTM recurrence (forward, default activations, gate order i,o,f,c) as ONE persistent kernel.
+// ONNX LSTM recurrence (forward, default activations, gate order i,o,f,c) as ONE persistent kernel, for the shapes that
+// lstm_cluster.cu leaves.
 //
 // The input projection P[T, B, 4H] = X * W^T of all steps is a tensor-core GEMM done beforehand; what
 // is left is the serial part: for t = 0..T-1, G = h_{t-1} * R^T + P_t, gates, c_t, h_t.  Launched per
