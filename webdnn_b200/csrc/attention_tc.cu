@@ -212,7 +212,7 @@ __device__ __forceinline__ float low_part(float x) { return x - __uint_as_float(
 // K [.., tk, dh] (strided) -> k_hi, k_lo [bh, tk, dh];  V -> vt_hi, vt_lo [bh, dh, tkp] (transposed, zero for
 // keys tk .. tkp-1).  One CTA per (head, 32 keys).
 template <int DH>
-__global__ void __launch_bounds__(256) attn_split_kv_kernel(const float* __restrict__ k, const float* __restrict__ v,
+__global__ void __launch_bounds__(256) attn_split_kv_kernel(const float* k, const float* v,
                                                             float* __restrict__ k_hi, float* __restrict__ k_lo,
                                                             float* __restrict__ vt_hi, float* __restrict__ vt_lo,
                                                             int heads, int tk, int tkp, int64_t k_sb, int64_t k_sh,
@@ -330,7 +330,7 @@ attention_tc_kernel(const AttTcProblem p, const __grid_constant__ CUtensorMap ma
 #pragma unroll
         for (int j = 0; j < 16; j += 4) {
           float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (qrow < p.tq) x = __ldg(reinterpret_cast<const float4*>(qp + c0 + j));
+          if (qrow < p.tq) x = pdl_ld(reinterpret_cast<const float4*>(qp + c0 + j));
           hi[j] = x.x; hi[j + 1] = x.y; hi[j + 2] = x.z; hi[j + 3] = x.w;
           lo[j] = low_part(x.x); lo[j + 1] = low_part(x.y); lo[j + 2] = low_part(x.z); lo[j + 3] = low_part(x.w);
         }

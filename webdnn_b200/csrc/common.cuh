@@ -128,7 +128,8 @@ struct DeviceGuard {
 
 // Programmatic dependent launch.  A kernel launched with wdc_launch_pdl may start while the grids before it finish: its
 // first statement is pdl_wait(), behind which everything they wrote is visible, and which also lets the next grid start.
-// Pointers that a kernel declares read-only go through pdl_after(), or the compiler might load ahead of the wait.
+// Such a kernel reads what earlier grids may have written with pdl_ld, an ordinary load that stays behind the wait: the
+// read-only path (__ldg) is for memory that nobody writes while the kernel is there, and it is there before the wait.
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
@@ -141,6 +142,32 @@ __device__ __forceinline__ T* pdl_after(T* p) {
   size_t g = __cvta_generic_to_global(p);
   asm volatile("" : "+l"(g)::"memory");
   return (T*)__cvta_global_to_generic(g);
+}
+__device__ __forceinline__ float pdl_ld(const float* p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint32_t pdl_ld(const uint32_t* p) {
+  uint32_t v;
+  asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ int32_t pdl_ld(const int32_t* p) { return (int32_t)pdl_ld((const uint32_t*)p); }
+__device__ __forceinline__ uint8_t pdl_ld(const uint8_t* p) {
+  uint32_t v;
+  asm volatile("ld.global.u8 %0, [%1];" : "=r"(v) : "l"(p));
+  return (uint8_t)v;
+}
+__device__ __forceinline__ float4 pdl_ld(const float4* p) {
+  float4 v;
+  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint4 pdl_ld(const uint4* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
 }
 template <class... P, class... A>
 void wdc_launch_pdl(wdc_context* ctx, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A... args) {

@@ -777,7 +777,7 @@ tc_igemm_kernel(const __grid_constant__ TcProblem p, const float* __restrict__ x
           const int ix = rix + j * p.dil_w;
           float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
           if (rowok && j < e.nchunks && (unsigned)ix < (unsigned)p.in_w)
-            v = __ldg(reinterpret_cast<const float4*>(src + j * p.dil_w * 4));
+            v = pdl_ld(reinterpret_cast<const float4*>(src + j * p.dil_w * 4));
           dst[j] = v;
         }
       } else {
@@ -785,12 +785,12 @@ tc_igemm_kernel(const __grid_constant__ TcProblem p, const float* __restrict__ x
         const bool ok2 = rowok && (unsigned)ix < (unsigned)p.in_w;
         if (ok2 && e.nchunks == 8) {
 #pragma unroll
-          for (int j = 0; j < 8; j++) dst[j] = __ldg(reinterpret_cast<const float4*>(src) + j);
+          for (int j = 0; j < 8; j++) dst[j] = pdl_ld(reinterpret_cast<const float4*>(src) + j);
         } else {
 #pragma unroll
           for (int j = 0; j < 8; j++) {
             float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (ok2 && j < e.nchunks) v = __ldg(reinterpret_cast<const float4*>(src) + j);
+            if (ok2 && j < e.nchunks) v = pdl_ld(reinterpret_cast<const float4*>(src) + j);
             dst[j] = v;
           }
         }
@@ -982,7 +982,7 @@ tc_igemm_kernel(const __grid_constant__ TcProblem p, const float* __restrict__ x
       // table and meet at a barrier of their own (id 1, 256 threads), so the producers are not held up
       const int used = p.tiles_n * p.tile_n + 64;
       for (int i = threadIdx.x - EPI_WARP0 * 32; i < used; i += n_epi * 32)
-        ss->shift_tab[i] = (p.shift && i < p.N) ? p.shift_mul * __ldg(p.shift + i) : 0.f;
+        ss->shift_tab[i] = (p.shift && i < p.N) ? p.shift_mul * pdl_ld(p.shift + i) : 0.f;
       asm volatile("bar.sync 1, %0;" ::"r"(n_epi * 32) : "memory");
     }
     if (p.tma_epi) {
@@ -1052,7 +1052,7 @@ tc_igemm_kernel(const __grid_constant__ TcProblem p, const float* __restrict__ x
           for (int j = 0; j < 64; j += 4) {
             float4 b4 = make_float4(0.f, 0.f, 0.f, 0.f);
             if (p.shift && j < ncols && nbase + j < p.N) {
-              b4 = __ldg(reinterpret_cast<const float4*>(p.shift + nbase + j));
+              b4 = pdl_ld(reinterpret_cast<const float4*>(p.shift + nbase + j));
               b4.x *= p.shift_mul; b4.y *= p.shift_mul; b4.z *= p.shift_mul; b4.w *= p.shift_mul;
             }
             acc[j] = b4.x;
@@ -1178,12 +1178,12 @@ tc_igemm_kernel(const __grid_constant__ TcProblem p, const float* __restrict__ x
           float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
           if (p.residual && !TC_DBG(p, 2) && m < p.M && col < p.N) {
             const float* rp = p.residual + m * p.res_stride + col;
-            if (vec) r = __ldg(reinterpret_cast<const float4*>(rp));
+            if (vec) r = pdl_ld(reinterpret_cast<const float4*>(rp));
             else {
-              r.x = __ldg(rp);
-              if (col + 1 < p.N) r.y = __ldg(rp + 1);
-              if (col + 2 < p.N) r.z = __ldg(rp + 2);
-              if (col + 3 < p.N) r.w = __ldg(rp + 3);
+              r.x = pdl_ld(rp);
+              if (col + 1 < p.N) r.y = pdl_ld(rp + 1);
+              if (col + 2 < p.N) r.z = pdl_ld(rp + 2);
+              if (col + 3 < p.N) r.w = pdl_ld(rp + 3);
             }
           }
           dst[i] = r;
@@ -1239,8 +1239,8 @@ tc_igemm_kernel(const __grid_constant__ TcProblem p, const float* __restrict__ x
 #pragma unroll
             for (int e = 0; e < 4; e++) {
               if (col + e < p.N) {
-                if (p.scale) sc[e] = __ldg(p.scale + col + e);
-                if (p.shift) sh[e] = p.shift_mul * __ldg(p.shift + col + e);
+                if (p.scale) sc[e] = pdl_ld(p.scale + col + e);
+                if (p.shift) sh[e] = p.shift_mul * pdl_ld(p.shift + col + e);
               }
             }
 #pragma unroll
@@ -1334,9 +1334,9 @@ __global__ void __launch_bounds__(256) split_tf32_transpose_kernel(const float* 
 // Second pass for the tiles whose reduction was cut into ranges: for tile `full_tiles + r`, block (r * splits + s)
 // of the workspace holds the raw partial sums of range s as 128 rows x tile_n columns.  The ranges are added in
 // ascending order (deterministic), then shift, residual and Relu are applied as in the fused epilogue.  N % 4 == 0.
-__global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restrict__ ws, float* __restrict__ y,
-                                                            const float* __restrict__ shift, float shift_mul,
-                                                            const float* __restrict__ residual, int64_t res_stride,
+__global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* ws, float* __restrict__ y,
+                                                            const float* shift, float shift_mul,
+                                                            const float* residual, int64_t res_stride,
                                                             float res_mul, int relu, int64_t M, int N, int tile_n,
                                                             int tiles_n, int full_tiles, int rest_tiles, int splits) {
   pdl_grid_wait();   // launched as a programmatic dependent of the contraction kernel
@@ -1354,7 +1354,7 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restr
     if (m >= M || n >= N) continue;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     if (shift) {
-      const float4 b = __ldg(reinterpret_cast<const float4*>(shift + n));
+      const float4 b = pdl_ld(reinterpret_cast<const float4*>(shift + n));
       acc = make_float4(shift_mul * b.x, shift_mul * b.y, shift_mul * b.z, shift_mul * b.w);
     }
     const float* src = ws + (((int64_t)r * splits) * TILE_M + row) * tile_n + c4 * 4;
@@ -1369,7 +1369,7 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restr
       if (s < splits) { acc.x += v[s].x; acc.y += v[s].y; acc.z += v[s].z; acc.w += v[s].w; }
     }
     if (residual) {
-      const float4 rr = __ldg(reinterpret_cast<const float4*>(residual + m * res_stride + n));
+      const float4 rr = pdl_ld(reinterpret_cast<const float4*>(residual + m * res_stride + n));
       acc.x = fmaf(res_mul, rr.x, acc.x); acc.y = fmaf(res_mul, rr.y, acc.y);
       acc.z = fmaf(res_mul, rr.z, acc.z); acc.w = fmaf(res_mul, rr.w, acc.w);
     }
@@ -1382,7 +1382,7 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restr
 
 // Stem mode operand preparation: 4 channels per pixel, 8 taps per filter row.
 // `plane` = 0: x is NHWC (a pixel's channels are adjacent); > 0: x is NCHW with `plane` pixels per channel plane.
-__global__ void pad_channels4_kernel(const float* __restrict__ x, float* __restrict__ x4, int64_t pixels, int cin,
+__global__ void pad_channels4_kernel(const float* x, float* __restrict__ x4, int64_t pixels, int cin,
                                      int64_t plane) {
   pdl_wait();
   x = pdl_after(x);
@@ -1392,17 +1392,17 @@ __global__ void pad_channels4_kernel(const float* __restrict__ x, float* __restr
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     const float* s = plane ? x + (i / plane) * plane * cin + i % plane : x + i * cin;
     const int64_t cs = plane ? plane : 1;
-    v.x = __ldg(s);
-    if (cin > 1) v.y = __ldg(s + cs);
-    if (cin > 2) v.z = __ldg(s + 2 * cs);
-    if (cin > 3) v.w = __ldg(s + 3 * cs);
+    v.x = pdl_ld(s);
+    if (cin > 1) v.y = pdl_ld(s + cs);
+    if (cin > 2) v.z = pdl_ld(s + 2 * cs);
+    if (cin > 3) v.w = pdl_ld(s + 3 * cs);
     reinterpret_cast<float4*>(x4)[i] = v;
   }
 }
 // Same with every image row shifted right by pad_l pixels into a zero-filled row of wp pixels: pixel pair
 // (2j, 2j+1) of the padded row is then the pair of taps (2j, 2j+1) of output column j for stride 2.
 // With hp > h the images are padded vertically too: pad_t zero rows above, hp - pad_t - h below.
-__global__ void pad_channels4_rows_kernel(const float* __restrict__ x, float* __restrict__ x4, int64_t images, int h,
+__global__ void pad_channels4_rows_kernel(const float* x, float* __restrict__ x4, int64_t images, int h,
                                           int hp, int pad_t, int w, int wp, int pad_l, int cin, int nchw) {
   pdl_wait();
   x = pdl_after(x);
@@ -1420,10 +1420,10 @@ __global__ void pad_channels4_rows_kernel(const float* __restrict__ x, float* __
       const int64_t plane = (int64_t)h * w;
       const float* s = nchw ? x + img * plane * cin + (int64_t)yy * w + px : x + ((img * h + yy) * w + px) * cin;
       const int64_t cs = nchw ? plane : 1;
-      v.x = __ldg(s);
-      if (cin > 1) v.y = __ldg(s + cs);
-      if (cin > 2) v.z = __ldg(s + 2 * cs);
-      if (cin > 3) v.w = __ldg(s + 3 * cs);
+      v.x = pdl_ld(s);
+      if (cin > 1) v.y = pdl_ld(s + cs);
+      if (cin > 2) v.z = pdl_ld(s + 2 * cs);
+      if (cin > 3) v.w = pdl_ld(s + 3 * cs);
     }
     reinterpret_cast<float4*>(x4)[i] = v;
   }

@@ -414,11 +414,11 @@ tc_small_kernel(const __grid_constant__ TcProblem p, const __grid_constant__ CUt
       out[i] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (live[i]) {
         if (p.shift) {
-          const float4 b = __ldg(reinterpret_cast<const float4*>(p.shift + n));
+          const float4 b = pdl_ld(reinterpret_cast<const float4*>(p.shift + n));
           out[i] = make_float4(p.shift_mul * b.x, p.shift_mul * b.y, p.shift_mul * b.z, p.shift_mul * b.w);
         }
         if (p.residual) {
-          const float4 x = __ldg(reinterpret_cast<const float4*>(p.residual + m * p.res_stride + n));
+          const float4 x = pdl_ld(reinterpret_cast<const float4*>(p.residual + m * p.res_stride + n));
           out[i].x = fmaf(p.res_mul, x.x, out[i].x);
           out[i].y = fmaf(p.res_mul, x.y, out[i].y);
           out[i].z = fmaf(p.res_mul, x.z, out[i].z);

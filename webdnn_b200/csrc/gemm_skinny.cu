@@ -32,7 +32,7 @@ struct SkinnyArgs {
 
 __device__ __forceinline__ void store_out(const SkinnyArgs& a, int64_t bz, int64_t m, int64_t n, float v) {
   v *= a.alpha;
-  if (a.C) v += __ldg(pdl_after(a.C) + m * a.sc0 + n * a.sc1) * a.beta;
+  if (a.C) v += pdl_ld(pdl_after(a.C) + m * a.sc0 + n * a.sc1) * a.beta;
   if (a.relu) v = v > 0.f ? v : (v == v ? 0.f : v);
   a.Y[(bz * a.m + m) * a.n + n] = v;
 }
@@ -87,10 +87,10 @@ __global__ void __launch_bounds__(ROW_WARPS * 32) skinny_rows_kernel(const Skinn
     if (VEC == 4) {
       float4 w[NC];
 #pragma unroll
-      for (int c = 0; c < NC; c++) w[c] = __ldg(reinterpret_cast<const float4*>(bp[c] + k));
+      for (int c = 0; c < NC; c++) w[c] = pdl_ld(reinterpret_cast<const float4*>(bp[c] + k));
 #pragma unroll
       for (int r = 0; r < MT; r++) {
-        const float4 x = __ldg(reinterpret_cast<const float4*>(ap[r] + k));
+        const float4 x = pdl_ld(reinterpret_cast<const float4*>(ap[r] + k));
 #pragma unroll
         for (int c = 0; c < NC; c++) {
           float& s = acc[r * NC + c];
@@ -103,10 +103,10 @@ __global__ void __launch_bounds__(ROW_WARPS * 32) skinny_rows_kernel(const Skinn
     } else {
       float w[NC];
 #pragma unroll
-      for (int c = 0; c < NC; c++) w[c] = __ldg(bp[c] + k);
+      for (int c = 0; c < NC; c++) w[c] = pdl_ld(bp[c] + k);
 #pragma unroll
       for (int r = 0; r < MT; r++) {
-        const float x = __ldg(ap[r] + k * a.sa1);
+        const float x = pdl_ld(ap[r] + k * a.sa1);
 #pragma unroll
         for (int c = 0; c < NC; c++) acc[r * NC + c] = fmaf(x, w[c], acc[r * NC + c]);
       }
@@ -143,13 +143,13 @@ __global__ void __launch_bounds__(COL_WARPS * 32) skinny_cols_kernel(const Skinn
 #pragma unroll
     for (int j = 0; j < COL_UNROLL; j++) {
       const int64_t k = k0 + j * COL_WARPS;
-      w[j] = k < a.k ? __ldg(bp + k * a.sb) : 0.f;
+      w[j] = k < a.k ? pdl_ld(bp + k * a.sb) : 0.f;
     }
     // lane j of the warp fetches A[r][k0 + 16 j]: one load per row, handed round by shuffles
 #pragma unroll
     for (int r = 0; r < MT; r++) {
       const int64_t k = k0 + (lane % COL_UNROLL) * COL_WARPS;
-      const float x = (r < rows && k < a.k) ? __ldg(A + r * a.sa0 + k * a.sa1) : 0.f;
+      const float x = (r < rows && k < a.k) ? pdl_ld(A + r * a.sa0 + k * a.sa1) : 0.f;
 #pragma unroll
       for (int j = 0; j < COL_UNROLL; j++)
         if (k0 + j * COL_WARPS < a.k) acc[r] = fmaf(__shfl_sync(0xffffffffu, x, j), w[j], acc[r]);

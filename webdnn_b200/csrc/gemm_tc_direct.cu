@@ -131,7 +131,7 @@ __device__ __forceinline__ void load_block(float* v, const float* base, int64_t 
 #pragma unroll
       for (int i = 0; i < ROWS / 32; i++) {
         if ((tid >> 3) + 32 * i < rows) {
-          const float4 q = __ldg(reinterpret_cast<const float4*>(p));
+          const float4 q = pdl_ld(reinterpret_cast<const float4*>(p));
           v[4 * i] = q.x; v[4 * i + 1] = q.y; v[4 * i + 2] = q.z; v[4 * i + 3] = q.w;
         }
         p += 32 * s_row;
@@ -143,7 +143,7 @@ __device__ __forceinline__ void load_block(float* v, const float* base, int64_t 
     if (k < klen) {
 #pragma unroll
       for (int i = 0; i < ROWS / 8; i++) {
-        if (warp + 8 * i < rows) v[i] = __ldg(p);
+        if (warp + 8 * i < rows) v[i] = pdl_ld(p);
         p += 8 * s_row;
       }
     }
@@ -155,7 +155,7 @@ __device__ __forceinline__ void load_block(float* v, const float* base, int64_t 
       if (k + t < klen) {
 #pragma unroll
         for (int i = 0; i < ROWS / 32; i++)
-          if (lane + 32 * i < rows) v[4 * i + t] = __ldg(p + 32 * i);
+          if (lane + 32 * i < rows) v[4 * i + t] = pdl_ld(p + 32 * i);
       }
       p += s_k;
     }
@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(THREADS, kLong && TN == 128 ? 1 : 2) gemm_tc_d
       if (r < a.m && col0 + c < a.n) {
         const float* pa = A + (int64_t)(r - m0) * a.sa_row;
         const float* pb = B + (int64_t)(col0 - n0 + c) * a.sb_row;
-        for (int k = 0; k < a.k; k++) s = fmaf(__ldg(pa + (int64_t)k * a.sa_k), __ldg(pb + (int64_t)k * a.sb_k), s);
+        for (int k = 0; k < a.k; k++) s = fmaf(pdl_ld(pa + (int64_t)k * a.sa_k), pdl_ld(pb + (int64_t)k * a.sb_k), s);
       }
       stg[lane * (COLS + 1) + c] = s;
     }
@@ -333,7 +333,7 @@ __global__ void __launch_bounds__(THREADS, kLong && TN == 128 ? 1 : 2) gemm_tc_d
       for (int c = lane; c < COLS; c += 32) {
         if (col0 + c < a.n) {
           float v = stg[r * (COLS + 1) + c] * a.alpha;
-          if (C) v += __ldg(C + (int64_t)(row0 + r) * a.sc0 + (int64_t)(col0 + c) * a.sc1) * a.beta;
+          if (C) v += pdl_ld(C + (int64_t)(row0 + r) * a.sc0 + (int64_t)(col0 + c) * a.sc1) * a.beta;
           if (a.relu) v = v > 0.f ? v : (v == v ? 0.f : v);
           Y[(int64_t)(row0 + r) * a.n + col0 + c] = v;
         }

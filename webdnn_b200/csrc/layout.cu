@@ -12,7 +12,7 @@ struct CopyShape {
 // division where the element count allows it (a 64-bit division per axis and element made a head split run at 43%
 // of the HBM copy rate).
 template <typename T, int M, typename I>
-__global__ void __launch_bounds__(256) strided_copy_kernel(const T* __restrict__ src, T* __restrict__ dst, int64_t n,
+__global__ void __launch_bounds__(256) strided_copy_kernel(const T* src, T* __restrict__ dst, int64_t n,
                                                            CopyShape sh) {
   pdl_wait();
   src = pdl_after(src);
@@ -34,7 +34,7 @@ __global__ void __launch_bounds__(256) strided_copy_kernel(const T* __restrict__
     }
     is += (int64_t)rem * sh.sstr[6 - M];
     id += (int64_t)rem * sh.dstr[6 - M];
-    dst[id] = __ldg(src + is);
+    dst[id] = pdl_ld(src + is);
   }
 }
 
@@ -61,7 +61,7 @@ static void launch_strided_copy(wdc_context* ctx, const T* s, T* d, int64_t n, c
 
 // dst[b][r][c] (dense, c innermost) <- src[b][c][r]: src element (b, r, c) at b*sb + c*rows + r.
 // 32x32 tiles through shared memory (padded against bank conflicts): both sides coalesced.
-__global__ void __launch_bounds__(256) transpose_tile_kernel(const uint32_t* __restrict__ src,
+__global__ void __launch_bounds__(256) transpose_tile_kernel(const uint32_t* src,
                                                              uint32_t* __restrict__ dst, int64_t batch,
                                                              int64_t rows, int64_t cols) {
   pdl_wait();
@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(256) transpose_tile_kernel(const uint32_t* __r
 // The same transpose in 64x64 tiles with 16-byte accesses on both sides (rows and cols multiples of 4, 16-byte
 // aligned buffers): a quarter of the memory instructions of the 32x32 kernel.  Shared-memory accesses are
 // scalar with a pitch of 65 words: at most two-way bank conflicts on either side.
-__global__ void __launch_bounds__(256) transpose_tile64_kernel(const float* __restrict__ src, float* __restrict__ dst,
+__global__ void __launch_bounds__(256) transpose_tile64_kernel(const float* src, float* __restrict__ dst,
                                                                int64_t batch, int64_t rows, int64_t cols) {
   pdl_wait();
   src = pdl_after(src);
@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(256) transpose_tile64_kernel(const float* __re
 #pragma unroll
     for (int k = 0; k < 4; k++) {   // src is [cols][rows], rows innermost
       const int64_t c = c0 + ty + 16 * k, r = r0 + 4 * tx;
-      v[k] = (c < cols && r < rows) ? __ldg(reinterpret_cast<const float4*>(s + c * rows + r))
+      v[k] = (c < cols && r < rows) ? pdl_ld(reinterpret_cast<const float4*>(s + c * rows + r))
                                     : make_float4(0.f, 0.f, 0.f, 0.f);
     }
 #pragma unroll
@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(256) transpose_tile64_kernel(const float* __re
 // image batch): one thread per position of the long axis, which is contiguous in src (narrow cols)
 // or in dst (narrow rows), so that side is coalesced per step and the other is covered by the
 // thread's short run of consecutive words.
-__global__ void __launch_bounds__(256) transpose_narrow_cols_kernel(const uint32_t* __restrict__ src,
+__global__ void __launch_bounds__(256) transpose_narrow_cols_kernel(const uint32_t* src,
                                                                     uint32_t* __restrict__ dst, int64_t batch,
                                                                     int64_t rows, int cols) {
   pdl_wait();
@@ -150,10 +150,10 @@ __global__ void __launch_bounds__(256) transpose_narrow_cols_kernel(const uint32
     int64_t b = i / rows, r = i - b * rows;
     const uint32_t* s = src + b * rows * cols + r;
     uint32_t* d = dst + i * cols;
-    for (int c = 0; c < cols; c++) d[c] = __ldg(s + (int64_t)c * rows);
+    for (int c = 0; c < cols; c++) d[c] = pdl_ld(s + (int64_t)c * rows);
   }
 }
-__global__ void __launch_bounds__(256) transpose_narrow_rows_kernel(const uint32_t* __restrict__ src,
+__global__ void __launch_bounds__(256) transpose_narrow_rows_kernel(const uint32_t* src,
                                                                     uint32_t* __restrict__ dst, int64_t batch,
                                                                     int rows, int64_t cols) {
   pdl_wait();
@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(256) transpose_narrow_rows_kernel(const uint32
     int64_t b = i / cols, c = i - b * cols;
     const uint32_t* s = src + (b * cols + c) * rows;
     uint32_t* d = dst + b * rows * cols + c;
-    for (int r = 0; r < rows; r++) d[(int64_t)r * cols] = __ldg(s + r);
+    for (int r = 0; r < rows; r++) d[(int64_t)r * cols] = pdl_ld(s + r);
   }
 }
 
@@ -259,8 +259,8 @@ extern "C" int wdc_strided_copy(wdc_context* ctx, const void* src, void* dst, in
   return wdc_check_launch(ctx, "strided_copy_kernel");
 }
 
-__global__ void __launch_bounds__(256) gather_kernel(const uint32_t* __restrict__ data,
-                                                     const int32_t* __restrict__ idx,
+__global__ void __launch_bounds__(256) gather_kernel(const uint32_t* data,
+                                                     const int32_t* idx,
                                                      uint32_t* __restrict__ out, int64_t outer,
                                                      int64_t axis_len, int64_t inner, int64_t n_idx) {
   pdl_wait();
@@ -271,11 +271,11 @@ __global__ void __launch_bounds__(256) gather_kernel(const uint32_t* __restrict_
   int64_t step = (int64_t)gridDim.x * blockDim.x;
   for (; i < n; i += step) {
     int64_t in = i % inner, k = (i / inner) % n_idx, o = i / (inner * n_idx);
-    int64_t j = __ldg(idx + k);
+    int64_t j = pdl_ld(idx + k);
     if (j < 0) j += axis_len;
     // out-of-range indices are clamped instead of read out of bounds
     j = j < 0 ? 0 : (j >= axis_len ? axis_len - 1 : j);
-    out[i] = __ldg(data + (o * axis_len + j) * inner + in);
+    out[i] = pdl_ld(data + (o * axis_len + j) * inner + in);
   }
 }
 

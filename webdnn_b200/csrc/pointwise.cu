@@ -76,7 +76,7 @@ __device__ __forceinline__ float unary_f32(float v, float p0, float p1) {
 }
 
 template <int OP>
-__global__ void __launch_bounds__(256) unary_f32_kernel(const float* __restrict__ src,
+__global__ void __launch_bounds__(256) unary_f32_kernel(const float* src,
                                                         float* __restrict__ dst, int64_t n,
                                                         float p0, float p1, int vec_ok) {
   pdl_wait();
@@ -88,27 +88,27 @@ __global__ void __launch_bounds__(256) unary_f32_kernel(const float* __restrict_
     const float4* s4 = reinterpret_cast<const float4*>(src);
     float4* d4 = reinterpret_cast<float4*>(dst);
     for (int64_t i = tid; i < n4; i += step) {
-      float4 v = __ldg(s4 + i);
+      float4 v = pdl_ld(s4 + i);
       v.x = unary_f32<OP>(v.x, p0, p1);
       v.y = unary_f32<OP>(v.y, p0, p1);
       v.z = unary_f32<OP>(v.z, p0, p1);
       v.w = unary_f32<OP>(v.w, p0, p1);
       d4[i] = v;
     }
-    for (int64_t i = (n4 << 2) + tid; i < n; i += step) dst[i] = unary_f32<OP>(__ldg(src + i), p0, p1);
+    for (int64_t i = (n4 << 2) + tid; i < n; i += step) dst[i] = unary_f32<OP>(pdl_ld(src + i), p0, p1);
   } else {
-    for (int64_t i = tid; i < n; i += step) dst[i] = unary_f32<OP>(__ldg(src + i), p0, p1);
+    for (int64_t i = tid; i < n; i += step) dst[i] = unary_f32<OP>(pdl_ld(src + i), p0, p1);
   }
 }
 
-__global__ void unary_i32_kernel(int op, const int32_t* __restrict__ src, int32_t* __restrict__ dst,
+__global__ void unary_i32_kernel(int op, const int32_t* src, int32_t* __restrict__ dst,
                                  int64_t n) {
   pdl_wait();
   src = pdl_after(src);
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t step = (int64_t)gridDim.x * blockDim.x;
   for (; i < n; i += step) {
-    int32_t v = __ldg(src + i);
+    int32_t v = pdl_ld(src + i);
     int32_t r;
     switch (op) {
       case WDC_U_ABS: r = v < 0 ? (int32_t)(0u - (uint32_t)v) : v; break;  // |INT_MIN| wraps
@@ -220,8 +220,8 @@ struct BinaryShape {
 // mode 0: both contiguous same shape; 1: b is a scalar; 2: a is a scalar;
 // 3: b repeats with period `period` along the innermost run (bias over the last axis)
 template <int OP>
-__global__ void __launch_bounds__(256) binary_f32_fast_kernel(const float* __restrict__ a,
-                                                              const float* __restrict__ b,
+__global__ void __launch_bounds__(256) binary_f32_fast_kernel(const float* a,
+                                                              const float* b,
                                                               float* __restrict__ out, int64_t n,
                                                               int mode, int64_t period, int vec_ok) {
   pdl_wait();
@@ -235,10 +235,10 @@ __global__ void __launch_bounds__(256) binary_f32_fast_kernel(const float* __res
     for (int64_t i = tid; i < n4; i += step) {
       float4 x, y;
       if (mode == 2) x = make_float4(sa, sa, sa, sa);
-      else x = __ldg(reinterpret_cast<const float4*>(a) + i);
+      else x = pdl_ld(reinterpret_cast<const float4*>(a) + i);
       if (mode == 1) y = make_float4(sb, sb, sb, sb);
-      else if (mode == 3) y = __ldg(reinterpret_cast<const float4*>(b + ((i << 2) % period)));
-      else y = __ldg(reinterpret_cast<const float4*>(b) + i);
+      else if (mode == 3) y = pdl_ld(reinterpret_cast<const float4*>(b + ((i << 2) % period)));
+      else y = pdl_ld(reinterpret_cast<const float4*>(b) + i);
       float4 r;
       r.x = binary_f32<OP>(x.x, y.x);
       r.y = binary_f32<OP>(x.y, y.y);
@@ -249,15 +249,15 @@ __global__ void __launch_bounds__(256) binary_f32_fast_kernel(const float* __res
     tid += n4 << 2;
   }
   for (int64_t i = tid; i < n; i += step) {
-    float x = __ldg(a + (mode == 2 ? 0 : i));
-    float y = __ldg(b + (mode == 1 ? 0 : mode == 3 ? i % period : i));
+    float x = pdl_ld(a + (mode == 2 ? 0 : i));
+    float y = pdl_ld(b + (mode == 1 ? 0 : mode == 3 ? i % period : i));
     out[i] = binary_f32<OP>(x, y);
   }
 }
 
 template <int OP>
-__global__ void __launch_bounds__(256) binary_f32_general_kernel(const float* __restrict__ a,
-                                                                 const float* __restrict__ b,
+__global__ void __launch_bounds__(256) binary_f32_general_kernel(const float* a,
+                                                                 const float* b,
                                                                  float* __restrict__ out, int64_t n,
                                                                  BinaryShape sh) {
   pdl_wait();
@@ -274,11 +274,11 @@ __global__ void __launch_bounds__(256) binary_f32_general_kernel(const float* __
       ia += c * sh.sa[d];
       ib += c * sh.sb[d];
     }
-    out[i] = binary_f32<OP>(__ldg(a + ia), __ldg(b + ib));
+    out[i] = binary_f32<OP>(pdl_ld(a + ia), pdl_ld(b + ib));
   }
 }
 
-__global__ void binary_i32_kernel(int op, const int32_t* __restrict__ a, const int32_t* __restrict__ b,
+__global__ void binary_i32_kernel(int op, const int32_t* a, const int32_t* b,
                                   int32_t* __restrict__ out, int64_t n, BinaryShape sh) {
   pdl_wait();
   a = pdl_after(a);
@@ -294,7 +294,7 @@ __global__ void binary_i32_kernel(int op, const int32_t* __restrict__ a, const i
       ia += c * sh.sa[d];
       ib += c * sh.sb[d];
     }
-    out[i] = binary_i32(op, __ldg(a + ia), __ldg(b + ib));
+    out[i] = binary_i32(op, pdl_ld(a + ia), pdl_ld(b + ib));
   }
 }
 
@@ -392,19 +392,19 @@ extern "C" int wdc_binary(wdc_context* ctx, int op, int dtype, const void* a, co
 }
 
 // --------------------------------------------------------------------------------- cast
-__global__ void cast_f32_i32_kernel(const float* __restrict__ s, int32_t* __restrict__ d, int64_t n) {
+__global__ void cast_f32_i32_kernel(const float* s, int32_t* __restrict__ d, int64_t n) {
   pdl_wait();
   s = pdl_after(s);
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t step = (int64_t)gridDim.x * blockDim.x;
-  for (; i < n; i += step) d[i] = to_int32((double)__ldg(s + i));
+  for (; i < n; i += step) d[i] = to_int32((double)pdl_ld(s + i));
 }
-__global__ void cast_i32_f32_kernel(const int32_t* __restrict__ s, float* __restrict__ d, int64_t n) {
+__global__ void cast_i32_f32_kernel(const int32_t* s, float* __restrict__ d, int64_t n) {
   pdl_wait();
   s = pdl_after(s);
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t step = (int64_t)gridDim.x * blockDim.x;
-  for (; i < n; i += step) d[i] = (float)__ldg(s + i);
+  for (; i < n; i += step) d[i] = (float)pdl_ld(s + i);
 }
 
 extern "C" int wdc_cast(wdc_context* ctx, int src_dtype, int dst_dtype, const void* src, void* dst,
@@ -428,9 +428,9 @@ extern "C" int wdc_cast(wdc_context* ctx, int src_dtype, int dst_dtype, const vo
 }
 
 // ---------------------------------------------------------------------- per-channel affine
-__global__ void __launch_bounds__(256) channel_affine_kernel(const float* __restrict__ x,
-                                                             const float* __restrict__ scale,
-                                                             const float* __restrict__ shift,
+__global__ void __launch_bounds__(256) channel_affine_kernel(const float* x,
+                                                             const float* scale,
+                                                             const float* shift,
                                                              float* __restrict__ y, int64_t n,
                                                              int64_t channels, int64_t inner, int relu,
                                                              int vec_ok) {
@@ -443,20 +443,20 @@ __global__ void __launch_bounds__(256) channel_affine_kernel(const float* __rest
   if (vec_ok) {  // inner == 1 (channels innermost, multiple of 4) or inner % 4 == 0
     int64_t n4 = n >> 2;
     for (int64_t i = tid; i < n4; i += step) {
-      float4 v = __ldg(reinterpret_cast<const float4*>(x) + i);
+      float4 v = pdl_ld(reinterpret_cast<const float4*>(x) + i);
       int64_t e = i << 2;
       float4 r;
       if (inner == 1) {
         int64_t c = e % channels;
-        float4 s = __ldg(reinterpret_cast<const float4*>(scale + c));
-        float4 t = __ldg(reinterpret_cast<const float4*>(shift + c));
+        float4 s = pdl_ld(reinterpret_cast<const float4*>(scale + c));
+        float4 t = pdl_ld(reinterpret_cast<const float4*>(shift + c));
         r.x = fmaf(v.x, s.x, t.x);
         r.y = fmaf(v.y, s.y, t.y);
         r.z = fmaf(v.z, s.z, t.z);
         r.w = fmaf(v.w, s.w, t.w);
       } else {
         int64_t c = (e / inner) % channels;
-        float s = __ldg(scale + c), t = __ldg(shift + c);
+        float s = pdl_ld(scale + c), t = pdl_ld(shift + c);
         r.x = fmaf(v.x, s, t);
         r.y = fmaf(v.y, s, t);
         r.z = fmaf(v.z, s, t);
@@ -528,7 +528,7 @@ __constant__ double kEightbitLevels[128] = {
     8.882811666e-1, 9.054686427e-1, 9.226561785e-1, 9.398436546e-1, 9.570311308e-1, 9.742186666e-1,
     9.914061427e-1, 1.0};
 
-__global__ void __launch_bounds__(256) decode_eightbit_kernel(const uint8_t* __restrict__ codes,
+__global__ void __launch_bounds__(256) decode_eightbit_kernel(const uint8_t* codes,
                                                               float* __restrict__ out, int64_t n, float scale) {
   pdl_wait();
   codes = pdl_after(codes);
@@ -543,7 +543,7 @@ __global__ void __launch_bounds__(256) decode_eightbit_kernel(const uint8_t* __r
   int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t step = (int64_t)gridDim.x * blockDim.x;
   for (; g < groups; g += step) {
-    const uint4 c = __ldg(reinterpret_cast<const uint4*>(codes) + g);
+    const uint4 c = pdl_ld(reinterpret_cast<const uint4*>(codes) + g);
     const uint32_t w[4] = {c.x, c.y, c.z, c.w};
     float4* dst = reinterpret_cast<float4*>(out) + g * 4;
 #pragma unroll
@@ -553,7 +553,7 @@ __global__ void __launch_bounds__(256) decode_eightbit_kernel(const uint8_t* __r
   }
   // tail of fewer than 16 codes
   for (int64_t i = groups * 16 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += step)
-    out[i] = table[__ldg(codes + i)];
+    out[i] = table[pdl_ld(codes + i)];
 }
 
 extern "C" int wdc_decode_eightbit(wdc_context* ctx, const void* codes, float* out, int64_t n, float scale) {

@@ -7,7 +7,7 @@
 #include "tape.cuh"
 
 template <bool IS_MAX, int VEC>
-__global__ void __launch_bounds__(256) pool2d_kernel(wdc_pool_desc d, const float* __restrict__ x,
+__global__ void __launch_bounds__(256) pool2d_kernel(wdc_pool_desc d, const float* x,
                                                      float* __restrict__ y, int c_fastest) {
   pdl_wait();
   x = pdl_after(x);
@@ -44,10 +44,10 @@ __global__ void __launch_bounds__(256) pool2d_kernel(wdc_pool_desc d, const floa
         const float* p = x + b * d.xs_n + c * d.xs_c + iny * d.xs_h + inx * d.xs_w;
         float val[VEC];
         if (VEC == 4) {
-          float4 t = __ldg(reinterpret_cast<const float4*>(p));
+          float4 t = pdl_ld(reinterpret_cast<const float4*>(p));
           val[0] = t.x; val[1 % VEC] = t.y; val[2 % VEC] = t.z; val[3 % VEC] = t.w;
         } else {
-          val[0] = __ldg(p);
+          val[0] = pdl_ld(p);
         }
 #pragma unroll
         for (int v = 0; v < VEC; v++) {
@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(256) pool2d_kernel(wdc_pool_desc d, const floa
 // image taps re-read the clamped pixel with a -inf substitute) before any comparison.
 // One thread = 4 channels of one output pixel.
 template <int KH, int KW>
-__global__ void __launch_bounds__(256) maxpool_cl_small_kernel(const float4* __restrict__ x, float4* __restrict__ y,
+__global__ void __launch_bounds__(256) maxpool_cl_small_kernel(const float4* x, float4* __restrict__ y,
                                                                int n_out, int chv, int in_h, int in_w, int out_h,
                                                                int out_w, int stride_h, int stride_w, int pad_t,
                                                                int pad_l) {
@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(256) maxpool_cl_small_kernel(const float4* __r
         const bool ok = (unsigned)iy < (unsigned)in_h && (unsigned)ix < (unsigned)in_w;
         const int cy = min(max(iy, 0), in_h - 1), cx = min(max(ix, 0), in_w - 1);
         in[ky * KW + kx] = ok;
-        v[ky * KW + kx] = __ldg(x + ((size_t)(b * in_h + cy) * in_w + cx) * chv + c);
+        v[ky * KW + kx] = pdl_ld(x + ((size_t)(b * in_h + cy) * in_w + cx) * chv + c);
       }
     }
     float4 m = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
@@ -173,7 +173,7 @@ extern "C" int wdc_avgpool2d(wdc_context* ctx, const wdc_pool_desc* d, const flo
 // Global average pool.  Channels-last: a warp's lanes are 32 consecutive (b, c), so every pixel it reads is coalesced,
 // and the 8 warps of a CTA share the pixels: one thread walking a 7x7 map alone is 49 dependent additions in double
 // behind a few loads at a time, 7 us for the 2048 channels of one image whatever the GPU has idle.
-__global__ void __launch_bounds__(256) gap_cl_kernel(const float* __restrict__ x, float* __restrict__ y,
+__global__ void __launch_bounds__(256) gap_cl_kernel(const float* x, float* __restrict__ y,
                                                      int64_t maps, int64_t ch, int64_t area,
                                                      int64_t xs_n, int64_t xs_p) {
   pdl_wait();
@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(256) gap_cl_kernel(const float* __restrict__ x
       const int64_t b = m / ch, c = m - b * ch;
       const float* p = x + b * xs_n + c;
 #pragma unroll 8
-      for (int64_t a = warp; a < area; a += 8) s += (double)__ldg(p + a * xs_p);
+      for (int64_t a = warp; a < area; a += 8) s += (double)pdl_ld(p + a * xs_p);
     }
     part[warp][lane] = s;
     __syncthreads();
@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(256) gap_cl_kernel(const float* __restrict__ x
 }
 
 // NCHW: one warp per (b, c), lanes stride the pixels.
-__global__ void __launch_bounds__(256) gap_warp_kernel(const float* __restrict__ x, float* __restrict__ y,
+__global__ void __launch_bounds__(256) gap_warp_kernel(const float* x, float* __restrict__ y,
                                                        int64_t batch, int64_t ch, int64_t area,
                                                        int64_t xs_n, int64_t xs_c, int64_t xs_p) {
   pdl_wait();
@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(256) gap_warp_kernel(const float* __restrict__
     int64_t b = row / ch, c = row % ch;
     const float* p = x + b * xs_n + c * xs_c;
     double s = 0;
-    for (int64_t a = lane; a < area; a += 32) s += (double)__ldg(p + a * xs_p);
+    for (int64_t a = lane; a < area; a += 32) s += (double)pdl_ld(p + a * xs_p);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (lane == 0) y[row] = (float)(s / (double)area);
@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(256) gap_warp_kernel(const float* __restrict__
 // so L lanes (4, 8 or 16) share a row and a warp works on 32 / L rows at once.  All of a row's loads are issued
 // before the first addition (up to 8 per lane), which is what keeps enough bytes in flight per SM.
 template <int L>
-__global__ void __launch_bounds__(256) gap_group_kernel(const float* __restrict__ x, float* __restrict__ y,
+__global__ void __launch_bounds__(256) gap_group_kernel(const float* x, float* __restrict__ y,
                                                         int64_t rows, int64_t ch, int area, int64_t xs_n,
                                                         int64_t xs_c, int64_t xs_p) {
   pdl_wait();
@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(256) gap_group_kernel(const float* __restrict_
 #pragma unroll
       for (int u = 0; u < 8; u++) {
         const int a = gl + u * L;
-        v[r][u] = (valid && a < area) ? __ldg(p + (int64_t)a * xs_p) : 0.f;
+        v[r][u] = (valid && a < area) ? pdl_ld(p + (int64_t)a * xs_p) : 0.f;
       }
     }
 #pragma unroll
@@ -276,7 +276,7 @@ __global__ void __launch_bounds__(256) gap_group_kernel(const float* __restrict_
 // words: conflict-free for odd areas, 2-way at worst for the even ones that matter).  Sums in double, like the others.
 constexpr int GAP_MAPS = 128;
 constexpr int GAP_MAX_AREA = 96;
-__global__ void __launch_bounds__(GAP_MAPS) gap_dense_kernel(const float* __restrict__ x, float* __restrict__ y,
+__global__ void __launch_bounds__(GAP_MAPS) gap_dense_kernel(const float* x, float* __restrict__ y,
                                                              int64_t rows, int area) {
   pdl_wait();
   x = pdl_after(x);
@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(GAP_MAPS) gap_dense_kernel(const float* __rest
 #pragma unroll
       for (int u = 0; u < 8; u++) {
         const int i = base + u * GAP_MAPS + (int)threadIdx.x;
-        r[u] = i < vec ? __ldg(reinterpret_cast<const float4*>(src) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        r[u] = i < vec ? pdl_ld(reinterpret_cast<const float4*>(src) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
 #pragma unroll
       for (int u = 0; u < 8; u++) {
@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(GAP_MAPS) gap_dense_kernel(const float* __rest
         if (i < vec) reinterpret_cast<float4*>(buf)[i] = r[u];
       }
     }
-    for (int i = (vec << 2) + threadIdx.x; i < words; i += blockDim.x) buf[i] = __ldg(src + i);
+    for (int i = (vec << 2) + threadIdx.x; i < words; i += blockDim.x) buf[i] = pdl_ld(src + i);
     __syncthreads();
     if ((int)threadIdx.x < maps) {
       const float* m = buf + threadIdx.x * area;

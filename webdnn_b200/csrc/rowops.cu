@@ -31,7 +31,7 @@ __device__ __forceinline__ void warp_sum_d(double (&v)[R]) {
 // ------------------------------------------------------------------------------ softmax
 // operators/cpu/operators/standard/softmax.ts:39-57: max, exp(v - max), sum, divide.
 template <int ITEMS>
-__global__ void __launch_bounds__(256) softmax_warp_kernel(const float* __restrict__ x,
+__global__ void __launch_bounds__(256) softmax_warp_kernel(const float* x,
                                                            float* __restrict__ y, int64_t outer,
                                                            int len) {
   pdl_wait();
@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(256) softmax_warp_kernel(const float* __restri
   }
 }
 
-__global__ void __launch_bounds__(512) softmax_block_kernel(const float* __restrict__ x,
+__global__ void __launch_bounds__(512) softmax_block_kernel(const float* x,
                                                             float* __restrict__ y, int64_t outer,
                                                             int64_t len) {
   pdl_wait();
@@ -126,7 +126,7 @@ __device__ __forceinline__ float block_reduce_f(float v, float* red, bool is_max
   return t;
 }
 template <int ITEMS>
-__global__ void __launch_bounds__(256) softmax_block_reg_kernel(const float* __restrict__ x, float* __restrict__ y,
+__global__ void __launch_bounds__(256) softmax_block_reg_kernel(const float* x, float* __restrict__ y,
                                                                 int64_t outer, int len) {
   pdl_wait();
   x = pdl_after(x);
@@ -232,7 +232,7 @@ __device__ __forceinline__ double red_finish(int kind, int final, double s, int6
 }
 
 // inner == 1: one warp per output element, lanes stride the reduced axis.
-__global__ void __launch_bounds__(256) reduce_rows_kernel(int kind, int final, const float* __restrict__ x,
+__global__ void __launch_bounds__(256) reduce_rows_kernel(int kind, int final, const float* x,
                                                           float* __restrict__ y, int64_t outer,
                                                           int64_t red, int64_t total) {
   pdl_wait();
@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(256) reduce_rows_kernel(int kind, int final, c
 }
 
 // inner > 1: one thread per (outer, inner) output, coalesced across inner.
-__global__ void __launch_bounds__(256) reduce_cols_kernel(int kind, int final, const float* __restrict__ x,
+__global__ void __launch_bounds__(256) reduce_cols_kernel(int kind, int final, const float* x,
                                                           float* __restrict__ y, int64_t outer,
                                                           int64_t red, int64_t inner, int64_t total) {
   pdl_wait();
@@ -307,9 +307,9 @@ extern "C" int wdc_reduce_axis(wdc_context* ctx, int kind, int final, const floa
 // 256); the result differs from the all-double sum by a few 1e-7 relative.  Two rows per warp iteration keep
 // twice the loads in flight.
 template <int ITEMS>
-__global__ void __launch_bounds__(256) layernorm_warp_kernel(const float* __restrict__ x,
-                                                             const float* __restrict__ gamma,
-                                                             const float* __restrict__ beta,
+__global__ void __launch_bounds__(256) layernorm_warp_kernel(const float* x,
+                                                             const float* gamma,
+                                                             const float* beta,
                                                              float* __restrict__ y, int64_t outer,
                                                              int len, float eps) {
   pdl_wait();
@@ -326,8 +326,8 @@ __global__ void __launch_bounds__(256) layernorm_warp_kernel(const float* __rest
 #pragma unroll
   for (int i = 0; i < KEPT; i++) {
     const int c = i * 32 + lane;
-    gk[i] = ITEMS <= 8 && gamma && c < len ? __ldg(gamma + c) : 1.f;
-    bk[i] = ITEMS <= 8 && beta && c < len ? __ldg(beta + c) : 0.f;
+    gk[i] = ITEMS <= 8 && gamma && c < len ? pdl_ld(gamma + c) : 1.f;
+    bk[i] = ITEMS <= 8 && beta && c < len ? pdl_ld(beta + c) : 0.f;
   }
   for (; row0 < outer; row0 += rstep) {
     float v[R][ITEMS];
@@ -340,7 +340,7 @@ __global__ void __launch_bounds__(256) layernorm_warp_kernel(const float* __rest
 #pragma unroll
       for (int i = 0; i < ITEMS; i++) {
         int c = i * 32 + lane;
-        v[r][i] = (live && c < len) ? __ldg(xr + c) : 0.f;
+        v[r][i] = (live && c < len) ? pdl_ld(xr + c) : 0.f;
         t += v[r][i];
       }
       s[r] = (double)t;
@@ -371,8 +371,8 @@ __global__ void __launch_bounds__(256) layernorm_warp_kernel(const float* __rest
         int c = i * 32 + lane;
         if (row0 + r < outer && c < len) {
           float o = v[r][i] * rden;                                                        // Div
-          if (gamma) o = o * (ITEMS <= 8 ? gk[i % KEPT] : __ldg(gamma + c));                // Mul
-          if (beta) o = o + (ITEMS <= 8 ? bk[i % KEPT] : __ldg(beta + c));                  // Add
+          if (gamma) o = o * (ITEMS <= 8 ? gk[i % KEPT] : pdl_ld(gamma + c));                // Mul
+          if (beta) o = o + (ITEMS <= 8 ? bk[i % KEPT] : pdl_ld(beta + c));                  // Add
           yr[c] = o;
         }
       }
@@ -392,9 +392,9 @@ __device__ __forceinline__ double block_sum_d(double v, double* scratch) {
   for (int i = 0; i < (int)(blockDim.x >> 5); i++) t += scratch[i];   // same order in every thread
   return t;
 }
-__global__ void __launch_bounds__(256) layernorm_block_kernel(const float* __restrict__ x,
-                                                              const float* __restrict__ gamma,
-                                                              const float* __restrict__ beta,
+__global__ void __launch_bounds__(256) layernorm_block_kernel(const float* x,
+                                                              const float* gamma,
+                                                              const float* beta,
                                                               float* __restrict__ y, int64_t outer, int64_t len,
                                                               float eps) {
   pdl_wait();
@@ -427,9 +427,9 @@ __global__ void __launch_bounds__(256) layernorm_block_kernel(const float* __res
 
 // Rows of 1025 .. 256 * ITEMS elements with the row held in the CTA's registers (one read of x).
 template <int ITEMS>
-__global__ void __launch_bounds__(256) layernorm_block_reg_kernel(const float* __restrict__ x,
-                                                                  const float* __restrict__ gamma,
-                                                                  const float* __restrict__ beta,
+__global__ void __launch_bounds__(256) layernorm_block_reg_kernel(const float* x,
+                                                                  const float* gamma,
+                                                                  const float* beta,
                                                                   float* __restrict__ y, int64_t outer, int len,
                                                                   float eps) {
   pdl_wait();
@@ -513,7 +513,7 @@ extern "C" int wdc_layernorm(wdc_context* ctx, const float* x, const float* gamm
 }
 
 // ------------------------------------------------------------------------------- argmax
-__global__ void __launch_bounds__(256) argmax_kernel(const float* __restrict__ x, int32_t* __restrict__ y,
+__global__ void __launch_bounds__(256) argmax_kernel(const float* x, int32_t* __restrict__ y,
                                                      int64_t outer, int64_t len, int select_last) {
   pdl_wait();
   x = pdl_after(x);

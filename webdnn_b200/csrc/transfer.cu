@@ -4,8 +4,8 @@
 // else can be queued, 12.7 GB/s for megabytes (605 us for an 800x800 image), where the link takes 50 GB/s from
 // page-locked memory.  Here the context keeps a ring of page-locked chunks: a transfer is cut into chunks, each is
 // copied by a few threads and sent (or received and copied) while its neighbours are on the link.  Page-locked
-// buffers of the caller's go straight to the link.  Small transfers leave the copy engines out: a kernel of the compute
-// stream reads or writes the page-locked memory, which saves the switch between the two.
+// buffers of the caller's go straight to the link.  Small results leave the copy engines out: a kernel of the compute
+// stream writes the page-locked memory, which saves the switch between the two.
 #include <string.h>
 
 #include <atomic>
@@ -189,7 +189,6 @@ bool page_locked(const void* p, int64_t bytes) {
 
 // Words of several buffers, copied by one launch.  Page-locked host memory on one side.
 __global__ void __launch_bounds__(256) io_copy_kernel(const wdc_io_list list) {
-  pdl_wait();
   for (int s = 0; s < list.n; s++) {
     const wdc_io_list::Part p = list.part[s];
     const int64_t vec = (((uintptr_t)p.dst | (uintptr_t)p.src) & 15) == 0 ? p.words / 4 : 0;
@@ -233,20 +232,6 @@ int wdc_stage_in(wdc_context* ctx, void* dst, const void* host, int64_t bytes) {
   int st = stager_of(ctx, &s);
   if (st != WDC_OK) return st;
   std::lock_guard<std::mutex> lk(s->mu);
-  if (bytes <= BY_KERNEL && bytes % 4 == 0) {
-    int i;
-    st = take_chunk(ctx, s, &i);
-    if (st != WDC_OK) return st;
-    memcpy(s->ring + i * CHUNK, host, (size_t)bytes);
-    wdc_io_list list = {};
-    list.n = 1;
-    list.part[0] = {(uint32_t*)dst, (const uint32_t*)(s->ring + i * CHUNK), bytes / 4};
-    wdc_launch_pdl(ctx, io_copy_kernel, wdc_io_grid(list), dim3(256), 0, list);
-    WDC_CUDA(ctx, cudaGetLastError());
-    WDC_CUDA(ctx, cudaEventRecord(s->done[i], ctx->stream));
-    s->busy[i] = true;
-    return WDC_OK;
-  }
   for (int64_t base = 0; base < bytes; base += CHUNKS * CHUNK) {   // a ring's worth at a time
     const int64_t part = bytes - base < CHUNKS * CHUNK ? bytes - base : CHUNKS * CHUNK;
     int index[CHUNKS];
@@ -296,7 +281,7 @@ int wdc_stage_out(wdc_context* ctx, int count, void* const* host, const void* co
       list.part[list.n++] = {(uint32_t*)at, (const uint32_t*)src[b], bytes[b] / 4};
       at += (bytes[b] + 15) / 16 * 16;
     }
-    wdc_launch_pdl(ctx, io_copy_kernel, wdc_io_grid(list), dim3(256), 0, list);
+    io_copy_kernel<<<wdc_io_grid(list), 256, 0, ctx->stream>>>(list);
     WDC_CUDA(ctx, cudaGetLastError());
     st = wdc_sync(ctx);
     if (st != WDC_OK) return st;
@@ -361,6 +346,12 @@ extern "C" int wdc_upload(wdc_context* ctx, void* dst, const void* host, int64_t
   if (bytes == 0) return WDC_OK;
   DeviceGuard g(ctx->device);
   wdc_tc_evict(ctx, dst, bytes);
+  // Not beside kernels in flight: a model's first run brings its weights into memory that the kernels before have just
+  // given back, and gains nothing from overlap.  (Repeated runs stage their inputs without coming through here.)
+  if (!ctx->capture_arena) {
+    WDC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    ctx->n_waits++;
+  }
   return wdc_stage_in(ctx, dst, host, bytes);
 }
 
