@@ -200,7 +200,17 @@ tc_small_kernel(const __grid_constant__ TcProblem p, const __grid_constant__ CUt
       const int seg = kb / SEG_KBLOCKS < nseg ? kb / SEG_KBLOCKS : nseg - 1;
       while (ok && seg >= drained + L::BUFS) drain();
       if (!ok) break;
-      ok = small_wait(full0 + (uint32_t)st * 8u, full_par, ss, p.status, 52);
+      // K block kb - T_ST: its MMAs have read the part of tensor memory that this one's parts go to.  With an odd number of
+      // stages they have also read this stage, which the other group waited for then: not before that may this group
+      // wait for the stage's next phase, or it takes the end of the phase before the last for it.  (Loads arrive in any
+      // order: block 1 there and block 0 not, and block 0's bytes were split as block 3's.)
+      const int old = kb - L::T_ST;
+      static_assert(L::STAGES % 2 == 0 || L::STAGES == L::T_ST, "a stage's phases are waited for one by one");
+      auto wait_old = [&]() {
+        return old < 0 || small_wait(empty0 + (uint32_t)(old % L::STAGES) * 8u, (uint32_t)((old / L::STAGES) & 1), ss, p.status, 53);
+      };
+      if (L::STAGES % 2) ok = wait_old();
+      ok = ok && small_wait(full0 + (uint32_t)st * 8u, full_par, ss, p.status, 52);
       if (!ok) break;
       const unsigned char* src = smem + st * L::STAGE + row_off;
       const uint32_t dst = t_lane + (uint32_t)(L::A_COL0 + ts * 64);
@@ -219,10 +229,7 @@ tc_small_kernel(const __grid_constant__ TcProblem p, const __grid_constant__ CUt
           }
         }
         if (h == 0) {
-          // the MMAs that read this part of tensor memory have completed: the commit of the K block T_ST before
-          const int old = kb - L::T_ST;
-          if (old >= 0)
-            ok = small_wait(empty0 + (uint32_t)(old % L::STAGES) * 8u, (uint32_t)((old / L::STAGES) & 1), ss, p.status, 53);
+          if (L::STAGES % 2 == 0) ok = wait_old();   // (with the first half of the row on its way)
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         }
