@@ -1,0 +1,113 @@
+"""What repeats a run for the host (tapes, graphs with their transfers) and what moves its data."""
+import ctypes
+from ctypes import c_void_p
+
+import numpy as np
+import pytest
+
+from webdnn_b200 import onnx_io, operator_table, zoo
+
+pytestmark = pytest.mark.gpu
+
+
+def _load(ctx, model, **options):
+    from webdnn_b200.runner import load
+    return load(model, backend_order=["cuda", "cpu"], backend_options={"cuda": {"context": ctx, **options}})
+
+
+def _model(nodes, inputs, outputs, inits=()):
+    value = lambda v: onnx_io.ValueInfo(v[0], v[2] if len(v) > 2 else onnx_io.FLOAT, list(v[1]))  # noqa: E731
+    g = onnx_io.Graph("g", nodes, [onnx_io.make_tensor(n, a) for n, a in inits], [value(v) for v in inputs],
+                      [value(v) for v in outputs])
+    return onnx_io.Model(g, opset_import=[("", 13)])
+
+
+def _cpu(a):
+    from webdnn_b200.backend import CPUTensor
+    return CPUTensor.from_array(np.ascontiguousarray(a))
+
+
+def _bits(a):
+    return np.ascontiguousarray(a).reshape(-1).view(np.uint32)
+
+
+def _two_outputs(rows):
+    """[rows, 40] and [rows, 40] -> their product's rectified halves, and an int32 index per row."""
+    make = onnx_io.make_node
+    rng = np.random.default_rng(rows)
+    return _model([make("MatMul", ["a", "w"], ["m"], name="m"), make("Add", ["m", "b"], ["s"], name="s"),
+                   make("Relu", ["s"], ["y"], name="r"), make("ArgMax", ["s"], ["i"], name="i", axis=-1, keepdims=0)],
+                  [("a", [rows, 40]), ("b", [rows, 64])], [("y", [rows, 64]), ("i", [rows], onnx_io.INT32)],
+                  [("w", rng.standard_normal((40, 64)).astype(np.float32))])
+
+
+def _tape_of(runner, on_device=False):
+    return [t for (dev, _), t in runner._tapes.items() if dev == on_device]
+
+
+def test_uploads_do_not_wait_for_kernels(cuda_context):
+    import time
+    ctx = cuda_context
+    big = ctx.empty_tensor([1 << 28])
+    dst = ctx._alloc(4 << 20)
+    pinned, pageable = ctx.pinned_array((1 << 20,), np.uint8), np.ones(4 << 20, np.uint8)
+    for host in (pinned, pageable[:4096], pageable):
+        ctx._call("wdc_upload", c_void_p(dst), host.ctypes.data_as(c_void_p), host.nbytes)   # (the ring exists from here on)
+        ctx.sync()
+        for _ in range(400):
+            ctx._call("wdc_fill_u32", c_void_p(big.ptr), ctypes.c_uint32(1), big.length)
+        t0 = time.perf_counter()
+        ctx._call("wdc_upload", c_void_p(dst), host.ctypes.data_as(c_void_p), host.nbytes)
+        t1 = time.perf_counter()
+        ctx.sync()
+        t2 = time.perf_counter()
+        assert t2 - t0 > 0.01 and t1 - t0 < 0.3 * (t2 - t0), (host.nbytes, t1 - t0, t2 - t0)
+    ctx._call("wdc_host_free", pinned.ctypes.data_as(c_void_p))
+    ctx._free(dst)
+    big.dispose()
+
+
+def test_taped_runs_that_nobody_waited_for(cuda_context):
+    """Inputs of later calls are brought into memory that the calls in flight have just given back."""
+    ctx = cuda_context
+    model = zoo.resnet50(48, 64, 32, (1, 1, 1, 1), 64, softmax=False)
+    runner = _load(ctx, model)
+    xs = [np.random.default_rng(i).standard_normal((48, 3, 64, 64)).astype(np.float32) for i in range(12)]
+    want = [runner.run([_cpu(x)])[0].numpy().copy() for x in xs]
+    for _ in range(3):
+        runner.run([_cpu(xs[0])], outputs_on_device=True)[0].dispose()
+    assert _tape_of(runner, True) != [None]
+    for _ in range(5):
+        queued = [runner.run([_cpu(x)], outputs_on_device=True)[0] for x in xs]
+        for q, w in zip(queued, want):
+            assert np.array_equal(_bits(q.get_data()), _bits(w))
+            q.dispose()
+        pending = []
+        for x, w in [*zip(xs, want), (None, None), (None, None)]:      # three in flight
+            if x is not None:
+                pending.append((runner.run([_cpu(x)], wait=False), w))
+            if len(pending) == 3 or x is None:
+                p, expected = pending.pop(0)
+                assert np.array_equal(_bits(p.result()[0].numpy()), _bits(expected))
+    runner.dispose()
+
+
+def test_first_results_in_used_memory(cuda_context):
+    """A model loaded into memory that other work has just given back gives the same bits at every call."""
+    ctx = cuda_context
+    rng = np.random.default_rng(0)
+    models = [zoo.resnet50(2, 64, 32, (1, 1, 1, 1), 64, softmax=False), zoo.resnet50(40, 64, 32, (1, 1, 1, 1), 64, softmax=False),
+              zoo.detr(batch=1, size=128, d=64, heads=2, enc_layers=1, dec_layers=1, ffn=128, queries=9, classes=7, width=16, blocks=(1, 1, 1, 1)),
+              zoo.mlp(33), zoo.lstm(9, 3, 16, 64)]
+    for i in range(60):
+        model = models[i % len(models)]
+        x = rng.standard_normal(model.graph.input[0].shape).astype(np.float32)
+        big = [ctx.empty_tensor([8 << 20]) for _ in range(4)]
+        for t in big:      # a quiet NaN, large values: whatever is read without having been written shows
+            ctx._call("wdc_fill_u32", c_void_p(t.ptr), ctypes.c_uint32([0x7fc00000, 0x7e000000, 0xc4fa0001][i % 3]), t.length)
+            t.dispose()
+        runner = _load(ctx, model)
+        results = [[o.numpy().copy() for o in runner.run([_cpu(x)])] for _ in range(3)]
+        for later in results[1:]:
+            assert all(np.array_equal(_bits(a), _bits(b)) for a, b in zip(results[0], later))
+        runner.dispose()

@@ -346,12 +346,6 @@ extern "C" int wdc_upload(wdc_context* ctx, void* dst, const void* host, int64_t
   if (bytes == 0) return WDC_OK;
   DeviceGuard g(ctx->device);
   wdc_tc_evict(ctx, dst, bytes);
-  // Not beside kernels in flight: a model's first run brings its weights into memory that the kernels before have just
-  // given back, and gains nothing from overlap.  (Repeated runs stage their inputs without coming through here.)
-  if (!ctx->capture_arena) {
-    WDC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    ctx->n_waits++;
-  }
   return wdc_stage_in(ctx, dst, host, bytes);
 }
 
