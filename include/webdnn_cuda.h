@@ -120,6 +120,10 @@ int wdc_sync(wdc_context* ctx);
  *   "split_k"   1 = small outputs with long reductions may be cut into K ranges (default), 0 = never;
  *   "pdl"       1 = contraction launches are programmatic dependent launches, so that a launch's set-up
  *                   overlaps the tail of the launch before it (default), 0 = plain stream order;
+ *   "small_tile" the contraction kernel for small outputs: 0 = where it is likely the faster one (default), 32 / 64 = with
+ *                   that tile width wherever it can run, -1 = never.  Results do not depend on it;
+ *   "attention_cluster" CTAs that share a query tile of the fused attention: 0 = chosen by size (default), 1, 2, 4 or 8 =
+ *                   that many, where there are as many chunks of keys;
  *   "nvtx"      1 = wdc_range_push / wdc_range_pop emit NVTX ranges (default 0).
  * Unknown names and out-of-range values return WDC_ERR_INVALID.  A captured graph keeps the options that were
  * in force while it was captured. */
@@ -133,7 +137,9 @@ void* wdc_stream(wdc_context* ctx);
 /* out[0..n): bytes_in_use, high_water_bytes, reserved_bytes, allocs, frees, launches,
  * h2d_bytes, d2h_bytes, tensor_core_launches (launches of the tcgen05 contraction kernel),
  * then, only when n > 9 (it costs a driver call): device_free_bytes, device_total_bytes as
- * cudaMemGetInfo reports them for the context's GPU (-1 if that query fails). */
+ * cudaMemGetInfo reports them for the context's GPU (-1 if that query fails), the last contraction's kernel
+ * (100 * tile width + 10 * CTAs per tile + 1 if it loads its weights early for the small-output kernel, else 0), CTAs
+ * per query tile of the last tensor-core attention. */
 int wdc_stats(wdc_context* ctx, int64_t* out, int n);
 int wdc_reset_stats(wdc_context* ctx);
 /* Per-family device timing.  While enabled, every contraction launch (wdc_gemm / wdc_conv2d) is
@@ -198,6 +204,11 @@ typedef struct wdc_gemm_desc {
 } wdc_gemm_desc;
 int wdc_gemm(wdc_context* ctx, const wdc_gemm_desc* d, const float* A, const float* B,
              const float* C, float* Y);
+/* n / columns products with the same A, their columns of B and Y beside one another, `columns` (a multiple of 4) each.
+ * Same results, bit for bit, as one call per product: the order in which a product's terms are added follows from its
+ * own size. */
+int wdc_gemm_columns(wdc_context* ctx, const wdc_gemm_desc* d, int64_t columns, const float* A, const float* B,
+                     const float* C, float* Y);
 
 /* wdc_conv2d replaces the conv_im2col / conv_matmul / conv_transpose / conv_bias pipeline
  * (src/shader/webgpu/shadersources/standard/conv_*.wgsl, operators/webgpu/operators/standard/

@@ -1,0 +1,137 @@
+"""Kernels that a rule on sizes chooses between: each of them where the rule would not, against the other, bit for bit where
+the order of the additions is the same."""
+from ctypes import byref, c_void_p
+
+import numpy as np
+import pytest
+
+from util import max_err_rel_linf
+
+pytestmark = pytest.mark.gpu
+
+
+def _put(ctx, a):
+    from webdnn_b200.backend import CPUTensor
+    return ctx.move_tensor(CPUTensor.from_array(np.ascontiguousarray(a)))
+
+
+def _conv(ctx, x, w, shift, res, pad, small_tile):
+    """x NHWC, w KRSC, on the device; the result and the kernel that computed it (see wdc_stats)."""
+    from webdnn_b200.lib import ConvDesc
+    n, h, wd, cin = x.dims
+    cout, k = w.dims[0], w.dims[1]
+    oh, ow = h + 2 * pad - k + 1, wd + 2 * pad - k + 1
+    y = ctx.empty_tensor([n, oh, ow, cout])
+    d = ConvDesc(batch=n, ch_in=cin, in_h=h, in_w=wd, ch_out=cout, k_h=k, k_w=k, out_h=oh, out_w=ow, stride_h=1, stride_w=1,
+                 pad_t=pad, pad_l=pad, dil_h=1, dil_w=1, group=1, relu=int(res is not None))
+    ctx.set_option("small_tile", small_tile)
+    try:
+        ctx.conv2d(d, x, w, None, shift, res, y)
+    finally:
+        ctx.set_option("small_tile", 0)
+    got = y.get_data().copy()
+    y.dispose()
+    return got.view(np.uint32), ctx.stats(device_memory=True)["last_contraction"]
+
+
+# [rows, columns, K blocks] that tc_igemm_kernel takes whole (in 1 .. 8 and more segments) or cuts into 2 .. 8 ranges: every
+# cluster size of both tile widths; a last K block, a last row tile and a last column tile that are not full
+@pytest.mark.parametrize("m,n,kblocks", [
+    (76, 4, 1), (50, 36, 5), (44, 4, 8), (37, 4, 14), (32, 8, 19), (36, 4, 20), (66, 4, 24), (70, 4, 30), (3488, 4, 32), (129, 68, 32),
+    (8261, 4, 54), (6105, 4, 41), (4061, 4, 36), (3333, 4, 36), (2780, 4, 36), (46, 4, 33), (33, 4, 40), (49, 100, 144),
+    (9841, 40, 1), (9884, 36, 9), (10109, 40, 12), (3136, 64, 18), (625, 256, 64), (320, 512, 144)])
+@pytest.mark.parametrize("ragged", [0, 12])
+@pytest.mark.parametrize("precision", ["tf32x3", "tf32x1"])
+def test_small_outputs_are_the_same_bits(cuda_context, m, n, kblocks, ragged, precision):
+    ctx = cuda_context
+    rng = np.random.default_rng(m + n)
+    k = 32 * kblocks - ragged
+    x, w = rng.standard_normal((1, 1, m, k)).astype(np.float32), rng.standard_normal((n, 1, 1, k)).astype(np.float32)
+    dx, dw = _put(ctx, x), _put(ctx, w)
+    shift, res = _put(ctx, rng.standard_normal(n).astype(np.float32)), _put(ctx, rng.standard_normal((m, n)).astype(np.float32))
+    ctx.declare_constant(dw)
+    ctx.set_precision(precision)
+    seen = set()
+    try:
+        for split_k in (1, 0):
+            ctx.set_option("split_k", split_k)
+            for s, r in ((None, None), (shift, None), (shift, res)):
+                want, kernel = _conv(ctx, dx, dw, s, r, 0, -1)
+                assert kernel == 0
+                for tile in (32, 64):
+                    got, kernel = _conv(ctx, dx, dw, s, r, 0, tile)
+                    seen.add(kernel // 10)
+                    assert np.array_equal(got, want), (split_k, tile, kernel)
+    finally:
+        ctx.set_option("split_k", 1)
+        ctx.set_precision("tf32x3")
+    assert any(s > 320 for s in seen) or kblocks < 8 or (m, n) == (9841, 40), seen
+    for t in (dx, dw, shift, res):
+        t.dispose()
+
+
+def test_every_cluster_size_is_taken(cuda_context):
+    """The shapes above do reach every variant of the small kernel."""
+    ctx = cuda_context
+    seen = set()
+    for m, n, kblocks in [(76, 4, 1), (44, 4, 8), (37, 4, 14), (32, 8, 19), (36, 4, 20), (66, 4, 24), (70, 4, 30), (3488, 4, 32),
+                          (9841, 40, 1), (8261, 4, 54), (6105, 4, 41), (4061, 4, 36), (3333, 4, 36), (2780, 4, 36), (46, 4, 33),
+                          (33, 4, 40)]:
+        dx, dw = ctx.empty_tensor([1, 1, m, 32 * kblocks]), ctx.empty_tensor([n, 1, 1, 32 * kblocks])
+        for t in (dx, dw):
+            ctx._call("wdc_fill_u32", c_void_p(t.ptr), 0, t.length)
+        ctx.declare_constant(dw)
+        for tile in (32, 64):
+            seen.add(_conv(ctx, dx, dw, None, None, 0, tile)[1] // 10)
+        dx.dispose()
+        dw.dispose()
+    assert {10 * t + c for t in (32, 64) for c in range(1, 9)} <= seen, seen
+
+
+# filter taps around the rotated start, short last blocks of a tap, padding
+@pytest.mark.parametrize("n,cin,cout,size,k", [(1, 64, 64, (56, 56), 3), (2, 100, 68, (9, 9), 3), (1, 36, 132, (20, 21), 3), (1, 512, 132, (7, 7), 3),
+                                               (5, 40, 36, (30, 17), 5), (3, 128, 128, (28, 28), 3)])
+def test_small_convolutions_are_the_same_bits(cuda_context, n, cin, cout, size, k):
+    ctx = cuda_context
+    rng = np.random.default_rng(cin + cout)
+    dx = _put(ctx, rng.standard_normal((n, *size, cin)).astype(np.float32))
+    dw = _put(ctx, rng.standard_normal((cout, k, k, cin)).astype(np.float32))
+    shift = _put(ctx, rng.standard_normal(cout).astype(np.float32))
+    ctx.declare_constant(dw)
+    want, kernel = _conv(ctx, dx, dw, shift, None, k // 2, -1)
+    assert kernel == 0
+    for tile in (32, 64, 32):      # the reads in between wait: later calls load their weights early
+        got, kernel = _conv(ctx, dx, dw, shift, None, k // 2, tile)
+        assert np.array_equal(got, want), (tile, kernel)
+    for t in (dx, dw, shift):
+        t.dispose()
+
+
+# products side by side: few rows, one and several waves of tiles of the small kernel, the whole-SM kernel
+@pytest.mark.parametrize("m", [5, 100, 625, 800, 5000])
+@pytest.mark.parametrize("k,columns,count", [(256, 256, 2), (256, 256, 6), (36, 100, 3), (1024, 64, 2)])
+def test_products_side_by_side_are_the_same_bits(cuda_context, m, k, columns, count):
+    from webdnn_b200.lib import GemmDesc
+    ctx = cuda_context
+    rng = np.random.default_rng(m + k)
+    a, b = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((k, columns * count)).astype(np.float32)
+    c = rng.standard_normal(columns * count).astype(np.float32)
+    da = _put(ctx, a)
+
+    def product(b, c, columns):
+        db, dc, n = _put(ctx, b), _put(ctx, c), b.shape[1]
+        ctx.declare_constant(db)
+        y = ctx.empty_tensor([m, n])
+        ctx.gemm(GemmDesc(batch=1, m=m, n=n, k=k, sab=0, sa0=k, sa1=1, sbb=0, sb0=n, sb1=1, sc0=0, sc1=1, alpha=1.0, beta=1.0, relu=0),
+                 da, db, dc, y, columns)
+        got = y.get_data().reshape(m, n).copy()
+        for t in (db, dc, y):
+            t.dispose()
+        return got
+
+    got = product(b, c, columns)
+    assert max_err_rel_linf(got, a.astype(np.float64) @ b + c) <= 2e-6
+    for i in range(count):
+        at = slice(i * columns, (i + 1) * columns)
+        assert np.array_equal(got[:, at].view(np.uint32), product(b[:, at], c[at], 0).view(np.uint32)), i
+    da.dispose()

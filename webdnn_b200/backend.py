@@ -320,12 +320,14 @@ class WebDNNCudaContext:
         return self._L.lib.wdc_stream(self.handle)
 
     def stats(self, device_memory: bool = False) -> Dict[str, int]:
-        """Arena and traffic counters; with device_memory also the GPU's free / total bytes (cudaMemGetInfo)."""
-        n = 11 if device_memory else 9
+        """Arena and traffic counters; with device_memory also the GPU's free / total bytes (cudaMemGetInfo) and what the
+        last contraction and the last attention ran with (see ``wdc_stats``)."""
+        n = 13 if device_memory else 9
         out = (ctypes.c_int64 * n)()
         self._call("wdc_stats", out, n)
         keys = ["bytes_in_use", "high_water_bytes", "reserved_bytes", "allocs", "frees", "launches",
-                "h2d_bytes", "d2h_bytes", "tensor_core_launches", "device_free_bytes", "device_total_bytes"]
+                "h2d_bytes", "d2h_bytes", "tensor_core_launches", "device_free_bytes", "device_total_bytes", "last_contraction",
+                "last_attention_cluster"]
         return dict(zip(keys[:n], list(out)))
 
     def reset_stats(self) -> None:
@@ -334,7 +336,7 @@ class WebDNNCudaContext:
     PRECISIONS = {"tf32x3": 0, "tf32x1": 1}
 
     def set_option(self, name: str, value: int) -> None:
-        """wdc_set_option: "precision" (0 tf32x3 / 1 tf32x1), "split_k", "pdl", "nvtx"."""
+        """wdc_set_option: "precision" (0 tf32x3 / 1 tf32x1), "split_k", "pdl", "small_tile", "attention_cluster", "nvtx"."""
         self._call("wdc_set_option", name.encode("utf-8"), int(value))
 
     def set_precision(self, precision: str) -> None:
@@ -544,9 +546,14 @@ class WebDNNCudaContext:
         self._call("wdc_binary", op, DTYPE_CODE[a.data_type], c_void_p(a.ptr), c_void_p(b.ptr),
                    c_void_p(out.ptr), len(dims), i64_array(dims), i64_array(sa), i64_array(sb))
 
-    def gemm(self, desc: GemmDesc, a: CudaTensor, b: CudaTensor, c: Optional[CudaTensor], y: CudaTensor) -> None:
-        self._call("wdc_gemm", byref(desc), c_void_p(a.ptr), c_void_p(b.ptr),
-                   c_void_p(c.ptr) if c is not None else None, c_void_p(y.ptr))
+    def gemm(self, desc: GemmDesc, a: CudaTensor, b: CudaTensor, c: Optional[CudaTensor], y: CudaTensor,
+             columns: int = 0) -> None:
+        """``columns``: the result's columns are several products side by side, that many each."""
+        operands = (c_void_p(a.ptr), c_void_p(b.ptr), c_void_p(c.ptr) if c is not None else None, c_void_p(y.ptr))
+        if columns:
+            self._call("wdc_gemm_columns", byref(desc), columns, *operands)
+        else:
+            self._call("wdc_gemm", byref(desc), *operands)
 
     def conv2d(self, desc: ConvDesc, x, w, scale, shift, residual, y) -> None:
         def p(t):

@@ -632,6 +632,8 @@ int launch(wdc_context* ctx, const wdc_attention_desc* d, const float* q, const 
     p.scale_log2 = d->scale * 1.4426950408889634f;
     p.status = ctx->status_word;
     p.cs = choose_cluster(ctx, ceil_div64(d->tq, BQ) * bh, tk, DH == 32 ? 2 : 1);
+    if (ctx->opt_attention_cluster && ctx->opt_attention_cluster <= ceil_div64(tk, BK)) p.cs = ctx->opt_attention_cluster;
+    ctx->last_attention_cluster = p.cs;
     cudaLaunchAttribute attr[2];
     int n_attr = 0;
     if (p.cs > 1) {

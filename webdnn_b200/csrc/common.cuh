@@ -55,6 +55,10 @@ struct wdc_context {
   int opt_precision = 0;                  // 0: tf32x3 (fp32-class accuracy), 1: tf32x1 (one pass, ~1e-3 relative)
   int opt_split_k = 1;                    // 1: small outputs with long reductions may be cut into K ranges
   int opt_pdl = 1;                        // 1: contraction launches use programmatic dependent launch
+  int opt_small_tile = 0;                 // tc_small_kernel: 0 where it is likely faster, 32 / 64 with that tile where it can, -1 never
+  int opt_attention_cluster = 0;          // 0: chosen by size; 1, 2, 4, 8: CTAs per query tile
+  int64_t last_attention_cluster = 0;     // what the last tensor-core attention ran with
+  int64_t last_contraction = 0;           // the last contraction's kernel: 100 * tile width + 10 * cluster + weights early, or 0
   int opt_nvtx = 0;                       // 1: wdc_range_push / wdc_range_pop emit NVTX ranges
   // second stream for host-to-device transfers that overlap the kernels of `stream`
   cudaStream_t copy_stream = nullptr;
@@ -220,7 +224,7 @@ static inline int grid_for(const wdc_context* ctx, int64_t work_items, int threa
 int wdc_tc_conv2d(wdc_context* ctx, const wdc_conv_desc* d, const float* x, const float* w,
                   const float* scale, const float* shift, const float* residual, float* y);
 int wdc_tc_gemm(wdc_context* ctx, const wdc_gemm_desc* d, const float* A, const float* B,
-                const float* C, float* Y);
+                const float* C, float* Y, int64_t columns = 0);   // columns: see wdc_gemm_columns
 // Few-row Gemm on the CUDA cores (gemm_skinny.cu); WDC_ERR_UNSUPPORTED for strides of B it does not take.
 int wdc_skinny_gemm(wdc_context* ctx, const wdc_gemm_desc* d, const float* A, const float* B, const float* C, float* Y);
 // Tensor-core Gemm that splits both operands as it loads them (gemm_tc_direct.cu): any strides, ragged K, batches.

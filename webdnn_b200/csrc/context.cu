@@ -566,6 +566,14 @@ extern "C" int wdc_set_option(wdc_context* ctx, const char* name, int64_t value)
     ctx->opt_split_k = value != 0;
   } else if (n == "pdl") {
     ctx->opt_pdl = value != 0;
+  } else if (n == "small_tile") {
+    if (value != 0 && value != 32 && value != 64 && value != -1)
+      return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_set_option: small_tile is 0, 32, 64 or -1, not %lld", (long long)value);
+    ctx->opt_small_tile = (int)value;
+  } else if (n == "attention_cluster") {
+    if (value != 0 && value != 1 && value != 2 && value != 4 && value != 8)
+      return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_set_option: attention_cluster is 0, 1, 2, 4 or 8, not %lld", (long long)value);
+    ctx->opt_attention_cluster = (int)value;
   } else if (n == "nvtx") {
     ctx->opt_nvtx = value != 0;
   } else {
@@ -590,9 +598,10 @@ extern "C" void* wdc_stream(wdc_context* ctx) { return ctx ? (void*)ctx->stream 
 
 extern "C" int wdc_stats(wdc_context* ctx, int64_t* out, int n) {
   if (!ctx || !out || n < 0) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_stats: bad argument");
-  int64_t v[11] = {ctx->arena.in_use, ctx->arena.high_water, ctx->arena.reserved, ctx->n_alloc,
+  int64_t v[13] = {ctx->arena.in_use, ctx->arena.high_water, ctx->arena.reserved, ctx->n_alloc,
                    ctx->n_free,       ctx->n_launch,         ctx->h2d_bytes,      ctx->d2h_bytes,
-                   ctx->n_tc_launch,  -1,                    -1};
+                   ctx->n_tc_launch,  -1,                    -1,                   ctx->last_contraction,
+                   ctx->last_attention_cluster};
   if (n > 9) {   // device-wide figures (every process and library on the GPU counts), asked only when wanted
     DeviceGuard g(ctx->device);
     size_t free_b = 0, total_b = 0;
@@ -603,7 +612,7 @@ extern "C" int wdc_stats(wdc_context* ctx, int64_t* out, int n) {
       cudaGetLastError();
     }
   }
-  for (int i = 0; i < n && i < 11; i++) out[i] = v[i];
+  for (int i = 0; i < n && i < 13; i++) out[i] = v[i];
   return WDC_OK;
 }
 

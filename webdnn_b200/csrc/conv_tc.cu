@@ -128,6 +128,13 @@ struct TcProblem {
                       //    (2j, 2j+1) are one 32-byte pixel pair: 4 loads of 128 x 32 bytes per K block
   int in_w_pad;       // c4 == 2: pixels per padded input row (even)
   int tiles_m, tiles_n;   // their product fits 31 bits (checked on the host)
+  // tc_small_kernel: K blocks of a part, and the order in which tc_igemm_kernel would walk a whole tile's K blocks:
+  // rotated by the CTA that would compute it, with tiles of rot_tile_n columns, rot_tiles_n beside one another in rot_n
+  // columns, dealt to rot_grid CTAs (rot_grid == 0: from the first K block on)
+  int part;
+  int rot_grid, rot_n, rot_tile_n, rot_tiles_n;
+  int w_row0;         // first row of the weight matrix
+  int64_t y_stride;   // elements from one row of the output to the next
   // epilogue
   const float* scale;     // per channel or null
   const float* shift;     // per channel or null
@@ -296,9 +303,6 @@ __device__ __forceinline__ void unit_of(const TcProblem& p, int u, int& tile, in
   kb0 = sp * p.kbs;
   kbn = p.kblocks - kb0 < p.kbs ? p.kblocks - kb0 : p.kbs;
 }
-
-// Programmatic dependent launch.  wait: everything the grids before this one wrote is visible afterwards (a no-op
-// for a launch without the attribute).  launch_dependents: the next grid of the stream may start its own set-up.
 
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred;
@@ -874,8 +878,8 @@ tc_igemm_kernel(const __grid_constant__ TcProblem p, const float* __restrict__ x
             const int tap = kr / p.cblocks;
             kx0 = tap * p.ch_in + (kr - tap * p.cblocks) * BLOCK_K;
           }
-          tma_load_2d(w_hi_ptr(stage), &map_w_hi, &ss->full_bar[stage], kx0, n0);
-          if (!p.single_pass) tma_load_2d(w_lo_ptr(stage), &map_w_lo, &ss->full_bar[stage], kx0, n0);
+          tma_load_2d(w_hi_ptr(stage), &map_w_hi, &ss->full_bar[stage], kx0, p.w_row0 + n0);
+          if (!p.single_pass) tma_load_2d(w_lo_ptr(stage), &map_w_lo, &ss->full_bar[stage], kx0, p.w_row0 + n0);
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
       }
@@ -1257,7 +1261,7 @@ tc_igemm_kernel(const __grid_constant__ TcProblem p, const float* __restrict__ x
                   if (p.relu) t = relu_nan(t);
                   o[e] = t;
                 }
-                float* yp = y + m * (int64_t)p.N + col;
+                float* yp = y + m * p.y_stride + col;
                 if (vec) *reinterpret_cast<float4*>(yp) = make_float4(o[0], o[1], o[2], o[3]);
                 else {
 #pragma unroll
@@ -1334,7 +1338,7 @@ __global__ void __launch_bounds__(256) split_tf32_transpose_kernel(const float* 
 // Second pass for the tiles whose reduction was cut into ranges: for tile `full_tiles + r`, block (r * splits + s)
 // of the workspace holds the raw partial sums of range s as 128 rows x tile_n columns.  The ranges are added in
 // ascending order (deterministic), then shift, residual and Relu are applied as in the fused epilogue.  N % 4 == 0.
-__global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* ws, float* __restrict__ y,
+__global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* ws, float* __restrict__ y, int64_t y_stride,
                                                             const float* shift, float shift_mul,
                                                             const float* residual, int64_t res_stride,
                                                             float res_mul, int relu, int64_t M, int N, int tile_n,
@@ -1376,7 +1380,7 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* ws, flo
     if (relu) {
       acc.x = relu_nan(acc.x); acc.y = relu_nan(acc.y); acc.z = relu_nan(acc.z); acc.w = relu_nan(acc.w);
     }
-    *reinterpret_cast<float4*>(y + m * N + n) = acc;
+    *reinterpret_cast<float4*>(y + m * y_stride + n) = acc;
   }
 }
 
@@ -1730,27 +1734,69 @@ void choose_tiling(const wdc_context* ctx, int64_t m, int64_t n, int kblocks, bo
   }
 }
 
+typedef void (*SmallKernel)(const TcProblem, const CUtensorMap, const CUtensorMap, const CUtensorMap, float*, int);
+struct SmallVariant {
+  SmallKernel kernel;
+  int smem;
+};
+template <int TN, int CS>
+SmallVariant small_variant() { return {tc_small_kernel<TN, CS>, SmallLayout<TN, CS>::SMEM}; }
+const SmallVariant small_variants[2][8] = {
+    {small_variant<32, 1>(), small_variant<32, 2>(), small_variant<32, 3>(), small_variant<32, 4>(),
+     small_variant<32, 5>(), small_variant<32, 6>(), small_variant<32, 7>(), small_variant<32, 8>()},
+    {small_variant<64, 1>(), small_variant<64, 2>(), small_variant<64, 3>(), small_variant<64, 4>(),
+     small_variant<64, 5>(), small_variant<64, 6>(), small_variant<64, 7>(), small_variant<64, 8>()}};
+constexpr int MAX_DEVICES = 64;
+
+// The variant's shared memory is allowed for on the context's device.
+bool small_ready(wdc_context* ctx, int wide, int cs) {
+  static bool ready[MAX_DEVICES][2][8] = {};
+  if (ctx->device < 0 || ctx->device >= MAX_DEVICES) return false;
+  bool& r = ready[ctx->device][wide][cs - 1];
+  const SmallVariant& v = small_variants[wide][cs - 1];
+  if (!r && cudaFuncSetAttribute(v.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return r = true;
+}
+
 // Tile width and cluster size of tc_small_kernel for an [M, N] output, and whether the launch is likely to be shorter
-// than the persistent kernel's with the tiling given (choose_tiling's).  Microseconds, fitted to the layers of ResNet-50
-// at one image (224 and 800 pixels) and of the DETR-style transformer, each launch behind others in a replayed graph:
-//   small       2.4 (32 columns) or 3.1 (64) + 0.006 per CTA, a K block 0.35 or 0.50, half as much again where two CTAs
-//               share an SM; a cluster adds 0.3 and its exchange, 16 bytes a clock and CTA.  At most two CTAs per SM,
-//               so nothing with more than 296 of them;
-//   persistent  3.6 + 0.03 per column of a tile (set-up, the tile's way out), a K block 0.55 whatever the width; a cut
-//               reduction 4 for the second launch, and the partial sums' way through L2.
-// Some of what it decides, us per launch (persistent -> small): [196, 2304] x 256 13.2 -> 7.2, [49, 512] x 2048 12.8 ->
-// 6.4, [100, 2048] x 256 11.8 -> 6.0, [1280, 1024] x 256 21.2 -> 10.3, [625, 2048] x 512 18.2 -> 15.6.
-bool choose_small(const wdc_context* ctx, const TcProblem& p, int tile_n, int splits, int full_tiles, int* tn, int* cs) {
+// than the persistent kernel's with the tiling given (choose_tiling's, for `n_one` of the N columns).  A tile is computed
+// as a whole, or in the parts that the persistent kernel adds up (see conv_tc_small.cuh), one CTA of a cluster each.
+// Nothing with more CTAs than two per SM, or seven eighths of that in clusters: a cluster lies within one of the GPU's
+// groups of SMs, and what does not come out even there leaves places empty (256 CTAs in clusters of 4 or 8 run at once,
+// 280 of 7 and 288 of 6 take 1.5 times as long: [625, 512] x 4608 31 us, 20 by the persistent kernel).
+// Microseconds, fitted to the layers of ResNet-50 at one image (224 and 800 pixels), at five of 250 (tf32x1) and of the
+// DETR-style transformer, launches back to back in a replayed graph; a K block's at tf32x3 / tf32x1:
+//   small       2.4 (32 columns) or 3.1 (64) + 0.006 per CTA, a K block 0.35 / 0.26 or 0.50 / 0.38, 1.45 / 1.25 times that
+//               where two CTAs share an SM; a cluster adds 0.3 and its exchange, 16 bytes a clock and CTA;
+//   persistent  4.4, 5.0 and 5.7 for tiles of 32, 64 and 128 columns, a K block 0.29 / 0.28, 0.35 / 0.29 and 0.46 / 0.32;
+//               a cut reduction 3.7 for the second launch, and the partial sums' way through L2.
+// Some of what it decides, us per launch (persistent -> small), all at tf32x3 but the last: [196, 256] x 2304 10.9 -> 7.0,
+// [49, 512] x 2048 10.3 -> 6.4, [100, 2048] x 256 7.5 -> 4.8, [784, 128] x 512 9.1 -> 4.5, [625, 256] x 2048 13.1 -> 11.1,
+// [320, 512] x 2048 12.5 -> 9.4; and not (persistent, small): [2500, 256] x 1024 16.2, 18.9; [625, 2048] x 512 13.2, 14.2.
+bool choose_small(const wdc_context* ctx, const TcProblem& p, int n_one, int tile_n, int splits, int full_tiles, int* tn, int* cs) {
   const int64_t tiles_m = ceil_div64(p.M, TILE_M);
-  const int sms = ctx->sm_count;
+  const int sms = ctx->sm_count, one = p.single_pass;
   const int rows = p.M < TILE_M ? (int)p.M : TILE_M;
+  if (splits > 1 && full_tiles > 0) return false;   // whole tiles and cut ones: their parts differ
+  const int parts = splits > 1 ? splits : segments_of(p.kblocks);
+  const int part = splits > 1 ? (p.kblocks + splits - 1) / splits : SEG_KBLOCKS;
+  const double small_kb[2][2] = {{0.35, 0.50}, {0.26, 0.38}}, shared[2] = {1.45, 1.25};
+  const double whole_kb[2][3] = {{0.29, 0.35, 0.46}, {0.28, 0.29, 0.32}}, whole_base[3] = {4.4, 5.0, 5.7};
   double best = 1e30;
-  for (int t = 32; t <= 64; t *= 2) {
+  for (int wide = 0; wide < 2; wide++) {
+    const int t = wide ? 64 : 32;
+    if (t > tile_n && splits == 1) break;           // its columns would be rotated differently
+    if (n_one < p.N && n_one % t != 0) continue;    // a tile would reach from one product into the next
+    if (ctx->opt_small_tile && t != ctx->opt_small_tile) continue;
     const int64_t tiles = tiles_m * ceil_div64(p.N, t);
-    for (int c = 1; c <= 8; c *= 2) {
-      const int kbs = (p.kblocks + c - 1) / c;
-      if (tiles * c > 2 * sms || (c - 1) * kbs >= p.kblocks || (c > 1 && !ctx->opt_split_k)) break;
-      double us = (t == 32 ? 2.4 : 3.1) + 0.006 * (double)(tiles * c) + kbs * (t == 32 ? 0.35 : 0.50) * (tiles * c > sms ? 1.45 : 1.0);
+    for (int c = 1; c <= parts; c += parts > 1 ? parts - 1 : 1) {
+      if (c == 1 && (splits > 1 || (parts > 1 && parts <= 8 && ctx->opt_small_tile && ctx->opt_split_k))) continue;
+      if (c > 8 || (c > 1 && !ctx->opt_split_k) || tiles * c > (c > 1 ? 7 * sms / 4 : 2 * sms)) break;
+      const int last = p.kblocks - (c - 1) * part, kbs = c == 1 || last > part ? last : part;
+      double us = (wide ? 3.1 : 2.4) + 0.006 * (double)(tiles * c) + kbs * small_kb[one][wide] * (tiles * c > sms ? shared[one] : 1.0);
       if (c > 1) us += 0.3 + rows * t * 4.0 * (c - 1) / c / 16 / 1900;
       if (us < best) {
         best = us;
@@ -1759,41 +1805,28 @@ bool choose_small(const wdc_context* ctx, const TcProblem& p, int tile_n, int sp
       }
     }
   }
-  const int64_t tiles = tiles_m * ceil_div64(p.N, tile_n);
-  double big = 3.6 + 0.03 * tile_n;
+  if (ctx->opt_small_tile) return best < 1e30;
+  const int64_t tiles = tiles_m * ceil_div64(n_one, tile_n);
+  const int w = tile_n == 128 ? 2 : tile_n == 64 ? 1 : 0;
+  double big = whole_base[w];
   if (splits == 1) {
-    big += (double)ceil_div64(tiles, sms) * p.kblocks * 0.55;
+    big += (double)ceil_div64(tiles, sms) * p.kblocks * whole_kb[one][w];
   } else {
-    const int64_t rest = tiles - full_tiles;
-    const int kbs = (p.kblocks + splits - 1) / splits;
-    big += ((double)(full_tiles / sms) * p.kblocks + (double)ceil_div64(rest * splits, sms) * kbs) * 0.55;
-    big += 4.0 + 2.0 * (double)(rest * splits) * TILE_M * tile_n * 4 / 6.5e6;
+    big += (double)ceil_div64(tiles * splits, sms) * part * whole_kb[one][w];
+    big += 3.7 + (double)(tiles * splits) * TILE_M * tile_n * 4 / 6.5e6;
   }
-  return best < big;
+  return best < big * ((double)p.N / n_one);
 }
 
-// A launch of tc_small_kernel: p.kblocks, tile counts and geometry are set; `tn` and `cs` chosen by the caller.
+// A launch of tc_small_kernel: p.kblocks, p.part and geometry are set; `tn` and `cs` chosen by choose_small.
 int launch_small(wdc_context* ctx, TcProblem& p, WeightEntry* we, const CUtensorMap& map_a, float* y, int tn, int cs) {
-  typedef void (*Kernel)(const TcProblem, const CUtensorMap, const CUtensorMap, const CUtensorMap, float*, int);
-  static const Kernel kernels[2][4] = {
-      {tc_small_kernel<32, 1>, tc_small_kernel<32, 2>, tc_small_kernel<32, 4>, tc_small_kernel<32, 8>},
-      {tc_small_kernel<64, 1>, tc_small_kernel<64, 2>, tc_small_kernel<64, 4>, tc_small_kernel<64, 8>}};
-  const int wide = tn == 64, ci = cs == 8 ? 3 : cs == 4 ? 2 : cs == 2 ? 1 : 0;
-  const Kernel kernel = kernels[wide][ci];
-  const int smem = wide ? SmallLayout<64>::SMEM : SmallLayout<32>::SMEM;
-  static bool attr_set[64][2][4] = {};
-  if (ctx->device < 0 || ctx->device >= 64) return WDC_ERR_UNSUPPORTED;
-  if (!attr_set[ctx->device][wide][ci]) {
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
-      cudaGetLastError();
-      return WDC_ERR_UNSUPPORTED;
-    }
-    attr_set[ctx->device][wide][ci] = true;
-  }
+  const int wide = tn == 64;
+  if (!small_ready(ctx, wide, cs)) return WDC_ERR_UNSUPPORTED;
+  const SmallKernel kernel = small_variants[wide][cs - 1].kernel;
+  const int smem = small_variants[wide][cs - 1].smem;
   p.tile_n = tn;
   p.tiles_m = (int)ceil_div64(p.M, TILE_M);
   p.tiles_n = (int)ceil_div64(p.N, tn);
-  p.kbs = (p.kblocks + cs - 1) / cs;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
@@ -1812,6 +1845,7 @@ int launch_small(wdc_context* ctx, TcProblem& p, WeightEntry* we, const CUtensor
   cudaError_t le = cudaLaunchKernelEx(&cfg, kernel, pc, we->map_hi[mi], we->map_lo[mi], map_a, y, we->settled ? 1 : 0);
   ctx->n_tc_launch++;
   ctx->n_launch++;
+  ctx->last_contraction = tn * 100 + cs * 10 + (we->settled ? 1 : 0);
   int s = wdc_check_cuda(ctx, le, "tc_small_kernel");
   if (s == WDC_OK) s = wdc_check_cuda(ctx, cudaGetLastError(), "tc_small_kernel");
   return s;
@@ -1830,8 +1864,39 @@ int weight_maps(wdc_context* ctx, WeightEntry* we, int tile_n) {
   return WDC_OK;
 }
 
+int launch_whole(wdc_context* ctx, TcProblem& p, WeightEntry* we, const float* x, float* y);
+
+// The columns p.w_row0 .. + p.N of the product, by the kernel that suits their number; results as if columns were
+// computed `n_one` at a time (see launch_tc).  With `small_only` false is returned where that is tc_igemm_kernel.
+bool launch_columns(wdc_context* ctx, TcProblem p, WeightEntry* we, const float* x, float* y, int n_one, bool small_only, int* status) {
+  // a split reduction needs the TMA paths on both sides (checked again in launch_whole) and no first-layer mode
+  const bool may_cut = !p.c4 && p.N % 4 == 0 && p.M < (1ll << 27) && tc_state(ctx)->encode_im2col != nullptr &&
+                       (((uintptr_t)p.shift | (uintptr_t)p.residual | (uintptr_t)y) & 15) == 0 &&
+                       (!p.residual || p.res_stride % 4 == 0);
+  const bool may_split = may_cut && ctx->opt_split_k;
+  choose_tiling(ctx, p.M, n_one, p.kblocks, may_split, &p.tile_n, &p.splits, &p.full_tiles);
+  int tn = 0, cs = 0;
+  CUtensorMap map_a;
+  if (may_cut && we->constant && ctx->opt_small_tile >= 0 &&
+      choose_small(ctx, p, n_one, p.tile_n, p.splits, p.full_tiles, &tn, &cs) && encode_a_map(tc_state(ctx), p, x, &map_a)) {
+    p.part = p.splits > 1 ? (p.kblocks + p.splits - 1) / p.splits : SEG_KBLOCKS;
+    p.rot_n = n_one;
+    p.rot_tile_n = p.tile_n;
+    p.rot_tiles_n = (int)ceil_div64(n_one, p.tile_n);
+    const int64_t tiles = ceil_div64(p.M, TILE_M) * p.rot_tiles_n;
+    p.rot_grid = p.splits > 1 ? 0 : tiles < ctx->sm_count ? (int)tiles : ctx->sm_count;
+    *status = weight_maps(ctx, we, tn);
+    if (*status == WDC_OK) *status = launch_small(ctx, p, we, map_a, y, tn, cs);
+    return true;
+  }
+  if (!small_only) *status = launch_whole(ctx, p, we, x, y);
+  return !small_only;
+}
+
+// `columns` > 0 (a divisor of p.N): the output's columns are several products beside one another, that many each.  Their
+// results are those of the products one by one: the order of the additions follows from a product's own size.
 int launch_tc(wdc_context* ctx, TcProblem& p, const float* x, const float* w, float* y, int c4_kw = 0,
-              int c4_cin = 0, bool w_k_major = true) {
+              int c4_cin = 0, bool w_k_major = true, int columns = 0) {
   WeightEntry* we = nullptr;
   int s = get_weight(ctx, w, p.scale, p.alpha, p.N, p.K, &we, p.c4 ? p.K / 32 : 0, c4_kw, c4_cin, w_k_major);
   if (s != WDC_OK) return s;
@@ -1840,36 +1905,30 @@ int launch_tc(wdc_context* ctx, TcProblem& p, const float* x, const float* w, fl
   p.kblocks = p.c4 ? p.K / BLOCK_K : p.k_h * p.k_w * p.cblocks;   // K blocks are counted per filter tap
   p.status = ctx->status_word;
   p.single_pass = ctx->opt_precision == 1 ? 1 : 0;
-  {
-    // a split reduction needs the TMA paths on both sides (checked again below) and no first-layer mode
-    const bool may_cut = !p.c4 && p.N % 4 == 0 && p.M < (1ll << 27) && tc_state(ctx)->encode_im2col != nullptr &&
-                         (((uintptr_t)p.shift | (uintptr_t)p.residual | (uintptr_t)y) & 15) == 0 &&
-                         (!p.residual || p.res_stride % 4 == 0);
-    const bool may_split = may_cut && ctx->opt_split_k;
-    choose_tiling(ctx, p.M, p.N, p.kblocks, may_split, &p.tile_n, &p.splits, &p.full_tiles);
-    int tn = 0, cs = 0;
-    bool small = may_cut && we->constant && choose_small(ctx, p, p.tile_n, p.splits, p.full_tiles, &tn, &cs);
-#ifdef WDC_TC_DEVELOP
-    if (const char* e = getenv("WDC_TC_SMALL")) {   // "tn,cs" forces the small kernel with that shape, "0,0" the other
-      sscanf(e, "%d,%d", &tn, &cs);
-      small = may_cut && we->constant && tn > 0;
-    }
-#endif
-    CUtensorMap map_a;
-    if (small && encode_a_map(tc_state(ctx), p, x, &map_a)) {
-      s = weight_maps(ctx, we, tn);
-      return s != WDC_OK ? s : launch_small(ctx, p, we, map_a, y, tn, cs);
-    }
+  p.y_stride = p.N;
+  const int n = p.N, n_one = columns > 0 ? columns : n;
+  if (launch_columns(ctx, p, we, x, y, n_one, n_one < n, &s) || n_one == n) return s;
+  for (int col = 0; col < n && s == WDC_OK; col += n_one) {
+    TcProblem q = p;
+    q.N = n_one;
+    q.w_row0 = col;
+    if (p.shift) q.shift = p.shift + col;
+    if (p.residual) q.residual = p.residual + col;
+    launch_columns(ctx, q, we, x, y + col, n_one, false, &s);
   }
+  return s;
+}
+
+// tc_igemm_kernel with the tiling that is set.
+int launch_whole(wdc_context* ctx, TcProblem& p, WeightEntry* we, const float* x, float* y) {
   const int mi = p.tile_n == 128 ? 2 : p.tile_n == 64 ? 1 : 0;
-  s = weight_maps(ctx, we, p.tile_n);
+  int s = weight_maps(ctx, we, p.tile_n);
   if (s != WDC_OK) return s;
   const CUtensorMap& w_map_hi = we->map_hi[mi];
   const CUtensorMap& w_map_lo = we->map_lo[mi];
   if (ceil_div64(p.M, TILE_M) * ceil_div64(p.N, p.tile_n) >= (1ll << 31) - 65536) return WDC_ERR_UNSUPPORTED;
   p.tiles_m = (int)ceil_div64(p.M, TILE_M);
   p.tiles_n = (int)ceil_div64(p.N, p.tile_n);
-  p.status = ctx->status_word;
   p.nap_ns = 100;
 #ifdef WDC_TC_DEVELOP
   {
@@ -1895,7 +1954,6 @@ int launch_tc(wdc_context* ctx, TcProblem& p, const float* x, const float* w, fl
     p.prof = prof_buf;
   }
 #endif
-  p.single_pass = ctx->opt_precision == 1 ? 1 : 0;
   TcState* st = tc_state(ctx);
   const int total_tiles = p.tiles_m * p.tiles_n;
   float* ws = nullptr;
@@ -1912,7 +1970,7 @@ int launch_tc(wdc_context* ctx, TcProblem& p, const float* x, const float* w, fl
     // (narrow tiles fed by TMA have four epilogue warps of tile_n columns each, all others eight of tile_n / 2)
     const int ncols = duo_mode(p, a_by_tma) ? p.tile_n : p.tile_n / 2, cw = ncols < 32 ? ncols : 32;
     bool can = (p.N % 4 == 0) && p.M < (1ll << 31) && !TC_DBG(p, 64) && (((uintptr_t)p.scale | (uintptr_t)p.shift) & 15) == 0;
-    if (can) can = encode_rows_map(st, &map_y, y, p.M, p.N, p.N, cw) == 0;
+    if (can) can = encode_rows_map(st, &map_y, y, p.M, p.N, p.y_stride, cw) == 0;
     if (can && p.residual)
       can = p.res_stride % 4 == 0 && encode_rows_map(st, &map_res, p.residual, p.M, p.N, p.res_stride, cw) == 0;
     p.tma_epi = can ? 1 : 0;
@@ -1958,6 +2016,7 @@ int launch_tc(wdc_context* ctx, TcProblem& p, const float* x, const float* w, fl
     le = cudaLaunchKernelEx(&cfg, tc_igemm_kernel<false>, pc, x, w_map_hi, w_map_lo, w_map_hi, map_y, map_res, map_ws, y);
   ctx->n_tc_launch++;
   ctx->n_launch++;
+  ctx->last_contraction = 0;
   s = wdc_check_cuda(ctx, le, "tc_igemm_kernel");
   if (s == WDC_OK) s = wdc_check_cuda(ctx, cudaGetLastError(), "tc_igemm_kernel");
 #ifdef WDC_TC_DEVELOP
@@ -1992,7 +2051,7 @@ int launch_tc(wdc_context* ctx, TcProblem& p, const float* x, const float* w, fl
       rc.stream = ctx->stream;
       rc.attrs = attr;
       rc.numAttrs = ctx->opt_pdl ? 1 : 0;
-      le = cudaLaunchKernelEx(&rc, splitk_reduce_kernel, (const float*)ws, y, p.shift, p.shift_mul, p.residual,
+      le = cudaLaunchKernelEx(&rc, splitk_reduce_kernel, (const float*)ws, y, p.y_stride, p.shift, p.shift_mul, p.residual,
                               p.res_stride, p.res_mul, p.relu, p.M, p.N, p.tile_n, p.tiles_n, p.full_tiles, rest_tiles,
                               p.splits);
       ctx->n_launch++;
@@ -2101,7 +2160,7 @@ int wdc_tc_conv2d(wdc_context* ctx, const wdc_conv_desc* d, const float* x, cons
 }
 
 int wdc_tc_gemm(wdc_context* ctx, const wdc_gemm_desc* d, const float* A, const float* B, const float* C,
-                float* Y) {
+                float* Y, int64_t columns) {
   // A [m, k] with k contiguous; B either [n, k] with k contiguous (Gemm transB=1, LSTM weights) or [k, n] with n
   // contiguous (MatMul, Gemm transB=0: transposed while it is split).  A batch whose B is shared (stride 0) and
   // whose A and Y are stacked without gaps is one tall matrix.
@@ -2136,5 +2195,5 @@ int wdc_tc_gemm(wdc_context* ctx, const wdc_gemm_desc* d, const float* A, const 
   p.cblocks = (int)((d->k + BLOCK_K - 1) / BLOCK_K);
   p.shift = shift; p.residual = residual; p.res_stride = res_stride;
   p.alpha = d->alpha; p.shift_mul = d->beta; p.res_mul = d->beta; p.relu = d->relu;
-  return launch_tc(ctx, p, A, B, Y, 0, 0, b_k_major);
+  return launch_tc(ctx, p, A, B, Y, 0, 0, b_k_major, (int)columns);
 }

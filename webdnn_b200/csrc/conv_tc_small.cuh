@@ -4,10 +4,11 @@
 // Such a launch is bound by latency.  The persistent kernel takes the whole SM (512 threads x 128 registers, 218 KB,
 // all of tensor memory), so a launch cannot begin its set-up while the one before it drains; its tiles walk the whole
 // reduction; and a reduction cut into ranges needs a second launch.  Here
-//   * a CTA computes one 128 x TN tile over one range of K and takes less than half an SM (352 threads x <= 88
-//     registers, 97 KB, 256 TMEM columns): under programmatic dependent launch the next launch's CTAs sit beside
-//     this one's, with barriers, tensor memory and the first weight tiles ready when the wait for this one ends;
-//   * the ranges of a tile are the CTAs of a thread-block cluster: each sends its partial sums to the CTA that
+//   * a CTA computes one 128 x TN tile over one part of K and takes less than half an SM (352 threads x <= 88
+//     registers, 256 TMEM columns, 96 KB of stages and, with 32 columns, up to 18 KB for the exchange): under
+//     programmatic dependent launch the next launch's CTAs sit beside this one's, with barriers, tensor memory and the
+//     first weight tiles ready when the wait for this one ends;
+//   * the parts of a tile are the CTAs of a thread-block cluster: each sends its partial sums to the CTA that
 //     finishes the row (st.async into distributed shared memory), which adds them in rank order and runs the epilogue;
 //   * a barrier operation answers after 150-250 cycles whatever it finds, and one warp's operations on the way of a
 //     K block add up: with separate rings for A, W and tensor memory the issuing lane's three waits and two commits
@@ -17,7 +18,11 @@
 //   * warps 0-7 split A into tensor memory in two groups that take alternate K blocks, and become the epilogue.
 // (The high part of A straight from its shared-memory tile would save the splitters half their work, but an MMA with
 // A in shared memory took about 64 cycles whatever its width: 730-880 cycles per K block.)
-// The products and the two-level accumulation are those of tc_igemm_kernel.
+// The products are those of tc_igemm_kernel, and so is the order of every addition, whatever the tile and the cluster: a
+// result does not depend on which of the two kernels a launch takes.  That matters where a network carries the last bits
+// on: a softmax over large scores is an argmax, and close rivals exchange places.  The parts are therefore the terms that
+// kernel adds up in fp32: where it takes a tile whole, its segments of SEG_KBLOCKS K blocks, walked from the same rotated
+// start and added behind the addend; where it cuts a tile, its ranges.
 
 constexpr int SM_SPLIT_WARPS = 8;
 constexpr int SM_A_WARP = 8, SM_W_WARP = 9, SM_MMA_WARP = 10;
@@ -25,8 +30,10 @@ constexpr int SM_THREADS = 352;
 constexpr int SM_EPI_THREADS = SM_SPLIT_WARPS * 32;
 constexpr int SM_TMEM_COLS = 256;
 
-template <int TN>
+// ROWS: rows of a tile that a CTA finishes, at most.
+template <int TN, int CS>
 struct SmallLayout {
+  static constexpr int ROWS = (TILE_M + CS - 1) / CS;
   static constexpr int W_BYTES = TN * 128;                 // one of the two parts of a weight tile
   static constexpr int STAGES = TN == 64 ? 3 : 4;
   static constexpr int STAGE = A_TILE_BYTES + 2 * W_BYTES;
@@ -40,9 +47,11 @@ struct SmallLayout {
   // SM and reuses the stages, for which the cluster has to meet after its last MMA.
   static constexpr bool OWN_EXCHANGE = TN == 32;
   static constexpr int EXCHANGE_OFF = OWN_EXCHANGE ? BYTES : 0;
-  static constexpr int SHARED_OFF = BYTES + (OWN_EXCHANGE ? TILE_M * TN * 4 : 0);
+  static constexpr int EXCHANGE = CS * ROWS * TN * 4;
+  static constexpr int SHARED_OFF = BYTES + (OWN_EXCHANGE ? EXCHANGE : 0);
   static constexpr int SMEM = SHARED_OFF + 256;            // no slack: the buffer itself is aligned (checked below)
-  static_assert(TILE_M * TN * 4 <= BYTES, "the exchanged sums fit the stages");
+  static_assert(EXCHANGE <= BYTES, "the exchanged sums fit the stages");
+  static_assert(2 * (SMEM + 1024) <= 228 * 1024, "two CTAs on an SM");
 };
 
 struct SmallShared {
@@ -94,23 +103,23 @@ __device__ __forceinline__ void tma_load_im2col_at(uint32_t dst, const CUtensorM
 }
 
 // Where the 16-byte cell (row, cell) of one source's sums lies in the exchange buffer of a CTA that finishes ROWS rows:
-// consecutive rows of a cell are consecutive words (one block per store of a warp), turned by the cell so that a row's
-// cells lie in different banks.
+// consecutive rows of a cell are consecutive words (one block per store of a warp), turned by the cell where ROWS is a
+// power of two, so that a row's cells lie in different banks.
 template <int ROWS>
 __device__ __forceinline__ uint32_t exchange_slot(uint32_t row, uint32_t cell) {
-  return cell * ROWS + (row ^ (cell & 7u));
+  return cell * ROWS + (ROWS % 8 == 0 ? row ^ (cell & 7u) : row);
 }
 
-// CS: CTAs of a cluster = ranges of K.  grid: tiles_m * tiles_n * CS.
+// CS: CTAs of a cluster = parts of K (1: the tile as a whole).  grid: tiles_m * tiles_n * CS.
 template <int TN, int CS>
 __global__ void __launch_bounds__(SM_THREADS, 2)
 tc_small_kernel(const __grid_constant__ TcProblem p, const __grid_constant__ CUtensorMap map_w_hi,
                 const __grid_constant__ CUtensorMap map_w_lo, const __grid_constant__ CUtensorMap map_a,
                 float* __restrict__ y, int w_early) {
-  using L = SmallLayout<TN>;
-  constexpr int ROWS = TILE_M / CS;                        // rows of the tile this CTA finishes, at most
+  using L = SmallLayout<TN, CS>;
+  constexpr int ROWS = L::ROWS;
   constexpr int CELLS = TN / 4;
-  constexpr int ITEMS = ROWS * CELLS / SM_EPI_THREADS > 0 ? ROWS * CELLS / SM_EPI_THREADS : 1;
+  constexpr int ITEMS = (ROWS * CELLS + SM_EPI_THREADS - 1) / SM_EPI_THREADS;
   constexpr int COLS = TN / 2;                             // accumulator columns of a warp
   extern __shared__ __align__(1024) unsigned char smem_small[];
   unsigned char* smem = smem_small;
@@ -119,9 +128,16 @@ tc_small_kernel(const __grid_constant__ TcProblem p, const __grid_constant__ CUt
   const int rank = (int)(blockIdx.x % CS), tile = (int)(blockIdx.x / CS);
   const int n0 = (tile % p.tiles_n) * TN;
   const int64_t m0 = (int64_t)(tile / p.tiles_n) * TILE_M;
-  const int kb0 = rank * p.kbs;                            // this CTA's range of K blocks (never empty)
-  const int nkb = p.kblocks - kb0 < p.kbs ? p.kblocks - kb0 : p.kbs;
+  // this CTA's part of the reduction (never empty): nkb K blocks from kb0 on, around the end where the tile is rotated
+  const int first_kb = CS == 1 ? 0 : rank * p.part;
+  const int nkb = rank == CS - 1 ? p.kblocks - first_kb : p.part;
   const int nseg = segments_of(nkb);
+  int kb0 = first_kb;
+  if (p.rot_grid) {
+    const uint32_t whole = (uint32_t)(tile / p.tiles_n) * (uint32_t)p.rot_tiles_n + (uint32_t)(n0 % p.rot_n / p.rot_tile_n);
+    kb0 += (int)(whole % (uint32_t)p.rot_grid * (uint32_t)p.kblocks / (uint32_t)p.rot_grid);
+    if (kb0 >= p.kblocks) kb0 -= p.kblocks;
+  }
   // the tile's rows that exist are finished in equal shares: the exchange is 16 bytes a clock, so rows past M stay out
   const int rows = p.M - m0 < TILE_M ? (int)(p.M - m0) : TILE_M;
   const int share = (rows + CS - 1) / CS;
@@ -190,7 +206,19 @@ tc_small_kernel(const __grid_constant__ TcProblem p, const __grid_constant__ CUt
       if (lane == 0) arrive_at(smem_u32(&ss->seg_empty[buf]));
       drained++;
     };
-    pdl_grid_wait();   // (before the residual and the output are touched; the tiles come after it anyway)
+    pdl_grid_wait();   // (before the addend, the residual and the output are touched; the tiles come after it anyway)
+    if (CS == 1 && p.shift) {
+#pragma unroll
+      for (int j = 0; j < COLS; j += 4) {
+        const int n = n0 + half * COLS + j;
+        if (n >= p.N) break;
+        const float4 b = pdl_ld(reinterpret_cast<const float4*>(p.shift + n));
+        acc[j] = p.shift_mul * b.x;
+        acc[j + 1] = p.shift_mul * b.y;
+        acc[j + 2] = p.shift_mul * b.z;
+        acc[j + 3] = p.shift_mul * b.w;
+      }
+    }
     const uint32_t full0 = smem_u32(&ss->full[0]), empty0 = smem_u32(&ss->empty[0]), tfull0 = smem_u32(&ss->t_full[0]);
     // stage and tensor-memory stage of K block kb; `old` = those of kb - T_ST, whose commit frees the latter
     int st = half, ts = half;
@@ -258,17 +286,19 @@ tc_small_kernel(const __grid_constant__ TcProblem p, const __grid_constant__ CUt
       int cb = kb0 - tap0 * p.cblocks, kx0 = tap0 * p.ch_in + cb * BLOCK_K;   // a tap's last block may be short
       uint32_t bar = smem_u32(&ss->full[0]), dst = smem_u32(smem) + (uint32_t)A_TILE_BYTES, par = 1;
       constexpr uint32_t to_empty = (uint32_t)(offsetof(SmallShared, empty) - offsetof(SmallShared, full));
-      int st = 0;
+      const int row0 = p.w_row0 + n0;
+      int st = 0, to_end = p.kblocks - kb0;
       for (int kb = 0; kb < nkb; kb++) {
         if (kb >= L::STAGES && !small_wait(bar + to_empty, par, ss, p.status, 54)) break;
         expect_at(bar, w_bytes);
-        tma_load_2d_at(dst, &map_w_hi, bar, kx0, n0);
-        if (!p.single_pass) tma_load_2d_at(dst + (uint32_t)L::W_BYTES, &map_w_lo, bar, kx0, n0);
+        tma_load_2d_at(dst, &map_w_hi, bar, kx0, row0);
+        if (!p.single_pass) tma_load_2d_at(dst + (uint32_t)L::W_BYTES, &map_w_lo, bar, kx0, row0);
         kx0 += BLOCK_K;
         if (++cb == p.cblocks) {
           cb = 0;
           kx0 += p.ch_in - p.cblocks * BLOCK_K;
         }
+        if (--to_end == 0) cb = kx0 = 0;
         bar += 8u;
         dst += (uint32_t)L::STAGE;
         if (++st == L::STAGES) {
@@ -294,7 +324,7 @@ tc_small_kernel(const __grid_constant__ TcProblem p, const __grid_constant__ CUt
       pdl_let_next_start();
       uint32_t bar = smem_u32(&ss->full[0]), dst = smem_u32(smem), par = 1;
       constexpr uint32_t to_empty = (uint32_t)(offsetof(SmallShared, empty) - offsetof(SmallShared, full));
-      int st = 0, dx = kx * p.dil_w, dy = ky * p.dil_h;
+      int st = 0, dx = kx * p.dil_w, dy = ky * p.dil_h, taps = p.k_h * p.k_w - tap0;
       for (int kb = 0; kb < nkb; kb++) {
         if (kb >= L::STAGES && !small_wait(bar + to_empty, par, ss, p.status, 55)) break;
         expect_at(bar, (uint32_t)A_TILE_BYTES);
@@ -304,6 +334,7 @@ tc_small_kernel(const __grid_constant__ TcProblem p, const __grid_constant__ CUt
           c0 = 0;
           dx += p.dil_w;
           if (++kx == p.k_w) { kx = 0; dx = 0; dy += p.dil_h; }
+          if (--taps == 0) kx = dx = dy = 0;
         }
         bar += 8u;
         dst += (uint32_t)L::STAGE;
@@ -411,7 +442,7 @@ tc_small_kernel(const __grid_constant__ TcProblem p, const __grid_constant__ CUt
       }
     }
     // residual and addend are on their way while the sums are
-    float4 out[ITEMS];
+    float4 out[ITEMS], res[ITEMS];
     bool live[ITEMS];
 #pragma unroll
     for (int i = 0; i < ITEMS; i++) {
@@ -420,17 +451,11 @@ tc_small_kernel(const __grid_constant__ TcProblem p, const __grid_constant__ CUt
       live[i] = r < mine && n < p.N;
       out[i] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (live[i]) {
-        if (p.shift) {
+        if (CS > 1 && p.shift) {
           const float4 b = pdl_ld(reinterpret_cast<const float4*>(p.shift + n));
           out[i] = make_float4(p.shift_mul * b.x, p.shift_mul * b.y, p.shift_mul * b.z, p.shift_mul * b.w);
         }
-        if (p.residual) {
-          const float4 x = pdl_ld(reinterpret_cast<const float4*>(p.residual + m * p.res_stride + n));
-          out[i].x = fmaf(p.res_mul, x.x, out[i].x);
-          out[i].y = fmaf(p.res_mul, x.y, out[i].y);
-          out[i].z = fmaf(p.res_mul, x.z, out[i].z);
-          out[i].w = fmaf(p.res_mul, x.w, out[i].w);
-        }
+        if (p.residual) res[i] = pdl_ld(reinterpret_cast<const float4*>(p.residual + m * p.res_stride + n));
       }
     }
     if (CS > 1) ok = sums_ok && small_wait(smem_u32(&ss->recv), 0, ss, p.status, 59);
@@ -444,17 +469,22 @@ tc_small_kernel(const __grid_constant__ TcProblem p, const __grid_constant__ CUt
         if (!live[i]) continue;
         const int item = threadIdx.x + i * SM_EPI_THREADS, r = item / CELLS, cell = item % CELLS;
         const unsigned char* src = smem + L::EXCHANGE_OFF + exchange_slot<ROWS>((uint32_t)r, (uint32_t)cell) * 16u;
-        float4 s = *reinterpret_cast<const float4*>(src);
+        float4 s = CS > 1 ? out[i] : *reinterpret_cast<const float4*>(src);
 #pragma unroll
-        for (int q = 1; q < CS; q++) {
+        for (int q = 0; CS > 1 && q < CS; q++) {
           const float4 v = *reinterpret_cast<const float4*>(src + q * (CELLS * ROWS * 16));
           s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
         }
-        s.x += out[i].x; s.y += out[i].y; s.z += out[i].z; s.w += out[i].w;
+        if (p.residual) {
+          s.x = fmaf(p.res_mul, res[i].x, s.x);
+          s.y = fmaf(p.res_mul, res[i].y, s.y);
+          s.z = fmaf(p.res_mul, res[i].z, s.z);
+          s.w = fmaf(p.res_mul, res[i].w, s.w);
+        }
         if (p.relu) {
           s.x = relu_nan(s.x); s.y = relu_nan(s.y); s.z = relu_nan(s.z); s.w = relu_nan(s.w);
         }
-        *reinterpret_cast<float4*>(y + (m0 + rank * share + r) * (int64_t)p.N + n0 + cell * 4) = s;
+        *reinterpret_cast<float4*>(y + (m0 + rank * share + r) * p.y_stride + n0 + cell * 4) = s;
       }
     }
   }

@@ -205,10 +205,8 @@ int wdc_simt_conv2d(wdc_context* ctx, const wdc_conv_desc* d, const float* x, co
 }
 
 // ------------------------------------------------------------------------ public entries
-extern "C" int wdc_gemm(wdc_context* ctx, const wdc_gemm_desc* d, const float* A, const float* B,
-                        const float* C, float* Y) {
-  if (!ctx) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_gemm: null context");
-  WDC_TAPE(ctx, wdc_gemm, tape_desc(d), A, B, C, Y);
+static int gemm_call(wdc_context* ctx, const wdc_gemm_desc* d, int64_t columns, const float* A, const float* B,
+                     const float* C, float* Y) {
   wdc_note_write(ctx, Y);
   WDC_REQUIRE(ctx, d != nullptr, "wdc_gemm: null descriptor");
   WDC_REQUIRE(ctx, d->batch >= 0 && d->m >= 0 && d->n >= 0 && d->k >= 0, "wdc_gemm: negative shape");
@@ -217,7 +215,7 @@ extern "C" int wdc_gemm(wdc_context* ctx, const wdc_gemm_desc* d, const float* A
   DeviceGuard g(ctx->device);
   ProfScope prof(ctx, 2.0 * (double)d->batch * (double)d->m * (double)d->n * (double)d->k);
   // Y = alpha*A*B + beta*Y (C aliasing the output) is served by the CUDA-core kernel's in-place mode only
-  int s = (C != nullptr && C == Y) ? WDC_ERR_UNSUPPORTED : wdc_tc_gemm(ctx, d, A, B, C, Y);
+  int s = (C != nullptr && C == Y) ? WDC_ERR_UNSUPPORTED : wdc_tc_gemm(ctx, d, A, B, C, Y, columns);
   if (s != WDC_ERR_UNSUPPORTED) return s;
   // Below 32 rows the tensor-core path declines (a 128-row tile would be three quarters empty and B would have to be
   // split first): such a product is a few dot products per column, bound by reading B.
@@ -229,6 +227,23 @@ extern "C" int wdc_gemm(wdc_context* ctx, const wdc_gemm_desc* d, const float* A
     if (s != WDC_ERR_UNSUPPORTED) return s;
   }
   return wdc_simt_gemm(ctx, d, A, B, C, Y);
+}
+
+extern "C" int wdc_gemm(wdc_context* ctx, const wdc_gemm_desc* d, const float* A, const float* B,
+                        const float* C, float* Y) {
+  if (!ctx) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_gemm: null context");
+  WDC_TAPE(ctx, wdc_gemm, tape_desc(d), A, B, C, Y);
+  return gemm_call(ctx, d, 0, A, B, C, Y);
+}
+
+extern "C" int wdc_gemm_columns(wdc_context* ctx, const wdc_gemm_desc* d, int64_t columns, const float* A, const float* B,
+                                const float* C, float* Y) {
+  if (!ctx) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_gemm_columns: null context");
+  WDC_TAPE(ctx, wdc_gemm_columns, tape_desc(d), columns, A, B, C, Y);
+  WDC_REQUIRE(ctx, d != nullptr, "wdc_gemm_columns: null descriptor");
+  WDC_REQUIRE(ctx, columns > 0 && columns % 4 == 0 && d->n % columns == 0,
+              "wdc_gemm_columns: %lld columns are not products of %lld (a multiple of 4)", (long long)d->n, (long long)columns);
+  return gemm_call(ctx, d, columns, A, B, C, Y);
 }
 
 extern "C" int wdc_conv2d(wdc_context* ctx, const wdc_conv_desc* d, const float* x, const float* w,

@@ -117,6 +117,7 @@ SIGNATURES = {
     "wdc_cast": (c_int, [c_void_p, c_int, c_int, c_void_p, c_void_p, c_int64]),
     "wdc_channel_affine": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int]),
     "wdc_gemm": (c_int, [c_void_p, POINTER(GemmDesc), c_void_p, c_void_p, c_void_p, c_void_p]),
+    "wdc_gemm_columns": (c_int, [c_void_p, POINTER(GemmDesc), c_int64, c_void_p, c_void_p, c_void_p, c_void_p]),
     "wdc_conv2d": (c_int, [c_void_p, POINTER(ConvDesc), c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]),
     "wdc_pack_conv_weight": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int64]),
     "wdc_maxpool2d": (c_int, [c_void_p, POINTER(PoolDesc), c_void_p, c_void_p]),

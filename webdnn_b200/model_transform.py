@@ -418,7 +418,8 @@ def _merge_projections(model: Model) -> None:
     """Linear layers of one tensor whose results only attention nodes read become one linear layer.
 
     A projection of 625 rows to 256 columns is a launch of 20 tiles, mostly latency: two cost twice one.  Side by side
-    they are one launch that fills the GPU better; the columns keep their own sums, so results do not change."""
+    they are one launch that fills the GPU better.  The ``columns`` attribute keeps a layer's additions in the order that
+    they have in the layer alone (``wdc_gemm_columns``), so results do not change by a bit."""
     g = model.graph
     if model.metadata_props.get("WebDNN2.WeightPaths"):
         return   # weights outside the graph may still be on their way
@@ -440,14 +441,14 @@ def _merge_projections(model: Model) -> None:
         return bool(users) and all(u.op_type == "CudaAttention" and
                                    {a.name: a.i for a in u.attribute}["heads"] > 0 for u in users)
 
-    groups: Dict[str, List[Node]] = {}
+    groups: Dict[tuple, List[Node]] = {}   # by tensor and width
     for n in g.node:
         if mergeable(n):
-            groups.setdefault(n.input[0], []).append(n)
+            groups.setdefault((n.input[0], inits[n.input[1]].dims[1]), []).append(n)
     place: Dict[str, tuple] = {}   # old result -> (merged result, first column, columns of the merged result)
     replace_at: Dict[int, Node] = {}
     removed = set()
-    for x, nodes in groups.items():
+    for (x, columns), nodes in groups.items():
         if len(nodes) < 2:
             continue
         ws = [np.asarray(inits[n.input[1]].array).reshape(inits[n.input[1]].dims) for n in nodes]
@@ -462,7 +463,8 @@ def _merge_projections(model: Model) -> None:
             col += w.shape[1]
             removed.add(id(n))
         replace_at[id(nodes[0])] = Node("CudaMatMulBias", [x, base + "_w", base + "_b"], [base], base,
-                                        [make_attr("relu", 0), make_attr("has_residual", 0)])
+                                        [make_attr("relu", 0), make_attr("has_residual", 0),
+                                         make_attr("columns", columns)])
     if not place:
         return
     new_nodes = []

@@ -226,16 +226,19 @@ class CudaMatMulBias(OperatorImpl):
     MatMul + Add [+ Relu | + Add], matmul.ts:11-111 and binary7.ts broadcasting for the reference semantics).
 
     With a residual the launch goes through ``wdc_conv2d`` as a 1x1 convolution over the rows (its epilogue takes a
-    per-column addend and a residual tensor together); W is transposed to [n, k] once and kept with the weight."""
+    per-column addend and a residual tensor together); W is transposed to [n, k] once and kept with the weight.
+    ``columns``: the weight is several layers' side by side, that many columns each (load-time merge of projections)."""
 
     def __init__(self):
         super().__init__("cuda")
         self.relu = False
         self.has_residual = False
+        self.columns = 0
 
     def initialize(self, attribute):
         self.relu = get_attr_int(attribute, "relu", 0) != 0
         self.has_residual = get_attr_int(attribute, "has_residual", 0) != 0
+        self.columns = get_attr_int(attribute, "columns", 0)
 
     def run(self, context, inputs, n_outputs):
         context.asserts_cuda_tensor_array(inputs)
@@ -264,7 +267,7 @@ class CudaMatMulBias(OperatorImpl):
         elif y.length:
             d = GemmDesc(batch=1, m=m, n=n, k=k, sab=0, sa0=k, sa1=1, sbb=0, sb0=n, sb1=1, sc0=0, sc1=1,
                          alpha=1.0, beta=1.0, relu=int(self.relu))
-            context.gemm(d, a, w, b, y)
+            context.gemm(d, a, w, b, y, self.columns)
         for t in owned:
             t.dispose()
         if res is not None and not fused_res:
