@@ -135,3 +135,33 @@ def test_products_side_by_side_are_the_same_bits(cuda_context, m, k, columns, co
         at = slice(i * columns, (i + 1) * columns)
         assert np.array_equal(got[:, at].view(np.uint32), product(b[:, at], c[at], 0).view(np.uint32)), i
     da.dispose()
+
+
+# CTAs per query tile, each of them; with all chunks of a CTA's keys scored -inf (a sum of products that overflows)
+@pytest.mark.parametrize("tq,tk,dh", [(130, 520, 32), (17, 2000, 32), (100, 640, 64)])
+@pytest.mark.parametrize("overflow", [False, True])
+def test_every_attention_cluster(cuda_context, tq, tk, dh, overflow):
+    from webdnn_b200.lib import AttentionDesc
+    ctx = cuda_context
+    rng = np.random.default_rng(tq + tk)
+    q, k, v = (2 * rng.standard_normal((1, t, dh)).astype(np.float32) for t in (tq, tk, tk))
+    if overflow:
+        q[:, :, 0], k[:, tk // 2:, 0], k[:, :tk // 2, 0] = 1e20, -1e20, 0.0
+    with np.errstate(over="ignore"):
+        s = (np.einsum("btc,bsc->bts", q.astype(np.float64), k) * dh ** -0.5).astype(np.float32).astype(np.float64)
+    p = np.exp(s - s.max(-1, keepdims=True))
+    want = p / p.sum(-1, keepdims=True) @ v
+    dq, dk, dv, y = _put(ctx, q), _put(ctx, k), _put(ctx, v), ctx.empty_tensor([1, tq, dh])
+    d = AttentionDesc(batch=1, heads=1, tq=tq, tk=tk, dh=dh, q_sb=tq * dh, q_sh=dh, q_st=dh, k_sb=tk * dh, k_sh=dh, k_st=dh,
+                      v_sb=tk * dh, v_sh=dh, v_st=dh, y_sb=tq * dh, y_sh=dh, y_st=dh, scale=dh ** -0.5)
+    try:
+        for cs in (1, 2, 4, 8):
+            ctx.set_option("attention_cluster", cs)
+            ctx._call("wdc_attention", byref(d), *(c_void_p(t.ptr) for t in (dq, dk, dv, y)))
+            got = y.get_data().reshape(want.shape)
+            assert ctx.stats(device_memory=True)["last_attention_cluster"] == cs
+            assert max_err_rel_linf(got, want) <= 1e-5, cs
+    finally:
+        ctx.set_option("attention_cluster", 0)
+    for t in (dq, dk, dv, y):
+        t.dispose()

@@ -361,10 +361,11 @@ attention_tc_kernel(const AttTcProblem p, const __grid_constant__ CUtensorMap ma
         mc = fmaxf(mc, s[c]);
       }
       const float m_new = fmaxf(m, mc);
-      const float alpha = exp2f(m - m_new);                 // 0 for the first chunk (m = -inf)
+      const float ref = m_new == -INFINITY ? 0.f : m_new;   // (every score so far is -inf: weights of 0, not NaN)
+      const float alpha = exp2f(m - ref);                   // 0 for the first chunk (m = -inf)
 #pragma unroll
       for (int c = 0; c < BK; c++) {
-        s[c] = exp2f(s[c] - m_new);
+        s[c] = exp2f(s[c] - ref);
         sum += s[c];
       }
       l = l * alpha + sum;
