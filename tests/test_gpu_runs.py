@@ -92,6 +92,55 @@ def test_taped_runs_that_nobody_waited_for(cuda_context):
     runner.dispose()
 
 
+def test_recurrence_inside_a_graph(cuda_context):
+    """The cluster recurrence is a cooperative launch: recorded and replayed like the others."""
+    runner = _load(cuda_context, zoo.lstm(20, 5, 24, 96), graphReplay=True)
+    rng = np.random.default_rng(0)
+    for _ in range(4):
+        x = rng.standard_normal((20, 5, 24)).astype(np.float32)
+        got = runner.run([_cpu(x)])
+        want = runner._run_nodes([_cpu(x)])
+        assert all(np.array_equal(_bits(g.numpy()), _bits(w.numpy())) for g, w in zip(got, want))
+    assert runner.graph_replays >= 2
+    runner.dispose()
+
+
+# an infinite weight, and one that rounding would make infinite; an infinite initial state: gates saturate as in fp32
+@pytest.mark.parametrize("batch,hidden", [(1, 32), (5, 100), (33, 256)])
+@pytest.mark.parametrize("where", ["R", "R_large", "h0"])
+def test_recurrence_with_infinities(cuda_context, batch, hidden, where):
+    ctx = cuda_context
+    seq, inp = 6, 8
+    rng = np.random.default_rng(hidden)
+    u = lambda *s: rng.uniform(-0.3, 0.3, s).astype(np.float32)  # noqa: E731
+    x, w, r, b, h0, c0 = u(seq, batch, inp), u(4 * hidden, inp), u(4 * hidden, hidden), u(8 * hidden), u(batch, hidden), u(batch, hidden)
+    if where == "R":
+        r[hidden + 3, 5], r[3, hidden - 1] = np.inf, -np.inf        # the output and the input gate of unit 3
+    elif where == "R_large":
+        r[hidden + 3, 5] = np.float32(3.4028e38)
+    else:
+        h0[batch - 1, 7] = np.inf
+    dev = [ctx.move_tensor(_cpu(a)) for a in (x, w, r, b, h0, c0)]
+    outs = [ctx.empty_tensor(s) for s in ((seq, batch, hidden), (batch, hidden), (batch, hidden))]
+    ctx._call("wdc_lstm", *(t.ptr for t in dev + outs), seq, batch, inp, hidden)
+    got = [o.get_data().reshape(o.dims) for o in outs]
+    sig = lambda v: 0.5 * (np.tanh(0.5 * v) + 1)  # noqa: E731
+    h, c, ys = h0.astype(np.float64), c0.astype(np.float64), []
+    with np.errstate(all="ignore"):
+        for t in range(seq):
+            g = x[t].astype(np.float64) @ w.T + h @ r.T.astype(np.float64) + b[:4 * hidden] + b[4 * hidden:]
+            i, o, f, cc = np.split(g, 4, axis=1)
+            c = sig(f) * c + sig(i) * np.tanh(cc)
+            h = sig(o) * np.tanh(c)
+            ys.append(h)
+    for a, e in zip(got, (np.stack(ys), h, c)):
+        assert np.array_equal(np.isnan(a), np.isnan(e))
+        assert np.all(np.abs(np.nan_to_num(a) - np.nan_to_num(e)) <= 1e-5)
+    assert np.isfinite(got[0]).any()
+    for t in dev + outs:
+        t.dispose()
+
+
 def test_first_results_in_used_memory(cuda_context):
     """A model loaded into memory that other work has just given back gives the same bits at every call."""
     ctx = cuda_context

@@ -18,7 +18,8 @@
 // exchange of h through L2 (store, poll), 1100 the 48 MMAs and their completion, 1500 the exchange of partial sums, 700
 // the sums and gates.
 // All clusters of a launch wait for one another, so the launch is cooperative (all resident or an error).
-// Products are 3xTF32 with rounded parts (2^-23 of a product), sums fp32; gates as in lstm_persistent.cu.
+// Products are 3xTF32 with rounded parts (2^-23 of a product), sums fp32; gates as in lstm_persistent.cu.  An infinite
+// element of R or h0 would meet low parts of either sign or zero: a CTA whose slice holds one sums with plain fp32 FMAs.
 // Waits are bounded (2 s): on expiry the CTA sets the context's status word and leaves at its next barrier; its
 // peers' waits expire in turn, and all meet at a last cluster barrier, so no CTA leaves while others may write to it.
 #include <math.h>
@@ -115,6 +116,7 @@ __device__ __forceinline__ void cluster_barrier() {
 __device__ __forceinline__ float high_part(float x) {
   return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u);
 }
+__device__ __forceinline__ bool not_finite(float x) { return (__float_as_uint(x) & 0x7f800000u) == 0x7f800000u; }
 __device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr) {   // K-major, 128B swizzle
   uint64_t d = 0;
   d |= (uint64_t)((saddr & 0x3FFFF) >> 4);
@@ -175,7 +177,27 @@ struct ClusterShared {
   unsigned long long recv_bar[2];
   unsigned int tmem_base;
   int abort;
+  int plain_r, plain_h;     // R's slice, or h0's, holds an element whose high part is not finite
 };
+
+// A step's sums of gate row `row` and `cols` batch rows from c0 on without the tensor cores, sent like the accumulator's.
+// h: the slice of h_{t-1} in global memory (null: zero); rows past nb are not used by anyone.
+__device__ __noinline__ void send_plain_sums(const float* R, const float* h, int H, int nb, int c0, int cols, int u0, int row, int k0,
+                                             int klen, uint32_t dst, uint32_t dst_step, uint32_t bar) {
+  const int unit = u0 + row / 4;
+  const float* r = R + ((size_t)(row & 3) * H + (unit < H ? unit : 0)) * H + k0;
+  for (int c = c0; c < c0 + cols; c += 4, dst += dst_step) {
+    float v[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int q = 0; q < 4 && unit < H && c + q < nb; q++) {
+      for (int k = 0; k < klen; k++) {
+        float x = 0.f;
+        if (h) asm volatile("ld.relaxed.gpu.global.f32 %0, [%1];" : "=f"(x) : "l"(h + (size_t)(c + q) * H + k) : "memory");
+        v[q] = fmaf(__ldg(r + k), x, v[q]);
+      }
+    }
+    send16(dst, bar, v);
+  }
+}
 
 // CS: CTAs of a cluster.  ITEMS: 16-byte words of h a thread brings in per step, at most.
 template <int CS, int ITEMS>
@@ -206,7 +228,7 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_cluster_kernel(const ClusterA
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&sh.recv_bar[0])));
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&sh.recv_bar[1])));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    sh.abort = 0;
+    sh.abort = sh.plain_r = sh.plain_h = 0;
   }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sh.tmem_base)),
@@ -226,6 +248,7 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_cluster_kernel(const ClusterA
     const int r = tid, unit = u0 + r / 4;
     const float* src = a.R + ((size_t)(r & 3) * H + unit) * H + k0;
     const uint32_t dst = tmem_a + ((uint32_t)(warp * 32) << 16);
+    bool plain = false;
     for (int c = 0; c < a.kc; c += 8) {
       float hi[8], lo[8];
 #pragma unroll
@@ -237,12 +260,14 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_cluster_kernel(const ClusterA
         for (int q = 0; q < 4; q++) {
           hi[j + q] = high_part(e[q]);
           lo[j + q] = e[q] - hi[j + q];
+          plain |= not_finite(hi[j + q]);
         }
       }
       tmem_st8(dst + (uint32_t)c, hi);
       tmem_st8(dst + (uint32_t)(a.kc + c), lo);
     }
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    if (plain) sh.plain_r = 1;
   }
   // Pairs (unit, batch row) this thread finishes: consecutive threads are consecutive units of one row, so that a
   // row's units leave in one store and arrive as the 16-byte words its readers ask for.
@@ -283,6 +308,11 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_cluster_kernel(const ClusterA
       const uint32_t row = (uint32_t)(i / chunks), ch = (uint32_t)(i % chunks);
       h_src[j] = (int)row * H + (int)ch * 4;
       h_dst[j] = (ch >> 3) * blk_bytes + row * 128u + (((ch & 7u) ^ (row & 7u)) << 4);
+      if (a.h0) {   // (later h are products of a sigmoid and a tanh)
+        const float4 e = *reinterpret_cast<const float4*>(a.h0 + (size_t)b0 * H + k0 + h_src[j]);
+        if (not_finite(high_part(e.x)) || not_finite(high_part(e.y)) || not_finite(high_part(e.z)) || not_finite(high_part(e.w)))
+          sh.plain_h = 1;
+      }
     }
   }
   const uint32_t step_bytes = 128u * (uint32_t)a.n * 4u;   // all rows this CTA finishes, from every CTA of the cluster
@@ -296,6 +326,7 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_cluster_kernel(const ClusterA
   cluster_barrier();                                       // barriers of every CTA are ready for the others' bytes
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
+  const bool plain_r = sh.plain_r != 0, plain_h = sh.plain_h != 0;
   const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(a.n >> 3) << 17) | ((128u >> 4) << 24);
   const uint64_t desc0 = make_smem_desc(smem_u32(h_hi));
   // where this thread's accumulator columns go: row r of the tile is finished by CTA r / ROWS of the cluster
@@ -405,7 +436,9 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_cluster_kernel(const ClusterA
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       uint32_t dst = recv_peer + (t & 1 ? parity_bytes : 0u);
       const uint32_t bar = bar_peer[t & 1];
-      for (int c = 0; c < cols; c += 16) {
+      const bool plain = plain_r || (t == 0 && plain_h);
+      if (plain) send_plain_sums(a.R, hsrc, H, nb, half * cols, cols, u0, my_row, k0, klen, dst, ROWS * 16u, bar);
+      for (int c = 0; c < cols && !plain; c += 16) {
         float v[16];
         tmem_ld8(d_src + (uint32_t)c, v);
         if (c + 8 < cols) tmem_ld8(d_src + (uint32_t)(c + 8), v + 8);
