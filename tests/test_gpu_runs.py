@@ -92,6 +92,68 @@ def test_taped_runs_that_nobody_waited_for(cuda_context):
     runner.dispose()
 
 
+def test_what_a_tape_must_not_keep(cuda_context):
+    """A custom operator runs every time, placement and precision may change, results may be inputs."""
+    from webdnn_b200.operators.cuda import OperatorImpl
+    ctx = cuda_context
+    calls = []
+
+    class Counted(OperatorImpl):
+        def __init__(self):
+            super().__init__("cuda")
+
+        def run(self, context, inputs, n_outputs):
+            calls.append(1)
+            y = context.empty_tensor(inputs[0].dims)
+            context._call("wdc_fill_u32", c_void_p(y.ptr), ctypes.c_uint32(len(calls)), y.length)
+            return [y]
+
+    operator_table.register_operators([operator_table.OperatorEntry("Counted", 1, None, "cuda", Counted)])
+    x = np.ones((40, 8), np.float32)
+    runner = _load(ctx, _model([onnx_io.make_node("Counted", ["x"], ["y"], name="c")], [("x", [40, 8])], [("y", [40, 8])]))
+    for i in range(5):
+        (y,) = runner.run([_cpu(x)])
+        assert len(calls) == i + 1 and np.all(_bits(y.numpy()) == i + 1)
+    runner.dispose()
+
+    make = onnx_io.make_node
+    runner = _load(ctx, _model([make("Relu", ["x"], ["r"], name="r"), make("Reshape", ["r", "s"], ["y"], name="y")],
+                               [("x", [40, 8])], [("y", [80, 4]), ("x", [40, 8])], [("s", np.array([80, 4], np.int64))]))
+    for i in range(4):      # a result that is an input
+        y, same = runner.run([_cpu(x * (i - 2))], outputs_on_device=True)
+        assert np.array_equal(y.get_data(), np.maximum(x * (i - 2), 0).reshape(-1)) and np.array_equal(same.get_data(), (x * (i - 2)).reshape(-1))
+    runner.dispose()
+
+    runner = _load(ctx, _two_outputs(70))
+    ins = [_cpu(np.random.default_rng(i).standard_normal((70, n)).astype(np.float32)) for i, n in ((0, 40), (1, 64))]
+    first = [runner.run(ins)[0].numpy().copy() for _ in range(3)][-1]
+    assert _tape_of(runner) != [None]
+    ctx.set_precision("tf32x1")
+    try:
+        rough = runner.run(ins)[0].numpy().copy()
+        assert np.array_equal(_bits(rough), _bits(runner._run_nodes(ins)[0].numpy()))
+    finally:
+        ctx.set_precision("tf32x3")
+    assert np.array_equal(_bits(runner.run(ins)[0].numpy()), _bits(first)) and not np.array_equal(rough, first)
+    runner.force_operator_backend_order["r"] = ["cpu"]
+    if any(n[0] == "r" for n in runner.node_backends):
+        with pytest.raises(RuntimeError):     # no cpu implementation of Relu: asked for, so tried
+            runner.run(ins)
+    runner.dispose()
+
+
+def test_more_signatures_than_tapes(cuda_context):
+    ctx = cuda_context
+    make = onnx_io.make_node
+    runner = _load(ctx, _model([make("Relu", ["x"], ["y"], name="r")], [("x", ["n", 8])], [("y", ["n", 8])]))
+    xs = [np.random.default_rng(n).standard_normal((n, 8)).astype(np.float32) for n in range(33, 33 + runner.MAX_TAPES + 6)]
+    for _ in range(3):
+        for x in xs:
+            assert np.array_equal(runner.run([_cpu(x)])[0].numpy(), np.maximum(x, 0))
+    assert len(runner._tapes) == runner.MAX_TAPES
+    runner.dispose()
+
+
 def test_recurrence_inside_a_graph(cuda_context):
     """The cluster recurrence is a cooperative launch: recorded and replayed like the others."""
     runner = _load(cuda_context, zoo.lstm(20, 5, 24, 96), graphReplay=True)

@@ -19,12 +19,23 @@ class OperatorEntry:
     backend: str
     factory: Callable[[], object]
     domain: Optional[str] = None
+    # run() does nothing but call entry points of the device library, with arguments that follow from the inputs' dims,
+    # dtypes and layouts: its calls may be noted and repeated without it (Runner's tapes).  The framework's own cuda
+    # operators are; a registered custom operator is called every time unless it says so.
+    repeatable: bool = False
 
 
 _registered: Dict[str, List[OperatorEntry]] = {}
+_version = 0    # counts changes of the registry
+
+
+def registry_version() -> int:
+    return _version
 
 
 def register_operators(entries: Sequence[OperatorEntry]) -> None:
+    global _version
+    _version += 1
     for e in entries:
         _registered.setdefault(e.op_type, []).append(e)
 
@@ -34,6 +45,8 @@ def registered_op_types(backend: str) -> List[str]:
 
 
 def clear_registry() -> None:
+    global _version
+    _version += 1
     _registered.clear()
 
 
@@ -58,7 +71,9 @@ def instantiate_operator(op_type: str, opset: int, backend_order: Sequence[str],
                     continue
                 if e.opset_max is not None and e.opset_max <= opset:
                     continue
-                return e.factory()
+                op = e.factory()
+                op.repeatable = e.repeatable
+                return op
         return None
 
     op = pick(local_order)

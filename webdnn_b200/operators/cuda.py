@@ -1168,4 +1168,6 @@ def get_op_entries() -> List[OperatorEntry]:
             entries.append(E(name, 13, None, "cuda", lambda n=name: CudaReduce(n, True)))
         else:
             entries.append(E(name, 1, None, "cuda", lambda n=name: CudaReduce(n, False)))
+    for e in entries:
+        e.repeatable = True
     return entries

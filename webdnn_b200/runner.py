@@ -17,6 +17,7 @@ assert that nothing ran on the host except shape bookkeeping.
 """
 from __future__ import annotations
 
+import copy
 import ctypes
 import json
 import logging
@@ -32,7 +33,7 @@ from .backend import (NP_DTYPE, CPUTensor, CudaTensor, EightbitCPUTensor, WebDNN
 from .model_transform import find_tensor_release_timing, model_transform
 from .onnx_io import FLOAT, INT32, INT64, Model, clip_long
 from .tensor_loader import TensorLoader
-from .operator_table import instantiate_operator, register_operators, registered_op_types
+from .operator_table import instantiate_operator, register_operators, registered_op_types, registry_version
 
 logger = logging.getLogger("WebDNN.runner")
 
@@ -80,7 +81,11 @@ class Runner:
         # runs that are not replayed as a graph: from its second use on, a signature's calls are taped, and later runs
         # repeat the tape with one call of the library.  None: this signature cannot be taped.
         self._tapes: Dict[tuple, Optional["TapedRun"]] = {}
-        self._untapeable = set()                  # signatures whose first run used the cpu backend
+        self._untapeable = set()                  # signatures whose first run used the cpu backend or a custom operator
+        self._repeatable = False                  # whether the last run's operators all are (OperatorEntry.repeatable)
+        # when the tapes were made: what a run's operators and placement follow from besides the model and the inputs
+        self._taped_under: Optional[tuple] = None
+    MAX_SIGNATURES = 4096                         # remembered at a time, where every call has dims of its own
     MAX_CAPTURED_SIGNATURES = 4                   # each recorded run keeps its own activation memory
     MAX_TAPES = 64                                # a tape is a list of calls on the host: some 20 KB for ResNet-50
     GRAPH_REPLAY_AUTO_BATCH = 32
@@ -238,17 +243,30 @@ class Runner:
             if cap is not None:
                 self.graph_replays += 1
                 return cap.run(inputs)
+        under = self._taped_under
+        if (under is None or under[0] != registry_version() or under[1] != self.backend_order or
+                under[2] != self.force_operator_backend_order or under[3] != self.tensor_move_options):
+            self._drop_tapes()
+            self._seen.clear()      # (a signature's next run is a first one again: it shows what may be taped)
+            self._taped_under = (registry_version(), *copy.deepcopy((self.backend_order, self.force_operator_backend_order,
+                                                                     self.tensor_move_options)))
         key = (outputs_on_device, sig)
         tape = self._tapes.get(key)
         if tape is not None:
             self.node_backends = tape.node_backends
+            self.node_performances = []
             return tape.run(inputs)
+        if len(self._seen) >= self.MAX_SIGNATURES:
+            self._seen.clear()
+            self._untapeable.clear()
         seen = self._seen.get(sig, 0)
         self._seen[sig] = seen + 1
-        if seen >= 1 and key not in self._tapes and sig not in self._untapeable:
+        if seen >= 1 and key not in self._tapes and sig not in self._untapeable \
+                and all(t.backend == "cuda" or t.data_type in ("float32", "int32") for t in inputs):
             return self._run_taping(inputs, key)
         results = self._run_nodes(inputs, False, outputs_on_device)
-        if seen == 0 and self.nodes_on("cpu"):
+        if seen == 0 and (self.nodes_on("cpu") or not self._repeatable or
+                          {vi.name for vi in self.model.graph.output} & {vi.name for vi in self.model.graph.input}):
             self._untapeable.add(sig)
         return results
 
@@ -289,7 +307,7 @@ class Runner:
             for t in moved:
                 t.dispose()
             raise
-        if all(isinstance(o, CudaTensor) for o in outs) and not self.nodes_on("cpu"):
+        if all(isinstance(o, CudaTensor) for o in outs) and not self.nodes_on("cpu") and self._repeatable:
             tape = ctx.tape_end(outs)
         else:
             ctx.tape_end(None)
@@ -339,6 +357,7 @@ class Runner:
         release_timing = find_tensor_release_timing(self.model, set(self.initializer_tensors))
         self.node_backends = []
         self.node_performances = []
+        self._repeatable = True
 
         for node in graph.node:
             t0 = time.perf_counter()
@@ -353,6 +372,7 @@ class Runner:
             operator = instantiate_operator(op_type, self.opset, order, current)
             if operator is None:
                 raise RuntimeError(f"Operator implementation for {op_type}, opset={self.opset} does not exist.")
+            self._repeatable &= getattr(operator, "repeatable", False)
             operator.initialize(node.attribute)
             requirement = operator.get_tensor_backend_requirement(len(node.input), len(node.output))
             operator_inputs = []
