@@ -84,8 +84,10 @@ int wdc_graph_run(wdc_context* ctx, wdc_graph* graph, int n_in, void* const* dst
  * counterpart in the reference either).  Unlike a graph it owns no device memory and takes new buffers every time.
  * wdc_tape_begin names the run's device inputs; every following call of this thread on the context executes and is
  * noted, allocations included, until wdc_tape_end names the run's results.  *tape is NULL when the run cannot be
- * repeated: it moved host data, waited, freed a buffer that is not its own, kept one that is no result, or returns an
- * input (n_out < 0: the recording is given up).  Device memory that is neither input nor allocated by the run (weights) is taken to stay where it is.
+ * repeated: it moved host data, waited, freed a buffer that is neither an input nor its own, kept one that is no
+ * result, or returns an input (n_out < 0: the recording is given up).  Device memory that is neither input nor allocated
+ * by the run (weights) is taken to stay where it is.  An input that the run frees is freed at that point of a repetition
+ * too where it came from host memory; a device input stays the caller's.
  * wdc_tape_run repeats the calls on new inputs (host memory where in_on_host[i] != 0).  out_host == NULL: out[]
  * receives the results' device buffers, which the caller frees; else the results are copied to out_host[], the call
  * waits for them and frees everything. */

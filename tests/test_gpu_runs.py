@@ -67,6 +67,35 @@ def test_uploads_do_not_wait_for_kernels(cuda_context):
     big.dispose()
 
 
+@pytest.mark.parametrize("rows", [40, 5000])      # results within and beyond what a kernel moves
+@pytest.mark.parametrize("on_device", [False, True])
+def test_tape_with_new_inputs(cuda_context, rows, on_device):
+    ctx = cuda_context
+    runner = _load(ctx, _two_outputs(rows))
+    rng = np.random.default_rng(1)
+    in_use = None
+    for i in range(6):
+        a, b = rng.standard_normal((rows, 40)).astype(np.float32), rng.standard_normal((rows, 64)).astype(np.float32)
+        where = [(0, 0), (1, 1), (0, 1), (1, 0)][i % 4]         # host and device inputs in one call
+        ins = [ctx.move_tensor(_cpu(x)) if d else _cpu(x) for x, d in zip((a, b), where)]
+        got = runner.run(ins, outputs_on_device=on_device)
+        assert runner.nodes_on("cpu") == [] and len(runner.node_backends) >= 2
+        want = runner._run_nodes([_cpu(a), _cpu(b)])
+        for g, w in zip(got, want):
+            assert g.backend == ("cuda" if on_device else "cpu") and g.data_type == w.data_type and list(g.dims) == list(w.dims)
+            assert np.array_equal(_bits(g.get_data()), _bits(w.numpy()))
+        for t in (*ins, *got):
+            if t.backend == "cuda":
+                t.dispose()
+        if i >= 1:
+            (tape,) = _tape_of(runner, on_device)
+            assert tape is not None
+            now = ctx.stats()["bytes_in_use"]
+            assert in_use in (None, now)
+            in_use = now
+    runner.dispose()
+
+
 def test_taped_runs_that_nobody_waited_for(cuda_context):
     """Inputs of later calls are brought into memory that the calls in flight have just given back."""
     ctx = cuda_context
@@ -152,6 +181,30 @@ def test_more_signatures_than_tapes(cuda_context):
             assert np.array_equal(runner.run([_cpu(x)])[0].numpy(), np.maximum(x, 0))
     assert len(runner._tapes) == runner.MAX_TAPES
     runner.dispose()
+
+
+def test_allocation_failing_in_the_middle_of_a_tape():
+    from webdnn_b200.backend import CudaBackendError, WebDNNCPUContext, WebDNNCudaContext
+    ctx = WebDNNCudaContext(WebDNNCPUContext(), arena_bytes=64 << 20)
+    ctx.initialize()
+    make = onnx_io.make_node
+    runner = _load(ctx, _model([make("Relu", ["x"], ["r"], name="r"), make("Exp", ["r"], ["e"], name="e"),
+                                make("Sqrt", ["e"], ["y"], name="y")], [("x", [1 << 20])], [("y", [1 << 20])]))
+    x = _cpu(np.linspace(-1, 1, 1 << 20).astype(np.float32))
+    want = [runner.run([x])[0].numpy().copy() for _ in range(3)][0]
+    assert _tape_of(runner) != [None]
+    before = ctx.stats()["bytes_in_use"]
+    hog = [ctx.empty_tensor([1 << 20]) for _ in range(14)]      # 56 of 64 MB: the input and one more fit
+    full = ctx.stats()["bytes_in_use"]
+    with pytest.raises(CudaBackendError):
+        runner.run([x])
+    for t in hog:
+        t.dispose()
+    assert full - before == 56 << 20
+    for _ in range(4):
+        assert np.array_equal(_bits(runner.run([x])[0].numpy()), _bits(want))
+    runner.dispose()
+    ctx.close()
 
 
 def test_recurrence_inside_a_graph(cuda_context):

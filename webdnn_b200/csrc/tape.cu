@@ -67,13 +67,16 @@ void wdc_tape_note_alloc(wdc_tape* t, void* p, int64_t bytes) {
 }
 void wdc_tape_note_free(wdc_tape* t, void* p) {
   auto it = t->live.find((char*)p);
-  if (it == t->live.end() || it->second.first < t->n_in) {   // not the run's own buffer
+  if (it == t->live.end()) {   // not the run's own buffer
     t->valid = false;
     return;
   }
   const int slot = it->second.first;
+  const bool input = slot < t->n_in;
   t->live.erase(it);
-  t->ops.push_back([slot](wdc_context* ctx, char** slots) {
+  t->ops.push_back([slot, input](wdc_context* ctx, char** slots) {
+    // an input is the run's own where it came from host memory: the caller keeps its device buffers
+    if (input && !slots[-1 - slot]) return (int)WDC_OK;
     void* q = slots[slot];
     slots[slot] = nullptr;
     return wdc_free(ctx, q);
@@ -86,32 +89,34 @@ extern "C" int wdc_tape_run(wdc_context* ctx, wdc_tape* tape, const void* const*
     return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_tape_run: bad argument");
   WDC_NO_TAPE(ctx);
   DeviceGuard g(ctx->device);
-  std::vector<char*> slots((size_t)tape->n_slots, nullptr);
+  // (in front of the slots, from the last one back: whether an input's buffer is the run's own)
+  std::vector<char*> buffers((size_t)(tape->n_in + tape->n_slots), nullptr);
+  char** const slots = buffers.data() + tape->n_in;
   int s = WDC_OK;
   for (int i = 0; i < tape->n_in && s == WDC_OK; i++) {
     if (!in_on_host[i]) {
-      slots[(size_t)i] = (char*)in[i];
+      slots[i] = (char*)in[i];
       continue;
     }
-    s = wdc_alloc(ctx, tape->in_bytes[(size_t)i], (void**)&slots[(size_t)i]);
-    if (s == WDC_OK && tape->in_bytes[(size_t)i] > 0)
-      s = wdc_stage_in(ctx, slots[(size_t)i], in[i], tape->in_bytes[(size_t)i]);
+    s = wdc_alloc(ctx, tape->in_bytes[(size_t)i], (void**)&slots[i]);
+    slots[-1 - i] = slots[i];
+    if (s == WDC_OK && tape->in_bytes[(size_t)i] > 0) s = wdc_stage_in(ctx, slots[i], in[i], tape->in_bytes[(size_t)i]);
   }
-  for (size_t k = 0; k < tape->ops.size() && s == WDC_OK; k++) s = tape->ops[k](ctx, slots.data());
+  for (size_t k = 0; k < tape->ops.size() && s == WDC_OK; k++) s = tape->ops[k](ctx, slots);
   for (int i = 0; i < tape->n_in; i++)   // stream-ordered: reused only by work queued after this run
-    if (in_on_host[i] && slots[(size_t)i]) {
-      wdc_free(ctx, slots[(size_t)i]);
-      slots[(size_t)i] = nullptr;
+    if (in_on_host[i] && slots[i]) {
+      wdc_free(ctx, slots[i]);
+      slots[i] = nullptr;
     }
   const int n_out = (int)tape->outs.size();
   if (s == WDC_OK) {
-    for (int i = 0; i < n_out; i++) out[i] = slots[(size_t)tape->outs[(size_t)i]];
+    for (int i = 0; i < n_out; i++) out[i] = slots[tape->outs[(size_t)i]];
     if (!out_host) return WDC_OK;
     s = wdc_stage_out(ctx, n_out, out_host, (const void* const*)out, out_bytes);
   }
   // results have been read, or a call failed: nothing of the run stays allocated
   for (int i = tape->n_in; i < tape->n_slots; i++)
-    if (slots[(size_t)i]) wdc_free(ctx, slots[(size_t)i]);
+    if (slots[i]) wdc_free(ctx, slots[i]);
   for (int i = 0; i < n_out; i++) out[i] = nullptr;
   return s;
 }

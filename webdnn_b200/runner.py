@@ -30,6 +30,7 @@ import numpy as np
 from . import onnx_io, tensor_loader
 from .backend import (NP_DTYPE, CPUTensor, CudaTensor, EightbitCPUTensor, WebDNNCPUContext, WebDNNCudaContext,
                       like_cpu_tensor)
+from .lib import WDC_ERR_OOM, CudaBackendError
 from .model_transform import find_tensor_release_timing, model_transform
 from .onnx_io import FLOAT, INT32, INT64, Model, clip_long
 from .tensor_loader import TensorLoader
@@ -255,7 +256,13 @@ class Runner:
         if tape is not None:
             self.node_backends = tape.node_backends
             self.node_performances = []
-            return tape.run(inputs)
+            try:
+                return tape.run(inputs)
+            except CudaBackendError as e:
+                if e.status != WDC_ERR_OOM:
+                    raise
+                # nothing of the run is left; node by node an input is brought in no earlier than it is needed
+                return self._run_nodes(inputs, False, outputs_on_device)
         if len(self._seen) >= self.MAX_SIGNATURES:
             self._seen.clear()
             self._untapeable.clear()
@@ -288,24 +295,27 @@ class Runner:
         ctx = self.backend_contexts["cuda"]
         moved = []
         dev_in = []
-        for t in inputs:
-            if t.backend == "cpu":
-                t = ctx.move_tensor(t)
-                moved.append(t)
-            else:
-                ctx.asserts_cuda_tensor(t)
-                ctx.wait_upload(t)
-            dev_in.append(t)
-        tape = None
-        ctx.tape_begin(dev_in)
         try:
-            outs = self._run_nodes(dev_in, outputs_on_device=True)
+            for t in inputs:
+                if t.backend == "cpu":
+                    t = ctx.move_tensor(t)
+                    moved.append(t)
+                else:
+                    ctx.asserts_cuda_tensor(t)
+                    ctx.wait_upload(t)
+                dev_in.append(t)
+            ctx.tape_begin(dev_in)
+        except Exception:
+            for t in moved:
+                t.dispose()
+            raise
+        tape = None
+        try:
+            outs = self._run_nodes(dev_in, outputs_on_device=True, owned=moved)
             if not outputs_on_device:
                 outs = self._canonical_outputs(outs)
         except Exception:
             ctx.tape_end(None)
-            for t in moved:
-                t.dispose()
             raise
         if all(isinstance(o, CudaTensor) for o in outs) and not self.nodes_on("cpu") and self._repeatable:
             tape = ctx.tape_end(outs)
@@ -322,8 +332,6 @@ class Runner:
                 results.append(o if o.backend == "cpu" else self.backend_contexts["cpu"].move_tensor(o, {}))
                 o.dispose()
             outs = results
-        for t in moved:
-            t.dispose()
         return outs
 
     def _drop_tapes(self) -> None:
@@ -333,10 +341,23 @@ class Runner:
         self._tapes.clear()
         self._untapeable.clear()
 
-    def _run_nodes(self, inputs, measure_performance: bool = False, outputs_on_device: bool = False):
-        """The run node by node."""
+    def _run_nodes(self, inputs, measure_performance: bool = False, outputs_on_device: bool = False, owned=()):
+        """The run node by node.  ``owned``: device inputs that are the run's, to be given back like its own tensors."""
+        tensors: Dict[str, Dict[str, object]] = {b: {} for b in BACKENDS}
+        borrowed = set()
+        try:
+            return self._run_nodes_in(tensors, borrowed, inputs, measure_performance, outputs_on_device, owned)
+        except Exception:
+            for backend in BACKENDS_WITHOUT_CPU:
+                for name, t in tensors[backend].items():
+                    if name in self.initializer_tensors:
+                        self.copied_initializer_tensors[backend][name] = t
+                    elif name not in borrowed:
+                        t.dispose()
+            raise
+
+    def _run_nodes_in(self, tensors_for_backends, borrowed, inputs, measure_performance, outputs_on_device, owned):
         graph = self.model.graph
-        tensors_for_backends: Dict[str, Dict[str, object]] = {b: {} for b in BACKENDS}
         for name, tensor in self.initializer_tensors.items():
             tensors_for_backends["cpu"][name] = tensor
         for backend, kv in self.copied_initializer_tensors.items():
@@ -345,10 +366,9 @@ class Runner:
 
         if len(self.inputs_without_initializer) != len(inputs):
             raise ValueError("length of inputs mismatch")
-        borrowed = set()
         for vi, t in zip(self.inputs_without_initializer, inputs):
             tensors_for_backends[t.backend][vi.name] = t
-            if t.backend != "cpu":
+            if t.backend != "cpu" and not any(t is o for o in owned):
                 borrowed.add(vi.name)  # caller-owned device tensor: never disposed here
                 wait = getattr(self.backend_contexts.get(t.backend), "wait_upload", None)
                 if wait is not None:
