@@ -45,6 +45,30 @@ def _tape_of(runner, on_device=False):
     return [t for (dev, _), t in runner._tapes.items() if dev == on_device]
 
 
+# around what a kernel moves (128 KB), what helper threads share (256 KB), a chunk (512 KB) and the ring (16 MB)
+@pytest.mark.parametrize("nbytes", [1, 3, 4, 4096, (128 << 10) - 4, 128 << 10, (128 << 10) + 4, (256 << 10) - 1, 256 << 10, (256 << 10) + 1,
+                                    (512 << 10) - 1, 512 << 10, (512 << 10) + 1, (16 << 20) - 1, 16 << 20, (16 << 20) + 1, 40_000_001])
+@pytest.mark.parametrize("pinned", [False, True])
+def test_round_trip(cuda_context, nbytes, pinned):
+    ctx = cuda_context
+    data = np.random.default_rng(nbytes).integers(0, 256, nbytes, dtype=np.uint8)
+    host = ctx.pinned_array((nbytes,), np.uint8) if pinned else np.empty(nbytes, np.uint8)
+    back = ctx.pinned_array((nbytes,), np.uint8) if pinned else np.empty(nbytes, np.uint8)
+    ptr = ctx._alloc(nbytes + 16)
+    for shift in (0, 4):     # the device side aligned to 16 bytes and not
+        host[:] = data
+        back[:] = 0
+        ctx._call("wdc_upload", c_void_p(ptr + shift), host.ctypes.data_as(c_void_p), nbytes)
+        if not pinned:
+            host[:] = 0      # a pageable source may be reused at once
+        ctx._call("wdc_download", back.ctypes.data_as(c_void_p), c_void_p(ptr + shift), nbytes)
+        assert np.array_equal(back, data)
+    ctx._free(ptr)
+    if pinned:
+        for a in (host, back):
+            ctx._call("wdc_host_free", a.ctypes.data_as(c_void_p))
+
+
 def test_uploads_do_not_wait_for_kernels(cuda_context):
     import time
     ctx = cuda_context
@@ -275,3 +299,42 @@ def test_first_results_in_used_memory(cuda_context):
         for later in results[1:]:
             assert all(np.array_equal(_bits(a), _bits(b)) for a, b in zip(results[0], later))
         runner.dispose()
+
+
+def test_copying_threads_of_all_contexts_stay_below_the_cpus():
+    """Large transfers of several contexts in a process that is bound to three CPUs."""
+    import os
+    import subprocess
+    import sys
+    code = """
+import os
+os.sched_setaffinity(0, set(sorted(os.sched_getaffinity(0))[:3]))
+import numpy as np
+from webdnn_b200.backend import CPUTensor, WebDNNCPUContext, WebDNNCudaContext
+contexts = []
+for i in range(3):
+    ctx = WebDNNCudaContext(WebDNNCPUContext())
+    ctx.initialize()
+    ctx.move_tensor(CPUTensor.from_array(np.ones(64, np.float32))).get_data()     # (whatever the driver starts for itself)
+    contexts.append(ctx)
+def threads():
+    return len(os.listdir("/proc/self/task"))
+before = threads()
+data = np.random.default_rng(0).standard_normal(4 << 20).astype(np.float32)
+for ctx in contexts:
+    t = ctx.move_tensor(CPUTensor.from_array(data))
+    assert np.array_equal(t.get_data(), data)
+assert 0 < threads() - before <= 2, (before, threads())
+for ctx in contexts:
+    ctx.close()
+ctx = WebDNNCudaContext(WebDNNCPUContext())
+ctx.initialize()
+ctx.move_tensor(CPUTensor.from_array(np.ones(64, np.float32))).get_data()
+before = threads()
+assert np.array_equal(ctx.move_tensor(CPUTensor.from_array(data)).get_data(), data)
+assert 0 < threads() - before <= 2, (before, threads())      # given back by the contexts that are gone
+ctx.close()
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    done = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr[-2000:]

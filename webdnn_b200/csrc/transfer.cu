@@ -6,10 +6,13 @@
 // copied by a few threads and sent (or received and copied) while its neighbours are on the link.  Page-locked
 // buffers of the caller's go straight to the link.  Small results leave the copy engines out: a kernel of the compute
 // stream writes the page-locked memory, which saves the switch between the two.
+#include <sched.h>
 #include <string.h>
 
 #include <atomic>
 #include <condition_variable>
+#include <exception>
+#include <new>
 #include <thread>
 
 #include "tape.cuh"
@@ -24,8 +27,19 @@ constexpr int64_t PINNED_CHECK = 256 << 10;   // asking the driver what a pointe
 constexpr int64_t BY_KERNEL = 128 << 10;      // up to here the link's latency, not its rate, is the time
 constexpr int MAX_HELPERS = 5;
 
+// CPUs this process may run on, and the helpers of all its contexts: together they stay below that number.
+int usable_cpus() {
+  cpu_set_t set;
+  CPU_ZERO(&set);
+  if (sched_getaffinity(0, sizeof(set), &set) == 0 && CPU_COUNT(&set) > 0) return CPU_COUNT(&set);
+  const unsigned n = std::thread::hardware_concurrency();
+  return n > 0 ? (int)n : 1;
+}
+std::atomic<int> helpers_alive{0};
+
 // memcpy by the caller and up to MAX_HELPERS threads that take pieces from a common counter: a helper that is still
-// asleep costs nothing, the caller takes its pieces.  Helpers poll for a while after a job, then sleep.
+// asleep costs nothing, the caller takes its pieces (all of them where no thread could be had).  Helpers poll for a while
+// after a job, then sleep.
 class CopyTeam {
  public:
   ~CopyTeam() {
@@ -35,6 +49,7 @@ class CopyTeam {
     }
     cv_.notify_all();
     for (auto& t : helpers_) t.join();
+    helpers_alive.fetch_sub((int)helpers_.size());
   }
   // dst[c] <- src in chunks of CHUNK bytes; sent(c) is called by the caller's thread, in order, as chunks are complete.
   template <class F>
@@ -45,7 +60,7 @@ class CopyTeam {
       sent(0);
       return;
     }
-    if (helpers_.empty()) start();
+    if (!started_) start();
     Job job;
     job.dst = dst;
     job.src = src;
@@ -98,9 +113,22 @@ class CopyTeam {
     return true;
   }
   void start() {
-    const unsigned cpus = std::thread::hardware_concurrency();
-    const int n = cpus > MAX_HELPERS ? MAX_HELPERS : cpus > 1 ? (int)cpus - 1 : 0;
-    for (int i = 0; i < n; i++) helpers_.emplace_back([this] { run(); });
+    started_ = true;
+    const int most = usable_cpus() - 1;
+    for (int i = 0; i < MAX_HELPERS; i++) {
+      bool made = false;
+      if (helpers_alive.fetch_add(1) < most) {
+        try {
+          helpers_.emplace_back([this] { run(); });
+          made = true;
+        } catch (const std::exception&) {   // no thread to be had
+        }
+      }
+      if (!made) {
+        helpers_alive.fetch_sub(1);
+        return;
+      }
+    }
   }
   void run() {
     uint64_t seen = 0;
@@ -135,7 +163,7 @@ class CopyTeam {
   std::atomic<uint64_t> seq_{0};
   std::atomic<int> asleep_{0};
   Job* job_ = nullptr;
-  bool stop_ = false;
+  bool started_ = false, stop_ = false;
 };
 
 }  // namespace
@@ -151,15 +179,27 @@ struct wdc_stager {
 
 namespace {
 
+void stager_free(wdc_stager* s) {
+  for (auto& ev : s->done)
+    if (ev) cudaEventDestroy(ev);
+  if (s->ring) cudaFreeHost(s->ring);
+  delete s;
+}
+
 int stager_of(wdc_context* ctx, wdc_stager** out) {
   std::lock_guard<std::mutex> lk(ctx->mu);
   if (!ctx->stager) {
-    wdc_stager* s = new wdc_stager();
+    wdc_stager* s = new (std::nothrow) wdc_stager();
+    if (!s) return wdc_fail(ctx, WDC_ERR_OOM, "page-locked staging memory: out of host memory");
     cudaError_t e = cudaMallocHost((void**)&s->ring, (size_t)(CHUNKS * CHUNK));
     for (auto& ev : s->done)
       if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+    if (e != cudaSuccess) {   // the next transfer tries again
+      cudaGetLastError();
+      stager_free(s);
+      return wdc_check_cuda(ctx, e, "page-locked staging memory");
+    }
     ctx->stager = s;
-    if (e != cudaSuccess) return wdc_check_cuda(ctx, e, "page-locked staging memory");
   }
   *out = ctx->stager;
   return WDC_OK;
@@ -210,12 +250,7 @@ dim3 wdc_io_grid(const wdc_io_list& list) {
 void* wdc_io_kernel() { return (void*)io_copy_kernel; }
 
 void wdc_stager_destroy(wdc_context* ctx) {
-  wdc_stager* s = ctx->stager;
-  if (!s) return;
-  for (auto& ev : s->done)
-    if (ev) cudaEventDestroy(ev);
-  if (s->ring) cudaFreeHost(s->ring);
-  delete s;
+  if (ctx->stager) stager_free(ctx->stager);
   ctx->stager = nullptr;
 }
 
