@@ -237,6 +237,7 @@ int wdc_stage_out(wdc_context* ctx, int count, void* const* host, const void* co
 void wdc_stager_destroy(wdc_context* ctx);
 void wdc_tape_note_alloc(struct wdc_tape* t, void* p, int64_t bytes);
 void wdc_tape_note_free(struct wdc_tape* t, void* p);
+void wdc_tape_forget(wdc_context* ctx);   // a recording of this thread on a context that goes away
 // Looks up the device address of wdc_lstm_static's scratch array for ctx's (current) device (lstm.cu).
 int wdc_lstm_static_setup(wdc_context* ctx);
 // Drops every cached hi/lo split whose source (weight matrix or per-channel scale vector) overlaps the

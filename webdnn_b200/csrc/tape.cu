@@ -1,6 +1,8 @@
 // Recording and repeating the calls of a run (see tape.cuh), and a captured graph's run with its host transfers.
 #include <string.h>
 
+#include <memory>
+
 #include "tape.cuh"
 
 thread_local wdc_tape* wdc_thread_tape = nullptr;
@@ -10,16 +12,28 @@ extern "C" int wdc_tape_begin(wdc_context* ctx, int n_in, void* const* in, const
     return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_tape_begin: bad argument");
   if (wdc_thread_tape) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_tape_begin: this thread is already recording a tape");
   if (ctx->capture_arena) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_tape_begin: a capture is open");
-  wdc_tape* t = new wdc_tape();
+  wdc_tape* t = new (std::nothrow) wdc_tape();
+  if (!t) return wdc_fail(ctx, WDC_ERR_OOM, "wdc_tape_begin: out of host memory");
   t->ctx = ctx;
   t->n_in = t->n_slots = n_in;
-  for (int i = 0; i < n_in; i++) {
-    t->in_bytes.push_back(bytes[i]);
-    // (an input passed twice, or an empty one, could not be told from its twin)
-    if (in[i] && bytes[i] > 0) t->valid &= t->live.insert({(char*)in[i], {i, bytes[i]}}).second;
+  try {
+    for (int i = 0; i < n_in; i++) {
+      t->in_bytes.push_back(bytes[i]);
+      // (an input passed twice, or an empty one, could not be told from its twin)
+      if (in[i] && bytes[i] > 0) t->valid &= t->live.insert({(char*)in[i], {i, bytes[i]}}).second;
+    }
+  } catch (const std::bad_alloc&) {
+    delete t;
+    return wdc_fail(ctx, WDC_ERR_OOM, "wdc_tape_begin: out of host memory");
   }
   wdc_thread_tape = t;
   return WDC_OK;
+}
+
+void wdc_tape_forget(wdc_context* ctx) {
+  if (!wdc_thread_tape || wdc_thread_tape->ctx != ctx) return;
+  delete wdc_thread_tape;
+  wdc_thread_tape = nullptr;
 }
 
 extern "C" int wdc_tape_end(wdc_context* ctx, int n_out, void* const* out, wdc_tape** tape) {
@@ -32,14 +46,18 @@ extern "C" int wdc_tape_end(wdc_context* ctx, int n_out, void* const* out, wdc_t
   size_t left = 0;
   for (auto& kv : t->live)
     if (kv.second.first >= t->n_in) left++;
-  std::vector<bool> taken((size_t)t->n_slots, false);
-  for (int i = 0; i < n_out && t->valid; i++) {
-    const wdc_tape::Ref r = t->ref(out[i]);
-    t->valid = r.slot >= t->n_in && r.offset == 0 && !taken[(size_t)r.slot];
-    if (t->valid) {
-      taken[(size_t)r.slot] = true;
-      t->outs.push_back(r.slot);
+  try {
+    std::vector<bool> taken((size_t)t->n_slots, false);
+    for (int i = 0; i < n_out && t->valid; i++) {
+      const wdc_tape::Ref r = t->ref(out[i]);
+      t->valid = r.slot >= t->n_in && r.offset == 0 && !taken[(size_t)r.slot];
+      if (t->valid) {
+        taken[(size_t)r.slot] = true;
+        t->outs.push_back(r.slot);
+      }
     }
+  } catch (const std::bad_alloc&) {
+    t->valid = false;
   }
   if (n_out < 0 || left != (size_t)n_out) t->valid = false;
   t->live.clear();
@@ -60,10 +78,14 @@ extern "C" int wdc_tape_destroy(wdc_context* ctx, wdc_tape* tape) {
 // What wdc_alloc and wdc_free note about themselves.
 void wdc_tape_note_alloc(wdc_tape* t, void* p, int64_t bytes) {
   const int slot = t->n_slots++;
-  t->live[(char*)p] = {slot, bytes > 0 ? bytes : 1};
-  t->ops.push_back([slot, bytes](wdc_context* ctx, char** slots) {
-    return wdc_alloc(ctx, bytes, (void**)&slots[slot]);
-  });
+  try {
+    t->live[(char*)p] = {slot, bytes > 0 ? bytes : 1};
+    t->ops.push_back([slot, bytes](wdc_context* ctx, char** slots) {
+      return wdc_alloc(ctx, bytes, (void**)&slots[slot]);
+    });
+  } catch (const std::bad_alloc&) {
+    t->valid = false;
+  }
 }
 void wdc_tape_note_free(wdc_tape* t, void* p) {
   auto it = t->live.find((char*)p);
@@ -74,13 +96,17 @@ void wdc_tape_note_free(wdc_tape* t, void* p) {
   const int slot = it->second.first;
   const bool input = slot < t->n_in;
   t->live.erase(it);
-  t->ops.push_back([slot, input](wdc_context* ctx, char** slots) {
-    // an input is the run's own where it came from host memory: the caller keeps its device buffers
-    if (input && !slots[-1 - slot]) return (int)WDC_OK;
-    void* q = slots[slot];
-    slots[slot] = nullptr;
-    return wdc_free(ctx, q);
-  });
+  try {
+    t->ops.push_back([slot, input](wdc_context* ctx, char** slots) {
+      // an input is the run's own where it came from host memory: the caller keeps its device buffers
+      if (input && !slots[-1 - slot]) return (int)WDC_OK;
+      void* q = slots[slot];
+      slots[slot] = nullptr;
+      return wdc_free(ctx, q);
+    });
+  } catch (const std::bad_alloc&) {
+    t->valid = false;
+  }
 }
 
 extern "C" int wdc_tape_run(wdc_context* ctx, wdc_tape* tape, const void* const* in, const int32_t* in_on_host,
@@ -90,8 +116,9 @@ extern "C" int wdc_tape_run(wdc_context* ctx, wdc_tape* tape, const void* const*
   WDC_NO_TAPE(ctx);
   DeviceGuard g(ctx->device);
   // (in front of the slots, from the last one back: whether an input's buffer is the run's own)
-  std::vector<char*> buffers((size_t)(tape->n_in + tape->n_slots), nullptr);
-  char** const slots = buffers.data() + tape->n_in;
+  std::unique_ptr<char*[]> buffers(new (std::nothrow) char*[(size_t)(tape->n_in + tape->n_slots)]());
+  if (!buffers) return wdc_fail(ctx, WDC_ERR_OOM, "wdc_tape_run: out of host memory");
+  char** const slots = buffers.get() + tape->n_in;
   int s = WDC_OK;
   for (int i = 0; i < tape->n_in && s == WDC_OK; i++) {
     if (!in_on_host[i]) {

@@ -8,6 +8,7 @@
 
 #include <functional>
 #include <map>
+#include <new>
 #include <tuple>
 #include <utility>
 #include <vector>
@@ -113,13 +114,18 @@ template <class F, class Kept, size_t... I>
 int tape_call(F fn, const Kept& kept, wdc_context* ctx, char** slots, std::index_sequence<I...>) {
   return fn(ctx, std::get<I>(kept).get(slots)...);
 }
+// (the entry points are C: a tape that does not fit in memory is given up)
 template <class F, class... A>
 void tape_note(wdc_tape* t, F fn, A... args) {
   typedef std::tuple<TapeArg<A>...> Kept;
-  const Kept kept{TapeArg<A>(*t, args)...};
-  t->ops.push_back([fn, kept](wdc_context* ctx, char** slots) {
-    return tape_call(fn, kept, ctx, slots, std::make_index_sequence<sizeof...(A)>());
-  });
+  try {
+    const Kept kept{TapeArg<A>(*t, args)...};
+    t->ops.push_back([fn, kept](wdc_context* ctx, char** slots) {
+      return tape_call(fn, kept, ctx, slots, std::make_index_sequence<sizeof...(A)>());
+    });
+  } catch (const std::bad_alloc&) {
+    t->valid = false;
+  }
 }
 
 // First statement of an entry point behind its null check.
