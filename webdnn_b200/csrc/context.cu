@@ -105,6 +105,7 @@ extern "C" int wdc_destroy(wdc_context* ctx) {
   if (!ctx) return WDC_OK;
   DeviceGuard g(ctx->device);
   cudaStreamSynchronize(ctx->stream);
+  wdc_tape_forget(ctx);
   wdc_tc_destroy(ctx);
   for (auto& s : ctx->arena.slabs) cudaFree(s.base);
   if (ctx->capture_arena) ctx->graph_arenas.push_back(ctx->capture_arena);
@@ -307,6 +308,7 @@ void wdc_forget_constants(wdc_context* ctx, const char* lo, const char* hi) {
 
 extern "C" int wdc_host_alloc(wdc_context* ctx, int64_t bytes, void** hptr) {
   if (!ctx || !hptr || bytes < 0) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_host_alloc: bad argument");
+  WDC_NO_TAPE(ctx);
   DeviceGuard g(ctx->device);
   WDC_CUDA(ctx, cudaMallocHost(hptr, (size_t)(bytes > 0 ? bytes : 1)));
   return WDC_OK;
@@ -314,6 +316,7 @@ extern "C" int wdc_host_alloc(wdc_context* ctx, int64_t bytes, void** hptr) {
 
 extern "C" int wdc_host_free(wdc_context* ctx, void* hptr) {
   if (!ctx) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_host_free: null context");
+  WDC_NO_TAPE(ctx);
   if (!hptr) return WDC_OK;
   DeviceGuard g(ctx->device);
   WDC_CUDA(ctx, cudaFreeHost(hptr));
@@ -363,6 +366,7 @@ extern "C" int wdc_upload_fresh_async(wdc_context* ctx, void* dst, const void* h
 
 extern "C" int wdc_wait_upload(wdc_context* ctx, int64_t ticket) {
   if (!ctx) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_wait_upload: null context");
+  WDC_NO_TAPE(ctx);
   if (ticket < 0 || ticket >= ctx->upload_seq)
     return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_wait_upload: unknown ticket %lld", (long long)ticket);
   // an event slot that has been reused marks a later transfer of the same in-order stream, which
@@ -399,6 +403,7 @@ static void arena_release(wdc_arena* a) {
 
 extern "C" int wdc_capture_end(wdc_context* ctx, wdc_graph** out) {
   if (!ctx || !out) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_capture_end: null argument");
+  WDC_NO_TAPE(ctx);
   *out = nullptr;
   if (!ctx->capture_arena) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_capture_end: no capture is open");
   DeviceGuard g(ctx->device);
@@ -431,6 +436,7 @@ extern "C" int wdc_capture_end(wdc_context* ctx, wdc_graph** out) {
 
 extern "C" int wdc_graph_launch(wdc_context* ctx, wdc_graph* graph) {
   if (!ctx || !graph || !graph->exec) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_graph_launch: bad argument");
+  WDC_NO_TAPE(ctx);
   if (ctx->capture_arena) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_graph_launch: a capture is open");
   if (graph->stale)
     return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_graph_launch: a weight or scale buffer the captured run uses was "
@@ -443,6 +449,7 @@ extern "C" int wdc_graph_launch(wdc_context* ctx, wdc_graph* graph) {
 
 extern "C" int wdc_graph_destroy(wdc_context* ctx, wdc_graph* graph) {
   if (!ctx) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_graph_destroy: null context");
+  WDC_NO_TAPE(ctx);
   if (!graph) return WDC_OK;
   DeviceGuard g(ctx->device);
   cudaStreamSynchronize(ctx->stream);
@@ -594,7 +601,11 @@ extern "C" int wdc_range_pop(wdc_context* ctx) {
   return WDC_OK;
 }
 
-extern "C" void* wdc_stream(wdc_context* ctx) { return ctx ? (void*)ctx->stream : nullptr; }
+extern "C" void* wdc_stream(wdc_context* ctx) {
+  if (!ctx) return nullptr;
+  WDC_NO_TAPE(ctx);   // (what the caller queues there is not noted)
+  return (void*)ctx->stream;
+}
 
 extern "C" int wdc_stats(wdc_context* ctx, int64_t* out, int n) {
   if (!ctx || !out || n < 0) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_stats: bad argument");
@@ -625,6 +636,7 @@ extern "C" int wdc_reset_stats(wdc_context* ctx) {
 
 extern "C" int wdc_profile_enable(wdc_context* ctx, int on) {
   if (!ctx) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_profile_enable: null context");
+  WDC_NO_TAPE(ctx);
   ctx->profile = on != 0;
   return WDC_OK;
 }
@@ -632,6 +644,7 @@ extern "C" int wdc_profile_enable(wdc_context* ctx, int on) {
 extern "C" int wdc_profile_read(wdc_context* ctx, int family, double* ms, int64_t* launches, double* flops) {
   if (!ctx || !ms || !launches || !flops || family != 0)
     return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_profile_read: bad argument");
+  WDC_NO_TAPE(ctx);
   DeviceGuard g(ctx->device);
   WDC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   double total = 0, fl = 0;
@@ -654,6 +667,9 @@ extern "C" int wdc_peer_copy(wdc_context* dst_ctx, void* dst, wdc_context* src_c
                              int64_t bytes) {
   if (!dst_ctx || !src_ctx || bytes < 0 || (bytes > 0 && (!dst || !src)))
     return wdc_fail(dst_ctx, WDC_ERR_INVALID, "wdc_peer_copy: bad argument");
+  TapeScope from_tape(src_ctx);
+  if (from_tape.tape) from_tape.tape->valid = false;
+  WDC_NO_TAPE(dst_ctx);
   wdc_note_write(dst_ctx, dst, bytes);
   if (bytes == 0) return WDC_OK;
   // Order the copy after everything already enqueued on the source stream, run it on the

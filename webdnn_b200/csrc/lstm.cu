@@ -113,6 +113,7 @@ extern "C" int wdc_lstm(wdc_context* ctx, const float* X, const float* W, const 
 // abort word, every CTA returns, and the context stays usable: the next wdc_sync reports WDC_ERR_DEVICE_WAIT once.
 extern "C" int wdc_selftest_device_wait(wdc_context* ctx, int64_t limit_ns) {
   if (!ctx) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_selftest_device_wait: null context");
+  WDC_NO_TAPE(ctx);
   WDC_REQUIRE(ctx, limit_ns >= 1000 && limit_ns <= 1000000000ll,
               "wdc_selftest_device_wait: limit of %lld ns is outside 1 us .. 1 s", (long long)limit_ns);
   DeviceGuard g(ctx->device);
