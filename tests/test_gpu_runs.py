@@ -231,6 +231,28 @@ def test_allocation_failing_in_the_middle_of_a_tape():
     ctx.close()
 
 
+# small and large inputs and results on one recorded graph, from the host and from the device in turn
+@pytest.mark.parametrize("rows,width", [(8, 64), (8, 8192), (32, 2048)])
+def test_graph_with_its_transfers(cuda_context, rows, width):
+    ctx = cuda_context
+    make = onnx_io.make_node
+    model = _model([make("Relu", ["x"], ["y"], name="r"), make("Add", ["y", "z"], ["s"], name="s"),
+                    make("ArgMax", ["s"], ["i"], name="i", axis=-1, keepdims=0)],
+                   [("x", [rows, width]), ("z", [rows, width])], [("y", [rows, width]), ("s", [rows, width]), ("i", [rows], onnx_io.INT32)])
+    runner = _load(ctx, model, graphReplay=True)
+    rng = np.random.default_rng(width)
+    for i in range(8):
+        x, z = (rng.standard_normal((rows, width)).astype(np.float32) for _ in range(2))
+        ins = [ctx.move_tensor(_cpu(a)) if i & bit and i > 2 else _cpu(a) for a, bit in ((x, 1), (z, 2))]
+        y, s, idx = runner.run(ins)
+        assert np.array_equal(y.numpy(), np.maximum(x, 0)) and np.array_equal(s.numpy(), np.maximum(x, 0) + z)
+        assert np.array_equal(idx.numpy(), np.argmax(np.maximum(x, 0) + z, -1))
+        p = runner.run([_cpu(x), _cpu(z)], wait=False)
+        assert np.array_equal(p.result()[1].numpy(), np.maximum(x, 0) + z)
+    assert runner.graph_replays > 6
+    runner.dispose()
+
+
 def test_recurrence_inside_a_graph(cuda_context):
     """The cluster recurrence is a cooperative launch: recorded and replayed like the others."""
     runner = _load(cuda_context, zoo.lstm(20, 5, 24, 96), graphReplay=True)
