@@ -195,6 +195,19 @@ def test_what_a_tape_must_not_keep(cuda_context):
     runner.dispose()
 
 
+def test_one_tensor_as_two_inputs(cuda_context):
+    ctx = cuda_context
+    runner = _load(ctx, _model([onnx_io.make_node("Sub", ["a", "b"], ["y"], name="s")], [("a", [50, 8]), ("b", [50, 8])], [("y", [50, 8])]))
+    for i in range(5):
+        a, b = (np.random.default_rng(10 * i + j).standard_normal((50, 8)).astype(np.float32) for j in (0, 1))
+        da, db = ctx.move_tensor(_cpu(a)), ctx.move_tensor(_cpu(b))
+        for x, y, want in ((da, da, a - a), (da, db, a - b), (db, da, b - a), (_cpu(a), _cpu(a), a - a)):
+            assert np.array_equal(runner.run([x, y])[0].numpy(), want)
+        da.dispose()
+        db.dispose()
+    runner.dispose()
+
+
 def test_more_signatures_than_tapes(cuda_context):
     ctx = cuda_context
     make = onnx_io.make_node

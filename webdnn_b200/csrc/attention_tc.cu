@@ -25,9 +25,10 @@
 // chunks, and the partial results (row maximum, row sum, unnormalised row) are combined through distributed shared
 // memory, each CTA finishing its part of the rows (choose_cluster).
 //
-// Warps: 0-3 row threads, 4 TMA producer (one elected lane), 5 MMA issuer.  With a head size of 32 a CTA needs 256 TMEM columns and 64 KB of shared memory, so two CTAs share an SM and
-// one's softmax overlaps the other's MMAs.  Every mbarrier wait is bounded (2 s): on expiry the CTA records a status
-// code, raises its abort flag, still meets its cluster, frees its TMEM and returns.  No multicast.
+// Warps: 0-3 row threads, 4 TMA producer (one elected lane), 5 MMA issuer.  With a head size of 32 a CTA needs 256 TMEM
+// columns and 64 KB of shared memory, so two CTAs share an SM and one's softmax overlaps the other's MMAs.  Every mbarrier
+// wait is bounded (2 s): on expiry the CTA records a status code, raises its abort flag, still meets its cluster, frees
+// its TMEM and returns.  No multicast.
 #include <cuda.h>
 
 #include <math.h>
