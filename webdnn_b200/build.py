@@ -10,7 +10,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB_PATH = os.path.join(HERE, "libwebdnn_cuda.so")
 SOURCES = ["context.cu", "transfer.cu", "tape.cu", "pointwise.cu", "rowops.cu", "pool.cu", "layout.cu", "gemm_simt.cu", "gemm_skinny.cu",
-           "conv_tc.cu", "gemm_tc_direct.cu", "lstm.cu", "lstm_persistent.cu", "lstm_cluster.cu", "extra_ops.cu", "attention.cu", "attention_tc.cu"]
+           "conv_tc.cu", "gemm_tc_direct.cu", "lstm.cu", "lstm_persistent.cu", "lstm_cluster.cu", "lstm_local.cu", "extra_ops.cu", "attention.cu", "attention_tc.cu"]
 # WDC_BUILD_DEVELOP=1 in the environment adds -DWDC_TC_DEVELOP: the contraction kernel then carries its development
 # knock-out switches (read from WDC_TC_DEBUG); the shipped build has none.
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",

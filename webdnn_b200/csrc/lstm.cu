@@ -1,6 +1,6 @@
 // ONNX LSTM (forward, default activations, gate order i,o,f,c).
 // Step 1: one GEMM projects all T steps of the input: P[T*Bt, 4H] = X * W^T.
-// Step 2: the recurrence, as one cooperative launch (lstm_cluster.cu, lstm_persistent.cu) when the shape
+// Step 2: the recurrence, as one launch (lstm_local.cu, lstm_cluster.cu, lstm_persistent.cu) when the shape
 // fits one; otherwise per time step G = h_{t-1} * R^T + P_t (GEMM with P_t as the C operand) and a
 // fused gate kernel that applies bias, sigmoid/tanh, updates c and h and writes Y_t.
 // Scratch (P, G, and the running h/c state) comes from the context arena.
@@ -16,6 +16,8 @@ int wdc_lstm_persistent(wdc_context* ctx, const float* P, const float* R, const 
                         int64_t selftest_wait_ns = 0);
 int wdc_lstm_cluster(wdc_context* ctx, const float* P, const float* R, const float* bias, const float* h0,
                      const float* c0, float* Y, float* Yh, float* Yc, int64_t T, int64_t Bt, int64_t H);
+int wdc_lstm_local(wdc_context* ctx, const float* P, const float* R, const float* bias, const float* h0, const float* c0,
+                   float* Y, float* Yh, float* Yc, int64_t T, int64_t Bt, int64_t H);
 
 __device__ __forceinline__ float sigmoid_ref(float x) { return (tanhf(x * 0.5f) + 1.f) * 0.5f; }
 
@@ -69,9 +71,10 @@ extern "C" int wdc_lstm(wdc_context* ctx, const float* X, const float* W, const 
       wdc_free(ctx, P);
       return s;
     }
-    // The whole recurrence as one launch when the shape fits one of two kernels: clusters with R in tensor memory
-    // (hidden sizes up to 768, any batch), else CTAs with R in shared memory (up to 1184, at most 64 rows).
-    s = wdc_lstm_cluster(ctx, P, R, bias, h0, c0, Y, Yh, Yc, T, Bt, H);
+    // The whole recurrence as one launch when the shape fits one of three kernels: R inside one cluster (hidden sizes up
+    // to 512), clusters that exchange h (up to 768, any batch), CTAs with R in shared memory (up to 1184, at most 64 rows).
+    s = wdc_lstm_local(ctx, P, R, bias, h0, c0, Y, Yh, Yc, T, Bt, H);
+    if (s == WDC_ERR_UNSUPPORTED) s = wdc_lstm_cluster(ctx, P, R, bias, h0, c0, Y, Yh, Yc, T, Bt, H);
     if (s == WDC_ERR_UNSUPPORTED) s = wdc_lstm_persistent(ctx, P, R, bias, h0, c0, Y, Yh, Yc, T, Bt, H);
     if (s != WDC_ERR_UNSUPPORTED) {
       wdc_free(ctx, P);

@@ -1,4 +1,5 @@
-// ONNX LSTM recurrence on the 5th-generation tensor cores, spread over the chip as thread-block clusters.
+// ONNX LSTM recurrence on the 5th-generation tensor cores, spread over the chip as thread-block clusters: hidden sizes whose R
+// does not fit one cluster (above 512; lstm_local.cu has the others, 2.0 us a step of [64, 512] where this takes 3.0).
 //
 // What bounds a recurrence is the chain of one step, not its arithmetic: h_t cannot start before h_{t-1} is known
 // everywhere.  lstm_persistent.cu spends 9 us on a step of [64, 512]: every CTA waits for a counter that all CTAs
@@ -508,8 +509,7 @@ bool few_items(int n, int kc) { return n * (kc / 4) <= 4 * THREADS; }
 Kernel kernel_of(int cs, int n, int kc) {
   const bool few = few_items(n, kc);
   if (cs == 8) return few ? lstm_cluster_kernel<8, 4> : lstm_cluster_kernel<8, 12>;
-  if (cs == 4) return few ? lstm_cluster_kernel<4, 4> : lstm_cluster_kernel<4, 12>;
-  return few ? lstm_cluster_kernel<2, 4> : lstm_cluster_kernel<2, 12>;
+  return few ? lstm_cluster_kernel<4, 4> : lstm_cluster_kernel<4, 12>;
 }
 
 size_t smem_of(int n, int kc) { return (size_t)n * ((kc + 31) / 32 * 256 + 2 * 128 * 4) + 1024; }
@@ -561,7 +561,7 @@ struct Plan {
 
 // The widest K split that fits: a wider cluster reads less of h per CTA and has a shorter product.
 Plan plan_of(wdc_context* ctx, int64_t Bt, int64_t H, int blocks) {
-  for (int cs = 8; cs >= 2; cs >>= 1) {
+  for (int cs = 8; cs >= 4; cs >>= 1) {
     Plan p;
     p.cs = cs;
     p.kc = (int)((ceil_div64(H, cs) + 7) / 8 * 8);

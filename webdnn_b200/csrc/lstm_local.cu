@@ -1,0 +1,711 @@
+// ONNX LSTM recurrence with the whole of R inside one thread-block cluster.
+//
+// What bounds a recurrence is the chain of one step.  lstm_cluster.cu spreads R over the chip, so that h crosses from
+// cluster to cluster through L2 (a store and a poll, 1850 cycles) and partial sums cross each cluster (1500 cycles).
+// Here a batch row's recurrence never leaves its cluster, and there is one exchange a step:
+//   * a CTA owns 32 hidden units (128 gate rows = the 128 lanes of an MMA) over the whole of K, a cluster the whole of R
+//     (up to 16 CTAs, 512 units); the batch is dealt to the clusters that fit on the chip, which run independently;
+//   * R fits because it is kept as two fp16 parts with a power of two per row (4 bytes an element, in tensor memory, the
+//     last low parts in shared memory), where TF32 parts take 8.  h is in (-1, 1) and has a constant scale.  Two parts of
+//     11 rounded bits carry 23 to 24 bits of the row's largest element (TF32 parts, cut by the tensor core: 22), and an
+//     fp16 MMA covers twice the K of a TF32 one in the same time: M 128 x N 16 x K 16 takes 9 cycles, N 32 takes 16;
+//   * h goes to every CTA of the cluster as 16-byte words in the layout of the MMA's B operand (no swizzle: 8 batch rows x
+//     8 units are 128 consecutive bytes), by st.async, whose mbarrier counts the bytes (a CTA takes in about 20 a clock:
+//     16 KB of 8 rows x 512 units 800 cycles).  Barriers for each four sources, so that the first MMAs overlap the last
+//     words, cost more than they gave (1.82 us a step for one, 1.82 to 1.74 for four at 16 rows, 1.49 to 1.63 at one);
+//   * two buffers of h by the parity of the step: a CTA sends h_t after it has all of h_{t-1}, which every CTA sent after
+//     its MMAs on h_{t-2}, the buffer's last reader, were complete.
+// Measured, start of a step to the next with lstm_cluster.cu and here: 256 units, batch 1, 1.63 -> 0.77 us; [64, 512] 3.0 ->
+// 1.95 us (of 3680 cycles the MMAs are 1330, the gates 850, the words on their way 1500: 20 KB into every CTA); 50 steps of
+// [1, 256] with the projection 98 -> 55 us, 128 of [64, 512] 434 -> 320 us.
+// Sums: hi*hi in one range of columns of the accumulator, hi*lo + lo*hi in another, added in fp32 after the last MMA.
+// h0 may be anything: its rows have a scale each.  A row of R, or an h0, with an infinite element or NaN has none: those
+// sums are plain fp32 FMAs.  Waits are bounded as in lstm_cluster.cu: on expiry a status word is set, the peers' waits expire in turn, and
+// all CTAs of the cluster meet at the last barrier.
+#include <cuda_fp16.h>
+#include <math.h>
+
+#include "common.cuh"
+
+namespace {
+
+constexpr int EPI_THREADS = 256;
+constexpr int THREADS = EPI_THREADS + 32;   // warps 0-7: gates; warp 8: issues the MMAs
+constexpr int UNITS = 32;                   // units of a CTA
+constexpr int MAX_CS = 16;
+constexpr int MAX_GROUPS = 4;               // 8-row groups of a cluster's batch rows
+constexpr int QUARTERS = MAX_CS / 4;
+constexpr int MAX_SMEM = 224 * 1024;
+constexpr int MIN_SMEM = 116 * 1024;        // all of tensor memory is taken: one CTA per SM
+constexpr float H_SCALE = 16384.f, H_UNSCALE = 1.f / 16384.f;
+constexpr unsigned long long WAIT_NS = 2000000000ull;
+
+struct LocalArgs {
+  const float* P;      // [T, B, 4H] input projection without bias
+  const float* R;      // [4H, H]
+  const float* bias;   // [8H] or null
+  const float* h0;     // [B, H] or null
+  const float* c0;
+  float* Y;            // [T, B, H]
+  float* Yh;
+  float* Yc;
+  int* status;
+  int T, B, H;
+  int cs;              // CTAs of a cluster: ceil(H / 32)
+  int per;             // batch rows of a cluster
+  int r_early;         // R and bias are constants: read before the grids in front have finished
+};
+
+struct LocalShared {
+  unsigned long long mma_bar;
+  unsigned long long full[2];
+  unsigned int tmem_base;
+  int plain_h;
+  float row_max[128];
+  float h0_unscale[8 * MAX_GROUPS];
+};
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.b32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ unsigned long long global_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+__device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, int* status, int code) {
+  const unsigned long long t0 = global_ns();
+  for (;;) {
+    for (int i = 0; i < 256; i++)
+      if (mbar_try_wait(bar, parity)) return true;
+    if (global_ns() - t0 > WAIT_NS) {
+      atomicCAS(status, 0, code);
+      return false;
+    }
+  }
+}
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* status, int code) {
+  for (int i = 0; i < 1024; i++)
+    if (mbar_try_wait(bar, parity)) return true;
+  return mbar_wait_slow(bar, parity, status, code);
+}
+__device__ __forceinline__ void expect_bytes(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ uint32_t map_to(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void send16(uint32_t dst, uint32_t bar, const uint4& v) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(dst),
+               "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ bool not_finite(float x) { return (__float_as_uint(x) & 0x7f800000u) == 0x7f800000u; }
+// Operand in shared memory, K-major without swizzle: 8 rows x 16 bytes are consecutive; `k_step` bytes between such
+// blocks along K, `row_step` along the rows.
+__device__ __forceinline__ uint64_t make_desc(uint32_t saddr, uint32_t k_step, uint32_t row_step) {
+  return (uint64_t)((saddr & 0x3FFFF) >> 4) | (uint64_t)(k_step >> 4) << 16 | (uint64_t)(row_step >> 4) << 32 | (uint64_t)1 << 46;
+}
+// The descriptors as their halves: only the low one (the start address) changes from MMA to MMA.
+__device__ __forceinline__ void mma_ts(uint32_t tmem_c, uint32_t tmem_a, uint32_t b_lo, uint32_t b_top, uint32_t idesc,
+                                       uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 d;\n\t"
+      "mov.b64 d, {%2, %3};\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], d, %4, p;\n\t}" ::"r"(tmem_c),
+      "r"(tmem_a), "r"(b_lo), "r"(b_top), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void mma_ts_more(uint32_t tmem_c, uint32_t tmem_a, uint32_t b_lo, uint32_t b_top, uint32_t idesc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 d;\n\t"
+      "mov.b64 d, {%2, %3};\n\t"
+      "setp.eq.b32 p, 0, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], d, %4, p;\n\t}" ::"r"(tmem_c),
+      "r"(tmem_a), "r"(b_lo), "r"(b_top), "r"(idesc)
+      : "memory");
+}
+__device__ __forceinline__ void mma_ss_more(uint32_t tmem_c, uint32_t a_lo, uint32_t a_top, uint32_t b_lo, uint32_t b_top,
+                                            uint32_t idesc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 d, a;\n\t"
+      "mov.b64 a, {%1, %2};\n\t"
+      "mov.b64 d, {%3, %4};\n\t"
+      "setp.eq.b32 p, 0, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], a, d, %5, p;\n\t}" ::"r"(tmem_c),
+      "r"(a_lo), "r"(a_top), "r"(b_lo), "r"(b_top), "r"(idesc)
+      : "memory");
+}
+__device__ __forceinline__ bool elect_one() {
+  uint32_t pred;
+  asm volatile(
+      "{\n\t.reg .pred P;\n\t"
+      "elect.sync _|P, 0xffffffff;\n\t"
+      "selp.b32 %0, 1, 0, P;\n\t}"
+      : "=r"(pred));
+  return pred != 0;
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* r) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]),
+               "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
+}
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, float* v) {
+  uint32_t* r = reinterpret_cast<uint32_t*>(v);
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(taddr)
+               : "memory");
+}
+// The gates without branches, so that a thread's calls overlap (five tanhf in a row took 700 cycles of a step of 2400).
+// e^x as 2^(x log2 e): its relative error, (|x| + 3) 2^-24, meets a factor below 0.25 in a sigmoid.
+// tanh: below 0.6 x + x^3 q(x^2), q fitted to equal ripple of the relative error (0.05 * 2^-24), above 1 - 2 / (e^2x + 1).
+__device__ __forceinline__ float exp_of(float x) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x * 1.44269504f));
+  return r;
+}
+__device__ __forceinline__ float inverse(float x) {                // of 1 .. infinity
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float sigmoid_fast(float x) { return inverse(1.f + exp_of(-x)); }
+__device__ __forceinline__ float tanh_fast(float x) {
+  const float m = fabsf(x), u = x * x;
+  float q = -0.00589514f;
+  q = fmaf(q, u, 0.02079596f);
+  q = fmaf(q, u, -0.05378383f);
+  q = fmaf(q, u, 0.13331924f);
+  q = fmaf(q, u, -0.33333298f);
+  const float small = fmaf(x * u, q, x), large = copysignf(fmaf(-2.f, inverse(exp_of(2.f * m) + 1.f), 1.f), x);
+  return m < 0.6f ? small : large;
+}
+// x = hi + lo in fp16 parts; the low part of a scaled element is at worst 2^-25, 2^-39 of the largest
+__device__ __forceinline__ void split_half(float x, __half* hi, __half* lo) {
+  *hi = __float2half_rn(x);
+  *lo = __float2half_rn(x - __half2float(*hi));
+}
+// Power of two that brings the largest magnitude `m` of a row into [2^13, 2^14) (a row of zeros or denormals: the largest
+// that leaves its inverse a normal number).
+__device__ __forceinline__ int row_exponent(float m) {
+  const int e = (int)(__float_as_uint(m) >> 23) - 127;
+  return min(13 - e, 100);
+}
+__device__ __forceinline__ float pow2(int e) { return __uint_as_float((uint32_t)(127 + e) << 23); }   // -126 <= e <= 127
+
+// h of one buffer: [source CTA][zeros? hi groups, lo groups][4 blocks of 8 units][8 batch rows][8 units], fp16.
+// An odd number of groups has a group of zeros in front: the MMA of the low parts of R has at least 16 columns and
+// adds to the range of columns that hi*lo is summed in; the zeros stand for the 8 columns in front of that range.
+template <int NG>
+struct LocalLayout {
+  static constexpr int ZERO = NG & 1;
+  static constexpr int GROUP = 512;                               // bytes of a group: 8 rows x 32 units
+  static constexpr int SRC = (ZERO + 2 * NG) * GROUP;
+  static constexpr int BUF = MAX_CS * SRC;                        // (fixed, so that operand addresses are constants)
+  static constexpr int D_COLS = 16 * NG;                          // hi*hi, then the cross products
+  static constexpr int STEPS_LO = (512 - D_COLS) / 8 - 2 * MAX_CS;   // k steps whose low parts of R are in tensor memory
+  static constexpr int LO_ROWS = 8 * (NG + ZERO);                 // columns of the MMA of the low parts
+  static constexpr int LO_COL0 = 8 * (NG - ZERO);
+  static constexpr int STAGE = 8 * NG * 128;                      // the eight warps' words on their way out
+};
+
+// The MMAs of four sources (two k steps each).  One block of straight-line code whose addresses are constant offsets from
+// bases in registers: 13 cycles an MMA.  With addresses computed for each it takes 28 to 65, with a block of constants for
+// every quarter and buffer behind a switch 25: the operands then pass through vector registers one by one.
+struct Issue {
+  uint32_t t_d, t_hi, t_lo;    // tensor memory: accumulator, high and low parts of R from these sources' columns on
+  uint32_t b, b_top;           // descriptor of their words
+  uint32_t r, r_top;           // descriptor of the low parts of R in shared memory
+};
+template <int NG, bool ALL>    // ALL: four sources, low parts in tensor memory
+__device__ __forceinline__ void issue_sources(const Issue& o, int n, int lo_in_tmem, uint32_t accumulate) {
+  using L = LocalLayout<NG>;
+  constexpr uint32_t ID_HI = (1u << 4) | ((uint32_t)(2 * NG) << 17) | ((128u >> 4) << 24);
+  constexpr uint32_t ID_LO = (1u << 4) | ((uint32_t)(L::LO_ROWS >> 3) << 17) | ((128u >> 4) << 24);
+#pragma unroll
+  for (int d = 0; d < 4; d++) {
+    if (ALL || d < n) {
+#pragma unroll
+      for (int j = 0; j < 2; j++) {
+        const int step = 2 * d + j;
+        const uint32_t b = o.b + (uint32_t)((d * L::SRC + 256 * j) >> 4), b_hi = b + (uint32_t)(L::ZERO * L::GROUP >> 4);
+        if (step == 0) mma_ts(o.t_d, o.t_hi, b_hi, o.b_top, ID_HI, accumulate);
+        else mma_ts_more(o.t_d, o.t_hi + (uint32_t)(8 * step), b_hi, o.b_top, ID_HI);
+        // (with zeros in front: their 8 columns have just been written by the MMA above, like the others)
+        if (ALL || step < lo_in_tmem) mma_ts_more(o.t_d + (uint32_t)L::LO_COL0, o.t_lo + (uint32_t)(8 * step), b, o.b_top, ID_LO);
+        else mma_ss_more(o.t_d + (uint32_t)L::LO_COL0, o.r + (uint32_t)((step - lo_in_tmem) * 256), o.r_top, b, o.b_top, ID_LO);
+      }
+    }
+  }
+}
+
+// Sum of a gate row over K with plain FMAs: row `r` of R against batch row `b` of h, from the operand or (step 0) h0.
+__device__ __noinline__ float plain_sum(const float* r, const float* h0, const unsigned char* buf, int src_bytes, int hi_off,
+                                        int lo_off, int b, int H) {
+  float s = 0.f;
+  for (int k = 0; k < H; k++) {
+    float x;
+    if (h0) {
+      x = h0[k];
+    } else {
+      const unsigned char* p = buf + (k >> 5) * src_bytes + (b >> 3) * 512 + ((k >> 3) & 3) * 128 + (b & 7) * 16 + (k & 7) * 2;
+      x = (__half2float(*reinterpret_cast<const __half*>(p + hi_off)) + __half2float(*reinterpret_cast<const __half*>(p + lo_off))) *
+          H_UNSCALE;
+    }
+    s = fmaf(r[k], x, s);
+  }
+  return s;
+}
+
+// The gates of GROUPS of a thread's NG cells (side by side: their chains of dependent operations overlap), h into `out`.
+template <int NG, int GROUPS>
+__device__ __forceinline__ void step_end(const float (&s)[NG][4], bool product, const float (&pin)[NG][4], const float (&bsum)[4],
+                                         const bool (&live)[NG], float (&c)[NG], float (&h)[NG], unsigned char* out) {
+  const bool up = (threadIdx.x & 2) != 0, odd = (threadIdx.x & 1) != 0;
+  float w[GROUPS][4] = {};
+  if (product) {
+    // a unit's four lanes hold a gate each of four batch rows: turned so that each holds four gates of a row
+    float x[GROUPS][2], r[GROUPS][2];
+#pragma unroll
+    for (int g = 0; g < GROUPS; g++) {
+      r[g][0] = __shfl_xor_sync(0xffffffffu, up ? s[g][0] : s[g][2], 2);
+      r[g][1] = __shfl_xor_sync(0xffffffffu, up ? s[g][1] : s[g][3], 2);
+    }
+#pragma unroll
+    for (int g = 0; g < GROUPS; g++) {
+      const float x00 = up ? r[g][0] : s[g][0], x01 = up ? r[g][1] : s[g][1], x10 = up ? s[g][2] : r[g][0], x11 = up ? s[g][3] : r[g][1];
+      x[g][0] = __shfl_xor_sync(0xffffffffu, odd ? x00 : x01, 1);
+      x[g][1] = __shfl_xor_sync(0xffffffffu, odd ? x10 : x11, 1);
+      w[g][0] = odd ? x[g][0] : x00;
+      w[g][1] = odd ? x01 : x[g][0];
+      w[g][2] = odd ? x[g][1] : x10;
+      w[g][3] = odd ? x11 : x[g][1];
+    }
+  }
+#pragma unroll
+  for (int g = 0; g < GROUPS; g++) {
+    const float it = sigmoid_fast(w[g][0] + (pin[g][0] + bsum[0])), ot = sigmoid_fast(w[g][1] + (pin[g][1] + bsum[1]));
+    const float ft = sigmoid_fast(w[g][2] + (pin[g][2] + bsum[2])), ct = tanh_fast(w[g][3] + (pin[g][3] + bsum[3]));
+    c[g] = ft * c[g] + it * ct;
+    h[g] = live[g] ? ot * tanh_fast(c[g]) : 0.f;
+  }
+#pragma unroll
+  for (int g = 0; g < GROUPS; g++) {
+    __half hi, lo;
+    split_half(h[g] * H_SCALE, &hi, &lo);
+    *reinterpret_cast<__half*>(out + g * 128) = hi;
+    *reinterpret_cast<__half*>(out + g * 128 + 64) = lo;
+  }
+}
+
+template <int NG>
+__global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs a) {
+  using L = LocalLayout<NG>;
+  extern __shared__ __align__(1024) unsigned char smem[];
+  __shared__ LocalShared sh;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int cs = a.cs, H = a.H;
+  const int rank = (int)(blockIdx.x % (unsigned)cs), cluster = (int)(blockIdx.x / (unsigned)cs);
+  const int b0 = cluster * a.per, nb = min(a.per, a.B - b0);
+  const int u0 = rank * UNITS;
+  const uint32_t buf_bytes = (uint32_t)L::BUF;
+  unsigned char* stage = smem + 2 * buf_bytes;
+  unsigned char* r_lo = stage + L::STAGE;                          // low parts of R past tensor memory: 4 KB a k step
+
+  if (tid == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&sh.mma_bar)));
+    for (int i = 0; i < 2; i++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&sh.full[i])));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    sh.plain_h = 0;
+  }
+  if (tid < 8 * MAX_GROUPS) sh.h0_unscale[tid] = 1.f;
+  if (warp == 8) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sh.tmem_base)),
+                 "r"(512));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  if (!a.r_early) pdl_grid_wait();
+
+  // Gate row r of the CTA = gate r % 4 of unit r / 4.  Its largest magnitude: eight lanes take 128 consecutive bytes of a
+  // row, a warp its rows 16 w .. 16 w + 15 (a thread per row, 16 bytes each, took 10 us more at 512 units).
+  const int row = (warp & 3) * 32 + lane, half = warp >> 2;
+  const int row_unit = u0 + row / 4;
+  const float* r_row = a.R + ((size_t)(row & 3) * H + (row_unit < H ? row_unit : 0)) * H;
+  if (warp < 8) {
+    for (int i = 0; i < 4; i++) {
+      const int r = warp * 16 + 4 * i + lane / 8, unit = u0 + r / 4, k1 = unit < H ? H : 0;
+      const float* src = a.R + ((size_t)(r & 3) * H + unit) * H;
+      uint32_t m = 0;                                              // (magnitudes compare like their bits)
+      for (int k = (lane & 7) * 4; k < k1; k += 256) {
+        uint4 v[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++)
+          v[j] = k + 32 * j < k1 ? *reinterpret_cast<const uint4*>(src + k + 32 * j) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for (int j = 0; j < 8; j++)
+          m = max(max(max(v[j].x & 0x7fffffffu, v[j].y & 0x7fffffffu), max(v[j].z & 0x7fffffffu, v[j].w & 0x7fffffffu)), m);
+      }
+#pragma unroll
+      for (int o = 1; o < 8; o <<= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+      if ((lane & 7) == 0) sh.row_max[r] = __uint_as_float(m);
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = sh.tmem_base;
+  const uint32_t tmem_hi = tmem + (uint32_t)L::D_COLS, tmem_lo = tmem_hi + (uint32_t)(16 * cs);
+  bool plain_row = false;
+  float unscale = 0.f;
+  if (warp < 8) {
+    const float m = sh.row_max[row];
+    plain_row = not_finite(m);
+    const int e = plain_row ? 0 : row_exponent(m);
+    const float scale = pow2(e);
+    unscale = pow2(-e) * H_UNSCALE;                                // (e <= 100: a normal number)
+    const uint32_t t_row = (uint32_t)((warp & 3) * 32) << 16;
+    // 64 columns at a time through shared memory (rows 272 bytes apart: no bank conflicts either way); warps w and w + 4 take
+    // 32 of them each of the rows 32 w .. 32 w + 31
+    float4* chunk = reinterpret_cast<float4*>(smem + 2 * buf_bytes - 128 * 272);
+    float4 next[8];
+    auto fetch = [&](int k) {
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        const int r = j * 16 + tid / 16, unit = u0 + r / 4, col = k + (tid & 15) * 4;
+        next[j] = unit < H && col < H ? *reinterpret_cast<const float4*>(a.R + ((size_t)(r & 3) * H + unit) * H + col)
+                                      : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    };
+    fetch(0);
+    for (int k = 0; k < cs * 32; k += 64) {
+#pragma unroll
+      for (int j = 0; j < 8; j++) chunk[(j * 16 + tid / 16) * 17 + (tid & 15)] = next[j];
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      if (k + 64 < cs * 32) fetch(k + 64);
+      for (int i = 0; i < 2; i++) {
+        const int j = k / 16 + half * 2 + i;                       // k step of 16
+        if (j >= 2 * cs) break;
+        uint32_t hi[8], lo[8];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          const float4 v = chunk[row * 17 + half * 8 + i * 4 + q];
+          const float x[4] = {v.x * scale, v.y * scale, v.z * scale, v.w * scale};
+          __half h[4], l[4];
+#pragma unroll
+          for (int c = 0; c < 4; c++) split_half(plain_row ? 0.f : x[c], &h[c], &l[c]);
+#pragma unroll
+          for (int c = 0; c < 2; c++) {
+            hi[q * 2 + c] = (uint32_t)__half_as_ushort(h[2 * c]) | (uint32_t)__half_as_ushort(h[2 * c + 1]) << 16;
+            lo[q * 2 + c] = (uint32_t)__half_as_ushort(l[2 * c]) | (uint32_t)__half_as_ushort(l[2 * c + 1]) << 16;
+          }
+        }
+        tmem_st8(tmem_hi + t_row + (uint32_t)(8 * j), hi);
+        if (j < L::STEPS_LO) {
+          tmem_st8(tmem_lo + t_row + (uint32_t)(8 * j), lo);
+        } else {
+          unsigned char* dst = r_lo + (size_t)(j - L::STEPS_LO) * 4096 + row * 16;
+          *reinterpret_cast<uint4*>(dst) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+          *reinterpret_cast<uint4*>(dst + 2048) = make_uint4(lo[4], lo[5], lo[6], lo[7]);
+        }
+      }
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+    }
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+  }
+  __syncthreads();
+  for (uint32_t i = (uint32_t)tid * 16u; i < 2u * buf_bytes; i += THREADS * 16u)   // rows past the batch stay zero
+    *reinterpret_cast<uint4*>(smem + i) = make_uint4(0, 0, 0, 0);
+  __syncthreads();
+  if (a.r_early) pdl_grid_wait();
+
+  // Cells of a thread: unit 8 (warp % 4) + lane / 4, batch rows 8 g + 4 (warp / 4) + lane % 4
+  const int unit = u0 + 8 * (warp & 3) + lane / 4, row0 = 4 * half + (lane & 3);
+  float c_reg[NG], h_reg[NG], bsum[4], pin[NG][4];
+  bool live[NG];
+#pragma unroll
+  for (int g = 0; g < 4; g++) bsum[g] = warp < 8 && unit < H && a.bias ? a.bias[g * H + unit] + a.bias[(4 + g) * H + unit] : 0.f;
+  const float* p_src = a.P + (size_t)(b0 + row0) * 4 * H + unit;
+  float* y_dst = a.Y + (size_t)(b0 + row0) * H + unit;
+#pragma unroll
+  for (int g = 0; g < NG; g++) {
+    live[g] = warp < 8 && unit < H && 8 * g + row0 < nb;
+    c_reg[g] = live[g] && a.c0 ? a.c0[(size_t)(b0 + 8 * g + row0) * H + unit] : 0.f;
+    h_reg[g] = 0.f;
+#pragma unroll
+    for (int q = 0; q < 4; q++) pin[g][q] = live[g] ? p_src[(size_t)8 * g * 4 * H + q * H] : 0.f;
+  }
+  constexpr int HI_OFF = L::ZERO * L::GROUP, LO_OFF = HI_OFF + NG * L::GROUP;
+  if (a.h0) {   // into buffer 0, each batch row with a scale of its own
+    for (int b = warp; b < nb; b += THREADS / 32) {
+      const float* src = a.h0 + (size_t)(b0 + b) * H;
+      uint32_t m = 0;
+      for (int k = lane; k < H; k += 32) m = max(m, __float_as_uint(src[k]) & 0x7fffffffu);
+      m = __reduce_max_sync(0xffffffffu, m);
+      if (not_finite(__uint_as_float(m))) {
+        if (lane == 0) sh.plain_h = 1;
+        continue;
+      }
+      const int e = row_exponent(__uint_as_float(m));
+      const float scale = pow2(e);
+      if (lane == 0) sh.h0_unscale[b] = pow2(-e);
+      for (int k = lane; k < H; k += 32) {
+        __half hi, lo;
+        split_half(src[k] * scale, &hi, &lo);
+        unsigned char* p = smem + (k >> 5) * L::SRC + (b >> 3) * 512 + ((k >> 3) & 3) * 128 + (b & 7) * 16 + (k & 7) * 2;
+        *reinterpret_cast<__half*>(p + HI_OFF) = hi;
+        *reinterpret_cast<__half*>(p + LO_OFF) = lo;
+      }
+    }
+  }
+  const uint32_t full0 = smem_u32(&sh.full[0]);
+  const int quarters = (cs + 3) / 4;
+  const uint32_t step_bytes = (uint32_t)cs * (uint32_t)nb * 128u;  // a source sends 128 for each batch row
+  if (tid == 0) {
+    expect_bytes(full0, step_bytes);
+    expect_bytes(full0 + 8u, step_bytes);
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // (zeros, h0 and low parts of R are read by the MMAs)
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  cluster_barrier();                                               // every CTA is ready for the others' words
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const bool plain_h = sh.plain_h != 0;
+  const uint32_t mma_bar = smem_u32(&sh.mma_bar);
+
+  if (warp == 8) {
+    const uint64_t b_desc = make_desc(smem_u32(smem), 128, L::GROUP), r_desc = make_desc(smem_u32(r_lo), 2048, 128);
+    if (elect_one()) {
+      for (int t = a.h0 ? 0 : 1; t < a.T; t++) {
+        const uint32_t bar = full0 + (t & 1 ? 8u : 0u);
+        if (t > 0) {
+          if (!mbar_wait(bar, (uint32_t)((t - 1) >> 1) & 1u, a.status, 94)) break;
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        for (int q = 0; q < quarters; q++) {
+          const int n = cs - 4 * q, lo_in_tmem = L::STEPS_LO - 8 * q;
+          const Issue o = {tmem, tmem_hi + (uint32_t)(64 * q), tmem_lo + (uint32_t)(64 * q),
+                           (uint32_t)b_desc + (uint32_t)(((t & 1) * L::BUF + 4 * q * L::SRC) >> 4), (uint32_t)(b_desc >> 32),
+                           (uint32_t)r_desc, (uint32_t)(r_desc >> 32)};
+          if (n >= 4 && lo_in_tmem >= 8) issue_sources<NG, true>(o, n, lo_in_tmem, q > 0 ? 1u : 0u);
+          else issue_sources<NG, false>(o, n, lo_in_tmem, q > 0 ? 1u : 0u);
+        }
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mma_bar) : "memory");
+        if (t > 0) expect_bytes(bar, step_bytes);                  // the words of step t + 2
+      }
+    }
+    __syncwarp();
+  } else {
+    const uint32_t t_row = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(4 * half);
+    // words on their way out: [group][hi, lo][4 batch rows][8 units] of this warp
+    unsigned char* out = stage + warp * (128 * NG);
+    unsigned char* my_out = out + (lane & 3) * 16 + (lane >> 2) * 2;
+    const int w_part = (lane >> 2) & 1, w_row = lane & 3, dist = lane >> 3;
+    uint32_t dst[QUARTERS];
+    uint32_t reach = 0;                                            // which of its up to four receivers there are
+    const uint32_t my_slot = smem_u32(smem) + (uint32_t)(rank * L::SRC + (w_part ? LO_OFF : HI_OFF) + (warp & 3) * 128 + (4 * half + w_row) * 16);
+    const uint32_t to_bar = full0 - my_slot;                       // from where the word goes to its barrier
+#pragma unroll
+    for (int i = 0; i < QUARTERS; i++) {
+      int peer = rank + dist + 4 * i;                              // (not all CTAs start with the same receiver)
+      if (dist + 4 * i < cs) reach |= 1u << i;
+      if (peer >= cs) peer -= cs;
+      dst[i] = map_to(my_slot, (uint32_t)(dist + 4 * i < cs ? peer : rank));
+    }
+    const bool any_plain = __any_sync(0xffffffffu, plain_row);
+    const bool some = 4 * half < nb;                               // (the last rows' warps may have nothing to do)
+    const bool last_empty = 8 * (NG - 1) + 4 * half >= nb;
+    uint32_t phase = 0;
+    for (int t = 0; t < a.T && some; t++) {
+      float s[NG][4];
+      const bool product = t > 0 || a.h0;
+      if (product) {
+        if (!__all_sync(0xffffffffu, mbar_wait(mma_bar, phase, a.status, 95))) break;
+        phase ^= 1u;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        float x[NG][4];
+#pragma unroll
+        for (int g = 0; g < NG; g++) {
+          tmem_ld4(t_row + (uint32_t)(8 * g), s[g]);
+          tmem_ld4(t_row + (uint32_t)(8 * NG + 8 * g), x[g]);
+        }
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+#pragma unroll
+        for (int g = 0; g < NG; g++)
+#pragma unroll
+          for (int j = 0; j < 4; j++) s[g][j] = (s[g][j] + x[g][j]) * unscale;
+        if (t == 0) {                                              // h0 has scales of its own
+#pragma unroll
+          for (int g = 0; g < NG; g++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) s[g][j] = s[g][j] * H_SCALE * sh.h0_unscale[8 * g + 4 * half + j];
+        }
+        if (any_plain || (t == 0 && plain_h)) {
+          bool ok = true;
+          if (t > 0)                                               // (this thread reads the others' words itself)
+            ok = mbar_wait(full0 + (t & 1 ? 8u : 0u), (uint32_t)((t - 1) >> 1) & 1u, a.status, 96);
+          const unsigned char* buf = smem + (t & 1 ? buf_bytes : 0u);
+#pragma unroll
+          for (int g = 0; g < NG; g++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+              const int b = 8 * g + 4 * half + j;
+              if (ok && (plain_row || (t == 0 && plain_h)) && b < nb && row_unit < H)
+                s[g][j] = plain_sum(r_row, t == 0 ? a.h0 + (size_t)(b0 + b) * H : nullptr, buf, L::SRC, HI_OFF, LO_OFF, b, H);
+            }
+          __syncwarp();
+        }
+      }
+      // (the last group of a warp's rows may be empty: a branch for all of its threads)
+      if (NG > 1 && last_empty) step_end<NG, (NG > 1 ? NG - 1 : 1)>(s, product, pin, bsum, live, c_reg, h_reg, my_out);
+      else step_end<NG, NG>(s, product, pin, bsum, live, c_reg, h_reg, my_out);
+      __syncwarp();
+      if (t + 1 < a.T) {
+        const uint32_t to = t & 1 ? 0u : buf_bytes, bar = to_bar + (t & 1 ? 0u : 8u);   // buffer and barrier of step t + 1
+#pragma unroll
+        for (int g = 0; g < NG; g++) {
+          if (8 * g + 4 * half + w_row < nb) {
+            const uint4 v = *reinterpret_cast<const uint4*>(out + g * 128 + (lane & 7) * 16);
+#pragma unroll
+            for (int i = 0; i < QUARTERS; i++)
+              if (reach >> i & 1u) send16(dst[i] + to + (uint32_t)(g * L::GROUP), dst[i] + bar, v);
+          }
+        }
+        __syncwarp();
+      }
+      p_src += (size_t)a.B * 4 * H;
+#pragma unroll
+      for (int g = 0; g < NG; g++) {
+        if (!live[g]) continue;
+        y_dst[(size_t)8 * g * H] = h_reg[g];
+        if (t + 1 < a.T) {
+#pragma unroll
+          for (int q = 0; q < 4; q++) pin[g][q] = p_src[(size_t)8 * g * 4 * H + q * H];
+        }
+      }
+      y_dst += (size_t)a.B * H;
+    }
+#pragma unroll
+    for (int g = 0; g < NG; g++) {
+      if (!live[g]) continue;
+      a.Yh[(size_t)(b0 + 8 * g + row0) * H + unit] = h_reg[g];
+      a.Yc[(size_t)(b0 + 8 * g + row0) * H + unit] = c_reg[g];
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  cluster_barrier();
+  if (warp == 8) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
+  }
+}
+
+typedef void (*Kernel)(const LocalArgs);
+
+Kernel kernel_of(int groups) {
+  switch (groups) {
+    case 1: return lstm_local_kernel<1>;
+    case 2: return lstm_local_kernel<2>;
+    case 3: return lstm_local_kernel<3>;
+    default: return lstm_local_kernel<4>;
+  }
+}
+
+template <int NG>
+size_t smem_of_groups(int cs) {
+  using L = LocalLayout<NG>;
+  const int in_smem = 2 * cs > L::STEPS_LO ? 2 * cs - L::STEPS_LO : 0;
+  return 2 * L::BUF + L::STAGE + (size_t)in_smem * 4096;
+}
+size_t smem_of(int cs, int groups) {
+  const size_t bytes = groups == 1 ? smem_of_groups<1>(cs) : groups == 2 ? smem_of_groups<2>(cs) : groups == 3 ? smem_of_groups<3>(cs) : smem_of_groups<4>(cs);
+  return bytes < MIN_SMEM ? MIN_SMEM : bytes;
+}
+
+void fill_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, int grid, int cs, size_t smem, cudaStream_t stream) {
+  *cfg = {};
+  cfg->gridDim = dim3((unsigned)grid);
+  cfg->blockDim = dim3(THREADS);
+  cfg->dynamicSmemBytes = smem;
+  cfg->stream = stream;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)cs;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg->attrs = attr;
+  cfg->numAttrs = 1;
+}
+
+// Clusters that can be resident at once (asked once per device and shape).
+int max_clusters(wdc_context* ctx, int cs, int groups) {
+  static std::mutex mu;
+  static std::map<std::pair<std::pair<int, int>, int>, int> known;
+  std::lock_guard<std::mutex> lk(mu);
+  const auto key = std::make_pair(std::make_pair(ctx->device, cs), groups);
+  auto it = known.find(key);
+  if (it != known.end()) return it->second;
+  int n = 0;
+  const Kernel kernel = kernel_of(groups);
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attr[2];
+  fill_config(&cfg, attr, cs, cs, smem_of(cs, groups), nullptr);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    n = 0;
+  }
+  known[key] = n;
+  return n;
+}
+
+}  // namespace
+
+// Runs the recurrence on the projected input P.  WDC_ERR_UNSUPPORTED: shape outside the kernel's range (nothing has been
+// written); any other non-zero status is an error.
+int wdc_lstm_local(wdc_context* ctx, const float* P, const float* R, const float* bias, const float* h0, const float* c0,
+                   float* Y, float* Yh, float* Yc, int64_t T, int64_t Bt, int64_t H) {
+  if (T < 4 || H < UNITS || H > MAX_CS * UNITS || H % 4 != 0) return WDC_ERR_UNSUPPORTED;
+  if (T > (1 << 24) || Bt > (1 << 20)) return WDC_ERR_UNSUPPORTED;
+  if (((uintptr_t)R & 15) != 0) return WDC_ERR_UNSUPPORTED;
+  LocalArgs a = {P, R, bias, h0, c0, Y, Yh, Yc, ctx->status_word, (int)T, (int)Bt, (int)H};
+  a.cs = (int)((H + UNITS - 1) / UNITS);
+  const int fit = max_clusters(ctx, a.cs, MAX_GROUPS);
+  if (!fit) return WDC_ERR_UNSUPPORTED;
+  const int64_t rounds = ceil_div64(Bt, (int64_t)fit * 8 * MAX_GROUPS);
+  a.per = (int)ceil_div64(Bt, rounds * fit);
+  const int groups = (a.per + 7) / 8, clusters = (int)ceil_div64(Bt, a.per);
+  if (!max_clusters(ctx, a.cs, groups)) return WDC_ERR_UNSUPPORTED;
+  a.r_early = ctx->opt_pdl && wdc_is_constant(ctx, R) && (!bias || wdc_is_constant(ctx, bias));
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attr[2];
+  fill_config(&cfg, attr, clusters * a.cs, a.cs, smem_of(a.cs, groups), ctx->stream);
+  cfg.numAttrs = ctx->opt_pdl ? 2 : 1;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kernel_of(groups), (const LocalArgs)a);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return WDC_ERR_UNSUPPORTED;
+  }
+  ctx->n_tc_launch++;
+  return wdc_check_launch(ctx, "lstm_local_kernel");
+}
