@@ -1,4 +1,4 @@
-"""Products with a handful of columns, on either side of the rule that sends them to the dot-product kernel (gemm_simt.cu)."""
+"""Products whose rows are no multiple of four columns, by the small tensor-core kernel (one CTA a tile, and clusters) and past it."""
 import numpy as np
 import pytest
 
@@ -8,8 +8,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("bias", [False, True])
-@pytest.mark.parametrize("m,k,n", [(32, 256, 1), (33, 512, 10), (64, 257, 15), (64, 512, 16), (64, 512, 17), (64, 255, 10),
-                                   (2048, 512, 10), (2049, 512, 10), (100, 1000, 3), (31, 512, 10)])
+@pytest.mark.parametrize("m,k,n", [(32, 256, 1), (33, 512, 10), (64, 260, 15), (64, 512, 17), (200, 64, 33), (130, 128, 35), (64, 36, 5),
+                                   (64, 1024, 62), (2048, 512, 10), (40000, 64, 3), (100, 1000, 3), (31, 512, 10)])
 def test_few_columns(cuda_context, m, k, n, bias):
     rng = np.random.default_rng(m + k + n)
     a, b = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((n, k)).astype(np.float32)

@@ -1874,10 +1874,14 @@ bool launch_columns(wdc_context* ctx, TcProblem p, WeightEntry* we, const float*
                        (((uintptr_t)p.shift | (uintptr_t)p.residual | (uintptr_t)y) & 15) == 0 &&
                        (!p.residual || p.res_stride % 4 == 0);
   const bool may_split = may_cut && ctx->opt_split_k;
+  // tc_small_kernel also stores rows of any length, a column at a time: [64, 512] x [512, 10], an MLP's last layer, 6.2 us where
+  // one tile that walks K alone and leaves through the plain epilogue takes 10.1 (from call to call), [20000, 512] x [512, 10] 13.6 for
+  // 16.2.
+  const bool ragged = !p.c4 && p.N % 4 != 0 && p.M < (1ll << 27) && tc_state(ctx)->encode_im2col != nullptr;
   choose_tiling(ctx, p.M, n_one, p.kblocks, may_split, &p.tile_n, &p.splits, &p.full_tiles);
   int tn = 0, cs = 0;
   CUtensorMap map_a;
-  if (may_cut && we->constant && ctx->opt_small_tile >= 0 &&
+  if ((may_cut || ragged) && we->constant && ctx->opt_small_tile >= 0 &&
       choose_small(ctx, p, n_one, p.tile_n, p.splits, p.full_tiles, &tn, &cs) && encode_a_map(tc_state(ctx), p, x, &map_a)) {
     p.part = p.splits > 1 ? (p.kblocks + p.splits - 1) / p.splits : SEG_KBLOCKS;
     p.rot_n = n_one;

@@ -110,6 +110,16 @@ __device__ __forceinline__ uint32_t exchange_slot(uint32_t row, uint32_t cell) {
   return cell * ROWS + (ROWS % 8 == 0 ? row ^ (cell & 7u) : row);
 }
 
+// Four columns from `n` on of a row of N that is `ragged` (N no multiple of 4: rows start anywhere, the last cell is short).
+__device__ __forceinline__ float4 small_cell(const float* p, int n, int N, bool ragged) {
+  if (!ragged) return pdl_ld(reinterpret_cast<const float4*>(p));
+  float4 v = make_float4(pdl_ld(p), 0.f, 0.f, 0.f);
+  if (n + 1 < N) v.y = pdl_ld(p + 1);
+  if (n + 2 < N) v.z = pdl_ld(p + 2);
+  if (n + 3 < N) v.w = pdl_ld(p + 3);
+  return v;
+}
+
 // CS: CTAs of a cluster = parts of K (1: the tile as a whole).  grid: tiles_m * tiles_n * CS.
 template <int TN, int CS>
 __global__ void __launch_bounds__(SM_THREADS, 2)
@@ -177,6 +187,7 @@ tc_small_kernel(const __grid_constant__ TcProblem p, const __grid_constant__ CUt
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   const uint32_t tmem_base = ss->tmem_base;
   const int q4 = warp & 3, half = warp >> 2;
+  const bool ragged = (p.N & 3) != 0;
   float acc[COLS];
   bool ok = true;
 
@@ -212,7 +223,7 @@ tc_small_kernel(const __grid_constant__ TcProblem p, const __grid_constant__ CUt
       for (int j = 0; j < COLS; j += 4) {
         const int n = n0 + half * COLS + j;
         if (n >= p.N) break;
-        const float4 b = pdl_ld(reinterpret_cast<const float4*>(p.shift + n));
+        const float4 b = small_cell(p.shift + n, n, p.N, ragged);
         acc[j] = p.shift_mul * b.x;
         acc[j + 1] = p.shift_mul * b.y;
         acc[j + 2] = p.shift_mul * b.z;
@@ -452,10 +463,10 @@ tc_small_kernel(const __grid_constant__ TcProblem p, const __grid_constant__ CUt
       out[i] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (live[i]) {
         if (CS > 1 && p.shift) {
-          const float4 b = pdl_ld(reinterpret_cast<const float4*>(p.shift + n));
+          const float4 b = small_cell(p.shift + n, n, p.N, ragged);
           out[i] = make_float4(p.shift_mul * b.x, p.shift_mul * b.y, p.shift_mul * b.z, p.shift_mul * b.w);
         }
-        if (p.residual) res[i] = pdl_ld(reinterpret_cast<const float4*>(p.residual + m * p.res_stride + n));
+        if (p.residual) res[i] = small_cell(p.residual + m * p.res_stride + n, n, p.N, ragged);
       }
     }
     if (CS > 1) ok = sums_ok && small_wait(smem_u32(&ss->recv), 0, ss, p.status, 59);
@@ -484,7 +495,16 @@ tc_small_kernel(const __grid_constant__ TcProblem p, const __grid_constant__ CUt
         if (p.relu) {
           s.x = relu_nan(s.x); s.y = relu_nan(s.y); s.z = relu_nan(s.z); s.w = relu_nan(s.w);
         }
-        *reinterpret_cast<float4*>(y + (m0 + rank * share + r) * p.y_stride + n0 + cell * 4) = s;
+        float* dst = y + (m0 + rank * share + r) * p.y_stride + n0 + cell * 4;
+        if (!ragged) {
+          *reinterpret_cast<float4*>(dst) = s;
+        } else {
+          const int left = p.N - n0 - cell * 4;
+          dst[0] = s.x;
+          if (left > 1) dst[1] = s.y;
+          if (left > 2) dst[2] = s.z;
+          if (left > 3) dst[3] = s.w;
+        }
       }
     }
   }

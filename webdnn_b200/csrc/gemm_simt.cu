@@ -214,15 +214,6 @@ static int gemm_call(wdc_context* ctx, const wdc_gemm_desc* d, int64_t columns, 
   WDC_REQUIRE(ctx, Y && (d->k == 0 || (A && B)), "wdc_gemm: null buffer");
   DeviceGuard g(ctx->device);
   ProfScope prof(ctx, 2.0 * (double)d->batch * (double)d->m * (double)d->n * (double)d->k);
-  // A handful of columns that the small tensor-core kernel cannot store (no multiple of 4; a classifier's last layer): a
-  // tile 128 wide would be nearly empty and walk the whole of K by itself.  As dot products spread over the chip [64, 512] x
-  // [512, 10] takes 4.9 us and not 9.8 from call to call, [2048, 512] x [512, 10] 7.3 and not 10.1; past that (20000 rows:
-  // 55 and 16) and for short reductions (4096 rows of 64: 7.2 and 5.2) the tile is the better one.
-  if (d->m >= 32 && d->n <= 16 && d->n % 4 != 0 && d->k >= 256 && d->m * d->k <= (1 << 20) && d->batch == 1 && d->sb0 == 1 &&
-      columns == 0 && (C == nullptr || C != Y)) {
-    const int s = wdc_skinny_gemm(ctx, d, A, B, C, Y);
-    if (s != WDC_ERR_UNSUPPORTED) return s;
-  }
   // Y = alpha*A*B + beta*Y (C aliasing the output) is served by the CUDA-core kernel's in-place mode only
   int s = (C != nullptr && C == Y) ? WDC_ERR_UNSUPPORTED : wdc_tc_gemm(ctx, d, A, B, C, Y, columns);
   if (s != WDC_ERR_UNSUPPORTED) return s;
