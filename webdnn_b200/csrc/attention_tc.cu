@@ -133,36 +133,22 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr) {
 __device__ __forceinline__ uint32_t make_idesc(int n) {
   return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(BQ >> 4) << 24);
 }
-// kAll: the whole warp runs the issuing loop, so that its addresses stay in uniform registers, and the lane whose `leader`
-// is 1 issues; else the calling lane does.
-template <bool kAll>
-__device__ __forceinline__ void umma_by(uint32_t leader, uint32_t tmem_c, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc,
-                                        uint32_t accumulate) {
-  if (kAll)
-    asm volatile(
-        "{\n\t.reg .pred p, e;\n\t"
-        "setp.ne.b32 e, %0, 0;\n\t"
-        "setp.ne.b32 p, %5, 0;\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::tf32 [%1], [%2], %3, %4, p;\n\t}"
-        :
-        : "r"(leader), "r"(tmem_c), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-        : "memory");
-  else
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}"
-        :
-        : "r"(tmem_c), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-__device__ __forceinline__ void commit_by(uint32_t leader, unsigned long long* bar) {
+// An MMA and a commit by one lane.  The issuing loop stands in a branch on elect.sync itself, where the compiler knows that
+// one lane is active and passes operands through uniform registers as they are; in a branch on a copy of the answer, or
+// with a predicate inside the instruction, it makes sure of their uniformity for every MMA (37 cycles each and 110 for a
+// commit, where the 24 MMAs of P V take 16 each).
+__device__ __forceinline__ void umma_one(uint32_t tmem_c, uint32_t tmem_a, uint32_t desc_lo, uint32_t desc_top, uint32_t idesc,
+                                         uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred e;\n\t"
-      "setp.ne.b32 e, %0, 0;\n\t"
-      "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%1];\n\t}" ::"r"(leader),
-      "r"(smem_u32(bar))
+      "{\n\t.reg .pred p;\n\t.reg .b64 d;\n\t"
+      "mov.b64 d, {%2, %3};\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], d, %4, p;\n\t}" ::"r"(tmem_c),
+      "r"(tmem_a), "r"(desc_lo), "r"(desc_top), "r"(idesc), "r"(accumulate)
       : "memory");
+}
+__device__ __forceinline__ void umma_commit_one(unsigned long long* bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
@@ -430,10 +416,7 @@ attention_tc_kernel(const AttTcProblem p, const __grid_constant__ CUtensorMap ma
     }
   } else {
     // ============================================================================ MMA issuer
-    // (where CTAs fill the GPU, one lane alone: the row threads lose more to a warp that polls than the issue loop gains)
-    const bool elected = elect_one();
-    const uint32_t leader = elected ? 1u : 0u;
-    if (kCluster || elected) {
+    if (elect_one()) {   // (see umma_one)
       const uint32_t idesc_s = make_idesc(BK), idesc_o = make_idesc(DH);
       const uint32_t t_qhi = tmem_base + L::Q_HI, t_qlo = tmem_base + L::Q_LO, t_s = tmem_base + L::S,
                      t_plo = tmem_base + L::P_LO, t_o = tmem_base + L::O;
@@ -450,39 +433,38 @@ attention_tc_kernel(const AttTcProblem p, const __grid_constant__ CUtensorMap ma
           if (!ok) break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t sb = smem_u32(stage_base + st * L::STAGE_BYTES);
+        const uint64_t desc = make_smem_desc(smem_u32(stage_base + st * L::STAGE_BYTES));
+        const uint32_t lo0 = (uint32_t)desc, top = (uint32_t)(desc >> 32);
 #pragma unroll
         for (int kb = 0; kb < L::KB; kb++) {
-          const uint64_t d_hi = make_smem_desc(sb + L::K_HI + kb * L::K_TILE);
-          const uint64_t d_lo = make_smem_desc(sb + L::K_LO + kb * L::K_TILE);
+          const uint32_t d_hi = lo0 + (uint32_t)((L::K_HI + kb * L::K_TILE) >> 4), d_lo = lo0 + (uint32_t)((L::K_LO + kb * L::K_TILE) >> 4);
 #pragma unroll
           for (int k8 = 0; k8 < 4; k8++) {
             const uint32_t acol = (uint32_t)(kb * 32 + k8 * 8);
-            const uint64_t adv = (uint64_t)(k8 * 2);
-            umma_by<kCluster>(leader, t_s, t_qlo + acol, d_hi + adv, idesc_s, (kb | k8) ? 1u : 0u);
-            umma_by<kCluster>(leader, t_s, t_qhi + acol, d_lo + adv, idesc_s, 1u);
-            umma_by<kCluster>(leader, t_s, t_qhi + acol, d_hi + adv, idesc_s, 1u);
+            const uint32_t adv = (uint32_t)(k8 * 2);
+            umma_one(t_s, t_qlo + acol, d_hi + adv, top, idesc_s, (kb | k8) ? 1u : 0u);
+            umma_one(t_s, t_qhi + acol, d_lo + adv, top, idesc_s, 1u);
+            umma_one(t_s, t_qhi + acol, d_hi + adv, top, idesc_s, 1u);
           }
         }
-        commit_by(leader, &sh->s_full);
+        umma_commit_one(&sh->s_full);
         ok = mbar_wait(&sh->p_ready, ph, sh, p.status, 77);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
         for (int blk = 0; blk < 2; blk++) {
-          const uint64_t d_hi = make_smem_desc(sb + L::V_HI + blk * L::V_TILE);
-          const uint64_t d_lo = make_smem_desc(sb + L::V_LO + blk * L::V_TILE);
+          const uint32_t d_hi = lo0 + (uint32_t)((L::V_HI + blk * L::V_TILE) >> 4), d_lo = lo0 + (uint32_t)((L::V_LO + blk * L::V_TILE) >> 4);
 #pragma unroll
           for (int k8 = 0; k8 < 4; k8++) {
             const uint32_t acol = (uint32_t)(blk * 32 + k8 * 8);
-            const uint64_t adv = (uint64_t)(k8 * 2);
-            umma_by<kCluster>(leader, t_o, t_plo + acol, d_hi + adv, idesc_o, (blk | k8) ? 1u : 0u);
-            umma_by<kCluster>(leader, t_o, t_s + acol, d_lo + adv, idesc_o, 1u);
-            umma_by<kCluster>(leader, t_o, t_s + acol, d_hi + adv, idesc_o, 1u);
+            const uint32_t adv = (uint32_t)(k8 * 2);
+            umma_one(t_o, t_plo + acol, d_hi + adv, top, idesc_o, (blk | k8) ? 1u : 0u);
+            umma_one(t_o, t_s + acol, d_lo + adv, top, idesc_o, 1u);
+            umma_one(t_o, t_s + acol, d_hi + adv, top, idesc_o, 1u);
           }
         }
-        commit_by(leader, &sh->kv_empty[st]);   // the stage's tiles have been read
-        commit_by(leader, &sh->o_full);
+        umma_commit_one(&sh->kv_empty[st]);   // the stage's tiles have been read
+        umma_commit_one(&sh->o_full);
       }
     }
   }
