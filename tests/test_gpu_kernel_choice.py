@@ -70,6 +70,47 @@ def test_small_outputs_are_the_same_bits(cuda_context, m, n, kblocks, ragged, pr
         t.dispose()
 
 
+# rows that are no multiple of four columns: tiles are not cut; one segment to eight of them and more; the addend comes last
+@pytest.mark.parametrize("m,n,k", [(76, 1, 32), (50, 35, 148), (64, 10, 512), (129, 67, 1024), (200, 33, 64), (2048, 10, 512),
+                                   (45, 62, 768), (66, 5, 640), (90, 6, 896), (33, 2, 1280), (4000, 63, 256)])
+@pytest.mark.parametrize("precision", ["tf32x3", "tf32x1"])
+def test_rows_of_any_length_are_the_same_bits(cuda_context, m, n, k, precision):
+    from webdnn_b200.lib import GemmDesc
+    ctx = cuda_context
+    rng = np.random.default_rng(m + n)
+    da, db = (_put(ctx, rng.standard_normal(s).astype(np.float32)) for s in ((m, k), (k, n)))
+    shift, full = _put(ctx, rng.standard_normal(n).astype(np.float32)), _put(ctx, rng.standard_normal((m, (n + 3) // 4 * 4)).astype(np.float32))
+    y = ctx.empty_tensor([m, n])
+    ctx.declare_constant(db)
+    ctx.set_precision(precision)
+    seen = set()
+
+    def product(c, beta, tile):
+        d = GemmDesc(batch=1, m=m, n=n, k=k, sab=0, sa0=k, sa1=1, sbb=0, sb0=n, sb1=1, sc0=0 if c is shift else full.dims[1],
+                     sc1=1, alpha=1.5, beta=beta, relu=int(beta != 1))
+        ctx.set_option("small_tile", tile)
+        ctx.gemm(d, da, db, c, y)
+        return y.get_data().copy().view(np.uint32), ctx.stats(device_memory=True)["last_contraction"]
+
+    try:
+        for split_k in (1, 0):
+            ctx.set_option("split_k", split_k)
+            for c, beta in ((None, 1.0), (shift, 1.0), (shift, 0.7), (full, 0.7)):
+                want, kernel = product(c, beta, -1)
+                assert kernel == 0
+                for tile in (32, 64):
+                    got, kernel = product(c, beta, tile)
+                    seen.add(kernel // 10)
+                    assert np.array_equal(got, want), (split_k, beta, tile, kernel)
+    finally:
+        ctx.set_option("small_tile", 0)
+        ctx.set_option("split_k", 1)
+        ctx.set_precision("tf32x3")
+    assert any(s % 10 == 1 for s in seen) and (any(s % 10 > 1 for s in seen) or not 256 <= k <= 1024), seen
+    for t in (da, db, shift, full, y):
+        t.dispose()
+
+
 def test_every_cluster_size_is_taken(cuda_context):
     """The shapes above do reach every variant of the small kernel."""
     ctx = cuda_context

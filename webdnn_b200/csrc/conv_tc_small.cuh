@@ -22,7 +22,8 @@
 // result does not depend on which of the two kernels a launch takes.  That matters where a network carries the last bits
 // on: a softmax over large scores is an argmax, and close rivals exchange places.  The parts are therefore the terms that
 // kernel adds up in fp32: where it takes a tile whole, its segments of SEG_KBLOCKS K blocks, walked from the same rotated
-// start and added behind the addend; where it cuts a tile, its ranges.
+// start and added behind the addend (rows of any length, which leave through that kernel's plain epilogue: in front of
+// it); where it cuts a tile, its ranges.
 
 constexpr int SM_SPLIT_WARPS = 8;
 constexpr int SM_A_WARP = 8, SM_W_WARP = 9, SM_MMA_WARP = 10;
@@ -218,12 +219,12 @@ tc_small_kernel(const __grid_constant__ TcProblem p, const __grid_constant__ CUt
       drained++;
     };
     pdl_grid_wait();   // (before the addend, the residual and the output are touched; the tiles come after it anyway)
-    if (CS == 1 && p.shift) {
+    if (CS == 1 && p.shift && !ragged) {
 #pragma unroll
       for (int j = 0; j < COLS; j += 4) {
         const int n = n0 + half * COLS + j;
         if (n >= p.N) break;
-        const float4 b = small_cell(p.shift + n, n, p.N, ragged);
+        const float4 b = pdl_ld(reinterpret_cast<const float4*>(p.shift + n));
         acc[j] = p.shift_mul * b.x;
         acc[j + 1] = p.shift_mul * b.y;
         acc[j + 2] = p.shift_mul * b.z;
@@ -453,7 +454,7 @@ tc_small_kernel(const __grid_constant__ TcProblem p, const __grid_constant__ CUt
       }
     }
     // residual and addend are on their way while the sums are
-    float4 out[ITEMS], res[ITEMS];
+    float4 out[ITEMS], res[ITEMS];   // out: the addend, in front of the sums or (rows of any length) behind them
     bool live[ITEMS];
 #pragma unroll
     for (int i = 0; i < ITEMS; i++) {
@@ -462,9 +463,9 @@ tc_small_kernel(const __grid_constant__ TcProblem p, const __grid_constant__ CUt
       live[i] = r < mine && n < p.N;
       out[i] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (live[i]) {
-        if (CS > 1 && p.shift) {
+        if ((CS > 1 || ragged) && p.shift) {
           const float4 b = small_cell(p.shift + n, n, p.N, ragged);
-          out[i] = make_float4(p.shift_mul * b.x, p.shift_mul * b.y, p.shift_mul * b.z, p.shift_mul * b.w);
+          out[i] = make_float4(__fmul_rn(p.shift_mul, b.x), __fmul_rn(p.shift_mul, b.y), __fmul_rn(p.shift_mul, b.z), __fmul_rn(p.shift_mul, b.w));
         }
         if (p.residual) res[i] = small_cell(p.residual + m * p.res_stride + n, n, p.N, ragged);
       }
@@ -480,11 +481,14 @@ tc_small_kernel(const __grid_constant__ TcProblem p, const __grid_constant__ CUt
         if (!live[i]) continue;
         const int item = threadIdx.x + i * SM_EPI_THREADS, r = item / CELLS, cell = item % CELLS;
         const unsigned char* src = smem + L::EXCHANGE_OFF + exchange_slot<ROWS>((uint32_t)r, (uint32_t)cell) * 16u;
-        float4 s = CS > 1 ? out[i] : *reinterpret_cast<const float4*>(src);
+        float4 s = CS == 1 ? *reinterpret_cast<const float4*>(src) : ragged ? make_float4(0.f, 0.f, 0.f, 0.f) : out[i];
 #pragma unroll
         for (int q = 0; CS > 1 && q < CS; q++) {
           const float4 v = *reinterpret_cast<const float4*>(src + q * (CELLS * ROWS * 16));
           s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+        }
+        if (ragged) {
+          s.x += out[i].x; s.y += out[i].y; s.z += out[i].z; s.w += out[i].w;
         }
         if (p.residual) {
           s.x = fmaf(p.res_mul, res[i].x, s.x);
