@@ -1739,21 +1739,22 @@ struct SmallVariant {
   SmallKernel kernel;
   int smem;
 };
-template <int TN, int CS>
-SmallVariant small_variant() { return {tc_small_kernel<TN, CS>, SmallLayout<TN, CS>::SMEM}; }
-const SmallVariant small_variants[2][8] = {
-    {small_variant<32, 1>(), small_variant<32, 2>(), small_variant<32, 3>(), small_variant<32, 4>(),
-     small_variant<32, 5>(), small_variant<32, 6>(), small_variant<32, 7>(), small_variant<32, 8>()},
-    {small_variant<64, 1>(), small_variant<64, 2>(), small_variant<64, 3>(), small_variant<64, 4>(),
-     small_variant<64, 5>(), small_variant<64, 6>(), small_variant<64, 7>(), small_variant<64, 8>()}};
+template <int TN, int CS, bool RAGGED>
+SmallVariant small_variant() { return {tc_small_kernel<TN, CS, RAGGED>, SmallLayout<TN, CS>::SMEM}; }
+#define SMALL_VARIANTS(TN, RAGGED)                                                                                               \
+  {small_variant<TN, 1, RAGGED>(), small_variant<TN, 2, RAGGED>(), small_variant<TN, 3, RAGGED>(), small_variant<TN, 4, RAGGED>(), \
+   small_variant<TN, 5, RAGGED>(), small_variant<TN, 6, RAGGED>(), small_variant<TN, 7, RAGGED>(), small_variant<TN, 8, RAGGED>()}
+const SmallVariant small_variants[2][2][8] = {   // [rows of any length][wide tile][CTAs of a cluster - 1]
+    {SMALL_VARIANTS(32, false), SMALL_VARIANTS(64, false)}, {SMALL_VARIANTS(32, true), SMALL_VARIANTS(64, true)}};
+#undef SMALL_VARIANTS
 constexpr int MAX_DEVICES = 64;
 
 // The variant's shared memory is allowed for on the context's device.
-bool small_ready(wdc_context* ctx, int wide, int cs) {
-  static bool ready[MAX_DEVICES][2][8] = {};
+bool small_ready(wdc_context* ctx, int ragged, int wide, int cs) {
+  static bool ready[MAX_DEVICES][2][2][8] = {};
   if (ctx->device < 0 || ctx->device >= MAX_DEVICES) return false;
-  bool& r = ready[ctx->device][wide][cs - 1];
-  const SmallVariant& v = small_variants[wide][cs - 1];
+  bool& r = ready[ctx->device][ragged][wide][cs - 1];
+  const SmallVariant& v = small_variants[ragged][wide][cs - 1];
   if (!r && cudaFuncSetAttribute(v.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem) != cudaSuccess) {
     cudaGetLastError();
     return false;
@@ -1820,10 +1821,10 @@ bool choose_small(const wdc_context* ctx, const TcProblem& p, int n_one, int til
 
 // A launch of tc_small_kernel: p.kblocks, p.part and geometry are set; `tn` and `cs` chosen by choose_small.
 int launch_small(wdc_context* ctx, TcProblem& p, WeightEntry* we, const CUtensorMap& map_a, float* y, int tn, int cs) {
-  const int wide = tn == 64;
-  if (!small_ready(ctx, wide, cs)) return WDC_ERR_UNSUPPORTED;
-  const SmallKernel kernel = small_variants[wide][cs - 1].kernel;
-  const int smem = small_variants[wide][cs - 1].smem;
+  const int wide = tn == 64, ragged = p.N % 4 != 0;
+  if (!small_ready(ctx, ragged, wide, cs)) return WDC_ERR_UNSUPPORTED;
+  const SmallKernel kernel = small_variants[ragged][wide][cs - 1].kernel;
+  const int smem = small_variants[ragged][wide][cs - 1].smem;
   p.tile_n = tn;
   p.tiles_m = (int)ceil_div64(p.M, TILE_M);
   p.tiles_n = (int)ceil_div64(p.N, tn);

@@ -111,9 +111,10 @@ __device__ __forceinline__ uint32_t exchange_slot(uint32_t row, uint32_t cell) {
   return cell * ROWS + (ROWS % 8 == 0 ? row ^ (cell & 7u) : row);
 }
 
-// Four columns from `n` on of a row of N that is `ragged` (N no multiple of 4: rows start anywhere, the last cell is short).
-__device__ __forceinline__ float4 small_cell(const float* p, int n, int N, bool ragged) {
-  if (!ragged) return pdl_ld(reinterpret_cast<const float4*>(p));
+// Four columns from `n` on of a row of N; RAGGED: N is no multiple of 4, rows start anywhere, the last cell is short.
+template <bool RAGGED>
+__device__ __forceinline__ float4 small_cell(const float* p, int n, int N) {
+  if (!RAGGED) return pdl_ld(reinterpret_cast<const float4*>(p));
   float4 v = make_float4(pdl_ld(p), 0.f, 0.f, 0.f);
   if (n + 1 < N) v.y = pdl_ld(p + 1);
   if (n + 2 < N) v.z = pdl_ld(p + 2);
@@ -122,7 +123,9 @@ __device__ __forceinline__ float4 small_cell(const float* p, int n, int N, bool 
 }
 
 // CS: CTAs of a cluster = parts of K (1: the tile as a whole).  grid: tiles_m * tiles_n * CS.
-template <int TN, int CS>
+// RAGGED: N is no multiple of 4.  Variants of their own: asked at run time, every launch of a network paid for the question
+// (ResNet-50, one image: 428 us a run as here, 434 with it).
+template <int TN, int CS, bool RAGGED>
 __global__ void __launch_bounds__(SM_THREADS, 2)
 tc_small_kernel(const __grid_constant__ TcProblem p, const __grid_constant__ CUtensorMap map_w_hi,
                 const __grid_constant__ CUtensorMap map_w_lo, const __grid_constant__ CUtensorMap map_a,
@@ -188,7 +191,6 @@ tc_small_kernel(const __grid_constant__ TcProblem p, const __grid_constant__ CUt
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   const uint32_t tmem_base = ss->tmem_base;
   const int q4 = warp & 3, half = warp >> 2;
-  const bool ragged = (p.N & 3) != 0;
   float acc[COLS];
   bool ok = true;
 
@@ -219,7 +221,7 @@ tc_small_kernel(const __grid_constant__ TcProblem p, const __grid_constant__ CUt
       drained++;
     };
     pdl_grid_wait();   // (before the addend, the residual and the output are touched; the tiles come after it anyway)
-    if (CS == 1 && p.shift && !ragged) {
+    if (CS == 1 && p.shift && !RAGGED) {
 #pragma unroll
       for (int j = 0; j < COLS; j += 4) {
         const int n = n0 + half * COLS + j;
@@ -463,11 +465,12 @@ tc_small_kernel(const __grid_constant__ TcProblem p, const __grid_constant__ CUt
       live[i] = r < mine && n < p.N;
       out[i] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (live[i]) {
-        if ((CS > 1 || ragged) && p.shift) {
-          const float4 b = small_cell(p.shift + n, n, p.N, ragged);
-          out[i] = make_float4(__fmul_rn(p.shift_mul, b.x), __fmul_rn(p.shift_mul, b.y), __fmul_rn(p.shift_mul, b.z), __fmul_rn(p.shift_mul, b.w));
+        if ((CS > 1 || RAGGED) && p.shift) {
+          const float4 b = small_cell<RAGGED>(p.shift + n, n, p.N);
+          out[i] = RAGGED ? make_float4(__fmul_rn(p.shift_mul, b.x), __fmul_rn(p.shift_mul, b.y), __fmul_rn(p.shift_mul, b.z), __fmul_rn(p.shift_mul, b.w))
+                          : make_float4(p.shift_mul * b.x, p.shift_mul * b.y, p.shift_mul * b.z, p.shift_mul * b.w);
         }
-        if (p.residual) res[i] = small_cell(p.residual + m * p.res_stride + n, n, p.N, ragged);
+        if (p.residual) res[i] = small_cell<RAGGED>(p.residual + m * p.res_stride + n, n, p.N);
       }
     }
     if (CS > 1) ok = sums_ok && small_wait(smem_u32(&ss->recv), 0, ss, p.status, 59);
@@ -481,13 +484,13 @@ tc_small_kernel(const __grid_constant__ TcProblem p, const __grid_constant__ CUt
         if (!live[i]) continue;
         const int item = threadIdx.x + i * SM_EPI_THREADS, r = item / CELLS, cell = item % CELLS;
         const unsigned char* src = smem + L::EXCHANGE_OFF + exchange_slot<ROWS>((uint32_t)r, (uint32_t)cell) * 16u;
-        float4 s = CS == 1 ? *reinterpret_cast<const float4*>(src) : ragged ? make_float4(0.f, 0.f, 0.f, 0.f) : out[i];
+        float4 s = CS == 1 ? *reinterpret_cast<const float4*>(src) : RAGGED ? make_float4(0.f, 0.f, 0.f, 0.f) : out[i];
 #pragma unroll
         for (int q = 0; CS > 1 && q < CS; q++) {
           const float4 v = *reinterpret_cast<const float4*>(src + q * (CELLS * ROWS * 16));
           s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
         }
-        if (ragged) {
+        if (RAGGED) {
           s.x += out[i].x; s.y += out[i].y; s.z += out[i].z; s.w += out[i].w;
         }
         if (p.residual) {
@@ -500,7 +503,7 @@ tc_small_kernel(const __grid_constant__ TcProblem p, const __grid_constant__ CUt
           s.x = relu_nan(s.x); s.y = relu_nan(s.y); s.z = relu_nan(s.z); s.w = relu_nan(s.w);
         }
         float* dst = y + (m0 + rank * share + r) * p.y_stride + n0 + cell * 4;
-        if (!ragged) {
+        if (!RAGGED) {
           *reinterpret_cast<float4*>(dst) = s;
         } else {
           const int left = p.N - n0 - cell * 4;
