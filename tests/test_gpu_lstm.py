@@ -62,3 +62,65 @@ def test_recurrence(cuda_context, seq, batch, hidden, state):
         assert np.array_equal(one.view(np.uint32), two.view(np.uint32))
     for t in dev + outs:
         t.dispose()
+
+
+def test_gates_are_no_further_off_than_by_tanhf(cuda_context):
+    """Sigmoid and tanh of the one-cluster kernel (sequences of 4 steps and more) and of the path for shorter ones, which calls
+    tanhf, against float64 on the same pre-activations: over magnitudes from 1e-5 to 40, by ranges.  Until the last step
+    the forget gate is open and the candidate 0, so that the cell is 1 or 0; then units 0 .. 15 give c = sigmoid(x) and the
+    others c = tanh(x), and h = tanh(c) with the output gate open."""
+    from ctypes import byref
+
+    from webdnn_b200.lib import GemmDesc
+    ctx = cuda_context
+    rng = np.random.default_rng(7)
+    batch, inp, hidden = 40000, 4, 32
+    x = np.exp(rng.uniform(np.log(1e-2), np.log(40), batch)).astype(np.float32)
+    x[:200] = np.nextafter(np.float32(1), np.float32(rng.choice([0, 2], 200))) * np.float32(1 + 1e-6) ** rng.integers(-9, 9, 200)
+    x[200:400] = np.float32(0.7) * np.float32(1 + 1e-6) ** rng.integers(-9, 9, 200)   # either side of where the forms change
+    x[400], x[401] = 3e38, np.nan
+    w = np.zeros((4, hidden, inp), np.float32)
+    sign = np.where(np.arange(16) % 2 == 0, 1, -1) * 2.0 ** -(np.arange(16) % 8 // 2 * 3)
+    sign[15] *= 16 * 512                                           # (3e38 times this is infinite)
+    w[2, :16, 0], w[3, 16:, 0] = sign, sign
+    w[2, :16, 1] = w[0, 16:, 2] = w[1, :, 2] = 1                   # gates held open by 100
+    c0 = np.zeros((batch, hidden), np.float32)
+    c0[:, :16] = 1
+    errors = {}
+    for seq in (4, 3):
+        xs = np.zeros((seq, batch, inp), np.float32)
+        xs[-1, :, 0], xs[:-1, :, 1], xs[:, :, 2] = x, 100, 100
+        dev = [ctx.move_tensor(CPUTensor.from_array(a)) for a in (xs, w.reshape(4 * hidden, inp), np.zeros((4 * hidden, hidden), np.float32), c0)]
+        outs = [ctx.empty_tensor(s) for s in ((seq, batch, hidden), (batch, hidden), (batch, hidden))]
+        ctx._call("wdc_lstm", dev[0].ptr, dev[1].ptr, dev[2].ptr, None, None, dev[3].ptr, *(o.ptr for o in outs), seq, batch, inp, hidden)
+        h, c = (o.get_data().reshape(o.dims).copy() for o in outs[1:])
+        p = ctx.empty_tensor([seq * batch, 4 * hidden])            # the projection, as wdc_lstm computes it
+        d = GemmDesc(batch=1, m=seq * batch, n=4 * hidden, k=inp, sab=0, sa0=inp, sa1=1, sbb=0, sb0=1, sb1=inp, sc0=0, sc1=0,
+                     alpha=1.0, beta=0.0, relu=0)
+        ctx._call("wdc_gemm", byref(d), dev[0].ptr, dev[1].ptr, None, p.ptr)
+        pre = p.get_data().reshape(seq, batch, 4, hidden)[-1].astype(np.float64)
+        for t in dev + outs + [p]:
+            t.dispose()
+        at = np.concatenate([pre[:, 2, :16], pre[:, 3, 16:]], axis=1)
+        nan = np.isnan(at)
+        assert nan[401].all() and np.isnan(c[401]).all() and np.isnan(h[401]).all() and not np.isnan(c[~nan]).any()
+        assert np.isinf(at[400]).any()
+        at, c, h = np.delete(at, 401, 0), np.delete(c, 401, 0).astype(np.float64), np.delete(h, 401, 0)
+        with np.errstate(over="ignore"):
+            want_s, want_t = 1 / (1 + np.exp(-at[:, :16])), np.tanh(at[:, 16:])
+        parts = [("sigmoid", np.abs(at[:, :16]), np.abs(c[:, :16] - want_s)),
+                 ("tanh", np.abs(at[:, 16:]), np.abs(c[:, 16:] - want_t) / np.abs(want_t)),
+                 ("tanh", np.abs(c), np.abs(h - np.tanh(c)) / np.maximum(np.abs(np.tanh(c)), 1e-30))]
+        for n, (name, mag, err) in enumerate(parts):
+            for lo, hi in ((1e-5, .25), (.25, .65), (.65, 1), (1, 2), (2, 4), (4, np.inf)):
+                e = err[(mag >= lo) & (mag <= hi)] * 2.0 ** 24
+                if e.size > 2000:
+                    errors.setdefault((n, name, lo), []).append((e.max(), np.sqrt(np.mean(e ** 2))))
+    assert len(errors) >= 14
+    # the largest errors over all floats in units of 2^-24, by tanhf 0.6, 0.9, 0.95, 1.4, 1.1, 0.8 and 1.9, 3.4, 2.95, 1.8, 1.1, 0.55
+    bounds = {"sigmoid": dict(zip((1e-5, .25, .65, 1, 2, 4), (.55, .61, .69, 1.3, .91, .6))),
+              "tanh": dict(zip((1e-5, .25, .65, 1, 2, 4), (1.04, 1.24, 2.9, 1.7, .87, .53)))}
+    for (n, name, lo), ((top, rms), (top_tanhf, rms_tanhf)) in errors.items():
+        assert top <= bounds[name][lo] and top_tanhf <= 3.4, (n, name, lo, top, top_tanhf)
+        # (two samples of a range differ by a share of a percent)
+        assert rms <= 1.01 * rms_tanhf, (n, name, lo, rms, rms_tanhf)

@@ -172,12 +172,18 @@ __device__ __forceinline__ void tmem_ld4(uint32_t taddr, float* v) {
                : "r"(taddr)
                : "memory");
 }
-// The gates without branches, so that a thread's calls overlap (five tanhf in a row took 700 cycles of a step of 2400).
-// e^x as 2^(x log2 e): its relative error, (|x| + 3) 2^-24, meets a factor below 0.25 in a sigmoid.
-// tanh: below 0.6 x + x^3 q(x^2), q fitted to equal ripple of the relative error (0.05 * 2^-24), above 1 - 2 / (e^2x + 1).
-__device__ __forceinline__ float exp_of(float x) {
+// The gates without branches, so that a thread's calls overlap (five tanhf in a row took 700 cycles of a step of 2400), and
+// no further from float64 than the forms by tanhf, 0.5 tanhf(0.5 x) + 0.5 and tanhf(x), at any magnitude.  Largest errors over
+// all floats in units of 2^-24, those forms' in brackets: the sigmoid's absolute one 0.54 [0.58] below 0.25, 0.68 [0.95] below 1,
+// 1.29 [1.38] to 1.25, 1.05 [1.16] to 2, 0.9 [1.03] past it; tanh's relative one 1.23 [3.33] below 0.65, 2.9 [2.9] to 1, 1.7 [1.8] to 1.25,
+// 0.86 [1.0] past 1.5.
+// Around zero both are odd polynomials, fitted to equal ripple by Lawson's reweighted least squares (C. L. Lawson, 1961): the
+// sigmoid's below 1 for its absolute error (0.03 * 2^-24 before rounding), tanh's below 0.7 for its relative one (0.02).  Past
+// that 1 / (1 + e^x) is small and so is what it is wrong by: the sigmoid is that or 1 minus it, and tanh(x) = 1 - 2 / (1 + e^2x).
+// e^x = 2^(x log2 e): the exponent's rounding costs (|x| log2 e) 2^-25, which tanh wins back as a factor 1 + l ln 2.
+__device__ __forceinline__ float exp2_of(float x) {
   float r;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x * 1.44269504f));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
 __device__ __forceinline__ float inverse(float x) {                // of 1 .. infinity
@@ -185,16 +191,29 @@ __device__ __forceinline__ float inverse(float x) {                // of 1 .. in
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
-__device__ __forceinline__ float sigmoid_fast(float x) { return inverse(1.f + exp_of(-x)); }
-__device__ __forceinline__ float tanh_fast(float x) {
+__device__ __forceinline__ float sigmoid_of(float x) {
   const float m = fabsf(x), u = x * x;
-  float q = -0.00589514f;
-  q = fmaf(q, u, 0.02079596f);
-  q = fmaf(q, u, -0.05378383f);
-  q = fmaf(q, u, 0.13331924f);
-  q = fmaf(q, u, -0.33333298f);
-  const float small = fmaf(x * u, q, x), large = copysignf(fmaf(-2.f, inverse(exp_of(2.f * m) + 1.f), 1.f), x);
-  return m < 0.6f ? small : large;
+  float q = 1.63452805e-05f;
+  q = fmaf(q, u, -0.000206102079f);
+  q = fmaf(q, u, 0.00208133925f);
+  q = fmaf(q, u, -0.0208329856f);
+  q = fmaf(q, u, 0.249999985f);
+  const float tail = inverse(1.f + exp2_of(m * 1.44269504f));
+  return m < 1.f ? fmaf(x, q, 0.5f) : x < 0.f ? tail : 1.f - tail;
+}
+__device__ __forceinline__ float tanh_of(float x) {
+  const float m = fabsf(x), u = x * x;
+  float q = 0.00189566764f;
+  q = fmaf(q, u, -0.00788331125f);
+  q = fmaf(q, u, 0.0215710606f);
+  q = fmaf(q, u, -0.0539209545f);
+  q = fmaf(q, u, 0.133329839f);
+  q = fmaf(q, u, -0.333333254f);
+  float y;
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(y) : "f"(2.f * m), "f"(80.f));
+  const float h = y * 1.44269504f, l = fmaf(y, 1.92596299e-8f, fmaf(y, 1.44269504f, -h));
+  const float e = exp2_of(h), tail = inverse(1.f + fmaf(e, l * 0.693147181f, e));
+  return copysignf(m < 0.7f ? fmaf(m * u, q, m) : fmaf(-2.f, tail, 1.f), x);
 }
 // x = hi + lo in fp16 parts; the low part of a scaled element is at worst 2^-25, 2^-39 of the largest
 __device__ __forceinline__ void split_half(float x, __half* hi, __half* lo) {
@@ -300,10 +319,10 @@ __device__ __forceinline__ void step_end(const float (&s)[NG][4], bool product, 
   }
 #pragma unroll
   for (int g = 0; g < GROUPS; g++) {
-    const float it = sigmoid_fast(w[g][0] + (pin[g][0] + bsum[0])), ot = sigmoid_fast(w[g][1] + (pin[g][1] + bsum[1]));
-    const float ft = sigmoid_fast(w[g][2] + (pin[g][2] + bsum[2])), ct = tanh_fast(w[g][3] + (pin[g][3] + bsum[3]));
+    const float it = sigmoid_of(w[g][0] + (pin[g][0] + bsum[0])), ot = sigmoid_of(w[g][1] + (pin[g][1] + bsum[1]));
+    const float ft = sigmoid_of(w[g][2] + (pin[g][2] + bsum[2])), ct = tanh_of(w[g][3] + (pin[g][3] + bsum[3]));
     c[g] = ft * c[g] + it * ct;
-    h[g] = live[g] ? ot * tanh_fast(c[g]) : 0.f;
+    h[g] = live[g] ? ot * tanh_of(c[g]) : 0.f;
   }
 #pragma unroll
   for (int g = 0; g < GROUPS; g++) {
