@@ -124,3 +124,33 @@ def test_gates_are_no_further_off_than_by_tanhf(cuda_context):
         assert top <= bounds[name][lo] and top_tanhf <= 3.4, (n, name, lo, top, top_tanhf)
         # (two samples of a range differ by a share of a percent)
         assert rms <= 1.01 * rms_tanhf, (n, name, lo, rms, rms_tanhf)
+
+
+# Rms errors that the TF32 parts and K slices of csrc/lstm_cluster.cu have at these sizes (random signs, one sign): the
+# one-cluster kernel is no further off.
+@pytest.mark.parametrize("hidden,mixed,one_sign", [(32, 1.09e-7, 0.91e-7), (64, 1.18e-7, 0.96e-7), (128, 1.60e-7, 1.31e-7), (256, 2.59e-7, 2.42e-7),
+                                                   (384, 3.65e-7, 3.66e-7), (480, 4.62e-7, 5.11e-7), (512, 9.14e-7, 1.19e-6)])
+@pytest.mark.parametrize("batch", [8, 200])
+def test_sums_are_no_further_off_than_tf32_parts(cuda_context, batch, hidden, mixed, one_sign):
+    """The first step's y = o tanh(i tanh(s)) with pre-activations so small that its relative error is that of the sum s (and of
+    the gates, 2^-24 each)."""
+    ctx = cuda_context
+    for positive, bound in ((False, mixed), (True, one_sign)):
+        off = size = 0.0
+        for seed in range(6 if batch < 100 else 2):
+            rng = np.random.default_rng(seed + hidden)
+            r = (rng.standard_normal((4 * hidden, hidden)) * 1e-4).astype(np.float32)
+            h0 = rng.uniform(-1, 1, (batch, hidden)).astype(np.float32)
+            if positive:
+                r, h0 = np.abs(r), np.abs(h0)
+            dev = [ctx.move_tensor(CPUTensor.from_array(a)) for a in (np.zeros((4, batch, 4), np.float32), np.zeros((4 * hidden, 4), np.float32), r, h0)]
+            outs = [ctx.empty_tensor(s) for s in ((4, batch, hidden), (batch, hidden), (batch, hidden))]
+            ctx._call("wdc_lstm", dev[0].ptr, dev[1].ptr, dev[2].ptr, None, dev[3].ptr, None, *(o.ptr for o in outs), 4, batch, 4, hidden)
+            got = outs[0].get_data().reshape(4, batch, hidden)[0].astype(np.float64)
+            i, o, f, g = np.split(h0.astype(np.float64) @ r.T.astype(np.float64), 4, axis=1)
+            want = np.tanh(np.tanh(g) / (1 + np.exp(-i))) / (1 + np.exp(-o))
+            off, size = off + np.sum((got - want) ** 2), size + np.sum(want ** 2)
+            for t in dev + outs:
+                t.dispose()
+        # (5 %: samples of a few thousand values in the smallest case)
+        assert np.sqrt(off / size) <= 1.05 * bound, (positive, np.sqrt(off / size), bound)

@@ -18,7 +18,12 @@
 // Measured, start of a step to the next with lstm_cluster.cu and here: 256 units, batch 1, 1.63 -> 0.77 us; [64, 512] 3.0 ->
 // 1.95 us (of 3680 cycles the MMAs are 1330, the gates 850, the words on their way 1500: 20 KB into every CTA); 50 steps of
 // [1, 256] with the projection 98 -> 55 us, 128 of [64, 512] 434 -> 320 us.
-// Sums: hi*hi in one range of columns of the accumulator, hi*lo + lo*hi in another, added in fp32 after the last MMA.
+// Sums: hi*hi in one range of columns of an accumulator, hi*lo + lo*hi in another, added in fp32 after the last MMA.  The tensor
+// core cuts every product off at the running sum's last bits, so a sum over K loses in proportion to K: the k steps go to four
+// accumulators in turn.  Rms error of a sum of 480 (512) products against 64 bits: mixed signs 6.2e-7 (6.6e-7) in one accumulator,
+// 2.1e-7 (2.1e-7) in four, 4.6e-7 (9.2e-7) by lstm_cluster.cu, whose CTAs sum slices of 60 (128); all of one sign 2.7e-6 (2.9e-6),
+// 4.9e-7 (5.3e-7), 5.1e-7 (1.2e-6).  Their columns push low parts of R into shared memory, where an MMA takes 45 cycles more
+// to read them: a step of [64, 512] 2.21 us in one accumulator, 2.30 in two, 2.50 in four; of [1, 256] 0.81, 0.80, 0.82.
 // h0 may be anything: its rows have a scale each.  A row of R, or an h0, with an infinite element or NaN has none: those
 // sums are plain fp32 FMAs.  Waits are bounded as in lstm_cluster.cu: on expiry a status word is set, the peers' waits expire in turn, and
 // all CTAs of the cluster meet at the last barrier.
@@ -231,30 +236,33 @@ __device__ __forceinline__ float pow2(int e) { return __uint_as_float((uint32_t)
 // h of one buffer: [source CTA][zeros? hi groups, lo groups][4 blocks of 8 units][8 batch rows][8 units], fp16.
 // An odd number of groups has a group of zeros in front: the MMA of the low parts of R has at least 16 columns and
 // adds to the range of columns that hi*lo is summed in; the zeros stand for the 8 columns in front of that range.
-template <int NG>
+// ACCS: accumulators that the k steps go to in turn.
+template <int NG, int ACCS>
 struct LocalLayout {
   static constexpr int ZERO = NG & 1;
   static constexpr int GROUP = 512;                               // bytes of a group: 8 rows x 32 units
   static constexpr int SRC = (ZERO + 2 * NG) * GROUP;
   static constexpr int BUF = MAX_CS * SRC;                        // (fixed, so that operand addresses are constants)
-  static constexpr int D_COLS = 16 * NG;                          // hi*hi, then the cross products
-  static constexpr int STEPS_LO = (512 - D_COLS) / 8 - 2 * MAX_CS;   // k steps whose low parts of R are in tensor memory
+  static constexpr int ACC = 16 * NG;                             // columns: hi*hi, then the cross products
+  static constexpr int D_COLS = ACC * ACCS;
   static constexpr int LO_ROWS = 8 * (NG + ZERO);                 // columns of the MMA of the low parts
   static constexpr int LO_COL0 = 8 * (NG - ZERO);
   static constexpr int STAGE = 8 * NG * 128;                      // the eight warps' words on their way out
+  // k steps whose low parts of R are in tensor memory
+  static __host__ __device__ constexpr int steps_lo(int cs) { return (512 - D_COLS) / 8 - 2 * cs < 2 * cs ? (512 - D_COLS) / 8 - 2 * cs : 2 * cs; }
 };
 
 // The MMAs of four sources (two k steps each).  One block of straight-line code whose addresses are constant offsets from
 // bases in registers: 13 cycles an MMA.  With addresses computed for each it takes 28 to 65, with a block of constants for
 // every quarter and buffer behind a switch 25: the operands then pass through vector registers one by one.
 struct Issue {
-  uint32_t t_d, t_hi, t_lo;    // tensor memory: accumulator, high and low parts of R from these sources' columns on
+  uint32_t t_d, t_hi, t_lo;    // tensor memory: accumulators, high and low parts of R from these sources' columns on
   uint32_t b, b_top;           // descriptor of their words
   uint32_t r, r_top;           // descriptor of the low parts of R in shared memory
 };
-template <int NG, bool ALL>    // ALL: four sources, low parts in tensor memory
-__device__ __forceinline__ void issue_sources(const Issue& o, int n, int lo_in_tmem, uint32_t accumulate) {
-  using L = LocalLayout<NG>;
+template <int NG, int ACCS, bool ALL>    // ALL: four sources, low parts in tensor memory
+__device__ __forceinline__ void issue_sources(const Issue& o, int q, int n, int lo_in_tmem) {
+  using L = LocalLayout<NG, ACCS>;
   constexpr uint32_t ID_HI = (1u << 4) | ((uint32_t)(2 * NG) << 17) | ((128u >> 4) << 24);
   constexpr uint32_t ID_LO = (1u << 4) | ((uint32_t)(L::LO_ROWS >> 3) << 17) | ((128u >> 4) << 24);
 #pragma unroll
@@ -263,12 +271,13 @@ __device__ __forceinline__ void issue_sources(const Issue& o, int n, int lo_in_t
 #pragma unroll
       for (int j = 0; j < 2; j++) {
         const int step = 2 * d + j;
+        const uint32_t t_acc = o.t_d + (uint32_t)(step % ACCS * L::ACC);
         const uint32_t b = o.b + (uint32_t)((d * L::SRC + 256 * j) >> 4), b_hi = b + (uint32_t)(L::ZERO * L::GROUP >> 4);
-        if (step == 0) mma_ts(o.t_d, o.t_hi, b_hi, o.b_top, ID_HI, accumulate);
-        else mma_ts_more(o.t_d, o.t_hi + (uint32_t)(8 * step), b_hi, o.b_top, ID_HI);
+        if (step < ACCS) mma_ts(t_acc, o.t_hi + (uint32_t)(8 * step), b_hi, o.b_top, ID_HI, q > 0 ? 1u : 0u);
+        else mma_ts_more(t_acc, o.t_hi + (uint32_t)(8 * step), b_hi, o.b_top, ID_HI);
         // (with zeros in front: their 8 columns have just been written by the MMA above, like the others)
-        if (ALL || step < lo_in_tmem) mma_ts_more(o.t_d + (uint32_t)L::LO_COL0, o.t_lo + (uint32_t)(8 * step), b, o.b_top, ID_LO);
-        else mma_ss_more(o.t_d + (uint32_t)L::LO_COL0, o.r + (uint32_t)((step - lo_in_tmem) * 256), o.r_top, b, o.b_top, ID_LO);
+        if (ALL || step < lo_in_tmem) mma_ts_more(t_acc + (uint32_t)L::LO_COL0, o.t_lo + (uint32_t)(8 * step), b, o.b_top, ID_LO);
+        else mma_ss_more(t_acc + (uint32_t)L::LO_COL0, o.r + (uint32_t)((step - lo_in_tmem) * 256), o.r_top, b, o.b_top, ID_LO);
       }
     }
   }
@@ -333,9 +342,9 @@ __device__ __forceinline__ void step_end(const float (&s)[NG][4], bool product, 
   }
 }
 
-template <int NG>
+template <int NG, int ACCS>
 __global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs a) {
-  using L = LocalLayout<NG>;
+  using L = LocalLayout<NG, ACCS>;
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ LocalShared sh;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -390,6 +399,7 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs 
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = sh.tmem_base;
   const uint32_t tmem_hi = tmem + (uint32_t)L::D_COLS, tmem_lo = tmem_hi + (uint32_t)(16 * cs);
+  const int steps_lo = L::steps_lo(cs);
   bool plain_row = false;
   float unscale = 0.f;
   if (warp < 8) {
@@ -435,10 +445,10 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs 
           }
         }
         tmem_st8(tmem_hi + t_row + (uint32_t)(8 * j), hi);
-        if (j < L::STEPS_LO) {
+        if (j < steps_lo) {
           tmem_st8(tmem_lo + t_row + (uint32_t)(8 * j), lo);
         } else {
-          unsigned char* dst = r_lo + (size_t)(j - L::STEPS_LO) * 4096 + row * 16;
+          unsigned char* dst = r_lo + (size_t)(j - steps_lo) * 4096 + row * 16;
           *reinterpret_cast<uint4*>(dst) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
           *reinterpret_cast<uint4*>(dst + 2048) = make_uint4(lo[4], lo[5], lo[6], lo[7]);
         }
@@ -518,12 +528,12 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs 
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         for (int q = 0; q < quarters; q++) {
-          const int n = cs - 4 * q, lo_in_tmem = L::STEPS_LO - 8 * q;
+          const int n = cs - 4 * q, lo_in_tmem = steps_lo - 8 * q;
           const Issue o = {tmem, tmem_hi + (uint32_t)(64 * q), tmem_lo + (uint32_t)(64 * q),
                            (uint32_t)b_desc + (uint32_t)(((t & 1) * L::BUF + 4 * q * L::SRC) >> 4), (uint32_t)(b_desc >> 32),
                            (uint32_t)r_desc, (uint32_t)(r_desc >> 32)};
-          if (n >= 4 && lo_in_tmem >= 8) issue_sources<NG, true>(o, n, lo_in_tmem, q > 0 ? 1u : 0u);
-          else issue_sources<NG, false>(o, n, lo_in_tmem, q > 0 ? 1u : 0u);
+          if (n >= 4 && lo_in_tmem >= 8) issue_sources<NG, ACCS, true>(o, q, n, lo_in_tmem);
+          else issue_sources<NG, ACCS, false>(o, q, n, lo_in_tmem);
         }
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mma_bar) : "memory");
         if (t > 0) expect_bytes(bar, step_bytes);                  // the words of step t + 2
@@ -559,12 +569,28 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs 
         phase ^= 1u;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         float x[NG][4];
+        constexpr int PART = NG == 1 ? ACCS : NG == 2 && ACCS % 2 == 0 ? 2 : 1;   // accumulators read at once
 #pragma unroll
-        for (int g = 0; g < NG; g++) {
-          tmem_ld4(t_row + (uint32_t)(8 * g), s[g]);
-          tmem_ld4(t_row + (uint32_t)(8 * NG + 8 * g), x[g]);
+        for (int i = 0; i < ACCS; i += PART) {
+          float hh[PART][NG][4], cross[PART][NG][4];
+#pragma unroll
+          for (int p = 0; p < PART; p++)
+#pragma unroll
+            for (int g = 0; g < NG; g++) {
+              tmem_ld4(t_row + (uint32_t)((i + p) * L::ACC + 8 * g), hh[p][g]);
+              tmem_ld4(t_row + (uint32_t)((i + p) * L::ACC + 8 * NG + 8 * g), cross[p][g]);
+            }
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int p = 0; p < PART; p++)
+#pragma unroll
+            for (int g = 0; g < NG; g++)
+#pragma unroll
+              for (int j = 0; j < 4; j++) {
+                s[g][j] = i + p ? s[g][j] + hh[p][g][j] : hh[p][g][j];
+                x[g][j] = i + p ? x[g][j] + cross[p][g][j] : cross[p][g][j];
+              }
         }
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
 #pragma unroll
         for (int g = 0; g < NG; g++)
@@ -639,25 +665,32 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs 
 
 typedef void (*Kernel)(const LocalArgs);
 
-Kernel kernel_of(int groups) {
-  switch (groups) {
-    case 1: return lstm_local_kernel<1>;
-    case 2: return lstm_local_kernel<2>;
-    case 3: return lstm_local_kernel<3>;
-    default: return lstm_local_kernel<4>;
-  }
+struct Variant {
+  Kernel kernel;
+  int zero, d_cols, buf, stage;
+};
+template <int NG, int ACCS>
+constexpr Variant variant() {
+  using L = LocalLayout<NG, ACCS>;
+  return {lstm_local_kernel<NG, ACCS>, L::ZERO, L::D_COLS, L::BUF, L::STAGE};
 }
+const Variant variants[MAX_GROUPS][2] = {   // [8-row groups - 1][more than one CTA a cluster]
+    {variant<1, 2>(), variant<1, 4>()}, {variant<2, 2>(), variant<2, 4>()}, {variant<3, 2>(), variant<3, 4>()}, {variant<4, 2>(), variant<4, 4>()}};
 
-template <int NG>
-size_t smem_of_groups(int cs) {
-  using L = LocalLayout<NG>;
-  const int in_smem = 2 * cs > L::STEPS_LO ? 2 * cs - L::STEPS_LO : 0;
-  return 2 * L::BUF + L::STAGE + (size_t)in_smem * 4096;
+// k steps whose low parts of R are in shared memory
+int steps_in_smem(const Variant& v, int cs) {
+  const int steps = 4 * cs - (512 - v.d_cols) / 8;
+  return steps < 0 ? 0 : steps;
 }
-size_t smem_of(int cs, int groups) {
-  const size_t bytes = groups == 1 ? smem_of_groups<1>(cs) : groups == 2 ? smem_of_groups<2>(cs) : groups == 3 ? smem_of_groups<3>(cs) : smem_of_groups<4>(cs);
+size_t smem_of(const Variant& v, int cs) {
+  const size_t bytes = 2 * (size_t)v.buf + v.stage + (size_t)steps_in_smem(v, cs) * 4096;
   return bytes < MIN_SMEM ? MIN_SMEM : bytes;
 }
+
+// Four accumulators, or one for each k step where there are two.
+const Variant& variant_of(int groups, int cs) { return variants[groups - 1][cs > 1]; }
+// 8-row groups of a cluster, at most: with four, 14 CTAs and more have no room for the low parts of R.
+int max_groups(int cs) { return cs <= 13 ? MAX_GROUPS : MAX_GROUPS - 1; }
 
 void fill_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, int grid, int cs, size_t smem, cudaStream_t stream) {
   *cfg = {};
@@ -675,21 +708,20 @@ void fill_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, int grid, i
 }
 
 // Clusters that can be resident at once (asked once per device and shape).
-int max_clusters(wdc_context* ctx, int cs, int groups) {
+int max_clusters(wdc_context* ctx, int cs, const Variant& v) {
   static std::mutex mu;
-  static std::map<std::pair<std::pair<int, int>, int>, int> known;
+  static std::map<std::pair<std::pair<int, int>, Kernel>, int> known;
   std::lock_guard<std::mutex> lk(mu);
-  const auto key = std::make_pair(std::make_pair(ctx->device, cs), groups);
+  const auto key = std::make_pair(std::make_pair(ctx->device, cs), v.kernel);
   auto it = known.find(key);
   if (it != known.end()) return it->second;
   int n = 0;
-  const Kernel kernel = kernel_of(groups);
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  cudaError_t e = cudaFuncSetAttribute(v.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(v.kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr[2];
-  fill_config(&cfg, attr, cs, cs, smem_of(cs, groups), nullptr);
-  if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg);
+  fill_config(&cfg, attr, cs, cs, smem_of(v, cs), nullptr);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, v.kernel, &cfg);
   if (e != cudaSuccess) {
     cudaGetLastError();
     n = 0;
@@ -709,18 +741,19 @@ int wdc_lstm_local(wdc_context* ctx, const float* P, const float* R, const float
   if (((uintptr_t)R & 15) != 0) return WDC_ERR_UNSUPPORTED;
   LocalArgs a = {P, R, bias, h0, c0, Y, Yh, Yc, ctx->status_word, (int)T, (int)Bt, (int)H};
   a.cs = (int)((H + UNITS - 1) / UNITS);
-  const int fit = max_clusters(ctx, a.cs, MAX_GROUPS);
+  const int fit = max_clusters(ctx, a.cs, variant_of(max_groups(a.cs), a.cs));
   if (!fit) return WDC_ERR_UNSUPPORTED;
-  const int64_t rounds = ceil_div64(Bt, (int64_t)fit * 8 * MAX_GROUPS);
+  const int64_t rounds = ceil_div64(Bt, (int64_t)fit * 8 * max_groups(a.cs));
   a.per = (int)ceil_div64(Bt, rounds * fit);
   const int groups = (a.per + 7) / 8, clusters = (int)ceil_div64(Bt, a.per);
-  if (!max_clusters(ctx, a.cs, groups)) return WDC_ERR_UNSUPPORTED;
+  const Variant& v = variant_of(groups, a.cs);
+  if (!max_clusters(ctx, a.cs, v)) return WDC_ERR_UNSUPPORTED;
   a.r_early = ctx->opt_pdl && wdc_is_constant(ctx, R) && (!bias || wdc_is_constant(ctx, bias));
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr[2];
-  fill_config(&cfg, attr, clusters * a.cs, a.cs, smem_of(a.cs, groups), ctx->stream);
+  fill_config(&cfg, attr, clusters * a.cs, a.cs, smem_of(v, a.cs), ctx->stream);
   cfg.numAttrs = ctx->opt_pdl ? 2 : 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, kernel_of(groups), (const LocalArgs)a);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, v.kernel, (const LocalArgs)a);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return WDC_ERR_UNSUPPORTED;
