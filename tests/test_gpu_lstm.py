@@ -1,6 +1,6 @@
 """The recurrence inside one cluster (csrc/lstm_local.cu): hidden sizes at the edges of its blocks of 32 units and of what
 tensor memory holds, batches at the edges of its groups of 8 rows and past what one round of clusters takes, initial states
-of any magnitude."""
+and weights of any magnitude, alone and side by side."""
 import numpy as np
 import pytest
 
@@ -27,7 +27,6 @@ def _reference(x, w, r, b, h, c):
     (20, 15, 256, None), (5, 121, 256, 1.0),                                 # one row a cluster; one past 8 rows
     (6, 1, 480, 1.0), (6, 90, 484, 1.0),                                     # the last sizes with 15 CTAs and the first with 16
     (6, 56, 512, None), (5, 57, 512, 1.0), (5, 113, 512, 1.0), (4, 169, 512, None), (4, 225, 512, 1.0), (4, 500, 512, None),
-    (6, 10, 512, 1e6), (6, 10, 64, 1e-6),                                    # rows of h0 have scales of their own
     (5, 4, 516, 1.0),                                                        # the first size that lstm_cluster.cu keeps
 ])
 def test_recurrence(cuda_context, seq, batch, hidden, state):
@@ -154,3 +153,63 @@ def test_sums_are_no_further_off_than_tf32_parts(cuda_context, batch, hidden, mi
                 t.dispose()
         # (5 %: samples of a few thousand values in the smallest case)
         assert np.sqrt(off / size) <= 1.05 * bound, (positive, np.sqrt(off / size), bound)
+
+
+@pytest.mark.parametrize("hidden,batch", [(36, 3), (64, 8), (256, 130), (416, 260), (480, 20), (512, 57), (512, 130)])
+@pytest.mark.parametrize("kind", ["weight 1e6", "weight 3e38", "wide weights", "few small", "h0 and weights", "tiny inputs"])
+def test_ranges_inside_rows(cuda_context, kind, batch, hidden):
+    """Elements of R and h0 that are far below the largest of their row count as much as where they are alone: a large weight
+    whose unit's output is 0 (its gate is shut), magnitudes spread over 12 decades in every row or in a few places, states
+    spread likewise, outputs of 1e-8."""
+    ctx = cuda_context
+    rng = np.random.default_rng(hidden + batch)
+    seq, inp, lim = 6, 12, 1 / np.sqrt(hidden)
+    u = lambda *s: rng.uniform(-lim, lim, s).astype(np.float32)  # noqa: E731
+    x, w, r, b = rng.standard_normal((seq, batch, inp)).astype(np.float32), u(4 * hidden, inp), u(4 * hidden, hidden), u(8 * hidden)
+    h0 = c0 = np.zeros((batch, hidden), np.float32)
+    if kind.startswith("weight"):
+        r[:, 3] = float(kind.split()[1])
+        r[hidden + 3], w[hidden + 3], b[hidden + 3], b[5 * hidden + 3] = 0, 0, -200, 0
+    if kind in ("wide weights", "h0 and weights"):
+        r *= (10.0 ** rng.uniform(-12, 0, r.shape)).astype(np.float32)
+    if kind == "few small":
+        at = rng.random(r.shape) < 0.002
+        r[at] *= np.float32(1e-11)
+        r[:, -1] *= np.float32(1e-11)
+    if kind == "h0 and weights":
+        h0 = (rng.standard_normal((batch, hidden)) * 10.0 ** rng.uniform(-12, 2, (batch, hidden))).astype(np.float32)
+        r[1::3, 0], h0[:, 0] = 1e8, 0                                # the small ones of both decide
+        c0 = rng.standard_normal((batch, hidden)).astype(np.float32)
+    if kind == "tiny inputs":
+        x *= np.float32(1e-7)
+        b[:] = 0
+    dev = [ctx.move_tensor(CPUTensor.from_array(a)) for a in (x, w, r, b, h0, c0)]
+    outs = [ctx.empty_tensor(s) for s in ((seq, batch, hidden), (batch, hidden), (batch, hidden))]
+    ctx._call("wdc_lstm", *(t.ptr for t in dev), *(o.ptr for o in outs), seq, batch, inp, hidden)
+    steps = 1 if kind == "h0 and weights" else seq                   # (a weight of 1e8 on h of 1 saturates the others)
+    got = outs[0].get_data().reshape(seq, batch, hidden)[:steps]
+    want = _reference(x, w, r, b, h0, c0)[0][:steps]
+    # 22 bits of every product and the gates' 2^-23: 2e-7 to 5e-7 over the steps
+    assert np.linalg.norm(got - want) <= 1e-6 * np.linalg.norm(want)
+    for t in dev + outs:
+        t.dispose()
+
+
+@pytest.mark.parametrize("hidden,batch", [(64, 10), (512, 10), (320, 130)])
+@pytest.mark.parametrize("state", [1e-30, 1e-6, 1.0, 1e6, 1e30])
+def test_initial_states_of_any_magnitude(cuda_context, state, batch, hidden):
+    """Rows of h0 have scales of their own: with R as much smaller as h0 is larger, a wrong one shows in the first step."""
+    ctx = cuda_context
+    rng = np.random.default_rng(hidden)
+    r = (rng.standard_normal((4 * hidden, hidden)) / np.sqrt(hidden) / state).astype(np.float32)
+    h0 = (rng.standard_normal((batch, hidden)) * state * 2.0 ** rng.uniform(-3, 1, (batch, 1))).astype(np.float32)
+    x, w, b, c0 = np.zeros((4, batch, 4), np.float32), np.zeros((4 * hidden, 4), np.float32), np.zeros(8 * hidden, np.float32), np.zeros((batch, hidden), np.float32)
+    dev = [ctx.move_tensor(CPUTensor.from_array(a)) for a in (x, w, r, h0)]
+    outs = [ctx.empty_tensor(s) for s in ((4, batch, hidden), (batch, hidden), (batch, hidden))]
+    ctx._call("wdc_lstm", dev[0].ptr, dev[1].ptr, dev[2].ptr, None, dev[3].ptr, None, *(o.ptr for o in outs), 4, batch, 4, hidden)
+    got = outs[0].get_data().reshape(4, batch, hidden)[0]
+    with np.errstate(over="ignore"):
+        want = _reference(x[:1], w, r, b, h0, c0)[0][0]
+    assert (np.abs(got - want).max(axis=1) <= 1e-6).all() and np.abs(want).max(axis=1).min() > 1e-2   # (zeros would not pass)
+    for t in dev + outs:
+        t.dispose()

@@ -7,8 +7,11 @@
 //     (up to 16 CTAs, 512 units); the batch is dealt to the clusters that fit on the chip, which run independently;
 //   * R fits because it is kept as two fp16 parts with a power of two per row (4 bytes an element, in tensor memory, the
 //     last low parts in shared memory), where TF32 parts take 8.  h is in (-1, 1) and has a constant scale.  Two parts of
-//     11 rounded bits carry 23 to 24 bits of the row's largest element (TF32 parts, cut by the tensor core: 22), and an
-//     fp16 MMA covers twice the K of a TF32 one in the same time: M 128 x N 16 x K 16 takes 9 cycles, N 32 takes 16;
+//     11 rounded bits carry 23 bits (TF32 parts, cut by the tensor core: 22), the low one with a scale of 2^13 of its own, so
+//     that elements down to 2^-28 of a row's largest have 22 bits.  What is smaller is left out of the parts, and the CTA that
+//     has such elements of R, or of h0, adds their products with fp32 FMAs (blocks of 8 units that hold one: some 500 cycles
+//     each).  h below 2^-29 is good to 2^-51 absolutely.  An fp16 MMA covers twice the K of a TF32 one in the same time: M 128
+//     x N 16 x K 16 takes 9 cycles, N 32 takes 16;
 //   * h goes to every CTA of the cluster as 16-byte words in the layout of the MMA's B operand (no swizzle: 8 batch rows x
 //     8 units are 128 consecutive bytes), by st.async, whose mbarrier counts the bytes (a CTA takes in about 20 a clock:
 //     16 KB of 8 rows x 512 units 800 cycles).  Barriers for each four sources, so that the first MMAs overlap the last
@@ -24,8 +27,8 @@
 // 2.1e-7 (2.1e-7) in four, 4.6e-7 (9.2e-7) by lstm_cluster.cu, whose CTAs sum slices of 60 (128); all of one sign 2.7e-6 (2.9e-6),
 // 4.9e-7 (5.3e-7), 5.1e-7 (1.2e-6).  Their columns push low parts of R into shared memory, where an MMA takes 45 cycles more
 // to read them: a step of [64, 512] 2.21 us in one accumulator, 2.30 in two, 2.50 in four; of [1, 256] 0.81, 0.80, 0.82.
-// h0 may be anything: its rows have a scale each.  A row of R, or an h0, with an infinite element or NaN has none: those
-// sums are plain fp32 FMAs.  Waits are bounded as in lstm_cluster.cu: on expiry a status word is set, the peers' waits expire in turn, and
+// h0 may be anything: its rows have a scale each.  A row of R, or an h0, with an infinite element or NaN has none: all of it
+// is left out of the parts.  Waits are bounded as in lstm_cluster.cu: on expiry a status word is set, the peers' waits expire in turn, and
 // all CTAs of the cluster meet at the last barrier.
 #include <cuda_fp16.h>
 #include <math.h>
@@ -43,6 +46,7 @@ constexpr int QUARTERS = MAX_CS / 4;
 constexpr int MAX_SMEM = 224 * 1024;
 constexpr int MIN_SMEM = 116 * 1024;        // all of tensor memory is taken: one CTA per SM
 constexpr float H_SCALE = 16384.f, H_UNSCALE = 1.f / 16384.f;
+constexpr float LO_SCALE = 8192.f, LO_UNSCALE = 1.f / 8192.f;   // of low parts against high ones
 constexpr unsigned long long WAIT_NS = 2000000000ull;
 
 struct LocalArgs {
@@ -64,10 +68,10 @@ struct LocalArgs {
 struct LocalShared {
   unsigned long long mma_bar;
   unsigned long long full[2];
+  unsigned long long small_r[4], small_h0;   // blocks of 8 units with elements outside the parts: of 32 rows of R, of h0
   unsigned int tmem_base;
-  int plain_h;
   float row_max[128];
-  float h0_unscale[8 * MAX_GROUPS];
+  float h0_unscale[8 * MAX_GROUPS], h0_limit[8 * MAX_GROUPS];
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -220,10 +224,16 @@ __device__ __forceinline__ float tanh_of(float x) {
   const float e = exp2_of(h), tail = inverse(1.f + fmaf(e, l * 0.693147181f, e));
   return copysignf(m < 0.7f ? fmaf(m * u, q, m) : fmaf(-2.f, tail, 1.f), x);
 }
-// x = hi + lo in fp16 parts; the low part of a scaled element is at worst 2^-25, 2^-39 of the largest
+// x = hi + lo / 2^13 in fp16 parts (|x| <= 2^14, so that |lo| <= 2^15): 23 bits, past 2^-15 at least 22, below that to 2^-37
 __device__ __forceinline__ void split_half(float x, __half* hi, __half* lo) {
   *hi = __float2half_rn(x);
-  *lo = __float2half_rn(x - __half2float(*hi));
+  *lo = __float2half_rn((x - __half2float(*hi)) * LO_SCALE);
+}
+// Elements that the parts would not hold to 22 bits: below a row's limit; a limit of NaN is for all of a row.
+__device__ __forceinline__ bool is_small(float v, float limit) { return v != 0.f && !(fabsf(v) >= limit); }
+__device__ __forceinline__ void add_blocks(unsigned long long* to, unsigned long long mine) {   // (the whole warp)
+  const uint32_t low = __reduce_or_sync(0xffffffffu, (uint32_t)mine), high = __reduce_or_sync(0xffffffffu, (uint32_t)(mine >> 32));
+  if ((threadIdx.x & 31) == 0 && (low | high)) atomicOr(to, (unsigned long long)high << 32 | low);
 }
 // Power of two that brings the largest magnitude `m` of a row into [2^13, 2^14) (a row of zeros or denormals: the largest
 // that leaves its inverse a normal number).
@@ -283,22 +293,49 @@ __device__ __forceinline__ void issue_sources(const Issue& o, int q, int n, int 
   }
 }
 
-// Sum of a gate row over K with plain FMAs: row `r` of R against batch row `b` of h, from the operand or (step 0) h0.
-__device__ __noinline__ float plain_sum(const float* r, const float* h0, const unsigned char* buf, int src_bytes, int hi_off,
-                                        int lo_off, int b, int H) {
-  float s = 0.f;
-  for (int k = 0; k < H; k++) {
-    float x;
-    if (h0) {
-      x = h0[k];
-    } else {
-      const unsigned char* p = buf + (k >> 5) * src_bytes + (b >> 3) * 512 + ((k >> 3) & 3) * 128 + (b & 7) * 16 + (k & 7) * 2;
-      x = (__half2float(*reinterpret_cast<const __half*>(p + hi_off)) + __half2float(*reinterpret_cast<const __half*>(p + lo_off))) *
-          H_UNSCALE;
+// Products of the elements of R that the parts leave out, for a gate row and four batch rows of h: `src` their high parts in
+// the first source's words, the low ones `lo_off` behind.  `blocks`: the blocks of 8 units to look at.
+__device__ __noinline__ float4 apart_sums(const float* r_row, float r_limit, unsigned long long blocks, int width, const unsigned char* src,
+                                          int src_bytes, int lo_off) {
+  float sum[4] = {0.f, 0.f, 0.f, 0.f};
+  for (; blocks; blocks &= blocks - 1) {
+    const int k = (__ffsll((long long)blocks) - 1) * 8;
+    float r[8];
+#pragma unroll
+    for (int c = 0; c < 8; c++) {
+      r[c] = k + c < width ? __ldg(r_row + k + c) : 0.f;
+      if (!is_small(r[c], r_limit)) r[c] = 0.f;
     }
-    s = fmaf(r[k], x, s);
+    const unsigned char* word = src + (k >> 5) * src_bytes + (k >> 3 & 3) * 128;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const uint4 hi = *reinterpret_cast<const uint4*>(word + j * 16), lo = *reinterpret_cast<const uint4*>(word + lo_off + j * 16);
+      const uint32_t wh[4] = {hi.x, hi.y, hi.z, hi.w}, wl[4] = {lo.x, lo.y, lo.z, lo.w};
+#pragma unroll
+      for (int c = 0; c < 8; c++) {
+        const __half h = __ushort_as_half((unsigned short)(wh[c / 2] >> (c & 1) * 16)), l = __ushort_as_half((unsigned short)(wl[c / 2] >> (c & 1) * 16));
+        if (r[c] != 0.f) sum[j] = fmaf(r[c], fmaf(__half2float(l), LO_UNSCALE, __half2float(h)) * H_UNSCALE, sum[j]);
+      }
+    }
   }
-  return s;
+  return make_float4(sum[0], sum[1], sum[2], sum[3]);
+}
+// The same for the first step, with four rows of h0 (`rows` of them exist) that have elements apart themselves.
+__device__ __noinline__ float4 apart_first(const float* r_row, float r_limit, unsigned long long blocks, int width, const float* h0,
+                                           const float* h0_limit, int rows) {
+  float sum[4] = {0.f, 0.f, 0.f, 0.f};
+  for (; blocks; blocks &= blocks - 1) {
+    const int k = (__ffsll((long long)blocks) - 1) * 8, end = min(k + 8, width);
+    for (int i = k; i < end; i++) {
+      const float r = __ldg(r_row + i);
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const float h = j < rows ? h0[(size_t)j * width + i] : 0.f;
+        if (j < rows && (is_small(r, r_limit) || is_small(h, h0_limit[j]))) sum[j] = fmaf(r, h, sum[j]);
+      }
+    }
+  }
+  return make_float4(sum[0], sum[1], sum[2], sum[3]);
 }
 
 // The gates of GROUPS of a thread's NG cells (side by side: their chains of dependent operations overlap), h into `out`.
@@ -360,7 +397,8 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs 
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&sh.mma_bar)));
     for (int i = 0; i < 2; i++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&sh.full[i])));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    sh.plain_h = 0;
+    for (int i = 0; i < 4; i++) sh.small_r[i] = 0;
+    sh.small_h0 = 0;
   }
   if (tid < 8 * MAX_GROUPS) sh.h0_unscale[tid] = 1.f;
   if (warp == 8) {
@@ -400,12 +438,12 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs 
   const uint32_t tmem = sh.tmem_base;
   const uint32_t tmem_hi = tmem + (uint32_t)L::D_COLS, tmem_lo = tmem_hi + (uint32_t)(16 * cs);
   const int steps_lo = L::steps_lo(cs);
-  bool plain_row = false;
-  float unscale = 0.f;
+  float unscale = 0.f, r_limit = 0.f;
   if (warp < 8) {
     const float m = sh.row_max[row];
-    plain_row = not_finite(m);
-    const int e = plain_row ? 0 : row_exponent(m);
+    const int e = not_finite(m) ? 0 : row_exponent(m);
+    r_limit = not_finite(m) ? __uint_as_float(0x7fffffffu) : pow2(-15 - e);   // (-114 <= e <= 100)
+    unsigned long long blocks = 0;
     const float scale = pow2(e);
     unscale = pow2(-e) * H_UNSCALE;                                // (e <= 100: a normal number)
     const uint32_t t_row = (uint32_t)((warp & 3) * 32) << 16;
@@ -434,10 +472,14 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs 
 #pragma unroll
         for (int q = 0; q < 4; q++) {
           const float4 v = chunk[row * 17 + half * 8 + i * 4 + q];
-          const float x[4] = {v.x * scale, v.y * scale, v.z * scale, v.w * scale};
+          const float x[4] = {v.x, v.y, v.z, v.w};
           __half h[4], l[4];
 #pragma unroll
-          for (int c = 0; c < 4; c++) split_half(plain_row ? 0.f : x[c], &h[c], &l[c]);
+          for (int c = 0; c < 4; c++) {
+            const bool small = is_small(x[c], r_limit);
+            split_half(small ? 0.f : x[c] * scale, &h[c], &l[c]);
+            if (small) blocks |= 1ull << (2 * j + (q >> 1));
+          }
 #pragma unroll
           for (int c = 0; c < 2; c++) {
             hi[q * 2 + c] = (uint32_t)__half_as_ushort(h[2 * c]) | (uint32_t)__half_as_ushort(h[2 * c + 1]) << 16;
@@ -456,6 +498,7 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs 
       asm volatile("bar.sync 1, 256;" ::: "memory");
     }
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    add_blocks(&sh.small_r[warp & 3], blocks);
   }
   __syncthreads();
   for (uint32_t i = (uint32_t)tid * 16u; i < 2u * buf_bytes; i += THREADS * 16u)   // rows past the batch stay zero
@@ -486,20 +529,25 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs 
       uint32_t m = 0;
       for (int k = lane; k < H; k += 32) m = max(m, __float_as_uint(src[k]) & 0x7fffffffu);
       m = __reduce_max_sync(0xffffffffu, m);
-      if (not_finite(__uint_as_float(m))) {
-        if (lane == 0) sh.plain_h = 1;
-        continue;
+      const bool finite = !not_finite(__uint_as_float(m));
+      const int e = finite ? row_exponent(__uint_as_float(m)) : 0;
+      const float scale = pow2(e), limit = finite ? pow2(-15 - e) : __uint_as_float(0x7fffffffu);
+      if (lane == 0) {
+        sh.h0_unscale[b] = pow2(-e);
+        sh.h0_limit[b] = limit;
       }
-      const int e = row_exponent(__uint_as_float(m));
-      const float scale = pow2(e);
-      if (lane == 0) sh.h0_unscale[b] = pow2(-e);
+      unsigned long long blocks = 0;
       for (int k = lane; k < H; k += 32) {
         __half hi, lo;
-        split_half(src[k] * scale, &hi, &lo);
+        const bool small = is_small(src[k], limit);
+        split_half(small ? 0.f : src[k] * scale, &hi, &lo);
+        if (small) blocks |= 1ull << (k >> 3);
         unsigned char* p = smem + (k >> 5) * L::SRC + (b >> 3) * 512 + ((k >> 3) & 3) * 128 + (b & 7) * 16 + (k & 7) * 2;
         *reinterpret_cast<__half*>(p + HI_OFF) = hi;
         *reinterpret_cast<__half*>(p + LO_OFF) = lo;
       }
+      __syncwarp();
+      add_blocks(&sh.small_h0, blocks);
     }
   }
   const uint32_t full0 = smem_u32(&sh.full[0]);
@@ -514,7 +562,7 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs 
   __syncthreads();
   cluster_barrier();                                               // every CTA is ready for the others' words
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const bool plain_h = sh.plain_h != 0;
+  const unsigned long long small_r = sh.small_r[warp & 3], small_h0 = sh.small_h0;
   const uint32_t mma_bar = smem_u32(&sh.mma_bar);
 
   if (warp == 8) {
@@ -557,7 +605,6 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs 
       if (peer >= cs) peer -= cs;
       dst[i] = map_to(my_slot, (uint32_t)(dist + 4 * i < cs ? peer : rank));
     }
-    const bool any_plain = __any_sync(0xffffffffu, plain_row);
     const bool some = 4 * half < nb;                               // (the last rows' warps may have nothing to do)
     const bool last_empty = 8 * (NG - 1) + 4 * half >= nb;
     uint32_t phase = 0;
@@ -595,26 +642,32 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs 
 #pragma unroll
         for (int g = 0; g < NG; g++)
 #pragma unroll
-          for (int j = 0; j < 4; j++) s[g][j] = (s[g][j] + x[g][j]) * unscale;
+          for (int j = 0; j < 4; j++) s[g][j] = fmaf(x[g][j], LO_UNSCALE, s[g][j]) * unscale;
         if (t == 0) {                                              // h0 has scales of its own
 #pragma unroll
           for (int g = 0; g < NG; g++)
 #pragma unroll
             for (int j = 0; j < 4; j++) s[g][j] = s[g][j] * H_SCALE * sh.h0_unscale[8 * g + 4 * half + j];
         }
-        if (any_plain || (t == 0 && plain_h)) {
+        const unsigned long long apart = t == 0 ? small_r | small_h0 : small_r;
+        if (apart) {                                               // products of what the parts do not hold, with plain FMAs
           bool ok = true;
           if (t > 0)                                               // (this thread reads the others' words itself)
             ok = mbar_wait(full0 + (t & 1 ? 8u : 0u), (uint32_t)((t - 1) >> 1) & 1u, a.status, 96);
-          const unsigned char* buf = smem + (t & 1 ? buf_bytes : 0u);
+          const int width = row_unit < H ? H : 0;
+          for (int g = 0; g < NG && ok; g++) {
+            const int b = 8 * g + 4 * half;
+            const float4 more = t == 0 ? apart_first(r_row, r_limit, apart, width, a.h0 + (size_t)(b0 + b) * H, sh.h0_limit + b, nb - b)
+                                       : apart_sums(r_row, r_limit, apart, width, smem + (t & 1 ? buf_bytes : 0u) + HI_OFF + g * L::GROUP + half * 64, L::SRC, NG * L::GROUP);
 #pragma unroll
-          for (int g = 0; g < NG; g++)
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-              const int b = 8 * g + 4 * half + j;
-              if (ok && (plain_row || (t == 0 && plain_h)) && b < nb && row_unit < H)
-                s[g][j] = plain_sum(r_row, t == 0 ? a.h0 + (size_t)(b0 + b) * H : nullptr, buf, L::SRC, HI_OFF, LO_OFF, b, H);
+            for (int i = 0; i < NG; i++) {                         // (s stays in registers)
+              if (i != g) continue;
+              s[i][0] += more.x;
+              s[i][1] += more.y;
+              s[i][2] += more.z;
+              s[i][3] += more.w;
             }
+          }
           __syncwarp();
         }
       }
