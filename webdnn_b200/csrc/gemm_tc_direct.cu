@@ -31,6 +31,7 @@ constexpr int TM = 128;              // rows of a tile = TMEM lanes
 constexpr int KB = 32;               // K block: one 128-byte swizzle row
 constexpr int SEG = 4;               // K blocks per TMEM segment
 constexpr int MAX_STAGES = 4;
+constexpr int SM_SMEM = 228 * 1024;
 constexpr unsigned long long WAIT_LIMIT_NS = 2000000000ull;
 
 struct DirectArgs {
@@ -448,10 +449,12 @@ int launch(wdc_context* ctx, DirectArgs a, int batch) {
   using L = DirectLayout<TN, kLong>;
   const dim3 grid((unsigned)((a.n + TN - 1) / TN), (unsigned)((a.m + TM - 1) / TM), (unsigned)batch);
   const int kblocks = (a.k + KB - 1) / KB;
-  // Short reductions of many tiles live on several CTAs per SM, one's output under the other's loads: one stage each
-  // (two stages at K = 64, [8, 850, 64] x [8, 64, 850]: one CTA an SM).  Otherwise as many as help.
-  const bool many = (int64_t)grid.x * grid.y * grid.z > ctx->sm_count;
-  a.stages = !kLong && many ? 1 : kblocks < L::STAGES ? kblocks : L::STAGES;
+  // Stages of short reductions: as many as leave room for all tiles at once ([16, 384, 128] x [16, 128, 384], 288 tiles: two
+  // 11.0 us, one 15.4).  More tiles than that live on three or four CTAs per SM, one's output under the other's loads, with one
+  // stage each (two at K = 64, [8, 850, 64] x [8, 64, 850]: one CTA an SM, 31.6 us and not 17.7).
+  const int64_t tiles = (int64_t)grid.x * grid.y * grid.z;
+  a.stages = kblocks < L::STAGES ? kblocks : L::STAGES;
+  while (!kLong && a.stages > 1 && tiles > (int64_t)ctx->sm_count * (SM_SMEM / (a.stages * L::STAGE + 2048))) a.stages--;
   const int smem = (a.stages * L::STAGE > L::OUT ? a.stages * L::STAGE : L::OUT) + 1024;
   static bool attr_set[64] = {};
   if (ctx->device < 0 || ctx->device >= 64) return WDC_ERR_UNSUPPORTED;
