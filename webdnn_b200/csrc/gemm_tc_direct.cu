@@ -14,10 +14,10 @@
 //     added in fp32 registers, one segment behind the MMAs;
 //   * the result leaves through shared memory, in rows of consecutive 16- or 8-byte words where N and Y allow.
 // Reductions of up to four K blocks are bound by a CTA's chain of latencies (load, split, MMA, output), so three or four CTAs
-// share an SM: [8, 850, 32] x [8, 32, 850] 20.4 -> 14.2 us a call (12 of them the host's), K = 64 32 -> 18 us, [64, 1024, 16]
-// x [64, 16, 1024] 162 -> 99 us.  Longer ones: [3, 100, 1000] x [3, 1000, 77] 39 -> 25 us, [8, 850, 256] x [8, 256, 850] 58 ->
-// 47, [64, 1024, 1024] x [64, 1024, 1024] 1460 -> 1240 us (2600 cycles a K block, of which shared memory alone takes
-// 1500: the MMAs read both operands there).
+// share an SM.  Device time, before the ring and with it: [8, 850, 32] x [8, 32, 850] 20.3 -> 9.6 us (a call from the host takes
+// 12), K = 64 31.6 -> 14.0, [64, 1024, 16] x [64, 16, 1024] 162 -> 74, [5, 1000, 32] x [5, 32, 77] 6.0 -> 4.3.  Longer ones: [3, 100, 1000]
+// x [3, 1000, 77] 39 -> 23, [8, 850, 256] x [8, 256, 850] 57 -> 43, [64, 1024, 1024] x [64, 1024, 1024] 1450 -> 1250 (2600 cycles a K
+// block, of which shared memory alone takes 1500: the MMAs read both operands there).
 // An infinite or NaN operand would meet low parts of
 // either sign or zero; a tile that contains one is recomputed with plain fp32 FMAs, which keeps IEEE results.
 // Waits are bounded (2 s, status word) like everywhere.
@@ -229,30 +229,42 @@ __device__ __forceinline__ bool store_block(const float* v, unsigned char* hi, u
   return bad;
 }
 
-// A warp's 32 rows x COLS columns of sums, staged in shared memory, to Y: V consecutive columns per lane.
-template <int V, int COLS, int PITCH>
+// A warp's 32 rows x COLS columns of sums, staged in shared memory, to Y: V consecutive columns per lane.  Several accesses of
+// a lane at a time, and the questions for an addend and a Relu (EXTRA) outside: one by one, with a branch each, the loads
+// from shared memory are a chain ([5, 1000, 32] x [5, 32, 77], 4-byte stores, 7.2 us and not 4.3).
+template <int V, bool EXTRA, int COLS, int PITCH>
 __device__ __forceinline__ void write_rows(const DirectArgs& a, const float* stg, float* Y, const float* C, int row0, int col0) {
   constexpr int LANES = COLS / V < 32 ? COLS / V : 32;             // of a row
   constexpr int ROWS = 32 / LANES;                                 // rows of an access
+  constexpr int PER_ROW = COLS / (LANES * V), ITEMS = 32 / ROWS * PER_ROW, BATCH = V == 4 ? 4 : 8;
+  static_assert(ITEMS % BATCH == 0, "whole batches");
   const int lane = threadIdx.x & 31, lr = lane / LANES, lc = lane % LANES * V;
-#pragma unroll 4
-  for (int r = lr; r < 32; r += ROWS) {
-    if (row0 + r >= a.m) break;
+  const int rows = a.m - row0, cols = a.n - col0 - lc;
+  Y += (int64_t)(row0 + lr) * a.n + col0 + lc;
+#pragma unroll 1
+  for (int i0 = 0; i0 < ITEMS; i0 += BATCH) {
+    float v[BATCH][V];
 #pragma unroll
-    for (int c = lc; c < COLS; c += LANES * V) {
-      if (col0 + c >= a.n) continue;
-      const float* src = stg + r * PITCH + c;
-      float* dst = Y + (int64_t)(row0 + r) * a.n + col0 + c;
-      float v[V];
+    for (int i = 0; i < BATCH; i++) {
+      const float* src = stg + (lr + (i0 + i) / PER_ROW * ROWS) * PITCH + lc + (i0 + i) % PER_ROW * (LANES * V);
+      if (V == 4) *reinterpret_cast<float4*>(v[i]) = *reinterpret_cast<const float4*>(src);
+      else if (V == 2) *reinterpret_cast<float2*>(v[i]) = *reinterpret_cast<const float2*>(src);
+      else v[i][0] = src[0];
+    }
+#pragma unroll
+    for (int i = 0; i < BATCH; i++) {
+      const int r = (i0 + i) / PER_ROW * ROWS, c = (i0 + i) % PER_ROW * (LANES * V);
+      if (lr + r >= rows || c >= cols) continue;
 #pragma unroll
       for (int j = 0; j < V; j++) {
-        v[j] = src[j] * a.alpha;
-        if (C) v[j] += pdl_ld(C + (int64_t)(row0 + r) * a.sc0 + (int64_t)(col0 + c + j) * a.sc1) * a.beta;
-        if (a.relu) v[j] = v[j] > 0.f ? v[j] : (v[j] == v[j] ? 0.f : v[j]);
+        v[i][j] *= a.alpha;
+        if (EXTRA && C) v[i][j] += pdl_ld(C + (int64_t)(row0 + lr + r) * a.sc0 + (int64_t)(col0 + lc + c + j) * a.sc1) * a.beta;
+        if (EXTRA && a.relu) v[i][j] = v[i][j] > 0.f ? v[i][j] : (v[i][j] == v[i][j] ? 0.f : v[i][j]);
       }
-      if (V == 4) *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1 % V], v[2 % V], v[3 % V]);
-      else if (V == 2) *reinterpret_cast<float2*>(dst) = make_float2(v[0], v[1 % V]);
-      else dst[0] = v[0];
+      float* dst = Y + (int64_t)r * a.n + c;
+      if (V == 4) *reinterpret_cast<float4*>(dst) = make_float4(v[i][0], v[i][1 % V], v[i][2 % V], v[i][3 % V]);
+      else if (V == 2) *reinterpret_cast<float2*>(dst) = make_float2(v[i][0], v[i][1 % V]);
+      else dst[0] = v[i][0];
     }
   }
 }
@@ -392,7 +404,7 @@ __global__ void __launch_bounds__(DirectLayout<TN, kLong>::THREADS, DirectLayout
         umma_tf32_ss(d, ah + adv, bl + adv, idesc, 1u);
         umma_tf32_ss(d, ah + adv, bh + adv, idesc, 1u);
       }
-      umma_commit(&sh.empty[st]);
+      if (kLong || kb + a.stages < kblocks) umma_commit(&sh.empty[st]);   // (nobody waits for the last ones)
       if (kb == kblocks - 1 || (kLong && in_seg == SEG - 1)) umma_commit(&sh.seg_full[buf]);
       if (++st == a.stages) { st = 0; par ^= 1u; }
     }
@@ -432,9 +444,15 @@ __global__ void __launch_bounds__(DirectLayout<TN, kLong>::THREADS, DirectLayout
     }
     __syncwarp();
     float* Y = a.Y + (int64_t)blockIdx.z * a.m * a.n;
-    if (a.vec == 4) write_rows<4, COLS, L::OUT_PITCH>(a, stg, Y, C, row0, col0);
-    else if (a.vec == 2) write_rows<2, COLS, L::OUT_PITCH>(a, stg, Y, C, row0, col0);
-    else write_rows<1, COLS, L::OUT_PITCH>(a, stg, Y, C, row0, col0);
+    if (C || a.relu) {
+      if (a.vec == 4) write_rows<4, true, COLS, L::OUT_PITCH>(a, stg, Y, C, row0, col0);
+      else if (a.vec == 2) write_rows<2, true, COLS, L::OUT_PITCH>(a, stg, Y, C, row0, col0);
+      else write_rows<1, true, COLS, L::OUT_PITCH>(a, stg, Y, C, row0, col0);
+    } else {
+      if (a.vec == 4) write_rows<4, false, COLS, L::OUT_PITCH>(a, stg, Y, C, row0, col0);
+      else if (a.vec == 2) write_rows<2, false, COLS, L::OUT_PITCH>(a, stg, Y, C, row0, col0);
+      else write_rows<1, false, COLS, L::OUT_PITCH>(a, stg, Y, C, row0, col0);
+    }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
