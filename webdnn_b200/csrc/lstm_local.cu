@@ -246,8 +246,9 @@ __device__ __forceinline__ float pow2(int e) { return __uint_as_float((uint32_t)
 // h of one buffer: [source CTA][zeros? hi groups, lo groups][4 blocks of 8 units][8 batch rows][8 units], fp16.
 // An odd number of groups has a group of zeros in front: the MMA of the low parts of R has at least 16 columns and
 // adds to the range of columns that hi*lo is summed in; the zeros stand for the 8 columns in front of that range.
-// ACCS: accumulators that the k steps go to in turn.
-template <int NG, int ACCS>
+// ACCS: accumulators that the k steps go to in turn.  TURNS: every other k step's low parts of R are in shared memory (where an
+// MMA takes 64 cycles to read them, part of it behind the others), not those that tensor memory has no room for.
+template <int NG, int ACCS, bool TURNS>
 struct LocalLayout {
   static constexpr int ZERO = NG & 1;
   static constexpr int GROUP = 512;                               // bytes of a group: 8 rows x 32 units
@@ -259,7 +260,9 @@ struct LocalLayout {
   static constexpr int LO_COL0 = 8 * (NG - ZERO);
   static constexpr int STAGE = 8 * NG * 128;                      // the eight warps' words on their way out
   // k steps whose low parts of R are in tensor memory
-  static __host__ __device__ constexpr int steps_lo(int cs) { return (512 - D_COLS) / 8 - 2 * cs < 2 * cs ? (512 - D_COLS) / 8 - 2 * cs : 2 * cs; }
+  static __host__ __device__ constexpr int steps_lo(int cs) {
+    return TURNS ? cs : (512 - D_COLS) / 8 - 2 * cs < 2 * cs ? (512 - D_COLS) / 8 - 2 * cs : 2 * cs;
+  }
 };
 
 // The MMAs of four sources (two k steps each).  One block of straight-line code whose addresses are constant offsets from
@@ -270,9 +273,9 @@ struct Issue {
   uint32_t b, b_top;           // descriptor of their words
   uint32_t r, r_top;           // descriptor of the low parts of R in shared memory
 };
-template <int NG, int ACCS, bool ALL>    // ALL: four sources, low parts in tensor memory
+template <int NG, int ACCS, bool TURNS, bool ALL>    // ALL: four sources, low parts in tensor memory
 __device__ __forceinline__ void issue_sources(const Issue& o, int q, int n, int lo_in_tmem) {
-  using L = LocalLayout<NG, ACCS>;
+  using L = LocalLayout<NG, ACCS, TURNS>;
   constexpr uint32_t ID_HI = (1u << 4) | ((uint32_t)(2 * NG) << 17) | ((128u >> 4) << 24);
   constexpr uint32_t ID_LO = (1u << 4) | ((uint32_t)(L::LO_ROWS >> 3) << 17) | ((128u >> 4) << 24);
 #pragma unroll
@@ -286,7 +289,9 @@ __device__ __forceinline__ void issue_sources(const Issue& o, int q, int n, int 
         if (step < ACCS) mma_ts(t_acc, o.t_hi + (uint32_t)(8 * step), b_hi, o.b_top, ID_HI, q > 0 ? 1u : 0u);
         else mma_ts_more(t_acc, o.t_hi + (uint32_t)(8 * step), b_hi, o.b_top, ID_HI);
         // (with zeros in front: their 8 columns have just been written by the MMA above, like the others)
-        if (ALL || step < lo_in_tmem) mma_ts_more(t_acc + (uint32_t)L::LO_COL0, o.t_lo + (uint32_t)(8 * step), b, o.b_top, ID_LO);
+        if (TURNS && j == 1) mma_ss_more(t_acc + (uint32_t)L::LO_COL0, o.r + (uint32_t)(d * 256), o.r_top, b, o.b_top, ID_LO);
+        else if (TURNS) mma_ts_more(t_acc + (uint32_t)L::LO_COL0, o.t_lo + (uint32_t)(8 * d), b, o.b_top, ID_LO);
+        else if (ALL || step < lo_in_tmem) mma_ts_more(t_acc + (uint32_t)L::LO_COL0, o.t_lo + (uint32_t)(8 * step), b, o.b_top, ID_LO);
         else mma_ss_more(t_acc + (uint32_t)L::LO_COL0, o.r + (uint32_t)((step - lo_in_tmem) * 256), o.r_top, b, o.b_top, ID_LO);
       }
     }
@@ -379,9 +384,9 @@ __device__ __forceinline__ void step_end(const float (&s)[NG][4], bool product, 
   }
 }
 
-template <int NG, int ACCS>
+template <int NG, int ACCS, bool TURNS>
 __global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs a) {
-  using L = LocalLayout<NG, ACCS>;
+  using L = LocalLayout<NG, ACCS, TURNS>;
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ LocalShared sh;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -487,10 +492,10 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs 
           }
         }
         tmem_st8(tmem_hi + t_row + (uint32_t)(8 * j), hi);
-        if (j < steps_lo) {
-          tmem_st8(tmem_lo + t_row + (uint32_t)(8 * j), lo);
+        if (TURNS ? (j & 1) == 0 : j < steps_lo) {
+          tmem_st8(tmem_lo + t_row + (uint32_t)(8 * (TURNS ? j >> 1 : j)), lo);
         } else {
-          unsigned char* dst = r_lo + (size_t)(j - steps_lo) * 4096 + row * 16;
+          unsigned char* dst = r_lo + (size_t)(TURNS ? j >> 1 : j - steps_lo) * 4096 + row * 16;
           *reinterpret_cast<uint4*>(dst) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
           *reinterpret_cast<uint4*>(dst + 2048) = make_uint4(lo[4], lo[5], lo[6], lo[7]);
         }
@@ -577,11 +582,11 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs 
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         for (int q = 0; q < quarters; q++) {
           const int n = cs - 4 * q, lo_in_tmem = steps_lo - 8 * q;
-          const Issue o = {tmem, tmem_hi + (uint32_t)(64 * q), tmem_lo + (uint32_t)(64 * q),
+          const Issue o = {tmem, tmem_hi + (uint32_t)(64 * q), tmem_lo + (uint32_t)((TURNS ? 32 : 64) * q),
                            (uint32_t)b_desc + (uint32_t)(((t & 1) * L::BUF + 4 * q * L::SRC) >> 4), (uint32_t)(b_desc >> 32),
-                           (uint32_t)r_desc, (uint32_t)(r_desc >> 32)};
-          if (n >= 4 && lo_in_tmem >= 8) issue_sources<NG, ACCS, true>(o, q, n, lo_in_tmem);
-          else issue_sources<NG, ACCS, false>(o, q, n, lo_in_tmem);
+                           (uint32_t)r_desc + (TURNS ? (uint32_t)(1024 * q) : 0u), (uint32_t)(r_desc >> 32)};
+          if (n >= 4 && (TURNS || lo_in_tmem >= 8)) issue_sources<NG, ACCS, TURNS, true>(o, q, n, lo_in_tmem);
+          else issue_sources<NG, ACCS, TURNS, false>(o, q, n, lo_in_tmem);
         }
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mma_bar) : "memory");
         if (t > 0) expect_bytes(bar, step_bytes);                  // the words of step t + 2
@@ -720,28 +725,36 @@ typedef void (*Kernel)(const LocalArgs);
 
 struct Variant {
   Kernel kernel;
-  int zero, d_cols, buf, stage;
+  int d_cols, buf, stage;
+  bool turns;
 };
-template <int NG, int ACCS>
+template <int NG, int ACCS, bool TURNS>
 constexpr Variant variant() {
-  using L = LocalLayout<NG, ACCS>;
-  return {lstm_local_kernel<NG, ACCS>, L::ZERO, L::D_COLS, L::BUF, L::STAGE};
+  using L = LocalLayout<NG, ACCS, TURNS>;
+  return {lstm_local_kernel<NG, ACCS, TURNS>, L::D_COLS, L::BUF, L::STAGE, TURNS};
 }
 const Variant variants[MAX_GROUPS][2] = {   // [8-row groups - 1][more than one CTA a cluster]
-    {variant<1, 2>(), variant<1, 4>()}, {variant<2, 2>(), variant<2, 4>()}, {variant<3, 2>(), variant<3, 4>()}, {variant<4, 2>(), variant<4, 4>()}};
+    {variant<1, 2, false>(), variant<1, 4, false>()}, {variant<2, 2, false>(), variant<2, 4, false>()},
+    {variant<3, 2, false>(), variant<3, 4, false>()}, {variant<4, 2, false>(), variant<4, 4, false>()}};
+const Variant two_groups_in_turns = variant<2, 4, true>();
 
 // k steps whose low parts of R are in shared memory
 int steps_in_smem(const Variant& v, int cs) {
   const int steps = 4 * cs - (512 - v.d_cols) / 8;
-  return steps < 0 ? 0 : steps;
+  return v.turns ? cs : steps < 0 ? 0 : steps;
 }
 size_t smem_of(const Variant& v, int cs) {
   const size_t bytes = 2 * (size_t)v.buf + v.stage + (size_t)steps_in_smem(v, cs) * 4096;
   return bytes < MIN_SMEM ? MIN_SMEM : bytes;
 }
 
-// Four accumulators, or one for each k step where there are two.
-const Variant& variant_of(int groups, int cs) { return variants[groups - 1][cs > 1]; }
+// Four accumulators, or one for each k step where there are two.  Two groups of rows on 15 and 16 CTAs have 12 and 16 k steps in
+// shared memory, and take every other one there: a step of [64, 480] 2.32 -> 2.28 us, of [64, 512] 2.47 -> 2.38 (with 8 of them, one
+// group on 16 CTAs, it is the other way round, 1.33 and 1.38, as there would be 16).
+const Variant& variant_of(int groups, int cs) {
+  const Variant& v = variants[groups - 1][cs > 1];
+  return groups == 2 && steps_in_smem(v, cs) > 8 ? two_groups_in_turns : v;
+}
 // 8-row groups of a cluster, at most: with four, 14 CTAs and more have no room for the low parts of R.
 int max_groups(int cs) { return cs <= 13 ? MAX_GROUPS : MAX_GROUPS - 1; }
 
