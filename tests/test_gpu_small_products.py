@@ -81,8 +81,9 @@ def test_two_activations_addend_and_non_finite(cuda_context):
     assert np.all(np.abs(got[m] - want[m]) <= 1e-5 * np.maximum(np.abs(want[m]), 1.0))
 
 
-# hidden sizes around the 32 units of a cluster and the K slices (8, 4 CTAs), batches around an MMA's 16 columns, the
-# spread over groups of clusters, and more rows than one launch takes; 3 steps, 28 and 800 units leave the kernel's range
+# hidden sizes around the 32 units of a CTA or a cluster, inside one cluster (up to 512) and across clusters (up to 768, their K
+# slices), batches around an MMA's columns, the spread over clusters, and more rows than one launch takes; 3 steps, 28 and
+# 800 units leave both kernels' range
 @pytest.mark.parametrize("seq,batch,inp,hidden,state", [
     (3, 3, 8, 32, False), (4, 1, 4, 32, False), (5, 2, 12, 28, True), (6, 3, 32, 36, True), (17, 16, 40, 64, False), (5, 17, 12, 100, True), (9, 96, 64, 216, True),
     (23, 5, 100, 344, False), (12, 64, 256, 512, True), (6, 70, 32, 512, False), (5, 33, 36, 516, True), (7, 96, 48, 768, True),

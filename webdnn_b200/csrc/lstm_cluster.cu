@@ -1,5 +1,5 @@
 // ONNX LSTM recurrence on the 5th-generation tensor cores, spread over the chip as thread-block clusters: hidden sizes whose R
-// does not fit one cluster (above 512; lstm_local.cu has the others, 2.0 us a step of [64, 512] where this takes 3.0).
+// does not fit one cluster (above 512; lstm_local.cu has the others, 2.4 us a step of [64, 512] where this takes 3.3).
 //
 // What bounds a recurrence is the chain of one step, not its arithmetic: h_t cannot start before h_{t-1} is known
 // everywhere.  lstm_persistent.cu spends 9 us on a step of [64, 512]: every CTA waits for a counter that all CTAs
@@ -14,10 +14,8 @@
 //     every thread sends its columns with st.async to the CTA that finishes its row, whose mbarrier counts the bytes.
 //     Two buffers and two barriers, by the parity of the step: a CTA reaches step t + 2 only after every CTA of the
 //     cluster has sent step t + 1, i.e. has read step t.
-// Measured on [128, 64, 256] with 512 hidden units: 1173 -> 442 us with the input projection (9.1 -> 3.4 us a step); 66
-// steps of [6, 176], which took the per-step path: 1867 -> 209 us.  Of a 64 x 512 step's 5500 cycles 1850 are the
-// exchange of h through L2 (store, poll), 1100 the 48 MMAs and their completion, 1500 the exchange of partial sums, 700
-// the sums and gates.
+// Measured: a step of [1, 544] 2.0 us, of [64, 544] 5.0 (two groups of rows fit the GPU), of [1,
+// 768] 2.2, of [64, 768] 5.8 (one group).
 // All clusters of a launch wait for one another, so the launch is cooperative (all resident or an error).
 // Products are 3xTF32 with rounded parts (2^-23 of a product), sums fp32; gates as in lstm_persistent.cu.  An infinite
 // element of R or h0 would meet low parts of either sign or zero: a CTA whose slice holds one sums with plain fp32 FMAs.
@@ -31,6 +29,10 @@ namespace {
 
 constexpr int THREADS = 256;
 constexpr int UNITS = 32;             // units of a cluster: 4 gate rows each
+constexpr int CS = 4;                 // CTAs of a cluster (17 clusters of 8, for the first size that gets here, do not fit the GPU)
+constexpr int UPC = UNITS / CS;       // units a CTA finishes
+constexpr int ROWS = 4 * UPC;         // their gate rows
+constexpr int PAIRS = 4;              // (unit, batch row) pairs a thread finishes, at most
 constexpr int D_COLS = 128;           // TMEM columns of the accumulator (batch rows of a launch, at most)
 constexpr int KC_MAX = (512 - D_COLS) / 2;   // K slice: high and low parts of R fill the rest of tensor memory
 constexpr int MAX_ITEMS = 12;         // 16-byte words of h a thread brings in per step, at most
@@ -200,12 +202,9 @@ __device__ __noinline__ void send_plain_sums(const float* R, const float* h, int
   }
 }
 
-// CS: CTAs of a cluster.  ITEMS: 16-byte words of h a thread brings in per step, at most.
-template <int CS, int ITEMS>
+// ITEMS: 16-byte words of h a thread brings in per step, at most.
+template <int ITEMS>
 __global__ void __launch_bounds__(THREADS, 1) lstm_cluster_kernel(const ClusterArgs a) {
-  constexpr int UPC = UNITS / CS;                          // units a CTA finishes
-  constexpr int ROWS = 4 * UPC;                            // their gate rows
-  constexpr int PAIRS = CS == 8 ? 2 : 4;                   // (unit, batch row) pairs a thread finishes, at most
   extern __shared__ unsigned char smem_raw[];
   __shared__ ClusterShared sh;
   unsigned char* h_hi = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -504,24 +503,19 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_cluster_kernel(const ClusterA
 
 typedef void (*Kernel)(const ClusterArgs);
 
-// words of h per thread of a launch with n batch rows and a K slice of kc
-bool few_items(int n, int kc) { return n * (kc / 4) <= 4 * THREADS; }
-Kernel kernel_of(int cs, int n, int kc) {
-  const bool few = few_items(n, kc);
-  if (cs == 8) return few ? lstm_cluster_kernel<8, 4> : lstm_cluster_kernel<8, 12>;
-  return few ? lstm_cluster_kernel<4, 4> : lstm_cluster_kernel<4, 12>;
-}
+// by the words of h per thread of a launch with n batch rows and a K slice of kc
+Kernel kernel_of(int n, int kc) { return n * (kc / 4) <= 4 * THREADS ? lstm_cluster_kernel<4> : lstm_cluster_kernel<12>; }
 
 size_t smem_of(int n, int kc) { return (size_t)n * ((kc + 31) / 32 * 256 + 2 * 128 * 4) + 1024; }
 
-void fill_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, int grid, int cs, size_t smem, cudaStream_t stream) {
+void fill_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, int grid, size_t smem, cudaStream_t stream) {
   *cfg = {};
   cfg->gridDim = dim3((unsigned)grid);
   cfg->blockDim = dim3(THREADS);
   cfg->dynamicSmemBytes = smem;
   cfg->stream = stream;
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)cs;
+  attr[0].val.clusterDim.x = CS;
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
   attr[1].id = cudaLaunchAttributeCooperative;
   attr[1].val.cooperative = 1;
@@ -529,8 +523,8 @@ void fill_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, int grid, i
   cfg->numAttrs = 2;
 }
 
-// Clusters of `cs` CTAs with `smem` bytes each that can be resident at once (asked once per device and shape).
-int max_clusters(wdc_context* ctx, Kernel kernel, int cs, size_t smem) {
+// Clusters whose CTAs have `smem` bytes each that can be resident at once (asked once per device and shape).
+int max_clusters(wdc_context* ctx, Kernel kernel, size_t smem) {
   static std::mutex mu;
   static std::map<std::pair<std::pair<int, Kernel>, size_t>, int> known;
   std::lock_guard<std::mutex> lk(mu);
@@ -541,7 +535,7 @@ int max_clusters(wdc_context* ctx, Kernel kernel, int cs, size_t smem) {
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM);
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr[2];
-  fill_config(&cfg, attr, cs, cs, smem, nullptr);
+  fill_config(&cfg, attr, CS, smem, nullptr);
   cfg.numAttrs = 1;
   if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg);
   if (e != cudaSuccess) {
@@ -554,42 +548,35 @@ int max_clusters(wdc_context* ctx, Kernel kernel, int cs, size_t smem) {
 
 struct Plan {
   Kernel kernel = nullptr;
-  int cs = 0, kc = 0, per = 0, n = 0;
+  int kc = 0, per = 0, n = 0;
   int fit = 0;            // groups of batch rows (each on `blocks` clusters) that are resident at once
   size_t smem = 0;
 };
 
-// The widest K split that fits: a wider cluster reads less of h per CTA and has a shorter product.
 Plan plan_of(wdc_context* ctx, int64_t Bt, int64_t H, int blocks) {
-  for (int cs = 8; cs >= 4; cs >>= 1) {
-    Plan p;
-    p.cs = cs;
-    p.kc = (int)((ceil_div64(H, cs) + 7) / 8 * 8);
-    if (p.kc > KC_MAX) break;
-    // batch rows per group: as few as spread the batch over the clusters that fit, at most what shared memory, the
-    // threads' words of h and their (unit, row) pairs allow
-    const int pairs = (cs == 8 ? 2 : 4) * THREADS / (UNITS / cs);
-    int most = pairs < D_COLS ? pairs : D_COLS;
-    while (most > 16 && (smem_of(most, p.kc) > (size_t)MAX_SMEM || most * (p.kc / 4) > MAX_ITEMS * THREADS)) most -= 16;
-    if (smem_of(most, p.kc) > (size_t)MAX_SMEM) continue;
-    if (most > Bt) most = (int)Bt;
-    const int most_n = (most + 15) / 16 * 16;
-    p.fit = max_clusters(ctx, kernel_of(cs, most_n, p.kc), cs, smem_of(most_n, p.kc)) / blocks;
-    if (!p.fit) continue;
-    int groups = (int)ceil_div64(Bt, 16);        // an MMA has at least 16 columns
-    if (groups > p.fit) groups = p.fit;
-    p.per = (int)ceil_div64(Bt, groups);
-    if (p.per > most) {                          // several launches: equal shares
-      const int64_t launches = ceil_div64(Bt, (int64_t)most * p.fit);
-      p.per = (int)ceil_div64(Bt, launches * p.fit);
-    }
-    p.n = (p.per + 15) / 16 * 16;
-    p.kernel = kernel_of(cs, p.n, p.kc);
-    p.smem = smem_of(p.n, p.kc);
-    if (max_clusters(ctx, p.kernel, cs, p.smem) / blocks < p.fit) continue;
-    return p;
+  Plan p;
+  p.kc = (int)((ceil_div64(H, CS) + 7) / 8 * 8);
+  // batch rows per group: as few as spread the batch over the clusters that fit, at most what shared memory, the
+  // threads' words of h and their (unit, row) pairs allow
+  int most = PAIRS * THREADS / UPC < D_COLS ? PAIRS * THREADS / UPC : D_COLS;
+  while (most > 16 && (smem_of(most, p.kc) > (size_t)MAX_SMEM || most * (p.kc / 4) > MAX_ITEMS * THREADS)) most -= 16;
+  if (smem_of(most, p.kc) > (size_t)MAX_SMEM) return Plan();
+  if (most > Bt) most = (int)Bt;
+  const int most_n = (most + 15) / 16 * 16;
+  p.fit = max_clusters(ctx, kernel_of(most_n, p.kc), smem_of(most_n, p.kc)) / blocks;
+  if (!p.fit) return Plan();
+  int groups = (int)ceil_div64(Bt, 16);        // an MMA has at least 16 columns
+  if (groups > p.fit) groups = p.fit;
+  p.per = (int)ceil_div64(Bt, groups);
+  if (p.per > most) {                          // several launches: equal shares
+    const int64_t launches = ceil_div64(Bt, (int64_t)most * p.fit);
+    p.per = (int)ceil_div64(Bt, launches * p.fit);
   }
-  return Plan();
+  p.n = (p.per + 15) / 16 * 16;
+  p.kernel = kernel_of(p.n, p.kc);
+  p.smem = smem_of(p.n, p.kc);
+  if (max_clusters(ctx, p.kernel, p.smem) / blocks < p.fit) return Plan();
+  return p;
 }
 
 }  // namespace
@@ -601,7 +588,7 @@ int wdc_lstm_cluster(wdc_context* ctx, const float* P, const float* R, const flo
   // One to three steps do not pay for filling Y and bringing R into tensor memory, and below 32 units most rows of the
   // MMA would be empty: the other paths keep those.
   if (T < 4 || H < UNITS) return WDC_ERR_UNSUPPORTED;
-  if (T > (1 << 24) || Bt > (1 << 20) || H % 4 != 0 || H > 8 * KC_MAX) return WDC_ERR_UNSUPPORTED;
+  if (T > (1 << 24) || Bt > (1 << 20) || H % 4 != 0 || H > CS * KC_MAX) return WDC_ERR_UNSUPPORTED;
   if ((((uintptr_t)R | (uintptr_t)Y | (uintptr_t)h0) & 15) != 0) return WDC_ERR_UNSUPPORTED;
   ClusterArgs a = {P, R, bias, h0, c0, Y, Yh, Yc, ctx->status_word, (int)T, (int)Bt, (int)H};
   a.blocks = (int)((H + UNITS - 1) / UNITS);
@@ -618,7 +605,7 @@ int wdc_lstm_cluster(wdc_context* ctx, const float* P, const float* R, const flo
     const int groups = (a.nb + a.per - 1) / a.per;
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[2];
-    fill_config(&cfg, attr, groups * a.blocks * p.cs, p.cs, p.smem, ctx->stream);
+    fill_config(&cfg, attr, groups * a.blocks * CS, p.smem, ctx->stream);
     cudaError_t e = cudaLaunchKernelEx(&cfg, p.kernel, (const ClusterArgs)a);
     if (e != cudaSuccess) {
       cudaGetLastError();
