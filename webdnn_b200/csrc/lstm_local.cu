@@ -9,8 +9,8 @@
 //     last low parts in shared memory), where TF32 parts take 8.  h is in (-1, 1) and has a constant scale.  Two parts of
 //     11 rounded bits carry 23 bits (TF32 parts, cut by the tensor core: 22), the low one with a scale of 2^13 of its own, so
 //     that elements down to 2^-28 of a row's largest have 22 bits.  What is smaller is left out of the parts, and the CTA that
-//     has such elements of R, or of h0, adds their products with fp32 FMAs (blocks of 8 units that hold one: some 500 cycles
-//     each).  h below 2^-29 is good to 2^-51 absolutely.  An fp16 MMA covers twice the K of a TF32 one in the same time: M 128
+//     has such elements of R, or of h0, adds their products with fp32 FMAs (one of them in R: a step of [64, 512] 2.37 -> 3.1
+//     us, of [1, 256] 0.82 -> 1.4, most of it the way to the element through L2).  h below 2^-29 is good to 2^-51 absolutely.  An fp16 MMA covers twice the K of a TF32 one in the same time: M 128
 //     x N 16 x K 16 takes 9 cycles, N 32 takes 16;
 //   * h goes to every CTA of the cluster as 16-byte words in the layout of the MMA's B operand (no swizzle: 8 batch rows x
 //     8 units are 128 consecutive bytes), by st.async, whose mbarrier counts the bytes (a CTA takes in about 20 a clock:
@@ -47,6 +47,7 @@ constexpr int MAX_SMEM = 224 * 1024;
 constexpr int MIN_SMEM = 116 * 1024;        // all of tensor memory is taken: one CTA per SM
 constexpr float H_SCALE = 16384.f, H_UNSCALE = 1.f / 16384.f;
 constexpr float LO_SCALE = 8192.f, LO_UNSCALE = 1.f / 8192.f;   // of low parts against high ones
+constexpr float SMALL = 1.f / 32768.f;   // what is below that, scaled, is left out of the parts
 constexpr unsigned long long WAIT_NS = 2000000000ull;
 
 struct LocalArgs {
@@ -68,10 +69,10 @@ struct LocalArgs {
 struct LocalShared {
   unsigned long long mma_bar;
   unsigned long long full[2];
-  unsigned long long small_r[4], small_h0;   // blocks of 8 units with elements outside the parts: of 32 rows of R, of h0
+  unsigned int small_r[4][MAX_CS], small_h0[MAX_CS];   // units with elements outside the parts: of 32 rows of R, of h0; by source
   unsigned int tmem_base;
   float row_max[128];
-  float h0_unscale[8 * MAX_GROUPS], h0_limit[8 * MAX_GROUPS];
+  float h0_unscale[8 * MAX_GROUPS];   // negative: all of the row is left out of the parts
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -231,9 +232,11 @@ __device__ __forceinline__ void split_half(float x, __half* hi, __half* lo) {
 }
 // Elements that the parts would not hold to 22 bits: below a row's limit; a limit of NaN is for all of a row.
 __device__ __forceinline__ bool is_small(float v, float limit) { return v != 0.f && !(fabsf(v) >= limit); }
-__device__ __forceinline__ void add_blocks(unsigned long long* to, unsigned long long mine) {   // (the whole warp)
-  const uint32_t low = __reduce_or_sync(0xffffffffu, (uint32_t)mine), high = __reduce_or_sync(0xffffffffu, (uint32_t)(mine >> 32));
-  if ((threadIdx.x & 31) == 0 && (low | high)) atomicOr(to, (unsigned long long)high << 32 | low);
+__device__ __forceinline__ uint32_t nonzero_words(const unsigned int* words) {                // bit i: word i of MAX_CS
+  uint32_t mask = 0;
+#pragma unroll
+  for (int i = 0; i < MAX_CS; i++) mask |= words[i] ? 1u << i : 0u;
+  return mask;
 }
 // Power of two that brings the largest magnitude `m` of a row into [2^13, 2^14) (a row of zeros or denormals: the largest
 // that leaves its inverse a normal number).
@@ -299,44 +302,43 @@ __device__ __forceinline__ void issue_sources(const Issue& o, int q, int n, int 
 }
 
 // Products of the elements of R that the parts leave out, for a gate row and four batch rows of h: `src` their high parts in
-// the first source's words, the low ones `lo_off` behind.  `blocks`: the blocks of 8 units to look at.
-__device__ __noinline__ float4 apart_sums(const float* r_row, float r_limit, unsigned long long blocks, int width, const unsigned char* src,
-                                          int src_bytes, int lo_off) {
+// the first source's words, the low ones `lo_off` behind.  `units`: the units that have such elements, `words` the words that
+// are not zero.
+__device__ __noinline__ float4 apart_sums(const float* r_row, float r_limit, const unsigned int* units, uint32_t words, int width,
+                                          const unsigned char* src, int src_bytes, int lo_off) {
   float sum[4] = {0.f, 0.f, 0.f, 0.f};
-  for (; blocks; blocks &= blocks - 1) {
-    const int k = (__ffsll((long long)blocks) - 1) * 8;
-    float r[8];
+  for (; words; words &= words - 1) {
+    const int w = __ffs((int)words) - 1;
+#pragma unroll 2
+    for (uint32_t left = units[w]; left; left &= left - 1) {
+      const int k = __ffs((int)left) - 1;
+      float r = w * 32 + k < width ? __ldg(r_row + w * 32 + k) : 0.f;
+      if (!is_small(r, r_limit)) r = 0.f;
+      const unsigned char* p = src + w * src_bytes + (k >> 3) * 128 + (k & 7) * 2;
 #pragma unroll
-    for (int c = 0; c < 8; c++) {
-      r[c] = k + c < width ? __ldg(r_row + k + c) : 0.f;
-      if (!is_small(r[c], r_limit)) r[c] = 0.f;
-    }
-    const unsigned char* word = src + (k >> 5) * src_bytes + (k >> 3 & 3) * 128;
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const uint4 hi = *reinterpret_cast<const uint4*>(word + j * 16), lo = *reinterpret_cast<const uint4*>(word + lo_off + j * 16);
-      const uint32_t wh[4] = {hi.x, hi.y, hi.z, hi.w}, wl[4] = {lo.x, lo.y, lo.z, lo.w};
-#pragma unroll
-      for (int c = 0; c < 8; c++) {
-        const __half h = __ushort_as_half((unsigned short)(wh[c / 2] >> (c & 1) * 16)), l = __ushort_as_half((unsigned short)(wl[c / 2] >> (c & 1) * 16));
-        if (r[c] != 0.f) sum[j] = fmaf(r[c], fmaf(__half2float(l), LO_UNSCALE, __half2float(h)) * H_UNSCALE, sum[j]);
+      for (int j = 0; j < 4; j++) {
+        const float h = __half2float(*reinterpret_cast<const __half*>(p + j * 16)), l = __half2float(*reinterpret_cast<const __half*>(p + lo_off + j * 16));
+        if (r != 0.f) sum[j] = fmaf(r, fmaf(l, LO_UNSCALE, h) * H_UNSCALE, sum[j]);
       }
     }
   }
   return make_float4(sum[0], sum[1], sum[2], sum[3]);
 }
 // The same for the first step, with four rows of h0 (`rows` of them exist) that have elements apart themselves.
-__device__ __noinline__ float4 apart_first(const float* r_row, float r_limit, unsigned long long blocks, int width, const float* h0,
-                                           const float* h0_limit, int rows) {
+__device__ __noinline__ float4 apart_first(const float* r_row, float r_limit, const unsigned int* units, const unsigned int* h0_units,
+                                           uint32_t words, int width, const float* h0, const float* h0_unscale, int rows) {
   float sum[4] = {0.f, 0.f, 0.f, 0.f};
-  for (; blocks; blocks &= blocks - 1) {
-    const int k = (__ffsll((long long)blocks) - 1) * 8, end = min(k + 8, width);
-    for (int i = k; i < end; i++) {
-      const float r = __ldg(r_row + i);
+  for (; words; words &= words - 1) {
+    const int w = __ffs((int)words) - 1;
+    for (uint32_t left = units[w] | h0_units[w]; left; left &= left - 1) {
+      const int k = w * 32 + __ffs((int)left) - 1;
+      if (k >= width) break;
+      const float r = __ldg(r_row + k);
 #pragma unroll
       for (int j = 0; j < 4; j++) {
-        const float h = j < rows ? h0[(size_t)j * width + i] : 0.f;
-        if (j < rows && (is_small(r, r_limit) || is_small(h, h0_limit[j]))) sum[j] = fmaf(r, h, sum[j]);
+        const float h = j < rows ? h0[(size_t)j * width + k] : 0.f;
+        const float limit = j < rows && h0_unscale[j] > 0.f ? h0_unscale[j] * SMALL : __uint_as_float(0x7fffffffu);
+        if (j < rows && (is_small(r, r_limit) || is_small(h, limit))) sum[j] = fmaf(r, h, sum[j]);
       }
     }
   }
@@ -402,9 +404,9 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs 
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&sh.mma_bar)));
     for (int i = 0; i < 2; i++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&sh.full[i])));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    for (int i = 0; i < 4; i++) sh.small_r[i] = 0;
-    sh.small_h0 = 0;
   }
+  if (tid < 4 * MAX_CS) sh.small_r[tid / MAX_CS][tid % MAX_CS] = 0;
+  if (tid < MAX_CS) sh.small_h0[tid] = 0;
   if (tid < 8 * MAX_GROUPS) sh.h0_unscale[tid] = 1.f;
   if (warp == 8) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sh.tmem_base)),
@@ -447,8 +449,7 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs 
   if (warp < 8) {
     const float m = sh.row_max[row];
     const int e = not_finite(m) ? 0 : row_exponent(m);
-    r_limit = not_finite(m) ? __uint_as_float(0x7fffffffu) : pow2(-15 - e);   // (-114 <= e <= 100)
-    unsigned long long blocks = 0;
+    r_limit = not_finite(m) ? __uint_as_float(0x7fffffffu) : pow2(-e) * SMALL;   // (-114 <= e <= 100)
     const float scale = pow2(e);
     unscale = pow2(-e) * H_UNSCALE;                                // (e <= 100: a normal number)
     const uint32_t t_row = (uint32_t)((warp & 3) * 32) << 16;
@@ -473,7 +474,7 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs 
       for (int i = 0; i < 2; i++) {
         const int j = k / 16 + half * 2 + i;                       // k step of 16
         if (j >= 2 * cs) break;
-        uint32_t hi[8], lo[8];
+        uint32_t hi[8], lo[8], units = 0;
 #pragma unroll
         for (int q = 0; q < 4; q++) {
           const float4 v = chunk[row * 17 + half * 8 + i * 4 + q];
@@ -483,7 +484,7 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs 
           for (int c = 0; c < 4; c++) {
             const bool small = is_small(x[c], r_limit);
             split_half(small ? 0.f : x[c] * scale, &h[c], &l[c]);
-            if (small) blocks |= 1ull << (2 * j + (q >> 1));
+            if (small) units |= 1u << (q * 4 + c);
           }
 #pragma unroll
           for (int c = 0; c < 2; c++) {
@@ -491,6 +492,7 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs 
             lo[q * 2 + c] = (uint32_t)__half_as_ushort(l[2 * c]) | (uint32_t)__half_as_ushort(l[2 * c + 1]) << 16;
           }
         }
+        if (units) atomicOr(&sh.small_r[warp & 3][j >> 1], units << (j & 1) * 16);
         tmem_st8(tmem_hi + t_row + (uint32_t)(8 * j), hi);
         if (TURNS ? (j & 1) == 0 : j < steps_lo) {
           tmem_st8(tmem_lo + t_row + (uint32_t)(8 * (TURNS ? j >> 1 : j)), lo);
@@ -503,7 +505,6 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs 
       asm volatile("bar.sync 1, 256;" ::: "memory");
     }
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-    add_blocks(&sh.small_r[warp & 3], blocks);
   }
   __syncthreads();
   for (uint32_t i = (uint32_t)tid * 16u; i < 2u * buf_bytes; i += THREADS * 16u)   // rows past the batch stay zero
@@ -536,23 +537,17 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs 
       m = __reduce_max_sync(0xffffffffu, m);
       const bool finite = !not_finite(__uint_as_float(m));
       const int e = finite ? row_exponent(__uint_as_float(m)) : 0;
-      const float scale = pow2(e), limit = finite ? pow2(-15 - e) : __uint_as_float(0x7fffffffu);
-      if (lane == 0) {
-        sh.h0_unscale[b] = pow2(-e);
-        sh.h0_limit[b] = limit;
-      }
-      unsigned long long blocks = 0;
+      const float scale = pow2(e), limit = finite ? pow2(-e) * SMALL : __uint_as_float(0x7fffffffu);
+      if (lane == 0) sh.h0_unscale[b] = finite ? pow2(-e) : -1.f;
       for (int k = lane; k < H; k += 32) {
         __half hi, lo;
         const bool small = is_small(src[k], limit);
         split_half(small ? 0.f : src[k] * scale, &hi, &lo);
-        if (small) blocks |= 1ull << (k >> 3);
+        if (small) atomicOr(&sh.small_h0[k >> 5], 1u << (k & 31));
         unsigned char* p = smem + (k >> 5) * L::SRC + (b >> 3) * 512 + ((k >> 3) & 3) * 128 + (b & 7) * 16 + (k & 7) * 2;
         *reinterpret_cast<__half*>(p + HI_OFF) = hi;
         *reinterpret_cast<__half*>(p + LO_OFF) = lo;
       }
-      __syncwarp();
-      add_blocks(&sh.small_h0, blocks);
     }
   }
   const uint32_t full0 = smem_u32(&sh.full[0]);
@@ -567,7 +562,7 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs 
   __syncthreads();
   cluster_barrier();                                               // every CTA is ready for the others' words
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const unsigned long long small_r = sh.small_r[warp & 3], small_h0 = sh.small_h0;
+  const uint32_t small_r = nonzero_words(sh.small_r[warp & 3]), small_h0 = nonzero_words(sh.small_h0);
   const uint32_t mma_bar = smem_u32(&sh.mma_bar);
 
   if (warp == 8) {
@@ -654,7 +649,7 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs 
 #pragma unroll
             for (int j = 0; j < 4; j++) s[g][j] = s[g][j] * H_SCALE * sh.h0_unscale[8 * g + 4 * half + j];
         }
-        const unsigned long long apart = t == 0 ? small_r | small_h0 : small_r;
+        const uint32_t apart = t == 0 ? small_r | small_h0 : small_r;
         if (apart) {                                               // products of what the parts do not hold, with plain FMAs
           bool ok = true;
           if (t > 0)                                               // (this thread reads the others' words itself)
@@ -662,8 +657,8 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs 
           const int width = row_unit < H ? H : 0;
           for (int g = 0; g < NG && ok; g++) {
             const int b = 8 * g + 4 * half;
-            const float4 more = t == 0 ? apart_first(r_row, r_limit, apart, width, a.h0 + (size_t)(b0 + b) * H, sh.h0_limit + b, nb - b)
-                                       : apart_sums(r_row, r_limit, apart, width, smem + (t & 1 ? buf_bytes : 0u) + HI_OFF + g * L::GROUP + half * 64, L::SRC, NG * L::GROUP);
+            const float4 more = t == 0 ? apart_first(r_row, r_limit, sh.small_r[warp & 3], sh.small_h0, apart, width, a.h0 + (size_t)(b0 + b) * H, sh.h0_unscale + b, nb - b)
+                                       : apart_sums(r_row, r_limit, sh.small_r[warp & 3], apart, width, smem + (t & 1 ? buf_bytes : 0u) + HI_OFF + g * L::GROUP + half * 64, L::SRC, NG * L::GROUP);
 #pragma unroll
             for (int i = 0; i < NG; i++) {                         // (s stays in registers)
               if (i != g) continue;
