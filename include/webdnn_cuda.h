@@ -337,9 +337,9 @@ int wdc_decode_eightbit(wdc_context* ctx, const void* codes, float* out, int64_t
  * ONNX LSTM, forward direction, default activations, no peepholes (not in the reference; ONNX
  * operator spec).  X [T, Bt, I], W [4H, I], R [4H, H], bias [8H] or NULL, h0/c0 [Bt, H] or NULL;
  * Y [T, 1, Bt, H], Yh/Yc [Bt, H].  Gate order i, o, f, c.  One tensor-core GEMM projects the
- * inputs of all steps; the recurrence runs as one cooperative kernel with R resident in tensor memory
- * (T >= 4, H >= 32, H % 4 == 0, slices that fit) or in shared memory (Bt <= 64, H % 32 == 0, slices
- * that fit), else as one GEMM + one gate kernel per step. */
+ * inputs of all steps; the recurrence runs as one launch with R resident in tensor memory (T >= 4,
+ * 32 <= H <= 768, H % 4 == 0) or in shared memory (Bt <= 64, H % 32 == 0, slices that fit), else as one
+ * GEMM + one gate kernel per step. */
 int wdc_lstm(wdc_context* ctx, const float* X, const float* W, const float* R, const float* bias,
              const float* h0, const float* c0, float* Y, float* Yh, float* Yc, int64_t T,
              int64_t Bt, int64_t I, int64_t H);

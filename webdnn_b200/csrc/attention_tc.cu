@@ -133,10 +133,9 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr) {
 __device__ __forceinline__ uint32_t make_idesc(int n) {
   return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(BQ >> 4) << 24);
 }
-// An MMA and a commit by one lane.  The issuing loop stands in a branch on elect.sync itself, where the compiler knows that
-// one lane is active and passes operands through uniform registers as they are; in a branch on a copy of the answer, or
-// with a predicate inside the instruction, it makes sure of their uniformity for every MMA (37 cycles each and 110 for a
-// commit, where the 24 MMAs of P V take 16 each).
+// An MMA and a commit by one lane.  The issuing loop stands in a branch on elect.sync itself: there the 24 MMAs of P V take
+// 16 cycles each to issue and a commit 20; in a branch on a copy of the answer, or with a predicate inside the instruction, 37
+// and 110.
 __device__ __forceinline__ void umma_one(uint32_t tmem_c, uint32_t tmem_a, uint32_t desc_lo, uint32_t desc_top, uint32_t idesc,
                                          uint32_t accumulate) {
   asm volatile(

@@ -429,9 +429,8 @@ __device__ __forceinline__ void arrive_at(uint32_t bar) {
 __device__ __forceinline__ void expect_at(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-// tcgen05.mma with A in tensor memory by the lane whose `leader` is 1.  The whole warp runs the issuing loop, so that
-// its addresses are the same in every lane and stay in uniform registers: in a branch of the elected lane alone the
-// arithmetic between two K blocks took longer than their MMAs.
+// tcgen05.mma with A in tensor memory by the lane whose `leader` is 1.  The whole warp runs the issuing loop:
+// in a branch of the elected lane alone the arithmetic between two K blocks took longer than their MMAs.
 __device__ __forceinline__ void umma_by(uint32_t leader, uint32_t tmem_c, uint32_t tmem_a, uint32_t desc_lo, uint32_t desc_hi,
                                         uint32_t idesc, uint32_t accumulate) {
   asm volatile(

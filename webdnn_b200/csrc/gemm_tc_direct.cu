@@ -32,6 +32,7 @@ constexpr int KB = 32;               // K block: one 128-byte swizzle row
 constexpr int SEG = 4;               // K blocks per TMEM segment
 constexpr int MAX_STAGES = 4;
 constexpr int SM_SMEM = 228 * 1024;
+constexpr int GROUP = 256;           // threads that load a K block
 constexpr unsigned long long WAIT_LIMIT_NS = 2000000000ull;
 
 struct DirectArgs {
@@ -43,7 +44,7 @@ struct DirectArgs {
   int m, n, k;
   int mode_a, mode_b;                // LOAD_*
   int stages;                        // K blocks in shared memory
-  int vec;                           // consecutive columns of an aligned access of Y and C
+  int vec;                           // consecutive columns of an aligned access of Y
   float alpha, beta;
   int relu;
   int* status;
@@ -137,21 +138,21 @@ __device__ __forceinline__ float high_part(float x) {
 }
 __device__ __forceinline__ bool not_finite(float x) { return (__float_as_uint(x) & 0x7f800000u) == 0x7f800000u; }
 
-// Registers of a thread's share of one K block of an operand with ROWS rows (THR threads share it; where it is small,
-// some have nothing):
+// Registers of a thread's share of one K block of an operand with ROWS rows (a group of threads shares it):
 //   LOAD_VEC4: K contiguous and 16-byte aligned: 8 threads x 16 bytes per row
 //   LOAD_K:    lanes along K (any strides; coalesced when K is contiguous)
 //   LOAD_ROW:  lanes along the rows (contiguous rows, e.g. B stored [k][n]); a thread holds 4 consecutive k of a row
-template <int ROWS, int THR>
+template <int ROWS>
 struct Share {
-  static constexpr int CELLS = ROWS * 8 / THR < 1 ? 1 : ROWS * 8 / THR;   // groups of four floats
+  static_assert(ROWS * 8 % GROUP == 0, "every thread has a share");
+  static constexpr int CELLS = ROWS * 8 / GROUP;                   // groups of four floats
   static constexpr int N = 4 * CELLS;
 };
-template <int ROWS, int THR>
+template <int ROWS>
 __device__ __forceinline__ void load_block(float* v, const float* base, int64_t s_row, int64_t s_k, int rows, int k0,
                                            int klen, int mode) {
-  using S = Share<ROWS, THR>;
-  const int tid = threadIdx.x % THR, warp = tid >> 5, lane = tid & 31;
+  using S = Share<ROWS>;
+  const int tid = threadIdx.x % GROUP, warp = tid >> 5, lane = tid & 31;
 #pragma unroll
   for (int i = 0; i < S::N; i++) v[i] = 0.f;
   if (mode == LOAD_VEC4) {
@@ -160,11 +161,11 @@ __device__ __forceinline__ void load_block(float* v, const float* base, int64_t 
     if (k < klen) {
 #pragma unroll
       for (int i = 0; i < S::CELLS; i++) {
-        if ((tid >> 3) + THR / 8 * i < rows) {
+        if ((tid >> 3) + 32 * i < rows) {
           const float4 q = pdl_ld(reinterpret_cast<const float4*>(p));
           v[4 * i] = q.x; v[4 * i + 1] = q.y; v[4 * i + 2] = q.z; v[4 * i + 3] = q.w;
         }
-        p += THR / 8 * s_row;
+        p += 32 * s_row;
       }
     }
   } else if (mode == LOAD_K) {
@@ -173,19 +174,19 @@ __device__ __forceinline__ void load_block(float* v, const float* base, int64_t 
     if (k < klen) {
 #pragma unroll
       for (int i = 0; i < S::N; i++) {
-        if (warp + THR / 32 * i < rows) v[i] = pdl_ld(p);
-        p += THR / 32 * s_row;
+        if (warp + 8 * i < rows) v[i] = pdl_ld(p);
+        p += 8 * s_row;
       }
     }
   } else {
-    const int k = k0 + (warp & 7) * 4, r0 = (warp >> 3) * 32 + lane;
-    const float* p = base + (int64_t)k * s_k + r0;
+    const int k = k0 + warp * 4;
+    const float* p = base + (int64_t)k * s_k + lane;
 #pragma unroll
     for (int t = 0; t < 4; t++) {
       if (k + t < klen) {
 #pragma unroll
         for (int i = 0; i < S::CELLS; i++)
-          if (r0 + THR / 8 * i < rows) v[4 * i + t] = pdl_ld(p + THR / 8 * i);
+          if (lane + 32 * i < rows) v[4 * i + t] = pdl_ld(p + 32 * i);
       }
       p += s_k;
     }
@@ -193,10 +194,10 @@ __device__ __forceinline__ void load_block(float* v, const float* base, int64_t 
 }
 
 // Writes the registers of load_block as the swizzled operand (high parts) and, `lo_off` bytes behind, its low parts.
-template <int ROWS, int THR>
+template <int ROWS>
 __device__ __forceinline__ bool store_block(const float* v, unsigned char* hi, uint32_t lo_off, int mode) {
-  using S = Share<ROWS, THR>;
-  const int tid = threadIdx.x % THR, warp = tid >> 5, lane = tid & 31;
+  using S = Share<ROWS>;
+  const int tid = threadIdx.x % GROUP, warp = tid >> 5, lane = tid & 31;
   float h[S::N];
   bool bad = false;
 #pragma unroll
@@ -207,8 +208,7 @@ __device__ __forceinline__ bool store_block(const float* v, unsigned char* hi, u
   if (mode == LOAD_K) {
 #pragma unroll
     for (int i = 0; i < S::N; i++) {
-      const uint32_t row = (uint32_t)(warp + THR / 32 * i);
-      if (row >= ROWS) break;
+      const uint32_t row = (uint32_t)(warp + 8 * i);
       const uint32_t off = row * 128u + ((((uint32_t)lane >> 2) ^ (row & 7u)) << 4) + ((uint32_t)lane & 3u) * 4u;
       *reinterpret_cast<float*>(hi + off) = h[i];
       *reinterpret_cast<float*>(hi + off + lo_off) = v[i] - h[i];
@@ -216,9 +216,8 @@ __device__ __forceinline__ bool store_block(const float* v, unsigned char* hi, u
   } else {
 #pragma unroll
     for (int i = 0; i < S::CELLS; i++) {
-      const uint32_t row = (uint32_t)((mode == LOAD_VEC4 ? tid >> 3 : (warp >> 3) * 32 + lane) + THR / 8 * i);
-      if (row >= ROWS) break;
-      const uint32_t chunk = (uint32_t)(mode == LOAD_VEC4 ? tid & 7 : warp & 7);
+      const uint32_t row = (uint32_t)((mode == LOAD_VEC4 ? tid >> 3 : lane) + 32 * i);
+      const uint32_t chunk = (uint32_t)(mode == LOAD_VEC4 ? tid & 7 : warp);
       const uint32_t off = row * 128u + ((chunk ^ (row & 7u)) << 4);
       const float *q = v + 4 * i, *g = h + 4 * i;
       *reinterpret_cast<float4*>(hi + off) = make_float4(g[0], g[1], g[2], g[3]);
@@ -277,7 +276,7 @@ struct DirectLayout {
   // Threads that load, split, add up and write (a warp more issues the MMAs).  A K block's way through a warp (wait,
   // split, write, proxy fence, arrive, ask for the next) takes 3000 cycles whatever the number of warps that share it, its
   // MMAs 800: where a CTA has the SM to itself, two groups of warps take alternate K blocks.
-  static constexpr int GROUP = 256, GROUPS = kLong ? 2 : 1;
+  static constexpr int GROUPS = kLong ? 2 : 1;
   static constexpr int LOADERS = GROUP * GROUPS, MMA_WARP = LOADERS / 32, THREADS = LOADERS + 32;
   static constexpr int CTAS = !kLong ? (TN == 32 ? 4 : 3) : 1;   // of an SM, at most
   static constexpr int COLS = TN * 128 / LOADERS < 16 ? 16 : TN * 128 / LOADERS;   // accumulator columns of a warp
@@ -289,7 +288,7 @@ struct DirectLayout {
 template <int TN, bool kLong>
 __global__ void __launch_bounds__(DirectLayout<TN, kLong>::THREADS, DirectLayout<TN, kLong>::CTAS) gemm_tc_direct_kernel(const DirectArgs a) {
   using L = DirectLayout<TN, kLong>;
-  constexpr int COLS = L::COLS, THR = L::GROUP, MMA_WARP = L::MMA_WARP;
+  constexpr int COLS = L::COLS, MMA_WARP = L::MMA_WARP;
   constexpr int NBUF = kLong ? 2 : 1;
   constexpr int TMEM_COLS = NBUF * TN < 32 ? 32 : NBUF * TN;
   extern __shared__ unsigned char smem_raw[];
@@ -303,7 +302,7 @@ __global__ void __launch_bounds__(DirectLayout<TN, kLong>::THREADS, DirectLayout
   if (tid < 2 * MAX_STAGES + 4) {
     unsigned long long* bar = tid < MAX_STAGES ? &sh.full[tid] : tid < 2 * MAX_STAGES ? &sh.empty[tid - MAX_STAGES]
                             : tid < 2 * MAX_STAGES + 2 ? &sh.seg_full[tid - 2 * MAX_STAGES] : &sh.seg_empty[tid - 2 * MAX_STAGES - 2];
-    const int count = tid < MAX_STAGES || tid >= 2 * MAX_STAGES + 2 ? tid < MAX_STAGES ? THR / 32 : L::OUT_WARPS : 1;
+    const int count = tid < MAX_STAGES || tid >= 2 * MAX_STAGES + 2 ? tid < MAX_STAGES ? GROUP / 32 : L::OUT_WARPS : 1;
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -317,11 +316,11 @@ __global__ void __launch_bounds__(DirectLayout<TN, kLong>::THREADS, DirectLayout
   const float* C = pdl_after(a.C);
   const float* A = pdl_after(a.A) + blockIdx.z * a.sab + (int64_t)m0 * a.sa_row;
   const float* B = pdl_after(a.B) + blockIdx.z * a.sbb + (int64_t)n0 * a.sb_row;
-  const int group = tid / THR;
-  float va[Share<TM, THR>::N], vb[Share<TN, THR>::N];
+  const int group = tid / GROUP;
+  float va[Share<TM>::N], vb[Share<TN>::N];
   if (warp < MMA_WARP && group < kblocks) {
-    load_block<TM, THR>(va, A, a.sa_row, a.sa_k, rows_a, group * KB, a.k, a.mode_a);
-    load_block<TN, THR>(vb, B, a.sb_row, a.sb_k, rows_b, group * KB, a.k, a.mode_b);
+    load_block<TM>(va, A, a.sa_row, a.sa_k, rows_a, group * KB, a.k, a.mode_a);
+    load_block<TN>(vb, B, a.sb_row, a.sb_k, rows_b, group * KB, a.k, a.mode_b);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -362,11 +361,11 @@ __global__ void __launch_bounds__(DirectLayout<TN, kLong>::THREADS, DirectLayout
       // the stage's last MMAs have read it (MMAs complete in order, so the release before that is long past)
       if (kb >= a.stages) ok = __all_sync(0xffffffffu, mbar_wait(&sh.empty[st], par, a.status, 81));
       if (!ok) break;
-      bad |= store_block<TM, THR>(va, sb, L::A_BYTES, a.mode_a);
-      bad |= store_block<TN, THR>(vb, sb + 2 * L::A_BYTES, L::B_BYTES, a.mode_b);
+      bad |= store_block<TM>(va, sb, L::A_BYTES, a.mode_a);
+      bad |= store_block<TN>(vb, sb + 2 * L::A_BYTES, L::B_BYTES, a.mode_b);
       if (kb + L::GROUPS < kblocks) {
-        load_block<TM, THR>(va, A, a.sa_row, a.sa_k, rows_a, (kb + L::GROUPS) * KB, a.k, a.mode_a);
-        load_block<TN, THR>(vb, B, a.sb_row, a.sb_k, rows_b, (kb + L::GROUPS) * KB, a.k, a.mode_b);
+        load_block<TM>(va, A, a.sa_row, a.sa_k, rows_a, (kb + L::GROUPS) * KB, a.k, a.mode_a);
+        load_block<TN>(vb, B, a.sb_row, a.sb_k, rows_b, (kb + L::GROUPS) * KB, a.k, a.mode_b);
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();

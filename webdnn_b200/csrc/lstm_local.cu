@@ -18,9 +18,9 @@
 //     words, cost more than they gave (1.82 us a step for one, 1.82 to 1.74 for four at 16 rows, 1.49 to 1.63 at one);
 //   * two buffers of h by the parity of the step: a CTA sends h_t after it has all of h_{t-1}, which every CTA sent after
 //     its MMAs on h_{t-2}, the buffer's last reader, were complete.
-// Measured, start of a step to the next with lstm_cluster.cu and here: 256 units, batch 1, 1.63 -> 0.77 us; [64, 512] 3.0 ->
-// 1.95 us (of 3680 cycles the MMAs are 1330, the gates 850, the words on their way 1500: 20 KB into every CTA); 50 steps of
-// [1, 256] with the projection 98 -> 55 us, 128 of [64, 512] 434 -> 320 us.
+// Measured, start of a step to the next with lstm_cluster.cu and here: 256 units, batch 1, 1.63 -> 0.82 us; [64, 512] 3.28 ->
+// 2.37 us (of 4500 cycles the words on their way are 1500, 20 KB into every CTA, and the gates 940); 50 steps of [1, 256] with the
+// projection 96 -> 58 us, 128 of [64, 512] 434 -> 343 us.
 // Sums: hi*hi in one range of columns of an accumulator, hi*lo + lo*hi in another, added in fp32 after the last MMA.  The tensor
 // core cuts every product off at the running sum's last bits, so a sum over K loses in proportion to K: the k steps go to four
 // accumulators in turn.  Rms error of a sum of 480 (512) products against 64 bits: mixed signs 6.2e-7 (6.6e-7) in one accumulator,
@@ -63,7 +63,7 @@ struct LocalArgs {
   int T, B, H;
   int cs;              // CTAs of a cluster: ceil(H / 32)
   int per;             // batch rows of a cluster
-  int r_early;         // R and bias are constants: read before the grids in front have finished
+  int r_early;         // R is read before the grids in front have finished: a constant that nothing still running writes
 };
 
 struct LocalShared {
@@ -270,7 +270,7 @@ struct LocalLayout {
 
 // The MMAs of four sources (two k steps each).  One block of straight-line code whose addresses are constant offsets from
 // bases in registers: 13 cycles an MMA.  With addresses computed for each it takes 28 to 65, with a block of constants for
-// every quarter and buffer behind a switch 25: the operands then pass through vector registers one by one.
+// every quarter and buffer behind a switch 25.
 struct Issue {
   uint32_t t_d, t_hi, t_lo;    // tensor memory: accumulators, high and low parts of R from these sources' columns on
   uint32_t b, b_top;           // descriptor of their words
@@ -312,7 +312,7 @@ __device__ __noinline__ float4 apart_sums(const float* r_row, float r_limit, con
 #pragma unroll 2
     for (uint32_t left = units[w]; left; left &= left - 1) {
       const int k = __ffs((int)left) - 1;
-      float r = w * 32 + k < width ? __ldg(r_row + w * 32 + k) : 0.f;
+      float r = w * 32 + k < width ? r_row[w * 32 + k] : 0.f;
       if (!is_small(r, r_limit)) r = 0.f;
       const unsigned char* p = src + w * src_bytes + (k >> 3) * 128 + (k & 7) * 2;
 #pragma unroll
@@ -333,7 +333,7 @@ __device__ __noinline__ float4 apart_first(const float* r_row, float r_limit, co
     for (uint32_t left = units[w] | h0_units[w]; left; left &= left - 1) {
       const int k = w * 32 + __ffs((int)left) - 1;
       if (k >= width) break;
-      const float r = __ldg(r_row + k);
+      const float r = r_row[k];
 #pragma unroll
       for (int j = 0; j < 4; j++) {
         const float h = j < rows ? h0[(size_t)j * width + k] : 0.f;
@@ -809,7 +809,10 @@ int wdc_lstm_local(wdc_context* ctx, const float* P, const float* R, const float
   const int groups = (a.per + 7) / 8, clusters = (int)ceil_div64(Bt, a.per);
   const Variant& v = variant_of(groups, a.cs);
   if (!max_clusters(ctx, a.cs, v)) return WDC_ERR_UNSUPPORTED;
-  a.r_early = ctx->opt_pdl && wdc_is_constant(ctx, R) && (!bias || wdc_is_constant(ctx, bias));
+  // A declared constant may have been written by the grid in front of the projection's: every kernel of the projection waits
+  // for the grids in front of it before it lets the next one start, so that one has finished by now.  (Only the projection,
+  // which is always launched in between, may still be running.)
+  a.r_early = ctx->opt_pdl && wdc_is_constant(ctx, R);
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr[2];
   fill_config(&cfg, attr, clusters * a.cs, a.cs, smem_of(v, a.cs), ctx->stream);
