@@ -351,6 +351,8 @@ int wdc_lstm(wdc_context* ctx, const float* X, const float* W, const float* R, c
  * The call itself returns WDC_OK; the next wdc_sync / wdc_download returns WDC_ERR_DEVICE_WAIT once, and the
  * context keeps working afterwards. */
 int wdc_selftest_device_wait(wdc_context* ctx, int64_t limit_ns);
+/* The same for the LSTM kernel whose CTAs exchange h inside a cluster. */
+int wdc_selftest_cluster_wait(wdc_context* ctx, int64_t limit_ns);
 
 /* wdc_lstm for callers that cannot allocate device memory while they run (a host that owns all GPU memory in
  * its own pool, a real-time loop, a sandbox without cudaMalloc): same arguments and results as wdc_lstm, but the

@@ -17,7 +17,7 @@ int wdc_lstm_persistent(wdc_context* ctx, const float* P, const float* R, const 
 int wdc_lstm_cluster(wdc_context* ctx, const float* P, const float* R, const float* bias, const float* h0,
                      const float* c0, float* Y, float* Yh, float* Yc, int64_t T, int64_t Bt, int64_t H);
 int wdc_lstm_local(wdc_context* ctx, const float* P, const float* R, const float* bias, const float* h0, const float* c0,
-                   float* Y, float* Yh, float* Yc, int64_t T, int64_t Bt, int64_t H);
+                   float* Y, float* Yh, float* Yc, int64_t T, int64_t Bt, int64_t H, int64_t selftest_wait_ns = 0);
 
 __device__ __forceinline__ float sigmoid_ref(float x) { return (tanhf(x * 0.5f) + 1.f) * 0.5f; }
 
@@ -110,17 +110,12 @@ extern "C" int wdc_lstm(wdc_context* ctx, const float* X, const float* W, const 
   return s;
 }
 
-// Self-test of the bounded device waits: runs the persistent recurrence kernel on a small zero-filled problem
-// (2 steps, batch 8, hidden 128: 32 CTAs) whose first step is told to wait for one arrival more than there are
-// CTAs, with `limit_ns` as the limit of every wait.  The wait runs out, the kernel records its status, raises its
-// abort word, every CTA returns, and the context stays usable: the next wdc_sync reports WDC_ERR_DEVICE_WAIT once.
-extern "C" int wdc_selftest_device_wait(wdc_context* ctx, int64_t limit_ns) {
-  if (!ctx) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_selftest_device_wait: null context");
-  WDC_NO_TAPE(ctx);
-  WDC_REQUIRE(ctx, limit_ns >= 1000 && limit_ns <= 1000000000ll,
-              "wdc_selftest_device_wait: limit of %lld ns is outside 1 us .. 1 s", (long long)limit_ns);
+// Self-tests of the bounded device waits, on a small zero-filled problem with `limit_ns` as the limit of every wait.  A wait
+// runs out, the kernel records its status, every CTA returns, and the context stays usable: the next wdc_sync reports
+// WDC_ERR_DEVICE_WAIT once.
+static int selftest_wait(wdc_context* ctx, int64_t limit_ns, const char* name, bool local, int64_t T, int64_t Bt, int64_t H) {
+  WDC_REQUIRE(ctx, limit_ns >= 1000 && limit_ns <= 1000000000ll, "%s: limit of %lld ns is outside 1 us .. 1 s", name, (long long)limit_ns);
   DeviceGuard g(ctx->device);
-  const int64_t T = 2, Bt = 8, H = 128;
   const int64_t n_p = T * Bt * 4 * H, n_r = 4 * H * H, n_y = T * Bt * H, n_s = Bt * H;
   float* buf = nullptr;
   int s = wdc_alloc(ctx, (n_p + n_r + n_y + 2 * n_s) * 4, (void**)&buf);
@@ -128,12 +123,26 @@ extern "C" int wdc_selftest_device_wait(wdc_context* ctx, int64_t limit_ns) {
   s = wdc_fill_u32(ctx, buf, 0u, n_p + n_r + n_y + 2 * n_s);
   if (s == WDC_OK) {
     float *P = buf, *R = P + n_p, *Y = R + n_r, *Yh = Y + n_y, *Yc = Yh + n_s;
-    s = wdc_lstm_persistent(ctx, P, R, nullptr, nullptr, nullptr, Y, Yh, Yc, T, Bt, H, limit_ns);
-    if (s == WDC_ERR_UNSUPPORTED)
-      s = wdc_fail(ctx, WDC_ERR_UNSUPPORTED, "wdc_selftest_device_wait: the persistent kernel cannot run on this device");
+    s = local ? wdc_lstm_local(ctx, P, R, nullptr, nullptr, nullptr, Y, Yh, Yc, T, Bt, H, limit_ns)
+              : wdc_lstm_persistent(ctx, P, R, nullptr, nullptr, nullptr, Y, Yh, Yc, T, Bt, H, limit_ns);
+    if (s == WDC_ERR_UNSUPPORTED) s = wdc_fail(ctx, WDC_ERR_UNSUPPORTED, "%s: the kernel cannot run on this device", name);
   }
   wdc_free(ctx, buf);   // stream-ordered
   return s;
+}
+// The persistent recurrence kernel (2 steps, batch 8, hidden 128: 32 CTAs) waits for one arrival more in its first step than
+// there are CTAs, and raises its abort word.
+extern "C" int wdc_selftest_device_wait(wdc_context* ctx, int64_t limit_ns) {
+  if (!ctx) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_selftest_device_wait: null context");
+  WDC_NO_TAPE(ctx);
+  return selftest_wait(ctx, limit_ns, "wdc_selftest_device_wait", false, 2, 8, 128);
+}
+// The recurrence inside one cluster (5 steps, batch 12, hidden 96: clusters of 3 CTAs) waits for a word of h more than its
+// CTAs send: the issuing warp's wait runs out, then the gates' for its MMAs, and the CTAs meet at the cluster's last barrier.
+extern "C" int wdc_selftest_cluster_wait(wdc_context* ctx, int64_t limit_ns) {
+  if (!ctx) return wdc_fail(ctx, WDC_ERR_INVALID, "wdc_selftest_cluster_wait: null context");
+  WDC_NO_TAPE(ctx);
+  return selftest_wait(ctx, limit_ns, "wdc_selftest_cluster_wait", true, 5, 12, 96);
 }
 
 // ------------------------------------------------------------------------------------------------

@@ -63,6 +63,8 @@ struct LocalArgs {
   int T, B, H;
   int cs;              // CTAs of a cluster: ceil(H / 32)
   int per;             // batch rows of a cluster
+  unsigned int beyond;          // bytes of h waited for beyond those that come: 0 (the self-test: one word)
+  unsigned long long wait_ns;   // limit of every wait (WAIT_NS; the self-test passes about a millisecond)
   int r_early;         // R is read before the grids in front have finished: a constant that nothing still running writes
 };
 
@@ -92,21 +94,21 @@ __device__ __forceinline__ unsigned long long global_ns() {
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
 }
-__device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, int* status, int code) {
+__device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, int* status, int code, unsigned long long limit_ns) {
   const unsigned long long t0 = global_ns();
   for (;;) {
     for (int i = 0; i < 256; i++)
       if (mbar_try_wait(bar, parity)) return true;
-    if (global_ns() - t0 > WAIT_NS) {
+    if (global_ns() - t0 > limit_ns) {
       atomicCAS(status, 0, code);
       return false;
     }
   }
 }
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* status, int code) {
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const LocalArgs& a, int code) {
   for (int i = 0; i < 1024; i++)
     if (mbar_try_wait(bar, parity)) return true;
-  return mbar_wait_slow(bar, parity, status, code);
+  return mbar_wait_slow(bar, parity, a.status, code, a.wait_ns);
 }
 __device__ __forceinline__ void expect_bytes(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
@@ -552,7 +554,7 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs 
   }
   const uint32_t full0 = smem_u32(&sh.full[0]);
   const int quarters = (cs + 3) / 4;
-  const uint32_t step_bytes = (uint32_t)cs * (uint32_t)nb * 128u;  // a source sends 128 for each batch row
+  const uint32_t step_bytes = (uint32_t)cs * (uint32_t)nb * 128u + a.beyond;  // a source sends 128 for each batch row
   if (tid == 0) {
     expect_bytes(full0, step_bytes);
     expect_bytes(full0 + 8u, step_bytes);
@@ -571,7 +573,7 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs 
       for (int t = a.h0 ? 0 : 1; t < a.T; t++) {
         const uint32_t bar = full0 + (t & 1 ? 8u : 0u);
         if (t > 0) {
-          if (!mbar_wait(bar, (uint32_t)((t - 1) >> 1) & 1u, a.status, 94)) break;
+          if (!mbar_wait(bar, (uint32_t)((t - 1) >> 1) & 1u, a, 94)) break;
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -612,7 +614,7 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs 
       float s[NG][4];
       const bool product = t > 0 || a.h0;
       if (product) {
-        if (!__all_sync(0xffffffffu, mbar_wait(mma_bar, phase, a.status, 95))) break;
+        if (!__all_sync(0xffffffffu, mbar_wait(mma_bar, phase, a, 95))) break;
         phase ^= 1u;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         float x[NG][4];
@@ -653,7 +655,7 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs 
         if (apart) {                                               // products of what the parts do not hold, with plain FMAs
           bool ok = true;
           if (t > 0)                                               // (this thread reads the others' words itself)
-            ok = mbar_wait(full0 + (t & 1 ? 8u : 0u), (uint32_t)((t - 1) >> 1) & 1u, a.status, 96);
+            ok = mbar_wait(full0 + (t & 1 ? 8u : 0u), (uint32_t)((t - 1) >> 1) & 1u, a, 96);
           const int width = row_unit < H ? H : 0;
           for (int g = 0; g < NG && ok; g++) {
             const int b = 8 * g + 4 * half;
@@ -796,7 +798,7 @@ int max_clusters(wdc_context* ctx, int cs, const Variant& v) {
 // Runs the recurrence on the projected input P.  WDC_ERR_UNSUPPORTED: shape outside the kernel's range (nothing has been
 // written); any other non-zero status is an error.
 int wdc_lstm_local(wdc_context* ctx, const float* P, const float* R, const float* bias, const float* h0, const float* c0,
-                   float* Y, float* Yh, float* Yc, int64_t T, int64_t Bt, int64_t H) {
+                   float* Y, float* Yh, float* Yc, int64_t T, int64_t Bt, int64_t H, int64_t selftest_wait_ns) {
   if (T < 4 || H < UNITS || H > MAX_CS * UNITS || H % 4 != 0) return WDC_ERR_UNSUPPORTED;
   if (T > (1 << 24) || Bt > (1 << 20)) return WDC_ERR_UNSUPPORTED;
   if (((uintptr_t)R & 15) != 0) return WDC_ERR_UNSUPPORTED;
@@ -809,6 +811,8 @@ int wdc_lstm_local(wdc_context* ctx, const float* P, const float* R, const float
   const int groups = (a.per + 7) / 8, clusters = (int)ceil_div64(Bt, a.per);
   const Variant& v = variant_of(groups, a.cs);
   if (!max_clusters(ctx, a.cs, v)) return WDC_ERR_UNSUPPORTED;
+  a.beyond = selftest_wait_ns > 0 ? 16u : 0u;
+  a.wait_ns = selftest_wait_ns > 0 ? (unsigned long long)selftest_wait_ns : WAIT_NS;
   // A declared constant may have been written by the grid in front of the projection's: every kernel of the projection waits
   // for the grids in front of it before it lets the next one start, so that one has finished by now.  (Only the projection,
   // which is always launched in between, may still be running.)
