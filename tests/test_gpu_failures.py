@@ -104,27 +104,23 @@ def test_null_and_invalid_arguments_return_a_status(cuda_context):
         ctx._call("wdc_alloc", -5, byref(c_void_p()))
     with pytest.raises(CudaBackendError, match="outside"):
         ctx._call("wdc_selftest_device_wait", c_int64(5))
-    with pytest.raises(CudaBackendError, match="outside"):
-        ctx._call("wdc_selftest_cluster_wait", c_int64(5))
     ctx.sync()     # none of the refused calls left anything behind
 
 
-# the persistent kernel waits for its step counter; in the one-cluster kernel the issuing warp for h, and the gates for its MMAs
-@pytest.mark.parametrize("entry,codes", [("wdc_selftest_device_wait", (61,)), ("wdc_selftest_cluster_wait", (94, 95))])
-def test_a_device_wait_that_runs_out_is_reported_and_the_context_survives(entry, codes):
-    """An LSTM kernel is told to wait for one CTA more than its grid has, or for one word more than its CTAs send, with a 1 ms
-    limit: the wait runs out, the kernel returns by itself, the next sync reports WDC_ERR_DEVICE_WAIT exactly once, and
-    the same context then runs the real LSTM correctly."""
+def test_a_device_wait_that_runs_out_is_reported_and_the_context_survives():
+    """The persistent LSTM kernel is told to wait for one CTA more than its grid has, with a 1 ms limit: the wait
+    runs out, the kernel returns by itself, the next sync reports WDC_ERR_DEVICE_WAIT exactly once, and the same
+    context then runs the real LSTM correctly."""
     import time
     from webdnn_b200.lib import CudaBackendError
     ctx = _new_context()
     try:
         ctx.sync()
         t0 = time.perf_counter()
-        ctx._call(entry, c_int64(1_000_000))
+        ctx._call("wdc_selftest_device_wait", c_int64(1_000_000))
         with pytest.raises(CudaBackendError) as e:
             ctx.sync()
-        assert e.value.status == 5 and any(f"kernel status {c}" in str(e.value) for c in codes)     # WDC_ERR_DEVICE_WAIT
+        assert e.value.status == 5 and "kernel status 61" in str(e.value)     # WDC_ERR_DEVICE_WAIT, the step counter
         assert time.perf_counter() - t0 < 5.0
         ctx.sync()                                                             # reported once, then clean
         model = zoo.lstm(6, 8, 16, 128)
@@ -132,6 +128,27 @@ def test_a_device_wait_that_runs_out_is_reported_and_the_context_survives(entry,
         want = ref_runner.run_model(model, [x])
         got = run_cuda(model, [x], ctx)
         for g, w in zip(got, want):
+            assert max_err_rel_linf(g, w) <= 1e-4
+    finally:
+        ctx.close()
+
+
+def test_a_wait_inside_a_cluster_that_runs_out_is_reported():
+    """The one-cluster LSTM kernel is told to wait for one word of h more than its CTAs send: the issuing warp's wait runs out (94),
+    then the gates' for its MMAs (95), with the same consequences as above."""
+    from webdnn_b200.lib import CudaBackendError
+    ctx = _new_context()
+    try:
+        with pytest.raises(CudaBackendError, match="outside"):
+            ctx._call("wdc_selftest_cluster_wait", c_int64(5))
+        ctx._call("wdc_selftest_cluster_wait", c_int64(1_000_000))
+        with pytest.raises(CudaBackendError) as e:
+            ctx.sync()
+        assert e.value.status == 5 and ("kernel status 94" in str(e.value) or "kernel status 95" in str(e.value))
+        ctx.sync()                                                             # reported once, then clean
+        model = zoo.lstm(6, 8, 16, 128)
+        x = zoo.make_input((6, 8, 16))
+        for g, w in zip(run_cuda(model, [x], ctx), ref_runner.run_model(model, [x])):
             assert max_err_rel_linf(g, w) <= 1e-4
     finally:
         ctx.close()

@@ -27,6 +27,7 @@ def _reference(x, w, r, b, h, c):
     (20, 15, 256, None), (5, 121, 256, 1.0),                                 # one row a cluster; one past 8 rows
     (6, 1, 480, 1.0), (6, 90, 484, 1.0),                                     # the last sizes with 15 CTAs and the first with 16
     (6, 56, 512, None), (5, 57, 512, 1.0), (5, 113, 512, 1.0), (4, 169, 512, None), (4, 225, 512, 1.0), (4, 500, 512, None),
+    (6, 10, 512, 1e6), (6, 10, 64, 1e-6),                                    # rows of h0 have scales of their own
     (5, 4, 516, 1.0),                                                        # the first size that lstm_cluster.cu keeps
 ])
 def test_recurrence(cuda_context, seq, batch, hidden, state):
@@ -211,5 +212,31 @@ def test_initial_states_of_any_magnitude(cuda_context, state, batch, hidden):
     with np.errstate(over="ignore"):
         want = _reference(x[:1], w, r, b, h0, c0)[0][0]
     assert (np.abs(got - want).max(axis=1) <= 1e-6).all() and np.abs(want).max(axis=1).min() > 1e-2   # (zeros would not pass)
+    for t in dev + outs:
+        t.dispose()
+
+
+# as tests/test_gpu_runs.py has it for smaller ones: the largest size inside one cluster, and sizes whose clusters exchange h
+@pytest.mark.parametrize("batch,hidden", [(3, 512), (5, 516), (20, 768)])
+@pytest.mark.parametrize("where", ["R", "R_large", "h0"])
+def test_infinities_in_many_units(cuda_context, where, batch, hidden):
+    ctx = cuda_context
+    seq, inp, lim = 6, 8, 0.3 * np.sqrt(256 / hidden)            # (a step passes on no more of an error than at 256 units)
+    rng = np.random.default_rng(hidden)
+    u = lambda *s: rng.uniform(-lim, lim, s).astype(np.float32)  # noqa: E731
+    x, w, r, b, h0, c0 = u(seq, batch, inp), u(4 * hidden, inp), u(4 * hidden, hidden), u(8 * hidden), u(batch, hidden), u(batch, hidden)
+    if where == "h0":
+        h0[batch - 1, 7] = np.inf
+    else:
+        r[hidden + 3, 5] = np.inf if where == "R" else np.float32(3.4028e38)
+        r[3, hidden - 1] = -np.inf if where == "R" else r[3, hidden - 1]
+    dev = [ctx.move_tensor(CPUTensor.from_array(a)) for a in (x, w, r, b, h0, c0)]
+    outs = [ctx.empty_tensor(s) for s in ((seq, batch, hidden), (batch, hidden), (batch, hidden))]
+    ctx._call("wdc_lstm", *(t.ptr for t in dev + outs), seq, batch, inp, hidden)
+    with np.errstate(all="ignore"):
+        wants = _reference(x, w, r, b, h0, c0)
+    for got, want in zip((o.get_data().reshape(o.dims) for o in outs), wants):
+        assert np.array_equal(np.isnan(got), np.isnan(want)) and np.isfinite(got).any()
+        assert np.all(np.abs(np.nan_to_num(got) - np.nan_to_num(want)) <= 1e-5)
     for t in dev + outs:
         t.dispose()

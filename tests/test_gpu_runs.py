@@ -266,11 +266,9 @@ def test_graph_with_its_transfers(cuda_context, rows, width):
     runner.dispose()
 
 
-# a launch of independent clusters, a cooperative one of clusters, a cooperative one of CTAs
-@pytest.mark.parametrize("hidden", [96, 544, 800])
-def test_recurrence_inside_a_graph(cuda_context, hidden):
-    """The recurrence's kernels, cooperative launches among them, are recorded and replayed like the others."""
-    runner = _load(cuda_context, zoo.lstm(20, 5, 24, hidden), graphReplay=True)
+def test_recurrence_inside_a_graph(cuda_context):
+    """The recurrence inside one cluster, a launch of clusters that are independent: recorded and replayed like the others."""
+    runner = _load(cuda_context, zoo.lstm(20, 5, 24, 96), graphReplay=True)
     rng = np.random.default_rng(0)
     for _ in range(4):
         x = rng.standard_normal((20, 5, 24)).astype(np.float32)
@@ -281,16 +279,27 @@ def test_recurrence_inside_a_graph(cuda_context, hidden):
     runner.dispose()
 
 
+# clusters that exchange h, and single CTAs: cooperative launches
+@pytest.mark.parametrize("hidden", [544, 800])
+def test_cooperative_recurrences_inside_a_graph(cuda_context, hidden):
+    runner = _load(cuda_context, zoo.lstm(20, 5, 24, hidden), graphReplay=True)
+    rng = np.random.default_rng(0)
+    for _ in range(4):
+        x = rng.standard_normal((20, 5, 24)).astype(np.float32)
+        got, want = runner.run([_cpu(x)]), runner._run_nodes([_cpu(x)])
+        assert all(np.array_equal(_bits(g.numpy()), _bits(w.numpy())) for g, w in zip(got, want))
+    assert runner.graph_replays >= 2
+    runner.dispose()
+
+
 # an infinite weight, and one that rounding would make infinite; an infinite initial state: gates saturate as in fp32
-# (hidden sizes of the kernel with R inside a cluster and, above 512, of the one whose clusters exchange h)
-@pytest.mark.parametrize("batch,hidden", [(1, 32), (5, 100), (33, 256), (3, 512), (5, 516), (20, 768)])
+@pytest.mark.parametrize("batch,hidden", [(1, 32), (5, 100), (33, 256)])
 @pytest.mark.parametrize("where", ["R", "R_large", "h0"])
 def test_recurrence_with_infinities(cuda_context, batch, hidden, where):
     ctx = cuda_context
     seq, inp = 6, 8
     rng = np.random.default_rng(hidden)
-    lim = 0.3 * min(1, np.sqrt(256 / hidden))   # (a step passes on errors of h times 0.6 lim sqrt(hidden): no more than at 256)
-    u = lambda *s: rng.uniform(-lim, lim, s).astype(np.float32)  # noqa: E731
+    u = lambda *s: rng.uniform(-0.3, 0.3, s).astype(np.float32)  # noqa: E731
     x, w, r, b, h0, c0 = u(seq, batch, inp), u(4 * hidden, inp), u(4 * hidden, hidden), u(8 * hidden), u(batch, hidden), u(batch, hidden)
     if where == "R":
         r[hidden + 3, 5], r[3, hidden - 1] = np.inf, -np.inf        # the output and the input gate of unit 3
