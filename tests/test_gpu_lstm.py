@@ -157,7 +157,7 @@ def test_sums_are_no_further_off_than_tf32_parts(cuda_context, batch, hidden, mi
 
 
 @pytest.mark.parametrize("hidden,batch", [(36, 3), (64, 8), (256, 130), (416, 260), (480, 20), (512, 57), (512, 130)])
-@pytest.mark.parametrize("kind", ["weight 1e6", "weight 3e38", "wide weights", "few small", "h0 and weights", "tiny inputs"])
+@pytest.mark.parametrize("kind", ["weight 1e6", "weight 1e8", "weight 1e10", "weight 3e38", "dead units", "wide weights", "few small", "h0 and weights", "tiny inputs"])
 def test_ranges_inside_rows(cuda_context, kind, batch, hidden):
     """Elements of R and h0 that are far below the largest of their row count as much as where they are alone: a large weight
     whose unit's output is 0 (its gate is shut), magnitudes spread over 12 decades in every row or in a few places, states
@@ -173,6 +173,10 @@ def test_ranges_inside_rows(cuda_context, kind, batch, hidden):
         r[hidden + 3], w[hidden + 3], b[hidden + 3], b[5 * hidden + 3] = 0, 0, -200, 0
     if kind in ("wide weights", "h0 and weights"):
         r *= (10.0 ** rng.uniform(-12, 0, r.shape)).astype(np.float32)
+    if kind == "dead units":
+        r[:, 1::2] *= np.float32(1e-11)
+        x[2:4], b[:] = 0, 0                                          # (and sums that only they decide)
+        r[::5, ::2] *= np.float32(1e-20)
     if kind == "few small":
         at = rng.random(r.shape) < 0.002
         r[at] *= np.float32(1e-11)

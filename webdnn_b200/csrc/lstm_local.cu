@@ -8,9 +8,11 @@
 //   * R fits because it is kept as two fp16 parts with a power of two per row (4 bytes an element, in tensor memory, the
 //     last low parts in shared memory), where TF32 parts take 8.  h is in (-1, 1) and has a constant scale.  Two parts of
 //     11 rounded bits carry 23 bits (TF32 parts, cut by the tensor core: 22), the low one with a scale of 2^13 of its own, so
-//     that elements down to 2^-28 of a row's largest have 22 bits.  What is smaller is left out of the parts, and the CTA that
-//     has such elements of R, or of h0, adds their products with fp32 FMAs (one of them in R: a step of [64, 512] 2.37 -> 3.1
-//     us, of [1, 256] 0.82 -> 1.4, most of it the way to the element through L2).  h below 2^-29 is good to 2^-51 absolutely.  An fp16 MMA covers twice the K of a TF32 one in the same time: M 128
+//     that elements down to 2^-28 of a row's largest have 22 bits.  Of what is smaller in R they miss up to 2^-49 of the largest.
+//     Where that can show, in a sum that is smaller than 2^24 times all of it, what is missing is added with fp32 FMAs, at the
+//     price of the elements' way through L2; elsewhere it costs a comparison (a step of [64, 512] 2.39 us without
+//     small elements, 2.49 with one unit's weights at 1e-12 of the others, 5.8 with 128 such units; always added they took 3.4 and 73).
+//     Small elements of h0 stay out of the parts and are added.  h below 2^-29 is good to 2^-51 absolutely.  An fp16 MMA covers twice the K of a TF32 one in the same time: M 128
 //     x N 16 x K 16 takes 9 cycles, N 32 takes 16;
 //   * h goes to every CTA of the cluster as 16-byte words in the layout of the MMA's B operand (no swizzle: 8 batch rows x
 //     8 units are 128 consecutive bytes), by st.async, whose mbarrier counts the bytes (a CTA takes in about 20 a clock:
@@ -47,7 +49,7 @@ constexpr int MAX_SMEM = 224 * 1024;
 constexpr int MIN_SMEM = 116 * 1024;        // all of tensor memory is taken: one CTA per SM
 constexpr float H_SCALE = 16384.f, H_UNSCALE = 1.f / 16384.f;
 constexpr float LO_SCALE = 8192.f, LO_UNSCALE = 1.f / 8192.f;   // of low parts against high ones
-constexpr float SMALL = 1.f / 32768.f;   // what is below that, scaled, is left out of the parts
+constexpr float SMALL = 1.f / 32768.f;   // below that, scaled, the parts have fewer than 22 bits
 constexpr unsigned long long WAIT_NS = 2000000000ull;
 
 struct LocalArgs {
@@ -71,9 +73,9 @@ struct LocalArgs {
 struct LocalShared {
   unsigned long long mma_bar;
   unsigned long long full[2];
-  unsigned int small_r[4][MAX_CS], small_h0[MAX_CS];   // units with elements outside the parts: of 32 rows of R, of h0; by source
+  unsigned int small_r[4][MAX_CS], small_h0[MAX_CS];   // units with small elements: of 32 rows of R, of h0; by source
   unsigned int tmem_base;
-  float row_max[128];
+  float row_max[128];                 // later: of pack_row
   float h0_unscale[8 * MAX_GROUPS];   // negative: all of the row is left out of the parts
 };
 
@@ -247,6 +249,19 @@ __device__ __forceinline__ int row_exponent(float m) {
   return min(13 - e, 100);
 }
 __device__ __forceinline__ float pow2(int e) { return __uint_as_float((uint32_t)(127 + e) << 23); }   // -126 <= e <= 127
+// A row's scale, and the limit of its small elements, by its largest magnitude: NaN where that is not finite.
+__device__ __forceinline__ int scale_exponent(float m) { return not_finite(m) ? 0 : row_exponent(m); }   // -114 .. 100
+// 2^24 times what the parts miss of a row, with the exponent of its largest magnitude in the last bits.  (One word for both: with 512
+// bytes more in front of them the operands in shared memory start 1 KB later, and a step of [64, 512] takes 2.56 us, not 2.37.)
+__device__ __forceinline__ float pack_row(float m, float error) {
+  return __uint_as_float((__float_as_uint(error * 0x1p24f) & ~0xffu) | __float_as_uint(m) >> 23);
+}
+__device__ __forceinline__ float error_of(float packed) {          // rounded up; infinite for a row that is not finite
+  const uint32_t bits = __float_as_uint(packed);
+  return (bits & 0xffu) == 0xffu ? __uint_as_float(0x7f800000u) : bits >> 8 ? __uint_as_float(bits | 0xffu) : 0.f;
+}
+__device__ __forceinline__ float row_magnitude(float packed) { return __uint_as_float((__float_as_uint(packed) & 0xffu) << 23); }   // for limit_of
+__device__ __forceinline__ float limit_of(float m) { return not_finite(m) ? __uint_as_float(0x7fffffffu) : pow2(-row_exponent(m)) * SMALL; }
 
 // h of one buffer: [source CTA][zeros? hi groups, lo groups][4 blocks of 8 units][8 batch rows][8 units], fp16.
 // An odd number of groups has a group of zeros in front: the MMA of the low parts of R has at least 16 columns and
@@ -303,48 +318,89 @@ __device__ __forceinline__ void issue_sources(const Issue& o, int q, int n, int 
   }
 }
 
-// Products of the elements of R that the parts leave out, for a gate row and four batch rows of h: `src` their high parts in
-// the first source's words, the low ones `lo_off` behind.  `units`: the units that have such elements, `words` the words that
-// are not zero.
-__device__ __noinline__ float4 apart_sums(const float* r_row, float r_limit, const unsigned int* units, uint32_t words, int width,
-                                          const unsigned char* src, int src_bytes, int lo_off) {
-  float sum[4] = {0.f, 0.f, 0.f, 0.f};
-  for (; words; words &= words - 1) {
-    const int w = __ffs((int)words) - 1;
-#pragma unroll 2
-    for (uint32_t left = units[w]; left; left &= left - 1) {
-      const int k = __ffs((int)left) - 1;
-      float r = w * 32 + k < width ? r_row[w * 32 + k] : 0.f;
-      if (!is_small(r, r_limit)) r = 0.f;
-      const unsigned char* p = src + w * src_bytes + (k >> 3) * 128 + (k & 7) * 2;
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const float h = __half2float(*reinterpret_cast<const __half*>(p + j * 16)), l = __half2float(*reinterpret_cast<const __half*>(p + lo_off + j * 16));
-        if (r != 0.f) sum[j] = fmaf(r, fmaf(l, LO_UNSCALE, h) * H_UNSCALE, sum[j]);
-      }
-    }
-  }
-  return make_float4(sum[0], sum[1], sum[2], sum[3]);
+// What the parts and their three products miss of an element that is small (x: scaled), times h: hi is off by at most 2^-25, lo
+// rounds that to 2^-38 or 2^-12 of itself, and lo * lo, 2^-12 of it, is left out.
+__device__ __forceinline__ float part_error(float x) {
+  const float m = fabsf(x);
+  return fminf(m, fmaf(fminf(m, 0x1p-25f), 0x1p-11f, 0x1p-38f));
 }
-// The same for the first step, with four rows of h0 (`rows` of them exist) that have elements apart themselves.
-__device__ __noinline__ float4 apart_first(const float* r_row, float r_limit, const unsigned int* units, const unsigned int* h0_units,
-                                           uint32_t words, int width, const float* h0, const float* h0_unscale, int rows) {
-  float sum[4] = {0.f, 0.f, 0.f, 0.f};
-  for (; words; words &= words - 1) {
-    const int w = __ffs((int)words) - 1;
-    for (uint32_t left = units[w] | h0_units[w]; left; left &= left - 1) {
-      const int k = w * 32 + __ffs((int)left) - 1;
-      if (k >= width) break;
-      const float r = r_row[k];
+// That for an element of R, to be added for h = h_hi + its low part: r h - (hi h + lo h_hi).
+struct Missing {
+  float rest, lo;      // r - hi, lo; unscaled
+};
+__device__ __forceinline__ Missing missing_of(float r, float r_limit, float scale, float unscale) {
+  if (!is_small(r, r_limit)) return {0.f, 0.f};
+  if (!(r_limit > 0.f)) return {r, 0.f};                           // all of its row is left out
+  __half hi, lo;
+  split_half(r * scale, &hi, &lo);
+  return {r - __half2float(hi) * unscale, __half2float(lo) * (LO_UNSCALE * unscale)};
+}
+
+// Whether what the parts miss (`error`: 2^24 times at most that) may show in a sum: above 2^-24 of it, or of 0.5 where the sum goes
+// into a sigmoid.
+__device__ __forceinline__ bool shows(float sum, float error) {
+  return !(error <= fmaxf(fabsf(sum), (threadIdx.x & 3) != 3 ? 0.5f : 0.f));
+}
+
+// A gate row's sums for 4 NG batch rows with what the parts miss of the row's small elements, where it may show.  h of the first step
+// is h0, whose own small elements are not in the parts at all.  (Rarely reached: by values, so that the step's sums stay in registers.)
+template <int NG>
+struct Sums {
+  float v[NG][4];
+};
+template <int NG, typename L>
+__device__ __noinline__ Sums<NG> with_missing(Sums<NG> s, const LocalArgs& a, const LocalShared* sh, const unsigned char* smem, int t) {
+  const int lane = threadIdx.x & 31, quarter = (threadIdx.x >> 5) & 3, half = threadIdx.x >> 7, row = quarter * 32 + lane;
+  const int b0 = (int)(blockIdx.x / (unsigned)a.cs) * a.per, nb = min(a.per, a.B - b0);
+  const int unit = (int)(blockIdx.x % (unsigned)a.cs) * UNITS + row / 4, width = unit < a.H ? a.H : 0;
+  const float* r_row = a.R + ((size_t)(row & 3) * a.H + (width ? unit : 0)) * a.H;
+  const float m = row_magnitude(sh->row_max[row]), r_limit = limit_of(m), error = error_of(sh->row_max[row]);
+  const float r_scale = pow2(scale_exponent(m)), r_unscale = pow2(-scale_exponent(m));
+  const unsigned int *r_units = sh->small_r[quarter], *h0_units = sh->small_h0;
+  const bool h0_small = t == 0 && nonzero_words(h0_units);
 #pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const float h = j < rows ? h0[(size_t)j * width + k] : 0.f;
-        const float limit = j < rows && h0_unscale[j] > 0.f ? h0_unscale[j] * SMALL : __uint_as_float(0x7fffffffu);
-        if (j < rows && (is_small(r, r_limit) || is_small(h, limit))) sum[j] = fmaf(r, h, sum[j]);
+  for (int g = 0; g < NG; g++) {
+    const int b = 8 * g + 4 * half;
+    uint32_t want = 0;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const float e = t == 0 ? error * H_SCALE * sh->h0_unscale[b + j] : error;                      // (|h| is below 1, h0 below that)
+      if (b + j < nb && (h0_small || shows(s.v[g][j], e))) want |= 1u << j;
+    }
+    if (!want) continue;
+    if (t > 0 && !mbar_wait(smem_u32(&sh->full[t & 1]), (uint32_t)((t - 1) >> 1) & 1u, a, 96)) break;   // (this thread reads the others' words itself)
+    float sum[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int w = 0; w < a.cs; w++) {
+#pragma unroll 2
+      for (uint32_t left = r_units[w] | (t == 0 ? h0_units[w] : 0u); left; left &= left - 1) {
+        const int k = __ffs((int)left) - 1;
+        const float r = w * 32 + k < width ? r_row[w * 32 + k] : 0.f;
+        const Missing q = missing_of(r, r_limit, r_scale, r_unscale);
+        const unsigned char* p = smem + (t & 1 ? L::BUF : 0) + L::ZERO * L::GROUP + g * L::GROUP + half * 64 + w * L::SRC + (k >> 3) * 128 + (k & 7) * 2;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          float unscale = H_UNSCALE;
+          if (t == 0) {
+            if (b + j >= nb) continue;
+            unscale = sh->h0_unscale[b + j];
+            if (h0_units[w] >> k & 1u) {
+              const float h = w * 32 + k < width ? a.h0[(size_t)(b0 + b + j) * a.H + w * 32 + k] : 0.f;
+              if (is_small(h, unscale > 0.f ? unscale * SMALL : __uint_as_float(0x7fffffffu))) {
+                sum[j] = fmaf(r, h, sum[j]);
+                continue;
+              }
+            }
+          }
+          const float h_hi = __half2float(*reinterpret_cast<const __half*>(p + j * 16)) * unscale;
+          const float h_lo = __half2float(*reinterpret_cast<const __half*>(p + NG * L::GROUP + j * 16)) * (LO_UNSCALE * unscale);
+          if (is_small(r, r_limit)) sum[j] = fmaf(-q.lo, h_hi, fmaf(q.rest, h_hi + h_lo, sum[j]));
+        }
       }
     }
+#pragma unroll
+    for (int j = 0; j < 4; j++) s.v[g][j] += want >> j & 1u ? sum[j] : 0.f;
   }
-  return make_float4(sum[0], sum[1], sum[2], sum[3]);
+  return s;
 }
 
 // The gates of GROUPS of a thread's NG cells (side by side: their chains of dependent operations overlap), h into `out`.
@@ -389,7 +445,7 @@ __device__ __forceinline__ void step_end(const float (&s)[NG][4], bool product, 
 }
 
 template <int NG, int ACCS, bool TURNS>
-__global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs a) {
+__global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const __grid_constant__ LocalArgs a) {
   using L = LocalLayout<NG, ACCS, TURNS>;
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ LocalShared sh;
@@ -420,8 +476,6 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs 
   // Gate row r of the CTA = gate r % 4 of unit r / 4.  Its largest magnitude: eight lanes take 128 consecutive bytes of a
   // row, a warp its rows 16 w .. 16 w + 15 (a thread per row, 16 bytes each, took 10 us more at 512 units).
   const int row = (warp & 3) * 32 + lane, half = warp >> 2;
-  const int row_unit = u0 + row / 4;
-  const float* r_row = a.R + ((size_t)(row & 3) * H + (row_unit < H ? row_unit : 0)) * H;
   if (warp < 8) {
     for (int i = 0; i < 4; i++) {
       const int r = warp * 16 + 4 * i + lane / 8, unit = u0 + r / 4, k1 = unit < H ? H : 0;
@@ -447,12 +501,13 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs 
   const uint32_t tmem = sh.tmem_base;
   const uint32_t tmem_hi = tmem + (uint32_t)L::D_COLS, tmem_lo = tmem_hi + (uint32_t)(16 * cs);
   const int steps_lo = L::steps_lo(cs);
-  float unscale = 0.f, r_limit = 0.f;
+  float unscale = 0.f;
   if (warp < 8) {
     const float m = sh.row_max[row];
-    const int e = not_finite(m) ? 0 : row_exponent(m);
-    r_limit = not_finite(m) ? __uint_as_float(0x7fffffffu) : pow2(-e) * SMALL;   // (-114 <= e <= 100)
-    const float scale = pow2(e);
+    const bool whole_row = not_finite(m);
+    const int e = scale_exponent(m);
+    const float r_limit = limit_of(m), scale = pow2(e);
+    float row_error = 0.f;
     unscale = pow2(-e) * H_UNSCALE;                                // (e <= 100: a normal number)
     const uint32_t t_row = (uint32_t)((warp & 3) * 32) << 16;
     // 64 columns at a time through shared memory (rows 272 bytes apart: no bank conflicts either way); warps w and w + 4 take
@@ -484,9 +539,11 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs 
           __half h[4], l[4];
 #pragma unroll
           for (int c = 0; c < 4; c++) {
-            const bool small = is_small(x[c], r_limit);
-            split_half(small ? 0.f : x[c] * scale, &h[c], &l[c]);
-            if (small) units |= 1u << (q * 4 + c);
+            split_half(whole_row ? 0.f : x[c] * scale, &h[c], &l[c]);
+            if (is_small(x[c], r_limit)) {
+              units |= 1u << (q * 4 + c);
+              row_error += part_error(x[c] * scale);
+            }
           }
 #pragma unroll
           for (int c = 0; c < 2; c++) {
@@ -507,6 +564,11 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs 
       asm volatile("bar.sync 1, 256;" ::: "memory");
     }
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    // what the parts miss of a row's small elements, of both warps
+    float* errors = reinterpret_cast<float*>(chunk);
+    if (half == 1) errors[row] = row_error;
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+    if (half == 0) sh.row_max[row] = pack_row(m, (row_error + errors[row]) * pow2(-e));
   }
   __syncthreads();
   for (uint32_t i = (uint32_t)tid * 16u; i < 2u * buf_bytes; i += THREADS * 16u)   // rows past the batch stay zero
@@ -537,10 +599,9 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs 
       uint32_t m = 0;
       for (int k = lane; k < H; k += 32) m = max(m, __float_as_uint(src[k]) & 0x7fffffffu);
       m = __reduce_max_sync(0xffffffffu, m);
-      const bool finite = !not_finite(__uint_as_float(m));
-      const int e = finite ? row_exponent(__uint_as_float(m)) : 0;
-      const float scale = pow2(e), limit = finite ? pow2(-e) * SMALL : __uint_as_float(0x7fffffffu);
-      if (lane == 0) sh.h0_unscale[b] = finite ? pow2(-e) : -1.f;
+      const int e = scale_exponent(__uint_as_float(m));
+      const float scale = pow2(e), limit = limit_of(__uint_as_float(m));
+      if (lane == 0) sh.h0_unscale[b] = limit > 0.f ? pow2(-e) : -1.f;
       for (int k = lane; k < H; k += 32) {
         __half hi, lo;
         const bool small = is_small(src[k], limit);
@@ -651,24 +712,18 @@ __global__ void __launch_bounds__(THREADS, 1) lstm_local_kernel(const LocalArgs 
 #pragma unroll
             for (int j = 0; j < 4; j++) s[g][j] = s[g][j] * H_SCALE * sh.h0_unscale[8 * g + 4 * half + j];
         }
-        const uint32_t apart = t == 0 ? small_r | small_h0 : small_r;
-        if (apart) {                                               // products of what the parts do not hold, with plain FMAs
-          bool ok = true;
-          if (t > 0)                                               // (this thread reads the others' words itself)
-            ok = mbar_wait(full0 + (t & 1 ? 8u : 0u), (uint32_t)((t - 1) >> 1) & 1u, a, 96);
-          const int width = row_unit < H ? H : 0;
-          for (int g = 0; g < NG && ok; g++) {
-            const int b = 8 * g + 4 * half;
-            const float4 more = t == 0 ? apart_first(r_row, r_limit, sh.small_r[warp & 3], sh.small_h0, apart, width, a.h0 + (size_t)(b0 + b) * H, sh.h0_unscale + b, nb - b)
-                                       : apart_sums(r_row, r_limit, sh.small_r[warp & 3], apart, width, smem + (t & 1 ? buf_bytes : 0u) + HI_OFF + g * L::GROUP + half * 64, L::SRC, NG * L::GROUP);
+        if (t == 0 ? small_r | small_h0 : small_r) {
+          const float error = error_of(sh.row_max[row]);
+          bool some_show = t == 0;                                 // (asked there)
 #pragma unroll
-            for (int i = 0; i < NG; i++) {                         // (s stays in registers)
-              if (i != g) continue;
-              s[i][0] += more.x;
-              s[i][1] += more.y;
-              s[i][2] += more.z;
-              s[i][3] += more.w;
-            }
+          for (int i = 0; i < 4 * NG; i++) some_show |= i / 4 * 8 + 4 * half + i % 4 < nb && shows(s[i / 4][i % 4], error);
+          if (some_show) {
+            Sums<NG> all;
+#pragma unroll
+            for (int i = 0; i < 4 * NG; i++) all.v[i / 4][i % 4] = s[i / 4][i % 4];
+            all = with_missing<NG, L>(all, a, &sh, smem, t);
+#pragma unroll
+            for (int i = 0; i < 4 * NG; i++) s[i / 4][i % 4] = all.v[i / 4][i % 4];
           }
           __syncwarp();
         }
