@@ -11,17 +11,17 @@
 //     that elements down to 2^-28 of a row's largest have 22 bits.  Of what is smaller in R they miss up to 2^-49 of the largest.
 //     Where that can show, in a sum that is smaller than 2^24 times all of it, what is missing is added with fp32 FMAs, at the
 //     price of the elements' way through L2; elsewhere it costs a comparison (a step of [64, 512] 2.39 us without
-//     small elements, 2.49 with one unit's weights at 1e-12 of the others, 5.8 with 128 such units; always added they took 3.4 and 73).
-//     Small elements of h0 stay out of the parts and are added.  h below 2^-29 is good to 2^-51 absolutely.  An fp16 MMA covers twice the K of a TF32 one in the same time: M 128
-//     x N 16 x K 16 takes 9 cycles, N 32 takes 16;
+//     small elements, 2.49 with one unit's weights at 1e-12 of the others, 5.8 with 128 such units; always added they took 3.4
+//     and 73).  Small elements of h0 stay out of the parts and are added.  h below 2^-29 is good to 2^-51 absolutely.  An fp16
+//     MMA covers twice the K of a TF32 one in the same time: M 128 x N 16 x K 16 takes 9 cycles, N 32 takes 16;
 //   * h goes to every CTA of the cluster as 16-byte words in the layout of the MMA's B operand (no swizzle: 8 batch rows x
 //     8 units are 128 consecutive bytes), by st.async, whose mbarrier counts the bytes (a CTA takes in about 20 a clock:
 //     16 KB of 8 rows x 512 units 800 cycles).  Barriers for each four sources, so that the first MMAs overlap the last
 //     words, cost more than they gave (1.82 us a step for one, 1.82 to 1.74 for four at 16 rows, 1.49 to 1.63 at one);
 //   * two buffers of h by the parity of the step: a CTA sends h_t after it has all of h_{t-1}, which every CTA sent after
 //     its MMAs on h_{t-2}, the buffer's last reader, were complete.
-// Measured, start of a step to the next with lstm_cluster.cu and here: 256 units, batch 1, 1.63 -> 0.82 us; [64, 512] 3.28 ->
-// 2.37 us (of 4500 cycles the words on their way are 1500, 20 KB into every CTA, and the gates 940); 50 steps of [1, 256] with the
+// Measured, start of a step to the next with lstm_cluster.cu and here: 256 units, batch 1, 1.63 -> 0.85 us; [64, 512] 3.28 ->
+// 2.39 us (of 4500 cycles the words on their way are 1500, 20 KB into every CTA, and the gates 940); 50 steps of [1, 256] with the
 // projection 96 -> 58 us, 128 of [64, 512] 434 -> 343 us.
 // Sums: hi*hi in one range of columns of an accumulator, hi*lo + lo*hi in another, added in fp32 after the last MMA.  The tensor
 // core cuts every product off at the running sum's last bits, so a sum over K loses in proportion to K: the k steps go to four
