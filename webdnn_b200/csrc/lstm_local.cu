@@ -11,7 +11,7 @@
 //     that elements down to 2^-28 of a row's largest have 22 bits.  Of what is smaller in R they miss up to 2^-49 of the largest.
 //     Where that can show, in a sum that is smaller than 2^24 times all of it, what is missing is added with fp32 FMAs, at the
 //     price of the elements' way through L2; elsewhere it costs a comparison (a step of [64, 512] 2.39 us without
-//     small elements, 2.49 with one unit's weights at 1e-12 of the others, 5.8 with 128 such units; always added they took 3.4
+//     small elements, 2.49 with one unit's weights at 1e-12 of the others, 5.6 with 128 such units; always added they took 3.4
 //     and 73).  Small elements of h0 stay out of the parts and are added.  h below 2^-29 is good to 2^-51 absolutely.  An fp16
 //     MMA covers twice the K of a TF32 one in the same time: M 128 x N 16 x K 16 takes 9 cycles, N 32 takes 16;
 //   * h goes to every CTA of the cluster as 16-byte words in the layout of the MMA's B operand (no swizzle: 8 batch rows x
@@ -370,30 +370,35 @@ __device__ __noinline__ Sums<NG> with_missing(Sums<NG> s, const LocalArgs& a, co
     if (!want) continue;
     if (t > 0 && !mbar_wait(smem_u32(&sh->full[t & 1]), (uint32_t)((t - 1) >> 1) & 1u, a, 96)) break;   // (this thread reads the others' words itself)
     float sum[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int w = 0; w < a.cs; w++) {
-#pragma unroll 2
-      for (uint32_t left = r_units[w] | (t == 0 ? h0_units[w] : 0u); left; left &= left - 1) {
-        const int k = __ffs((int)left) - 1;
-        const float r = w * 32 + k < width ? r_row[w * 32 + k] : 0.f;
-        const Missing q = missing_of(r, r_limit, r_scale, r_unscale);
-        const unsigned char* p = smem + (t & 1 ? L::BUF : 0) + L::ZERO * L::GROUP + g * L::GROUP + half * 64 + w * L::SRC + (k >> 3) * 128 + (k & 7) * 2;
+    for (int w8 = 0; w8 < 4 * a.cs; w8++) {                        // eight units: 32 bytes of a row, together
+      const uint32_t of_h0 = t == 0 ? h0_units[w8 >> 2] >> (w8 & 3) * 8 & 0xffu : 0u, units = (r_units[w8 >> 2] >> (w8 & 3) * 8 & 0xffu) | of_h0;
+      if (!units) continue;
+      float r[8];
+#pragma unroll
+      for (int i = 0; i < 8; i += 4)                               // (H is a multiple of 4, rows are 16-byte aligned)
+        *reinterpret_cast<float4*>(r + i) = w8 * 8 + i < width ? *reinterpret_cast<const float4*>(r_row + w8 * 8 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+      const unsigned char* p = smem + (t & 1 ? L::BUF : 0) + (L::ZERO + g) * L::GROUP + half * 64 + (w8 >> 2) * L::SRC + (w8 & 3) * 128;
+#pragma unroll
+      for (int i = 0; i < 8; i++) {
+        if (!(units >> i & 1u)) continue;
+        const Missing q = missing_of(r[i], r_limit, r_scale, r_unscale);
 #pragma unroll
         for (int j = 0; j < 4; j++) {
           float unscale = H_UNSCALE;
           if (t == 0) {
             if (b + j >= nb) continue;
             unscale = sh->h0_unscale[b + j];
-            if (h0_units[w] >> k & 1u) {
-              const float h = w * 32 + k < width ? a.h0[(size_t)(b0 + b + j) * a.H + w * 32 + k] : 0.f;
+            if (of_h0 >> i & 1u) {
+              const float h = w8 * 8 + i < width ? a.h0[(size_t)(b0 + b + j) * a.H + w8 * 8 + i] : 0.f;
               if (is_small(h, unscale > 0.f ? unscale * SMALL : __uint_as_float(0x7fffffffu))) {
-                sum[j] = fmaf(r, h, sum[j]);
+                sum[j] = fmaf(r[i], h, sum[j]);
                 continue;
               }
             }
           }
-          const float h_hi = __half2float(*reinterpret_cast<const __half*>(p + j * 16)) * unscale;
-          const float h_lo = __half2float(*reinterpret_cast<const __half*>(p + NG * L::GROUP + j * 16)) * (LO_UNSCALE * unscale);
-          if (is_small(r, r_limit)) sum[j] = fmaf(-q.lo, h_hi, fmaf(q.rest, h_hi + h_lo, sum[j]));
+          const float h_hi = __half2float(*reinterpret_cast<const __half*>(p + j * 16 + i * 2)) * unscale;
+          const float h_lo = __half2float(*reinterpret_cast<const __half*>(p + NG * L::GROUP + j * 16 + i * 2)) * (LO_UNSCALE * unscale);
+          if (is_small(r[i], r_limit)) sum[j] = fmaf(-q.lo, h_hi, fmaf(q.rest, h_hi + h_lo, sum[j]));
         }
       }
     }
